@@ -80,7 +80,7 @@ def draw(rng):
     elif kind in ("cascade", "batch"):
         steps = rng.randint(30, 120) if precision == "mixed" else rng.randint(10, 30)
         energy = round(rng.uniform(200.0, 1000.0 if n < 30 else 5000.0), 1)
-        replicas = rng.randint(2, 8) if kind == "batch" else 1
+        replicas = rng.randint(2, 6) if kind == "batch" else 1
     return _case(None, kind, precision, cells, n_ele, steps, energy, replicas)
 
 
@@ -301,8 +301,9 @@ def run(s):
         s["batch"].run(steps)
     else:
         s["boxes"][0].ctx.simulate(steps)
-    return [dict(b.fetch(a), inter={f: b.inter[f] for f in ("type", "x", "v", "f", "rho", "df")})
-            for b, a in zip(s["boxes"], s["back"])]
+    out = {"boxes": [b.fetch(a) for b, a in zip(s["boxes"], s["back"])]}
+    out["inter"] = {f: np.stack([b.inter[f] for b in s["boxes"]]) for f in ("type", "x", "v", "f", "rho", "df")}
+    return out
 
 
 # ---- what a pass cannot do without ------------------------------------------------------------------
