@@ -41,6 +41,9 @@ struct mg_context {
     Slots s{};
     Inter in{};
     PotTables pt{};
+    FixParams fp{};                 // fixed-point pair arithmetic of the FP64 form (on when the tables suit it)
+    void *fix_mem = nullptr;        // its tables
+    bool fix_built = false;         // tables made for the potential in use (by the first FP64 state)
     bool pot_ready = false;
     HostPotential hp;               // the spline coefficients in use
     int types_ok_mask = 0;          // bit t set: the potential has the element of atom type t
@@ -99,6 +102,7 @@ struct mg_context {
     LaunchCtx lc() const {
         LaunchCtx l{stream, num_sms};
         l.nt = &nt;
+        l.fp = !mixed() && fp.on && s.fix ? &fp : nullptr;
         l.rho_order = tune[precision][0][0];
         l.rho_block = tune[precision][0][1];
         l.rho_apt = tune[precision][0][2];
@@ -235,7 +239,7 @@ void seq_compute_eam(mg_context *ctx, bool kick, bool with_manage_prefix, int ma
 // next one (both only act when no inter atoms exist, which the kernels check on the device)
 void seq_step(mg_context *ctx, Timer *t, bool fused_prev = false, bool fuse_next = false) {
     if (t) t->mark(0);
-    launch_step_head(ctx->lc(), ctx->d_sp);
+    launch_step_head(ctx->lc(), ctx->d_sp, ctx->s.skin);
     seq_firststep(ctx, true, t, fused_prev);
     seq_compute_eam(ctx, true, true, MANAGE_DECIDE | MANAGE_CLEAR_GHOST | MANAGE_EXCHANGE | MANAGE_BORDER, t, fuse_next);
 }
@@ -248,7 +252,57 @@ mg_status require_ready(mg_context *ctx) {
     return MG_OK;
 }
 
+// The FP64 form's fixed-point tables and arrays (40 bytes per slot), made for the first FP64 state that comes
+// in under a potential. Where the tables do not suit the potential, or the arrays do not fit the device,
+// the passes run in FP64.
+void ensure_fix(mg_context *ctx) {
+    if (ctx->mixed() || !ctx->pot_ready || ctx->fix_built) return;
+    ctx->fix_built = true;
+    const HostPotential &hp = ctx->hp;
+    int ele_of_type[3];
+    for (int t = 0; t < 3; t++) ele_of_type[t] = std::max(0, hp.ele(type_key(t)));
+    FixParams fp;
+    FixTables ft;
+    if (!build_fixed(hp, ele_of_type, ctx->g.a0, ctx->g.rc / ctx->g.a0, std::max(ctx->n_pruned, ctx->n_full - ctx->n_pruned), fp, ft)) return;
+    Slots &s = ctx->s;
+    const size_t ns = static_cast<size_t>(ctx->g.n_slots);
+    const size_t n[3] = {ft.rho.size(), ft.zg.size(), ft.phi.size()};
+    void *tab = nullptr, *rec = s.fix, *df = s.dfq;
+    cudaError_t e = cudaMalloc(&tab, (n[0] + n[1] + n[2]) * sizeof(FixPoly));
+    if (e == cudaSuccess && !rec) e = cudaMalloc(&rec, ns * sizeof(FixRec));
+    if (e == cudaSuccess && !df) e = cudaMalloc(&df, ns * sizeof(i64));
+    FixPoly *d = static_cast<FixPoly *>(tab);
+    const FixPoly *src[3] = {ft.rho.data(), ft.zg.data(), ft.phi.data()};
+    const FixPoly *at[3];
+    for (int k = 0; k < 3; k++) {
+        at[k] = d;
+        if (e == cudaSuccess) e = cudaMemcpy(d, src[k], n[k] * sizeof(FixPoly), cudaMemcpyHostToDevice);
+        if (d) d += n[k];
+    }
+    if (e == cudaSuccess && !s.dfq) e = cudaMemsetAsync(df, 0, ns * sizeof(i64), ctx->stream);
+    if (e != cudaSuccess) {
+        cudaGetLastError();
+        cudaFree(tab);
+        if (rec != s.fix) cudaFree(rec);
+        if (df != s.dfq) cudaFree(df);
+        return;
+    }
+    if (!s.fix) ctx->dev_allocs.push_back(rec);
+    if (!s.dfq) ctx->dev_allocs.push_back(df);
+    s.fix = static_cast<FixRec *>(rec);
+    s.dfq = static_cast<i64 *>(df);
+    ctx->fix_mem = tab;
+    fp.rho = at[0];
+    fp.zg = at[1];
+    fp.phi = at[2];
+    ctx->fp = fp;
+    launch_skin_dirty(ctx->lc(), s);  // FP64 passes before this kept no lists
+    ctx->graph_stale = true;  // graphs captured without them
+    ctx->gen++;
+}
+
 mg_status ensure_aos(mg_context *ctx) {
+    ensure_fix(ctx);
     if (ctx->d_aos) return MG_OK;
     MG_CK(dalloc(ctx, &ctx->d_aos, static_cast<size_t>(ctx->g.n_slots)));
     return MG_OK;
@@ -370,6 +424,9 @@ mg_status install_potential(mg_context *ctx, const HostPotential &hp) {
     pt.F_vf = d_vf + base_F; pt.F_dff = d_df + base_F;
     pt.z_vf = d_vf + base_z; pt.z_dff = d_df + base_z;
     pt.zr8 = d_zr;
+    if (ctx->fix_mem) { cudaFree(ctx->fix_mem); ctx->fix_mem = nullptr; }
+    ctx->fp = FixParams{};
+    ctx->fix_built = false;
     ctx->hp = hp;
     ctx->pot_ready = true;
     ctx->graph_stale = true;
@@ -631,6 +688,7 @@ mg_status mg_destroy(mg_context *ctx) {
     if (ctx->copy_out) cudaStreamDestroy(ctx->copy_out);
     for (void *p : ctx->dev_allocs) cudaFree(p);
     if (ctx->pot_mem) cudaFree(ctx->pot_mem);
+    if (ctx->fix_mem) cudaFree(ctx->fix_mem);
     if (ctx->stream) cudaStreamDestroy(ctx->stream);
     delete ctx;
     return MG_OK;
@@ -912,6 +970,7 @@ mg_status mg_prepare(mg_context *ctx) {
     if (!ctx) return MG_ERR_ARG;
     mg_status st = require_ready(ctx);
     if (st != MG_OK) return st;
+    ensure_fix(ctx);
     // exchangeAtomFirst, clearForce, computeEam (src/simulation.cpp:137-145); the lattice passes assign
     // instead of accumulate, which is what clearForce + accumulate gives
     seq_compute_eam(ctx, false, false, 0, nullptr);
@@ -1314,7 +1373,7 @@ static mg_status step_host_overlapped(mg_context *ctx, mg_atom_element *atoms, m
     MG_CK(cudaEventRecord(ctx->pipe_ev[ev], ctx->stream));
     MG_CK(cudaStreamWaitEvent(ctx->copy_in, ctx->pipe_ev[ev++], 0));
     launch_set_counts(lc, ctx->in, 0);
-    launch_step_head(lc, ctx->d_sp);
+    launch_step_head(lc, ctx->d_sp, ctx->s.skin);
     launch_far_clear(lc, g, ctx->in);  // the previous far list's marks, which decide clears
     launch_spec_begin(lc, ctx->in);
     std::vector<size_t> in_ev(S);
@@ -1357,6 +1416,7 @@ static mg_status step_host_overlapped(mg_context *ctx, mg_atom_element *atoms, m
         launch_firststep(lc, g, ctx->s, ctx->in, ctx->d_sp, true, t0, t1);
         launch_spec_decide(lc, g, ctx->s, ctx->in, t0, t1);
         launch_ghost_copy_planes(lc, g, ctx->s, k0, k1);
+        launch_fix_records(lc, g, ctx->s, static_cast<int>((g.gz + k0) * plane), static_cast<int>((g.gz + k1) * plane));
         // slabs 1 .. SS - 2 in order once the planes within 3 of them are in; then the forces of slabs
         // 2 .. SS - 3 whose neighbour slabs have their density, and their finished planes go out
         while (next_rho <= SS - 2 && last_plane(next_rho) + 3 < k1) {
@@ -1380,12 +1440,14 @@ static mg_status step_host_overlapped(mg_context *ctx, mg_atom_element *atoms, m
     }
     // the seam: ghost planes, the end slabs' density and ghost df, then their forces
     launch_ghost_copy_planes(lc, g, ctx->s, -1, -1);
+    launch_fix_records(lc, g, ctx->s, 0, static_cast<int>(g.gz * plane));
+    launch_fix_records(lc, g, ctx->s, static_cast<int>((g.gz + K) * plane), g.n_slots);
     rho_slab(0);
     rho_slab(SS - 1);
     launch_ghost_df_planes(lc, g, ctx->s, ctx->in, mx, 0, planes_from(1));
     launch_ghost_df_planes(lc, g, ctx->s, ctx->in, mx, df_hi, K);
     launch_ghost_df_planes(lc, g, ctx->s, ctx->in, mx, -1, -1);
-    if (mx) launch_skin_advance(lc, ctx->s);  // after the last density slab
+    if (mx || lc.fp) launch_skin_advance(lc, ctx->s);  // after the last density slab
     force_slab(1);
     force_slab(0);
     if ((st = flush(0, out_lo)) != MG_OK) return st;
@@ -1468,7 +1530,7 @@ static mg_status step_host_pipelined(mg_context *ctx, mg_atom_element *atoms, mg
     MG_CK(cudaEventRecord(ctx->pipe_ev[ev], ctx->stream));
     MG_CK(cudaStreamWaitEvent(ctx->copy_in, ctx->pipe_ev[ev++], 0));
     launch_set_counts(lc, ctx->in, 0);
-    launch_step_head(lc, ctx->d_sp);
+    launch_step_head(lc, ctx->d_sp, ctx->s.skin);
     for (int c = 0; c < S; c++) {
         const int z0 = c == 0 ? 0 : g.gz + local_plane_bound(c);
         const int z1 = c == S - 1 ? g.Sz : g.gz + local_plane_bound(c + 1);
@@ -1546,6 +1608,7 @@ static mg_status step_host_pipelined(mg_context *ctx, mg_atom_element *atoms, mg
             launch_ghost_df_planes(lc, g, ctx->s, ctx->in, mx, df_done, k);
             df_done = k;
         };
+        launch_fix_records(lc, g, ctx->s);
         rho_slab(0);
         rho_slab(1);
         // planes of slabs 1 .. S - 2 go out after their force; the plane cut by u[1] waits for slab 0
@@ -1558,7 +1621,7 @@ static mg_status step_host_pipelined(mg_context *ctx, mg_atom_element *atoms, mg
             if ((st = flush(z_done, z_to)) != MG_OK) return st;
             z_done = std::max(z_done, z_to);
         }
-        if (mx) launch_skin_advance(lc, ctx->s);  // after the last density slab (no firststep since)
+        if (mx || lc.fp) launch_skin_advance(lc, ctx->s);  // after the last density slab (no firststep since)
         launch_ghost_df_planes(lc, g, ctx->s, ctx->in, mx, -1, -1);
         launch_lat_force_sites(lc, g, ctx->s, ctx->in, ctx->pt, ctx->d_sp, true, mx, u[SS - 1], u[SS], true);
         if ((st = flush(z_done, g.Sz)) != MG_OK) return st;

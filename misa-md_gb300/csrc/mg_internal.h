@@ -8,6 +8,7 @@
 #include <vector>
 
 #include "../../include/misa_gb300.h"
+#include "mg_fixed.h"
 
 namespace mg {
 
@@ -94,7 +95,7 @@ struct SkinState {
     float acc;                       // the sum of the per-step maxima of |du| since the build
     int dirty;                       // a record changed outside firststep: the next pass rebuilds
     int rebuilt;                     // the last density pass rebuilt every group's list
-    int pad;
+    int wild;                        // FP64 form: an atom is too far from its site for the fixed-point records
     unsigned long long rebuilds;     // density passes that rebuilt every group's list
     unsigned long long passes;       // density passes with the group lists
 };
@@ -115,6 +116,9 @@ struct Slots {
                              // site of the group had inside rc + skin when the list was last built
     SkinState *skin;
     float *df32;             // F'(rho) in float
+    // FP64 form, the same layout (null: the passes run in FP64 throughout):
+    FixRec *fix;             // fixed-point coordinates and type of the positions the density pass is about to read
+    i64 *dfq;                // F'(rho) in fixed point, written wherever df is
 };
 
 // Inter-atom lists (local list in list order; ghost list in receive order).
@@ -217,6 +221,14 @@ bool read_setfl(const std::string &path, HostPotential &p, std::string &err);
 bool build_potential(int n_ele, const int32_t *zs, int nrho, double drho, int nr, double dr, double cutoff,
                      const double *F, const double *rho, const double *rphi, HostPotential &p, std::string &err);
 
+// Scales and tables of the fixed-point pair arithmetic for a lattice (a0, cutoff factor, the most candidates
+// summed at a time) and a potential; false when the tables do not suit it (mg_fixed.cpp states the bounds).
+struct FixTables {
+    std::vector<FixPoly> rho, zg, phi;
+};
+bool build_fixed(const HostPotential &hp, const int ele_of_type[3], double a0, double rcf, int n_part, FixParams &fp,
+                 FixTables &tab);
+
 // Offset tables (restatement of NeighbourIndex::make, src/atom/neighbour_index.inl:13-76) plus the
 // real-space site vector (in units of a0) of every entry.
 struct OffsetTable {
@@ -245,6 +257,7 @@ struct LaunchCtx {
     int rho_order = 0, rho_block = 256, rho_apt = 1;        // gather thread order, block size and atoms per thread
     int force_order = 0, force_block = 256, force_apt = 1;  // of the density and force passes (mg_autotune)
     const NeighTables *nt = nullptr;         // the context's offset tables
+    const FixParams *fp = nullptr;           // FP64 form: scales and tables of the fixed-point pair arithmetic
 };
 
 // Mass table shared by all contexts (atom types are fixed).
@@ -270,6 +283,9 @@ void launch_site_table(const LaunchCtx &lc, const Geom &g, double *site_half);
 void launch_decide_scan(const LaunchCtx &lc, const Geom &g, Slots s, Inter in);
 // after a deciding firststep: the displaced slots in scan order into in.displaced, count in CNT_DISPLACED
 void launch_displaced_collect(const LaunchCtx &lc, const Geom &g, Inter in);
+// FP64 form: the fixed-point records of the slots [s0, s1) (s1 < 0: to the end), after every change of a
+// position and before the density pass (the force hook: before the force pass)
+void launch_fix_records(const LaunchCtx &lc, const Geom &g, Slots s, int s0 = 0, int s1 = -1);
 // far-atom neighbourhood marks: clear those of the current far list / set them (grid-wide)
 void launch_far_clear(const LaunchCtx &lc, const Geom &g, Inter in);
 void launch_far_mark(const LaunchCtx &lc, const Geom &g, Inter in);
@@ -312,7 +328,7 @@ void launch_lat_force_sites(const LaunchCtx &lc, const Geom &g, Slots s, Inter i
                             bool mixed, int u0, int u1, bool lists = false);
 void launch_secondstep(const LaunchCtx &lc, const Geom &g, Slots s, Inter in, StepParams *sp, bool lattice);
 // step head: records the step's dt and, in variable mode, sets dt from the last kick's max |v|
-void launch_step_head(const LaunchCtx &lc, StepParams *sp);
+void launch_step_head(const LaunchCtx &lc, StepParams *sp, SkinState *skin);
 // out[0] = steps taken, out[1] = simulated time
 void launch_clock_sample(const LaunchCtx &lc, const StepParams *sp, double *out);
 // set the timestep rule and dt / dt/(2m) (dx_max <= 0: fixed dt)

@@ -33,6 +33,9 @@ void set_mass_table(cudaStream_t stream) {
     cudaStreamSynchronize(stream);
 }
 
+// the fixed-point form's parameters of a launch (off when the context has none)
+inline FixParams fix_params(const LaunchCtx &lc) { return lc.fp ? *lc.fp : FixParams{}; }
+
 // ------------------------------------------------------------------------------------------------
 // index helpers
 // ------------------------------------------------------------------------------------------------
@@ -326,7 +329,7 @@ __device__ __forceinline__ void kahan(float &sum, float &comp, float term) {
 // AoS <-> SoA (the reference's AtomElement array crosses the boundary as raw records)
 // ------------------------------------------------------------------------------------------------
 __global__ void k_unpack_aos(Geom g, const mg_atom_element *aos, Slots s, Inter in, int types_ok_mask, bool mixed, int s0,
-                             int s1) {
+                             int s1, FixParams fp) {
     const int t = s0 + blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= s1) return;
     mg_atom_element a = aos[t];
@@ -347,6 +350,7 @@ __global__ void k_unpack_aos(Geom g, const mg_atom_element *aos, Slots s, Inter 
         s.u4[sidx(g, t)] = a.type < 0 ? vacant_u4() : make_u4(g, a.x[0], a.x[1], a.x[2], xs, ys, zs, a.type);
     }
     if (mixed) s.df32[sidx(g, t)] = (float) a.df;
+    else if (fp.on) s.dfq[sidx(g, t)] = fix_df(fp, a.df);
 }
 
 __global__ void k_pack_aos(Geom g, mg_atom_element *aos, Slots s, int fields, bool mixed, int s0, int s1) {
@@ -377,8 +381,9 @@ void launch_unpack_aos(const LaunchCtx &lc, const Geom &g, const mg_atom_element
     if (s1 < 0) s1 = g.n_slots;
     if (s1 <= s0) return;
     const int b = 256;
-    k_unpack_aos<<<(s1 - s0 + b - 1) / b, b, 0, lc.stream>>>(g, aos, s, in, types_ok_mask, mixed, s0, s1);
+    k_unpack_aos<<<(s1 - s0 + b - 1) / b, b, 0, lc.stream>>>(g, aos, s, in, types_ok_mask, mixed, s0, s1, fix_params(lc));
     launch_skin_dirty(lc, s);
+    if (lc.fp) cudaMemsetAsync(&s.skin->wild, 0, sizeof(int), lc.stream);
 }
 __global__ void k_set_counts(Inter in, int n_inter) {
     in.cnt[CNT_INTER] = n_inter;
@@ -724,13 +729,21 @@ void launch_ghost_copy_planes(const LaunchCtx &lc, const Geom &g, Slots s, int k
 
 // forward df (DfEmbedPacker, src/pack/df_embed_packer.cpp): lattice ghosts and ghost inter atoms
 template <bool MIXED>
+__device__ __forceinline__ void ghost_df_one(const Geom &g, const Slots &s, int gs, int os) {
+    if (MIXED) {
+        s.df32[sidx(g, gs)] = s.df32[sidx(g, os)];
+    } else {
+        s.df[gs] = s.df[os];
+        if (s.dfq) s.dfq[sidx(g, gs)] = s.dfq[sidx(g, os)];
+    }
+}
+template <bool MIXED>
 __global__ void k_ghost_df(Geom g, Slots s, Inter in) {
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t < g.n_ghost_slots) {
         const int gs = ghost_slot(g, t);
         const int os = owner_slot(g, gs);
-        if (MIXED) s.df32[sidx(g, gs)] = s.df32[sidx(g, os)];
-        else s.df[gs] = s.df[os];
+        ghost_df_one<MIXED>(g, s, gs, os);
     }
     const int ng = in.cnt[CNT_GHOST];
     for (int q = t; q < ng; q += gridDim.x * blockDim.x) in.gdf[q] = in.df[in.groot[q]];
@@ -750,8 +763,7 @@ __global__ void k_ghost_df_planes(Geom g, Slots s, Inter in, int k0, int k1) {
         if (t < 2 * g.gz * g.Sy * g.Sx) {
             const int gs = ghost_slot(g, t);  // the z-ghost planes come first in the ghost enumeration
             const int os = owner_slot(g, gs);
-            if (MIXED) s.df32[sidx(g, gs)] = s.df32[sidx(g, os)];
-            else s.df[gs] = s.df[os];
+            ghost_df_one<MIXED>(g, s, gs, os);
         }
         const int ng = in.cnt[CNT_GHOST];
         for (int q = t; q < ng; q += gridDim.x * blockDim.x) in.gdf[q] = in.df[in.groot[q]];
@@ -772,8 +784,7 @@ __global__ void k_ghost_df_planes(Geom g, Slots s, Inter in, int k0, int k1) {
     }
     const int gs = lin(g, X, Y, Z);
     const int os = owner_slot(g, gs);
-    if (MIXED) s.df32[sidx(g, gs)] = s.df32[sidx(g, os)];
-    else s.df[gs] = s.df[os];
+    ghost_df_one<MIXED>(g, s, gs, os);
 }
 void launch_ghost_df_planes(const LaunchCtx &lc, const Geom &g, Slots s, Inter in, bool mixed, int k0, int k1) {
     const int b = 256;
@@ -801,6 +812,13 @@ __device__ __forceinline__ bool near_f32(const Geom &g, f2 uixy, float uiz, floa
     return dx * dx + dy * dy + dz * dz < g.rc2_pre;
 }
 
+// rho_tj(r) of one pair inside the cutoff
+__device__ __forceinline__ double rho_term_fp64(const PotTables &pt, double r2, int tj) {
+    const double r = r2 * rsqrt(r2);
+    int m; double p;
+    locate_d(r, pt.inv_dr, pt.nr, m, p);
+    return val_d(pt.rho_v + tj * pt.nr, m, p);
+}
 template <int PAR>
 __device__ __forceinline__ double rho_sum_fp64(const NeighTables &nt, const Geom &g, const Slots &s, const PotTables &pt, int sl,
                                                int si, float4 ui, double xi, double yi, double zi, int q0, int q1) {
@@ -815,22 +833,13 @@ __device__ __forceinline__ double rho_sum_fp64(const NeighTables &nt, const Geom
         const int tj = __float_as_int(uj.w);
         const double dx = xi - s.x[sj], dy = yi - s.y[sj], dz = zi - s.z[sj];
         const double r2 = dx * dx + dy * dy + dz * dz;
-        if (r2 < g.rc2) {
-            const double r = r2 * rsqrt(r2);
-            int m; double p;
-            locate_d(r, pt.inv_dr, pt.nr, m, p);
-            acc += val_d(pt.rho_v + tj * pt.nr, m, p);
-        }
+        if (r2 < g.rc2) acc += rho_term_fp64(pt, r2, tj);
     }
     return acc;
 }
-
-__device__ __forceinline__ void k_lat_rho_fp64_site(int t, const NeighTables &nt, const Geom &g, const Slots &s, const Inter &in, const PotTables &pt, bool hook, int order) {
-    int par;
-    const int sl = gather_slot(g, t, order, par);
-    if (sl < 0) return;
-    const int ti = s.type[sl];
-    if (ti < 0) { s.rho[sl] = 0.0; return; }
+// the density of one atom, all in FP64
+__device__ __forceinline__ double rho_atom_fp64(const NeighTables &nt, const Geom &g, const Slots &s, const Inter &in,
+                                                const PotTables &pt, int sl, int par) {
     const double xi = s.x[sl], yi = s.y[sl], zi = s.z[sl];
     const int si = sidx(g, sl);
     const float4 ui = s.u4[si];
@@ -842,6 +851,16 @@ __device__ __forceinline__ void k_lat_rho_fp64_site(int t, const NeighTables &nt
         acc += par ? rho_sum_fp64<1>(nt, g, s, pt, sl, si, ui, xi, yi, zi, np, nf)
                    : rho_sum_fp64<0>(nt, g, s, pt, sl, si, ui, xi, yi, zi, np, nf);
     }
+    return acc;
+}
+
+__device__ __forceinline__ void k_lat_rho_fp64_site(int t, const NeighTables &nt, const Geom &g, const Slots &s, const Inter &in, const PotTables &pt, bool hook, int order) {
+    int par;
+    const int sl = gather_slot(g, t, order, par);
+    if (sl < 0) return;
+    const int ti = s.type[sl];
+    if (ti < 0) { s.rho[sl] = 0.0; return; }
+    const double acc = rho_atom_fp64(nt, g, s, in, pt, sl, par);
     s.rho[sl] = acc;
     if (!hook && lattice_only(in)) {
         int m; double p;
@@ -1017,6 +1036,210 @@ __global__ void __launch_bounds__(512, 4) k_lat_rho_mixed(const __grid_constant_
         k_lat_rho_mixed_site(t, true, nt, g, s, in, pt, hook, order, false, true);
 }
 
+
+// ------------------------------------------------------------------------------------------------
+// FP64 form in fixed point (mg_fixed.h): the pair sums in 64-bit integers. Bound by integer issue and by the
+// table records' L1 wavefronts. A pair costs about 60 (density) and 110 (force) integer and single-precision
+// operations at one or two issue slots each; its FP64 operations cost 64 slots apiece, which bound the FP64
+// loops (2M atoms, step: 14.2 -> 2.1 ms; 300k atoms: 2.2 -> 0.50 ms; 16k atoms: 0.32 -> 0.14 ms). They stay
+// for the cases below and for tables the fixed point does not suit. Its errors are half the FP64 loops'
+// (thermal crystals against 113-bit arithmetic: force rms 2.4e-15 -> 1.1e-15 of the rms force).
+// The group lists of the mixed form serve here as well: 66 candidates are visited instead of 112.
+// Pairs closer than the tables reach (hot crystals, cascades) are kept per thread and summed in FP64 after
+// the loop; an atom with more than four of them, or with an F'(rho) too large for its fixed-point
+// range, is done in FP64 altogether, and so is every atom of a pass while some atom is too far from its
+// site for the wrapped coordinates (an uploaded state before its first decide).
+// ------------------------------------------------------------------------------------------------
+// The records of the slots [s0, s1): 25 bytes read and 32 written per slot, bound by HBM (0.2 ms at 16M
+// atoms of a 10 ms step), so that a candidate costs one 32-byte load instead of three 8-byte loads and
+// three conversions per pair.
+__global__ void k_fix_records(Geom g, Slots s, FixParams fp, int s0, int s1) {
+    const int t = s0 + blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= s1) return;
+    const int si = sidx(g, t);
+    const float4 u = s.u4[si];
+    const int ty = __float_as_int(u.w);
+    FixRec r;
+    r.type = ty;
+    if (ty >= 0) {
+        r.x = fix_coord(s.x[t], fp.kx);
+        r.y = fix_coord(s.y[t], fp.kx);
+        r.z = fix_coord(s.z[t], fp.kx);
+        // 1.2 half-lattice units: recombined atoms sit up to sqrt(5) / 2 of them from their site
+        if (!(fmaxf(fmaxf(fabsf(u.x), fabsf(u.y)), fabsf(u.z)) <= 1.2f) || u.x != u.x || u.y != u.y || u.z != u.z) s.skin->wild = 1;
+    } else {
+        const int X = t % g.Sx, q = t / g.Sx, Y = q % g.Sy, Z = q / g.Sy;
+        double xs, ys, zs;
+        site_of(g, X, Y, Z, xs, ys, zs);
+        const unsigned long long away = 1ull << 63;
+        r.x = (i64) ((unsigned long long) fix_coord(xs, fp.kx) ^ away);
+        r.y = (i64) ((unsigned long long) fix_coord(ys, fp.kx) ^ away);
+        r.z = (i64) ((unsigned long long) fix_coord(zs, fp.kx) ^ away);
+    }
+    longlong2 *o = reinterpret_cast<longlong2 *>(s.fix + si);
+    o[0] = make_longlong2(r.x, r.y);
+    o[1] = make_longlong2(r.z, r.type);
+}
+void launch_fix_records(const LaunchCtx &lc, const Geom &g, Slots s, int s0, int s1) {
+    if (!lc.fp) return;
+    if (s1 < 0) s1 = g.n_slots;
+    if (s1 <= s0) return;
+    k_fix_records<<<(s1 - s0 + 255) / 256, 256, 0, lc.stream>>>(g, s, *lc.fp, s0, s1);
+}
+
+// one 32-byte read-only load each
+__device__ __forceinline__ FixRec ld_fix_rec(const FixRec *p) {
+    FixRec r;
+    asm("ld.global.nc.v4.b64 {%0, %1, %2, %3}, [%4];" : "=l"(r.x), "=l"(r.y), "=l"(r.z), "=l"(r.type) : "l"(p));
+    return r;
+}
+__device__ __forceinline__ FixPoly ld_fix_poly(const FixPoly *p) {
+    FixPoly r;
+    i64 w;
+    asm("ld.global.nc.v4.b64 {%0, %1, %2, %3}, [%4];" : "=l"(r.c0), "=l"(r.c1), "=l"(r.c2), "=l"(w) : "l"(p));
+    r.c3 = (int) w;
+    r.c4 = fix_hi(w);
+    return r;
+}
+// the candidates closer than the tables reach: up to four candidate numbers, one byte each
+__device__ __forceinline__ void fix_note_near(unsigned &near, int q) {
+    near = near >> 24 ? 0xffffffffu : (near << 8) | (unsigned) (q + 1);
+}
+constexpr unsigned kFixNearMany = 0xffffffffu;  // more than fit (a candidate number is below 255)
+
+// an atom's density over its near pairs, or (many) over all pairs, in FP64
+__device__ __noinline__ double rho_near_fp64(const NeighTables &nt, const Geom &g, const Slots &s, const Inter &in,
+                                             const PotTables &pt, int sl, int par, unsigned near) {
+    if (near == kFixNearMany) return rho_atom_fp64(nt, g, s, in, pt, sl, par);
+    double acc = 0.0;
+    for (; near; near >>= 8) {
+        const int sj = sl + (par ? nt.lat[1][(near & 255u) - 1] : nt.lat[0][(near & 255u) - 1]);
+        const double dx = s.x[sl] - s.x[sj], dy = s.y[sl] - s.y[sj], dz = s.z[sl] - s.z[sj];
+        acc += rho_term_fp64(pt, dx * dx + dy * dy + dz * dz, s.type[sj]);
+    }
+    return acc;
+}
+
+// candidate q of the atom at (xb, yb, zb) (biased)
+template <int PAR>
+__device__ __forceinline__ void rho_fix_candidate(const NeighTables &nt, const Slots &s, const FixParams &fp, int si, i64 xb, i64 yb,
+                                                  i64 zb, int q, i64 &acc, unsigned &near) {
+    const FixRec j = ld_fix_rec(s.fix + si + __float_as_int(nt.cand[PAR][q].w));
+    const i64 r2 = fix_r2(fix_delta(xb - j.x, yb - j.y, zb - j.z), fp.b0);
+    if ((unsigned long long) (r2 - fp.lo) < (unsigned long long) (fp.rc2 - fp.lo)) {
+        int m;
+        const FixCoord t = fix_locate(fp, r2, m);
+        acc += fix_poly(ld_fix_poly(fp.rho + (int) j.type * fp.nr1 + m), t, fp.e3_rho);
+    } else if ((unsigned long long) r2 < (unsigned long long) fp.lo) {
+        fix_note_near(near, q);
+    }
+}
+// the candidates [q0, q1) after the single-precision test; NOTED: bit j of the result marks candidate
+// q0 + j within rc + skin (q1 - q0 <= 32)
+template <int PAR, bool NOTED>
+__device__ __forceinline__ unsigned rho_fix_range(const NeighTables &nt, const Geom &g, const Slots &s, const FixParams &fp, int si,
+                                                  float4 ui, i64 xb, i64 yb, i64 zb, int q0, int q1, i64 &acc, unsigned &near) {
+    const f2 uixy = f2_pack(ui.x, ui.y);
+    unsigned nb = 0;
+#pragma unroll 1
+    for (int q = q0; q < q1; q++) {
+        const float4 D = nt.cand[PAR][q];
+        f2 dxy; float dz;
+        const float r2 = pair_r2(uixy, ui.z, D, __ldg(s.u4 + si + __float_as_int(D.w)), dxy, dz);
+        if (NOTED && r2 < g.rcs2_h) nb |= 1u << (q - q0);
+        if (r2 < g.rc2_pre) rho_fix_candidate<PAR>(nt, s, fp, si, xb, yb, zb, q, acc, near);
+    }
+    return nb;
+}
+template <int PAR>
+__device__ __forceinline__ void rho_fix_listed(const NeighTables &nt, const Slots &s, const FixParams &fp, int si, i64 xb, i64 yb,
+                                               i64 zb, int q0, unsigned word, i64 &acc, unsigned &near) {
+    for (unsigned w = word; w; w &= w - 1) rho_fix_candidate<PAR>(nt, s, fp, si, xb, yb, zb, q0 + __ffs(w) - 1, acc, near);
+}
+
+// the pair sum over the candidates the tables bound (the pruned ones), and over the tail of a far atom's
+// neighbourhood: each fits the integers by itself. lists, full: as k_lat_rho_mixed_site.
+template <int PAR>
+__device__ __forceinline__ double rho_fix_atom(const NeighTables &nt, const Geom &g, const Slots &s, const FixParams &fp, int si,
+                                               float4 ui, const FixRec &me, bool lists, bool full, unsigned *list, unsigned live,
+                                               bool far, unsigned &near) {
+    const i64 xb = me.x + kFixBias, yb = me.y + kFixBias, zb = me.z + kFixBias;
+    const int np = nt.npruned;
+    i64 acc = 0;
+    if (lists && !full) {
+        const uint4 n4 = *reinterpret_cast<const uint4 *>(list);
+        for (int k = 0; k * 32 < np; k++)
+            rho_fix_listed<PAR>(nt, s, fp, si, xb, yb, zb, 32 * k, k == 0 ? n4.x : k == 1 ? n4.y : k == 2 ? n4.z : n4.w, acc, near);
+    } else if (lists) {
+        const bool leader = (int) (threadIdx.x & 31) == __ffs(live) - 1;
+        for (int k = 0; k * 32 < np; k++) {
+            const unsigned nb = rho_fix_range<PAR, true>(nt, g, s, fp, si, ui, xb, yb, zb, 32 * k, min(32 * k + 32, np), acc, near);
+            const unsigned any = __reduce_or_sync(live, nb);
+            if (leader) list[k] = any;
+        }
+    } else {
+        rho_fix_range<PAR, false>(nt, g, s, fp, si, ui, xb, yb, zb, 0, np, acc, near);
+    }
+    double rho = (double) acc * fp.rho_unit;
+    if (far) {
+        acc = 0;
+        rho_fix_range<PAR, false>(nt, g, s, fp, si, ui, xb, yb, zb, np, nt.nfull, acc, near);
+        rho += (double) acc * fp.rho_unit;
+    }
+    return rho;
+}
+__device__ __forceinline__ void k_lat_rho_fix_site(int t, bool valid, const NeighTables &nt, const Geom &g, const Slots &s,
+                                                   const Inter &in, const PotTables &pt, const FixParams &fp, bool hook, int order,
+                                                   bool lists, bool full, bool wild) {
+    int par = 0, u = 0;
+    const int sl = valid ? gather_site(g, t, order, par, u) : -1;
+    const int si = sl >= 0 ? sidx(g, sl) : 0;
+    const float4 ui = sl >= 0 ? s.u4[si] : vacant_u4();
+    const int ti = __float_as_int(ui.w);
+    const unsigned live = lists ? __ballot_sync(0xffffffffu, ti >= 0) : 0u;
+    const bool far = sl >= 0 && in.far_flag[sl];
+    if (lists && !full) full = __any_sync(0xffffffffu, far);
+    if (sl < 0) return;
+    if (ti < 0) { s.rho[sl] = 0.0; return; }
+    double rho = 0.0;
+    unsigned near = kFixNearMany;
+    if (!wild) {
+        near = 0u;
+        const FixRec me = ld_fix_rec(s.fix + si);
+        unsigned *list = group_list(g, s, par, u);
+        rho = par ? rho_fix_atom<1>(nt, g, s, fp, si, ui, me, lists, full, list, live, far, near)
+                  : rho_fix_atom<0>(nt, g, s, fp, si, ui, me, lists, full, list, live, far, near);
+    }
+    if (near) rho = rho_near_fp64(nt, g, s, in, pt, sl, par, near) + (near == kFixNearMany ? 0.0 : rho);
+    s.rho[sl] = rho;
+    if (!hook && lattice_only(in)) {
+        int m; double p;
+        locate_d(rho, pt.inv_drho, pt.nrho, m, p);
+        const double df = der_d(pt.F_d + ti * pt.nrho, m, p);
+        s.df[sl] = df;
+        s.dfq[si] = fix_df(fp, df);
+    }
+}
+template <bool LOOP>  // LOOP: several sites per thread, one grid stride apart (no group lists)
+__global__ void __launch_bounds__(512, 2) k_lat_rho_fix(const __grid_constant__ NeighTables nt, const __grid_constant__ Geom g,
+                                                        const __grid_constant__ Slots s, const __grid_constant__ Inter in,
+                                                        const __grid_constant__ PotTables pt, const __grid_constant__ FixParams fp,
+                                                        bool hook, int order, int tbase, int nthreads, bool lists) {
+    const int t0 = tbase + blockIdx.x * blockDim.x + threadIdx.x;  // threads [tbase, nthreads)
+    const bool wild = s.skin->wild != 0;  // the same in every thread of the grid: set before the pass
+    if (LOOP) {
+        for (int t = t0; t < nthreads; t += gridDim.x * blockDim.x)
+            k_lat_rho_fix_site(t, true, nt, g, s, in, pt, fp, hook, order, false, true, wild);
+        return;
+    }
+    const bool full = lists && !wild && skin_full(g, s);
+    if (lists && blockIdx.x == 0 && threadIdx.x == 0) {
+        if (wild) s.skin->dirty = 1;  // groups near a recombined atom did not rebuild their lists
+        else if (full) s.skin->rebuilt = 1;
+    }
+    k_lat_rho_fix_site(t0, t0 < nthreads, nt, g, s, in, pt, fp, hook, order, lists && !wild, full, wild);
+}
+
 // atoms per thread: each thread takes rho_apt sites, one grid stride apart (the stride is a multiple
 // of 64, so warps keep their parity and thread order)
 // The passes can keep and use per-group candidate lists when every warp of both passes covers one
@@ -1034,9 +1257,11 @@ static void launch_lat_rho_threads(const LaunchCtx &lc, const Geom &g, Slots s, 
     if (n <= 0) return;
     if (lc.rho_apt > 1) {
         if (mixed) k_lat_rho_mixed<true><<<n, b, 0, lc.stream>>>(*lc.nt, g, s, in, t, hook, order, tb, te, false);
+        else if (lc.fp) k_lat_rho_fix<true><<<n, b, 0, lc.stream>>>(*lc.nt, g, s, in, t, *lc.fp, hook, order, tb, te, false);
         else k_lat_rho_fp64<true><<<n, b, 0, lc.stream>>>(*lc.nt, g, s, in, t, hook, order, tb, te);
     } else {
         if (mixed) k_lat_rho_mixed<false><<<n, b, 0, lc.stream>>>(*lc.nt, g, s, in, t, hook, order, tb, te, lists);
+        else if (lc.fp) k_lat_rho_fix<false><<<n, b, 0, lc.stream>>>(*lc.nt, g, s, in, t, *lc.fp, hook, order, tb, te, lists);
         else k_lat_rho_fp64<false><<<n, b, 0, lc.stream>>>(*lc.nt, g, s, in, t, hook, order, tb, te);
     }
 }
@@ -1064,13 +1289,16 @@ __global__ void __launch_bounds__(kSkinSlots) k_skin_advance(SkinState *k) {
 void launch_skin_advance(const LaunchCtx &lc, Slots s) { k_skin_advance<<<1, kSkinSlots, 0, lc.stream>>>(s.skin); }
 void launch_skin_dirty(const LaunchCtx &lc, Slots s) { cudaMemsetAsync(&s.skin->dirty, 1, 1, lc.stream); }
 
-// A mixed pass with the group lists is followed by the skin's advance. A mixed pass without them
-// leaves the lists behind the positions, so the next pass with them rebuilds them.
+// whether a pass can use the group lists: the mixed form, and the FP64 form's fixed-point passes
+static bool has_lists(const LaunchCtx &lc, bool mixed) { return mixed || lc.fp; }
+// A pass with the group lists is followed by the skin's advance. A pass without them leaves the lists
+// behind the positions, so the next pass with them rebuilds them.
 void launch_lat_rho(const LaunchCtx &lc, const Geom &g, Slots s, Inter in, PotTables t, bool mixed, bool hook, bool lists) {
-    const bool v = lists && mixed && !hook && lists_ok(lc, g);
+    const bool v = lists && has_lists(lc, mixed) && !hook && lists_ok(lc, g);
+    if (!mixed) launch_fix_records(lc, g, s);
     launch_lat_rho_threads(lc, g, s, in, t, mixed, hook, 0, gather_threads(g, lc.rho_order), v);
     if (v) launch_skin_advance(lc, s);
-    else if (mixed) launch_skin_dirty(lc, s);
+    else if (has_lists(lc, mixed)) launch_skin_dirty(lc, s);
 }
 // thread range of the sites [u0, u1) of both parities (u0, u1 multiples of 32, or u1 = n_local_half)
 static void site_threads(const Geom &g, int order, int u0, int u1, int tb[2], int te[2], int &nr) {
@@ -1089,14 +1317,14 @@ void launch_lat_rho_sites(const LaunchCtx &lc, const Geom &g, Slots s, Inter in,
     if (u1 <= u0) return;
     int tb[2], te[2], nr;
     site_threads(g, lc.rho_order, u0, u1, tb, te, nr);
-    const bool v = lists && mixed && lists_ok(lc, g);
+    const bool v = lists && has_lists(lc, mixed) && lists_ok(lc, g);
     for (int r = 0; r < nr; r++) launch_lat_rho_threads(lc, g, s, in, t, mixed, false, tb[r], te[r], v);
-    if (!v && mixed) launch_skin_dirty(lc, s);  // the caller advances the skin after the last slab
+    if (!v && has_lists(lc, mixed)) launch_skin_dirty(lc, s);  // the caller advances the skin after the last slab
 }
 
 // dF/drho when inter atoms added density after the lattice pass (or for the df hook)
 template <bool MIXED>
-__global__ void k_lat_df(Geom g, Slots s, Inter in, PotTables pt, bool hook) {
+__global__ void k_lat_df(Geom g, Slots s, Inter in, PotTables pt, bool hook, FixParams fp) {
     if (!hook && lattice_only(in)) return;  // already fused into the density pass
     for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < g.n_local; t += gridDim.x * blockDim.x) {
         int i, j, k;
@@ -1110,15 +1338,17 @@ __global__ void k_lat_df(Geom g, Slots s, Inter in, PotTables pt, bool hook) {
         } else {
             int m; double p;
             locate_d(s.rho[sl], pt.inv_drho, pt.nrho, m, p);
-            s.df[sl] = der_d(pt.F_d + ti * pt.nrho, m, p);
+            const double df = der_d(pt.F_d + ti * pt.nrho, m, p);
+            s.df[sl] = df;
+            if (fp.on) s.dfq[sidx(g, sl)] = fix_df(fp, df);
         }
     }
 }
 void launch_lat_df(const LaunchCtx &lc, const Geom &g, Slots s, Inter in, PotTables t, bool mixed, bool hook) {
     const int b = 256;
     const int n = hook ? (g.n_local + b - 1) / b : std::max(1, std::min(lc.num_sms * 8, (g.n_local + b - 1) / b));
-    if (mixed) k_lat_df<true><<<n, b, 0, lc.stream>>>(g, s, in, t, hook);
-    else k_lat_df<false><<<n, b, 0, lc.stream>>>(g, s, in, t, hook);
+    if (mixed) k_lat_df<true><<<n, b, 0, lc.stream>>>(g, s, in, t, hook, FixParams{});
+    else k_lat_df<false><<<n, b, 0, lc.stream>>>(g, s, in, t, hook, fix_params(lc));
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -1127,11 +1357,26 @@ void launch_lat_df(const LaunchCtx &lc, const Geom &g, Slots s, Inter in, PotTab
 // is fused, and inside a fused graph (mixed form) so is the next loop body's firststep.
 // fpair = -(F'_i rho'_j(r) + F'_j rho'_i(r) + phi'_ij(r)) / r, phi = (r phi) / r.
 // ------------------------------------------------------------------------------------------------
+// fpair of one pair inside the cutoff
+__device__ __forceinline__ double fpair_fp64(const PotTables &pt, double r2, int ti, int tj, double dfi, double dfj) {
+    const double rinv = rsqrt(r2);
+    const double r = r2 * rinv;
+    int m; double p;
+    locate_d(r, pt.inv_dr, pt.nr, m, p);
+    const double rhojp = der_d(pt.rho_d + tj * pt.nr, m, p);
+    const double rhoip = (tj == ti) ? rhojp : der_d(pt.rho_d + ti * pt.nr, m, p);
+    const int pr = (ti * 3 + tj) * pt.nr;
+    const double zv = val_d(pt.z_v + pr, m, p);
+    const double zp = der_d(pt.z_d + pr, m, p);
+    const double phi = zv * rinv;
+    const double phip = zp * rinv - phi * rinv;
+    const double psip = dfi * rhojp + dfj * rhoip + phip;
+    return -psip * rinv;
+}
 template <int PAR>
 __device__ __forceinline__ void force_sum_fp64(const NeighTables &nt, const Geom &g, const Slots &s, const PotTables &pt, int sl, int ti,
                                                int si, float4 ui, double xi, double yi, double zi, double dfi, int q0, int q1,
                                                double &fx, double &fy, double &fz) {
-    const Knot64 *rho_di = pt.rho_d + ti * pt.nr;
     const f2 uixy = f2_pack(ui.x, ui.y);
 #pragma unroll 2
     for (int q = q0; q < q1; q++) {
@@ -1143,23 +1388,42 @@ __device__ __forceinline__ void force_sum_fp64(const NeighTables &nt, const Geom
         const double dx = xi - s.x[sj], dy = yi - s.y[sj], dz = zi - s.z[sj];
         const double r2 = dx * dx + dy * dy + dz * dz;
         if (r2 < g.rc2) {
-            const double rinv = rsqrt(r2);
-            const double r = r2 * rinv;
-            int m; double p;
-            locate_d(r, pt.inv_dr, pt.nr, m, p);
-            const double rhojp = der_d(pt.rho_d + tj * pt.nr, m, p);
-            const double rhoip = (tj == ti) ? rhojp : der_d(rho_di, m, p);
-            const int pr = (ti * 3 + tj) * pt.nr;
-            const double zv = val_d(pt.z_v + pr, m, p);
-            const double zp = der_d(pt.z_d + pr, m, p);
-            const double phi = zv * rinv;
-            const double phip = zp * rinv - phi * rinv;
-            const double psip = dfi * rhojp + s.df[sj] * rhoip + phip;
-            const double fpair = -psip * rinv;
+            const double fpair = fpair_fp64(pt, r2, ti, tj, dfi, s.df[sj]);
             fx += dx * fpair;
             fy += dy * fpair;
             fz += dz * fpair;
         }
+    }
+}
+// the lattice force on one atom, all in FP64
+__device__ __forceinline__ void force_atom_fp64(const NeighTables &nt, const Geom &g, const Slots &s, const Inter &in,
+                                                const PotTables &pt, int sl, int ti, int par, double &fx, double &fy,
+                                                double &fz) {
+    const double xi = s.x[sl], yi = s.y[sl], zi = s.z[sl];
+    const double dfi = s.df[sl];
+    const int si = sidx(g, sl);
+    const float4 ui = s.u4[si];
+    fx = 0.0; fy = 0.0; fz = 0.0;
+    const int np = nt.npruned;
+    if (par) force_sum_fp64<1>(nt, g, s, pt, sl, ti, si, ui, xi, yi, zi, dfi, 0, np, fx, fy, fz);
+    else force_sum_fp64<0>(nt, g, s, pt, sl, ti, si, ui, xi, yi, zi, dfi, 0, np, fx, fy, fz);
+    if (in.far_flag[sl]) {
+        const int nf = nt.nfull;
+        if (par) force_sum_fp64<1>(nt, g, s, pt, sl, ti, si, ui, xi, yi, zi, dfi, np, nf, fx, fy, fz);
+        else force_sum_fp64<0>(nt, g, s, pt, sl, ti, si, ui, xi, yi, zi, dfi, np, nf, fx, fy, fz);
+    }
+}
+// stores the force and takes the second half-kick where the lattice pass may
+__device__ __forceinline__ void force_done_fp64(const Slots &s, const Inter &in, StepParams *sp, int sl, int ti, double fx,
+                                                double fy, double fz, bool kick, bool hook) {
+    s.fx[sl] = fx; s.fy[sl] = fy; s.fz[sl] = fz;
+    if (kick && !hook && kick_in_lattice_pass(in, sl)) {
+        const double c = dt_inv_m_of(sp, ti);
+        const double vx = __dadd_rn(s.vx[sl], __dmul_rn(c, fx));
+        const double vy = __dadd_rn(s.vy[sl], __dmul_rn(c, fy));
+        const double vz = __dadd_rn(s.vz[sl], __dmul_rn(c, fz));
+        s.vx[sl] = vx; s.vy[sl] = vy; s.vz[sl] = vz;
+        if (variable_dt(sp)) note_vmax2(sp, speed2(vx, vy, vz));
     }
 }
 
@@ -1170,28 +1434,9 @@ __device__ __forceinline__ void k_lat_force_fp64_site(int t, const NeighTables &
     if (sl < 0) return;
     const int ti = s.type[sl];
     if (ti < 0) { s.fx[sl] = 0.0; s.fy[sl] = 0.0; s.fz[sl] = 0.0; return; }
-    const double xi = s.x[sl], yi = s.y[sl], zi = s.z[sl];
-    const double dfi = s.df[sl];
-    const int si = sidx(g, sl);
-    const float4 ui = s.u4[si];
-    double fx = 0.0, fy = 0.0, fz = 0.0;
-    const int np = nt.npruned;
-    if (par) force_sum_fp64<1>(nt, g, s, pt, sl, ti, si, ui, xi, yi, zi, dfi, 0, np, fx, fy, fz);
-    else force_sum_fp64<0>(nt, g, s, pt, sl, ti, si, ui, xi, yi, zi, dfi, 0, np, fx, fy, fz);
-    if (in.far_flag[sl]) {
-        const int nf = nt.nfull;
-        if (par) force_sum_fp64<1>(nt, g, s, pt, sl, ti, si, ui, xi, yi, zi, dfi, np, nf, fx, fy, fz);
-        else force_sum_fp64<0>(nt, g, s, pt, sl, ti, si, ui, xi, yi, zi, dfi, np, nf, fx, fy, fz);
-    }
-    s.fx[sl] = fx; s.fy[sl] = fy; s.fz[sl] = fz;
-    if (kick && !hook && kick_in_lattice_pass(in, sl)) {
-        const double c = dt_inv_m_of(sp, ti);
-        const double vx = __dadd_rn(s.vx[sl], __dmul_rn(c, fx));
-        const double vy = __dadd_rn(s.vy[sl], __dmul_rn(c, fy));
-        const double vz = __dadd_rn(s.vz[sl], __dmul_rn(c, fz));
-        s.vx[sl] = vx; s.vy[sl] = vy; s.vz[sl] = vz;
-        if (variable_dt(sp)) note_vmax2(sp, speed2(vx, vy, vz));
-    }
+    double fx, fy, fz;
+    force_atom_fp64(nt, g, s, in, pt, sl, ti, par, fx, fy, fz);
+    force_done_fp64(s, in, sp, sl, ti, fx, fy, fz, kick, hook);
 }
 template <bool LOOP>  // LOOP: several sites per thread, one grid stride apart
 __global__ void __launch_bounds__(512) k_lat_force_fp64(const __grid_constant__ NeighTables nt, Geom g, Slots s, Inter in, PotTables pt,
@@ -1203,6 +1448,138 @@ __global__ void __launch_bounds__(512) k_lat_force_fp64(const __grid_constant__ 
         return;
     }
     for (int t = t0; t < nthreads; t += gridDim.x * blockDim.x) k_lat_force_fp64_site(t, nt, g, s, in, pt, sp, kick, hook, order);
+}
+
+// ---- FP64 form in fixed point: see the density pass ----
+struct FixForce {
+    i64 x, y, z;     // sum of (x_i - x_j) (F'_i rho'_j + F'_j rho'_i + phi') / r: minus the force
+    int df_hi;       // largest upper word of F'_i + F'_j met
+    unsigned near;
+};
+// an atom's force over its near pairs, or (many) over all pairs, in FP64
+__device__ __noinline__ double3 force_near_fp64(const NeighTables &nt, const Geom &g, const Slots &s, const Inter &in,
+                                                const PotTables &pt, int sl, int ti, int par, unsigned near) {
+    double fx = 0.0, fy = 0.0, fz = 0.0;
+    if (near == kFixNearMany) {
+        force_atom_fp64(nt, g, s, in, pt, sl, ti, par, fx, fy, fz);
+    } else {
+        for (; near; near >>= 8) {
+            const int sj = sl + (par ? nt.lat[1][(near & 255u) - 1] : nt.lat[0][(near & 255u) - 1]);
+            const double dx = s.x[sl] - s.x[sj], dy = s.y[sl] - s.y[sj], dz = s.z[sl] - s.z[sj];
+            const double fpair = fpair_fp64(pt, dx * dx + dy * dy + dz * dz, ti, s.type[sj], s.df[sl], s.df[sj]);
+            fx += dx * fpair;
+            fy += dy * fpair;
+            fz += dz * fpair;
+        }
+    }
+    return make_double3(fx, fy, fz);
+}
+template <int PAR>
+__device__ __forceinline__ void force_fix_candidate(const NeighTables &nt, const Slots &s, const FixParams &fp, int si, int ti, i64 xb,
+                                                    i64 yb, i64 zb, i64 dfb, int q, FixForce &a) {
+    const int oj = si + __float_as_int(nt.cand[PAR][q].w);
+    const FixRec j = ld_fix_rec(s.fix + oj);
+    const FixDelta d = fix_delta(xb - j.x, yb - j.y, zb - j.z);
+    const i64 r2 = fix_r2(d, fp.b0);
+    if ((unsigned long long) (r2 - fp.lo) < (unsigned long long) (fp.rc2 - fp.lo)) {
+        const i64 dfj = __ldg(s.dfq + oj);
+        int m;
+        const FixCoord t = fix_locate(fp, r2, m);
+        const int tj = (int) j.type;
+        const FixPoly *rec = fp.zg + 2 * ((ti * 3 + tj) * fp.nr1 + m);
+        const i64 gj = fix_poly(ld_fix_poly(rec), t, fp.e3_g);
+        i64 f = fix_poly(ld_fix_poly(rec + 1), t, fp.e3_h);
+        const i64 both = dfb + dfj;  // biased
+        a.df_hi = max(a.df_hi, fix_hi(both));
+        if (tj == ti) {
+            f = fix_mul_add(fix_hi(both), fix_lo(both), fix_hi(gj), fix_lo(gj), f);
+        } else {
+            const i64 gi = fix_poly(ld_fix_poly(fp.zg + 2 * ((tj * 3 + ti) * fp.nr1 + m)), t, fp.e3_g);
+            const i64 djb = dfj + kFixBias;
+            f = fix_mul_add(fix_hi(dfb), fix_lo(dfb), fix_hi(gj), fix_lo(gj), f);
+            f = fix_mul_add(fix_hi(djb), fix_lo(djb), fix_hi(gi), fix_lo(gi), f);
+        }
+        const int fh = fix_hi(f), fl = fix_lo(f);
+        a.x = fix_mul_add(d.xh, d.xl, fh, fl, a.x);
+        a.y = fix_mul_add(d.yh, d.yl, fh, fl, a.y);
+        a.z = fix_mul_add(d.zh, d.zl, fh, fl, a.z);
+    } else if ((unsigned long long) r2 < (unsigned long long) fp.lo) {
+        fix_note_near(a.near, q);
+    }
+}
+template <int PAR>
+__device__ __forceinline__ void force_fix_range(const NeighTables &nt, const Geom &g, const Slots &s, const FixParams &fp, int si,
+                                                int ti, float4 ui, i64 xb, i64 yb, i64 zb, i64 dfb, int q0, int q1, FixForce &a) {
+    const f2 uixy = f2_pack(ui.x, ui.y);
+#pragma unroll 1
+    for (int q = q0; q < q1; q++) {
+        const float4 D = nt.cand[PAR][q];
+        if (near_f32(g, uixy, ui.z, D, __ldg(s.u4 + si + __float_as_int(D.w))))
+            force_fix_candidate<PAR>(nt, s, fp, si, ti, xb, yb, zb, dfb, q, a);
+    }
+}
+template <int PAR>
+__device__ __forceinline__ void force_fix_atom(const NeighTables &nt, const Geom &g, const Slots &s, const FixParams &fp, int si,
+                                               int ti, const FixRec &me, const unsigned *list, bool far, FixForce &a, double3 &f) {
+    const i64 xb = me.x + kFixBias, yb = me.y + kFixBias, zb = me.z + kFixBias, dfb = s.dfq[si] + kFixBias;
+    const int np = nt.npruned;
+    if (list) {
+        for (int k = 0; k * 32 < np; k++)
+            for (unsigned w = list[k]; w; w &= w - 1)
+                force_fix_candidate<PAR>(nt, s, fp, si, ti, xb, yb, zb, dfb, 32 * k + __ffs(w) - 1, a);
+    } else {
+        force_fix_range<PAR>(nt, g, s, fp, si, ti, s.u4[si], xb, yb, zb, dfb, 0, np, a);
+    }
+    f = make_double3(-(double) a.x * fp.f_unit, -(double) a.y * fp.f_unit, -(double) a.z * fp.f_unit);
+    if (far) {  // each part fits the integers by itself
+        a.x = 0; a.y = 0; a.z = 0;
+        force_fix_range<PAR>(nt, g, s, fp, si, ti, s.u4[si], xb, yb, zb, dfb, np, nt.nfull, a);
+        f.x -= (double) a.x * fp.f_unit;
+        f.y -= (double) a.y * fp.f_unit;
+        f.z -= (double) a.z * fp.f_unit;
+    }
+}
+__device__ __forceinline__ void k_lat_force_fix_site(int t, const NeighTables &nt, const Geom &g, const Slots &s, const Inter &in,
+                                                     const PotTables &pt, const FixParams &fp, StepParams *sp, bool kick, bool hook,
+                                                     int order, bool lists, bool wild) {
+    int par, u;
+    const int sl = gather_site(g, t, order, par, u);
+    if (sl < 0) return;
+    const int si = sidx(g, sl);
+    const FixRec me = ld_fix_rec(s.fix + si);
+    const int ti = (int) me.type;
+    if (ti < 0) { s.fx[sl] = 0.0; s.fy[sl] = 0.0; s.fz[sl] = 0.0; return; }
+    FixForce a{0, 0, 0, 0, kFixNearMany};
+    double3 f{0.0, 0.0, 0.0};
+    if (!wild) {
+        a.near = 0u;
+        const unsigned *list = lists ? group_list(g, s, par, u) : nullptr;
+        const bool far = in.far_flag[sl];
+        if (par) force_fix_atom<1>(nt, g, s, fp, si, ti, me, list, far, a, f);
+        else force_fix_atom<0>(nt, g, s, fp, si, ti, me, list, far, a, f);
+        if (a.df_hi >= kFixBadHi) a.near = kFixNearMany;
+    }
+    if (a.near) {
+        const double3 n = force_near_fp64(nt, g, s, in, pt, sl, ti, par, a.near);
+        if (a.near == kFixNearMany) f = n;
+        else { f.x += n.x; f.y += n.y; f.z += n.z; }
+    }
+    force_done_fp64(s, in, sp, sl, ti, f.x, f.y, f.z, kick, hook);
+}
+template <bool LOOP>  // LOOP: several sites per thread, one grid stride apart (no group lists)
+__global__ void __launch_bounds__(512, 2) k_lat_force_fix(const __grid_constant__ NeighTables nt, const __grid_constant__ Geom g,
+                                                          const __grid_constant__ Slots s, const __grid_constant__ Inter in,
+                                                          const __grid_constant__ PotTables pt, const __grid_constant__ FixParams fp,
+                                                          StepParams *sp, bool kick, bool hook, int order, int tbase, int nthreads,
+                                                          bool lists) {
+    const int t0 = tbase + blockIdx.x * blockDim.x + threadIdx.x;  // threads [tbase, nthreads)
+    const bool wild = s.skin->wild != 0;
+    if (!LOOP) {
+        if (t0 < nthreads) k_lat_force_fix_site(t0, nt, g, s, in, pt, fp, sp, kick, hook, order, lists && !wild, wild);
+        return;
+    }
+    for (int t = t0; t < nthreads; t += gridDim.x * blockDim.x)
+        k_lat_force_fix_site(t, nt, g, s, in, pt, fp, sp, kick, hook, order, false, wild);
 }
 
 // Compensated force sums of the mixed form: each pair term d * fpair is added by Kahan's method
@@ -1377,23 +1754,26 @@ static void launch_lat_force_threads(const LaunchCtx &lc, const Geom &g, Slots s
     const bool fuse = fuse_next && mixed && kick && !hook;
     if (lc.force_apt > 1) {
         if (mixed) k_lat_force_mixed<true><<<n, b, 0, lc.stream>>>(*lc.nt, g, s, in, t, p, kick, hook, order, tb, te, fuse, false);
+        else if (lc.fp) k_lat_force_fix<true><<<n, b, 0, lc.stream>>>(*lc.nt, g, s, in, t, *lc.fp, p, kick, hook, order, tb, te, false);
         else k_lat_force_fp64<true><<<n, b, 0, lc.stream>>>(*lc.nt, g, s, in, t, p, kick, hook, order, tb, te);
     } else {
         if (mixed) k_lat_force_mixed<false><<<n, b, 0, lc.stream>>>(*lc.nt, g, s, in, t, p, kick, hook, order, tb, te, fuse, lists);
+        else if (lc.fp) k_lat_force_fix<false><<<n, b, 0, lc.stream>>>(*lc.nt, g, s, in, t, *lc.fp, p, kick, hook, order, tb, te, lists);
         else k_lat_force_fp64<false><<<n, b, 0, lc.stream>>>(*lc.nt, g, s, in, t, p, kick, hook, order, tb, te);
     }
 }
 void launch_lat_force(const LaunchCtx &lc, const Geom &g, Slots s, Inter in, PotTables t, StepParams *p, bool kick,
                       bool mixed, bool hook, bool fuse_next, bool lists) {
+    if (hook && !mixed) launch_fix_records(lc, g, s);
     launch_lat_force_threads(lc, g, s, in, t, p, kick, mixed, hook, 0, gather_threads(g, lc.force_order), fuse_next,
-                             lists && mixed && !hook && lists_ok(lc, g));
+                             lists && has_lists(lc, mixed) && !hook && lists_ok(lc, g));
 }
 void launch_lat_force_sites(const LaunchCtx &lc, const Geom &g, Slots s, Inter in, PotTables t, StepParams *p, bool kick,
                             bool mixed, int u0, int u1, bool lists) {
     if (u1 <= u0) return;
     int tb[2], te[2], nr;
     site_threads(g, lc.force_order, u0, u1, tb, te, nr);
-    const bool v = lists && mixed && lists_ok(lc, g);
+    const bool v = lists && has_lists(lc, mixed) && lists_ok(lc, g);
     for (int r = 0; r < nr; r++) launch_lat_force_threads(lc, g, s, in, t, p, kick, mixed, false, tb[r], te[r], false, v);
 }
 
@@ -1460,7 +1840,7 @@ void launch_set_step(const LaunchCtx &lc, StepParams *sp, double dt, double dx_m
 }
 // One block of kVmaxSlots threads: reduce and clear the max words, then (variable mode)
 // dt = clamp(dx_max / sqrt(max |v|^2), dt_min, dt_max); record dt and advance the clock.
-__global__ void __launch_bounds__(kVmaxSlots) k_step_head(StepParams *p) {
+__global__ void __launch_bounds__(kVmaxSlots) k_step_head(StepParams *p, SkinState *skin) {
     __shared__ unsigned long long part[kVmaxSlots / 32];
     const unsigned long long b = p->vmax2[threadIdx.x];
     p->vmax2[threadIdx.x] = 0ull;
@@ -1470,6 +1850,7 @@ __global__ void __launch_bounds__(kVmaxSlots) k_step_head(StepParams *p) {
     if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = ((unsigned long long) mhi << 32) | mlo;
     __syncthreads();
     if (threadIdx.x != 0) return;
+    skin->wild = 0;  // the step's records find out again
     unsigned long long m = 0ull;
     for (int w = 0; w < kVmaxSlots / 32; w++) m = part[w] > m ? part[w] : m;
     if (p->dx_max > 0.0) {
@@ -1484,7 +1865,9 @@ __global__ void __launch_bounds__(kVmaxSlots) k_step_head(StepParams *p) {
     p->time = __dadd_rn(p->time, p->dt);
     p->steps = k + 1;
 }
-void launch_step_head(const LaunchCtx &lc, StepParams *sp) { k_step_head<<<1, kVmaxSlots, 0, lc.stream>>>(sp); }
+void launch_step_head(const LaunchCtx &lc, StepParams *sp, SkinState *skin) {
+    k_step_head<<<1, kVmaxSlots, 0, lc.stream>>>(sp, skin);
+}
 // steps taken and simulated time into a sample record (stage machine thermo output)
 __global__ void k_clock_sample(const StepParams *p, double *out) {
     out[0] = (double) p->steps;
