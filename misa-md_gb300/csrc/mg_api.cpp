@@ -97,8 +97,10 @@ struct mg_context {
     uint64_t stage_dump_interval = 0;
     std::string origin_path;
 
-    // [precision][rho, force] = {thread order, block size, atoms per thread}
-    int tune[2][2][3] = {{{0, 256, 1}, {0, 256, 1}}, {{0, 256, 1}, {0, 256, 1}}};
+    // [precision][rho, force] = {thread order, block size, atoms per thread}. Order 1 until an autotune: its
+    // warps cover whole 32-site groups in every box, so the group lists serve boxes with an odd number of sites
+    // of a parity as well (order 0 visits all 112 candidates there).
+    int tune[2][2][3] = {{{1, 256, 1}, {1, 256, 1}}, {{1, 256, 1}, {1, 256, 1}}};
     LaunchCtx lc() const {
         LaunchCtx l{stream, num_sms};
         l.nt = &nt;
