@@ -390,11 +390,11 @@ mg_status install_potential(mg_context *ctx, const HostPotential &hp) {
             const HostSpline &rb = hp.rho[ele_of_type[b]];
             for (size_t m = 0; m < nr; m++) {
                 float *r = &zr[8 * ((a * 3 + b) * nr + m)];
-                // interleaved for a packed Horner step: {c0, d0, c1, d1, c2, d2, c3, 0}
+                // interleaved for a packed Horner step: {c0, d0, c1, d1, c2, d2, c3, 3 c3}
                 r[0] = (float) z.c0[m]; r[1] = (float) rb.d0[m];
                 r[2] = (float) z.c1[m]; r[3] = (float) rb.d1[m];
                 r[4] = (float) z.c2[m]; r[5] = (float) rb.d2[m];
-                r[6] = (float) z.c3[m]; r[7] = 0.0f;
+                r[6] = (float) z.c3[m]; r[7] = 3.0f * r[6];
             }
         }
     }
@@ -419,6 +419,7 @@ mg_status install_potential(mg_context *ctx, const HostPotential &hp) {
     pt.inv_dr_f = (float) pt.inv_dr;
     pt.inv_drho_f = (float) pt.inv_drho;
     pt.h_inv_dr_f = (float) (0.5 * ctx->g.a0 * pt.inv_dr);
+    pt.knot_max_f = 8388608.0f + (float) (hp.nr - 1);
     pt.rho_v = d_vd + base_rho; pt.rho_d = d_dd + base_rho;
     pt.F_v = d_vd + base_F; pt.F_d = d_dd + base_F;
     pt.z_v = d_vd + base_z; pt.z_d = d_dd + base_z;

@@ -170,10 +170,11 @@ struct PotTables {
     int nr, nrho;
     double inv_dr, inv_drho;
     float inv_dr_f, inv_drho_f, h_inv_dr_f;   // h_inv_dr_f = (a0/2) / dr
+    float knot_max_f;                         // 2^23 + nr - 1
     const Knot64 *rho_v, *rho_d, *F_v, *F_d, *z_v, *z_d;
     const float4 *rho_vf, *rho_dff, *F_vf, *F_dff, *z_vf, *z_dff;
     // force pass, mixed form: per type pair (ti * 3 + tj) and knot one 32-byte record
-    // {r*phi c0, rho_tj' d0, c1, d1, c2, d2, c3, 0}; r*phi' comes from the value coefficients
+    // {r*phi c0, rho_tj' d0, c1, d1, c2, d2, c3, 3 c3}; r*phi' comes from the value coefficients
     const float *zr8;
 };
 
