@@ -52,6 +52,7 @@ struct mg_context {
     OffsetTable offs;
     std::vector<int> lat_order[2];  // reordered full table (pruned entries first), linear offsets
     NeighTables nt{};               // the tables as the kernels receive them
+    float4 *d_cand = nullptr;       // nt.cand in device memory
     int n_full = 0, n_pruned = 0;
     cudaStream_t stream = nullptr;
     int num_sms = 1;
@@ -101,9 +102,12 @@ struct mg_context {
     // warps cover whole 32-site groups in every box, so the group lists serve boxes with an odd number of sites
     // of a parity as well (order 0 visits all 112 candidates there).
     int tune[2][2][3] = {{{1, 256, 1}, {1, 256, 1}}, {{1, 256, 1}, {1, 256, 1}}};
+    int share = 1;                  // contexts stepping side by side (while a batch captures)
     LaunchCtx lc() const {
         LaunchCtx l{stream, num_sms};
+        l.share = share;
         l.nt = &nt;
+        l.cand = d_cand;
         l.fp = !mixed() && fp.on && s.fix ? &fp : nullptr;
         l.rho_order = tune[precision][0][0];
         l.rho_block = tune[precision][0][1];
@@ -342,6 +346,8 @@ mg_status upload_tables(mg_context *ctx) {
                                         int_bits_as_float(delta));
         }
     }
+    if (!ctx->d_cand) MG_CK(dalloc(ctx, &ctx->d_cand, static_cast<size_t>(2 * kMaxFull)));
+    MG_CK(cudaMemcpy(ctx->d_cand, nt.cand, sizeof(nt.cand), cudaMemcpyHostToDevice));
     set_mass_table(ctx->stream);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) { ctx->err = std::string("mass table: ") + cudaGetErrorString(e); return MG_ERR_CUDA; }
@@ -1861,10 +1867,12 @@ mg_status capture_batch(mg_batch *b, int steps, cudaGraphExec_t *exec, int *n_no
     for (size_t r = 0; r < b->ctxs.size() && e == cudaSuccess; r++) {
         mg_context *ctx = b->ctxs[r];
         e = cudaStreamWaitEvent(ctx->stream, b->ev_fork, 0);
+        ctx->share = static_cast<int>(b->ctxs.size());
         for (int k = 0; k < steps && e == cudaSuccess; k++) {
             seq_step(ctx, nullptr);
             e = cudaGetLastError();
         }
+        ctx->share = 1;
         if (e == cudaSuccess) e = cudaEventRecord(b->ev_ctx[r], ctx->stream);
         if (e == cudaSuccess) e = cudaStreamWaitEvent(b->stream, b->ev_ctx[r], 0);
     }

@@ -258,7 +258,9 @@ struct LaunchCtx {
     int rho_order = 0, rho_block = 256, rho_apt = 1;        // gather thread order, block size and atoms per thread
     int force_order = 0, force_block = 256, force_apt = 1;  // of the density and force passes (mg_autotune)
     const NeighTables *nt = nullptr;         // the context's offset tables
+    const float4 *cand = nullptr;            // its cand[2][kMaxFull] in device memory
     const FixParams *fp = nullptr;           // FP64 form: scales and tables of the fixed-point pair arithmetic
+    int share = 1;                           // contexts that step side by side (a batch's members)
 };
 
 // Mass table shared by all contexts (atom types are fixed).

@@ -981,6 +981,18 @@ __device__ __forceinline__ unsigned *group_list(const Geom &g, const Slots &s, i
     return s.near + kListWords * (par * ((g.n_local_half + 31) >> 5) + (u >> 5));
 }
 
+// stores the density and, where nothing adds to it afterwards, F'(rho)
+__device__ __forceinline__ void rho_done_mixed(const Slots &s, const Inter &in, const PotTables &pt, int sl, int si, int ti, float sum,
+                                               float comp, bool hook) {
+    const double rho = (double) sum - (double) comp;
+    s.rho[sl] = rho;
+    if (!hook && lattice_only(in)) {
+        int m; float p;
+        locate_f((float) rho, pt.inv_drho_f, pt.nrho, m, p);
+        s.df32[si] = der_f(pt.F_dff + ti * pt.nrho, m, p);
+    }
+}
+
 // lists: use the group lists (all 32 lanes of the warp call this, with valid false for threads past
 // the end; the warp covers one 32-site group of one parity). full: visit every pruned candidate and
 // rebuild the group's list; else visit the listed candidates only.
@@ -1029,13 +1041,7 @@ __device__ __forceinline__ void k_lat_rho_mixed_site(int t, bool valid, const Ne
         if (par) rho_sum_mixed<1>(nt, g, s, pt, si, ui, np, nf, sum, comp);
         else rho_sum_mixed<0>(nt, g, s, pt, si, ui, np, nf, sum, comp);
     }
-    const double rho = (double) sum - (double) comp;
-    s.rho[sl] = rho;
-    if (!hook && lattice_only(in)) {
-        int m; float p;
-        locate_f((float) rho, pt.inv_drho_f, pt.nrho, m, p);
-        s.df32[si] = der_f(pt.F_dff + ti * pt.nrho, m, p);
-    }
+    rho_done_mixed(s, in, pt, sl, si, ti, sum, comp, hook);
 }
 template <bool LOOP>  // LOOP: several sites per thread, one grid stride apart (no group lists)
 __global__ void __launch_bounds__(512, 4) k_lat_rho_mixed(const __grid_constant__ NeighTables nt, Geom g, Slots s, Inter in, PotTables pt, bool hook, int order, int tbase,
@@ -1051,6 +1057,169 @@ __global__ void __launch_bounds__(512, 4) k_lat_rho_mixed(const __grid_constant_
         k_lat_rho_mixed_site(t, true, nt, g, s, in, pt, hook, order, false, true);
 }
 
+
+
+// ------------------------------------------------------------------------------------------------
+// Small boxes and thin slabs: one block of W warps per 32-site group. A warp of the whole-group passes walks
+// about 66 candidates one after another, each a chain of dependent loads and some 90 dependent instructions,
+// so a pass lasts 30 to 70 us however few atoms it has. Here the W warps share a group's candidates, W streams
+// of them at a time, and what the terms add up to stays what the whole-group passes give, bit for bit.
+// FP64 form: the sums are integers, so each warp takes all 32 sites and a share of the candidates.
+// Mixed form: compensated sums depend on their order. A warp takes 32 / W sites, its lanes W consecutive
+// candidates of each, and every lane adds the W terms of its site up in candidate order, by shuffles; no term
+// goes through memory.
+// ------------------------------------------------------------------------------------------------
+constexpr int kSplitSegment = 32 * kListWords;  // candidates listed at a time
+struct SplitList {
+    unsigned words[kListWords];
+    float4 rec[kSplitSegment];                  // the listed candidates' records, in candidate order
+    unsigned char num[kSplitSegment];           // and their numbers, from the segment's first
+};
+// the block's group: sites u0 + 32 (b / 2) .. + 31 of parity b & 1, one per lane of each warp
+struct SplitSite {
+    int par, u, sl, si, ti;
+    float4 ui;
+};
+__device__ __forceinline__ SplitSite split_site(const Geom &g, const Slots &s, int u0, int u1) {
+    SplitSite a;
+    a.par = blockIdx.x & 1;
+    a.u = u0 + 32 * (blockIdx.x >> 1) + (threadIdx.x & 31);
+    a.sl = -1;
+    a.si = 0;
+    a.ui = vacant_u4();
+    if (a.u < u1) {
+        const int r = a.u / g.nxh;
+        a.sl = lin(g, 2 * (a.u % g.nxh) + a.par + g.gx, r % g.by + g.gy, r / g.by + g.gz);
+        a.si = sidx(g, a.sl);
+        a.ui = s.u4[a.si];
+    }
+    a.ti = __float_as_int(a.ui.w);
+    return a;
+}
+// Lists the candidates [q0, q1) (at most kSplitSegment; cand: the records of the group's parity) that some site
+// with `mine` set has within r2max: those of the words `known`, or (null) by looking. Returns their number. All
+// threads of the block call it.
+template <int W>
+__device__ __forceinline__ int split_list(const float4 *cand, const Slots &s, const SplitSite &a, bool mine, int q0, int q1,
+                                          float r2max, const unsigned *known, SplitList &sh) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    unsigned w[kListWords];
+    if (known) {
+        const uint4 v = *reinterpret_cast<const uint4 *>(known);
+        w[0] = v.x; w[1] = v.y; w[2] = v.z; w[3] = v.w;
+        __syncthreads();  // the previous list is done with
+    } else {
+        __syncthreads();
+        if (threadIdx.x < kListWords) sh.words[threadIdx.x] = 0u;
+        __syncthreads();
+        const f2 uixy = f2_pack(a.ui.x, a.ui.y);
+#pragma unroll 4
+        for (int q = q0 + warp; q < q1; q += W) {
+            const float4 D = __ldg(cand + q);
+            const float4 uj = __ldg(s.u4 + a.si + (a.sl >= 0 ? __float_as_int(D.w) : 0));
+            f2 dxy; float dz;
+            const float r2 = pair_r2(uixy, a.ui.z, D, uj, dxy, dz);
+            if (__any_sync(0xffffffffu, mine && r2 < r2max) && lane == 0)
+                atomicOr(&sh.words[(q - q0) >> 5], 1u << ((q - q0) & 31));
+        }
+        __syncthreads();
+#pragma unroll
+        for (int k = 0; k < kListWords; k++) w[k] = sh.words[k];
+    }
+    int n = 0;
+#pragma unroll
+    for (int k = 0; k < kListWords; k++) {
+        if (k % W == warp && (w[k] >> lane) & 1u) {
+            const int r = n + __popc(w[k] & ((1u << lane) - 1u));
+            sh.rec[r] = __ldg(cand + q0 + 32 * k + lane);
+            sh.num[r] = (unsigned char) (32 * k + lane);
+        }
+        n += __popc(w[k]);
+    }
+    __syncthreads();
+    return n;
+}
+// a term outside the cutoff: a NaN that no arithmetic gives
+constexpr unsigned kSplitNone = 0x7fffdeadu;
+__device__ __forceinline__ bool split_none(float v) { return __float_as_uint(v) == kSplitNone; }
+// The mixed form's view: lane l of a warp takes stream l / P of site P * warp + l % P (P = 32 / W).
+template <int W>
+struct SplitLane {
+    static constexpr int P = 32 / W;
+    int si, ti, stream;
+    bool in, mine;
+    f2 uixy;
+    float uiz;
+    __device__ __forceinline__ SplitLane(const SplitSite &a) {
+        const int lane = threadIdx.x & 31, from = P * (threadIdx.x >> 5) + lane % P;
+        stream = lane / P;
+        si = __shfl_sync(0xffffffffu, a.si, from);
+        ti = max(__shfl_sync(0xffffffffu, a.ti, from), 0);
+        in = __shfl_sync(0xffffffffu, a.sl, from) >= 0;
+        uixy = f2_pack(__shfl_sync(0xffffffffu, a.ui.x, from), __shfl_sync(0xffffffffu, a.ui.y, from));
+        uiz = __shfl_sync(0xffffffffu, a.ui.z, from);
+        mine = true;
+    }
+};
+
+// Density, mixed form (500 groups: 26 -> 12 us).
+template <int W>
+__device__ __forceinline__ void rho_mixed_split(const float4 *cand, int np, int nf, const Geom &g, const Slots &s, const Inter &in,
+                                                const PotTables &pt, const SplitSite &a, bool hook, bool lists, bool full, bool far,
+                                                SplitList &sh, float2 *out) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int end = __any_sync(0xffffffffu, far) ? nf : np;
+    SplitLane<W> b(a);
+    constexpr int P = SplitLane<W>::P;
+    const bool b_far = __shfl_sync(0xffffffffu, far, P * warp + lane % P);
+    float sum = 0.f, comp = 0.f;
+    int q1;
+    for (int q0 = 0; q0 < end; q0 = q1) {
+        const bool tail = q0 >= np;
+        q1 = min(q0 + kSplitSegment, tail ? end : np);
+        unsigned *list = lists && !tail ? group_list(g, s, a.par, a.u) : nullptr;
+        const int n = split_list<W>(cand, s, a, !tail || far, q0, q1, list ? g.rcs2_h : g.rc2_h, full ? nullptr : list, sh);
+        if (full && list && threadIdx.x < kListWords) list[threadIdx.x] = sh.words[threadIdx.x];
+        const bool mine = !tail || b_far;
+#pragma unroll 2
+        for (int c0 = 0; c0 < n; c0 += W) {
+            const float4 D = sh.rec[min(c0 + b.stream, n - 1)];
+            const float4 uj = __ldg(s.u4 + b.si + (b.in ? __float_as_int(D.w) : 0));
+            f2 dxy; float dz;
+            const float r2 = pair_r2(b.uixy, b.uiz, D, uj, dxy, dz);
+            // outside the cutoff the knot stays on the table, and its value is not used
+            const float v = rho_term_mixed(pt, r2, max(__float_as_int(uj.w), 0));
+            const float t = c0 + b.stream < n && mine && r2 < g.rc2_h ? v : __uint_as_float(kSplitNone);
+#pragma unroll
+            for (int k = 0; k < W; k++) {
+                const float tk = __shfl_sync(0xffffffffu, t, P * k + lane % P);
+                if (!split_none(tk)) kahan(sum, comp, tk);
+            }
+        }
+    }
+    if (b.stream == 0) out[P * warp + lane % P] = make_float2(sum, comp);
+    __syncthreads();
+    if (warp != 0 || a.sl < 0) return;
+    if (a.ti < 0) { s.rho[a.sl] = 0.0; return; }
+    rho_done_mixed(s, in, pt, a.sl, a.si, a.ti, out[lane].x, out[lane].y, hook);
+}
+template <int W>
+__global__ void __launch_bounds__(32 * W) k_lat_rho_mixed_split(const float4 *cand, int np, int nf, Geom g, Slots s, Inter in, PotTables pt,
+                                                                bool hook, int u0, int u1, bool lists) {
+    __shared__ SplitList sh;
+    __shared__ float2 out[32];
+    bool full = lists && skin_full(g, s);
+    if (full && blockIdx.x == 0 && threadIdx.x == 0) s.skin->rebuilt = 1;
+    const SplitSite a = split_site(g, s, u0, u1);
+    if (!__any_sync(0xffffffffu, a.ti >= 0)) {  // the same in every warp of the block
+        if (threadIdx.x < 32 && a.sl >= 0) s.rho[a.sl] = 0.0;
+        return;
+    }
+    // as in the whole-group pass: a marked site makes its group rebuild its list
+    const bool marked = a.sl >= 0 && in.far_flag[a.sl];
+    full = full || __any_sync(0xffffffffu, marked);
+    rho_mixed_split<W>(cand + a.par * kMaxFull, np, nf, g, s, in, pt, a, hook, lists, full, marked && a.ti >= 0, sh, out);
+}
 
 // ------------------------------------------------------------------------------------------------
 // FP64 form in fixed point (mg_fixed.h): the pair sums in 64-bit integers. Bound by integer issue and by the
@@ -1121,6 +1290,13 @@ __device__ __forceinline__ void fix_note_near(unsigned &near, int q) {
     near = near >> 24 ? 0xffffffffu : (near << 8) | (unsigned) (q + 1);
 }
 constexpr unsigned kFixNearMany = 0xffffffffu;  // more than fit (a candidate number is below 255)
+// the near candidates of a later part of the list joined to those of an earlier one
+__device__ __forceinline__ void fix_join_near(unsigned &near, unsigned more) {
+    if (more == kFixNearMany) near = kFixNearMany;
+    else
+        for (int sh = 24; sh >= 0; sh -= 8)
+            if ((more >> sh) & 255u) fix_note_near(near, (int) ((more >> sh) & 255u) - 1);
+}
 
 // an atom's density over its near pairs, or (many) over all pairs, in FP64
 __device__ __noinline__ double rho_near_fp64(const NeighTables &nt, const Geom &g, const Slots &s, const Inter &in,
@@ -1135,11 +1311,10 @@ __device__ __noinline__ double rho_near_fp64(const NeighTables &nt, const Geom &
     return acc;
 }
 
-// candidate q of the atom at (xb, yb, zb) (biased)
-template <int PAR>
-__device__ __forceinline__ void rho_fix_candidate(const NeighTables &nt, const Slots &s, const FixParams &fp, int si, i64 xb, i64 yb,
+// candidate q, at index oj, of the atom at (xb, yb, zb) (biased)
+__device__ __forceinline__ void rho_fix_candidate(const Slots &s, const FixParams &fp, int oj, i64 xb, i64 yb,
                                                   i64 zb, int q, i64 &acc, unsigned &near) {
-    const FixRec j = ld_fix_rec(s.fix + si + __float_as_int(nt.cand[PAR][q].w));
+    const FixRec j = ld_fix_rec(s.fix + oj);
     const i64 r2 = fix_r2(fix_delta(xb - j.x, yb - j.y, zb - j.z), fp.b0);
     if ((unsigned long long) (r2 - fp.lo) < (unsigned long long) (fp.rc2 - fp.lo)) {
         int m;
@@ -1149,6 +1324,8 @@ __device__ __forceinline__ void rho_fix_candidate(const NeighTables &nt, const S
         fix_note_near(near, q);
     }
 }
+// within this the FP64 form's lists hold a pair: rc + skin, and (skin 0) whatever the single-precision test lets by
+__device__ __forceinline__ float fix_list_r2(const Geom &g) { return fmaxf(g.rcs2_h, g.rc2_pre); }
 // the candidates [q0, q1) after the single-precision test; NOTED: bit j of the result marks candidate
 // q0 + j within rc + skin (q1 - q0 <= 32)
 template <int PAR, bool NOTED>
@@ -1161,15 +1338,18 @@ __device__ __forceinline__ unsigned rho_fix_range(const NeighTables &nt, const G
         const float4 D = nt.cand[PAR][q];
         f2 dxy; float dz;
         const float r2 = pair_r2(uixy, ui.z, D, __ldg(s.u4 + si + __float_as_int(D.w)), dxy, dz);
-        if (NOTED && r2 < g.rcs2_h) nb |= 1u << (q - q0);
-        if (r2 < g.rc2_pre) rho_fix_candidate<PAR>(nt, s, fp, si, xb, yb, zb, q, acc, near);
+        if (NOTED && r2 < fix_list_r2(g)) nb |= 1u << (q - q0);
+        if (r2 < g.rc2_pre) rho_fix_candidate(s, fp, si + __float_as_int(D.w), xb, yb, zb, q, acc, near);
     }
     return nb;
 }
 template <int PAR>
 __device__ __forceinline__ void rho_fix_listed(const NeighTables &nt, const Slots &s, const FixParams &fp, int si, i64 xb, i64 yb,
                                                i64 zb, int q0, unsigned word, i64 &acc, unsigned &near) {
-    for (unsigned w = word; w; w &= w - 1) rho_fix_candidate<PAR>(nt, s, fp, si, xb, yb, zb, q0 + __ffs(w) - 1, acc, near);
+    for (unsigned w = word; w; w &= w - 1) {
+        const int q = q0 + __ffs(w) - 1;
+        rho_fix_candidate(s, fp, si + __float_as_int(nt.cand[PAR][q].w), xb, yb, zb, q, acc, near);
+    }
 }
 
 // the pair sum over the candidates the tables bound (the pruned ones), and over the tail of a far atom's
@@ -1203,6 +1383,20 @@ __device__ __forceinline__ double rho_fix_atom(const NeighTables &nt, const Geom
     }
     return rho;
 }
+// adds the near pairs, stores the density and, where nothing adds to it afterwards, F'(rho)
+__device__ __forceinline__ void rho_done_fix(const NeighTables &nt, const Geom &g, const Slots &s, const Inter &in, const PotTables &pt,
+                                             const FixParams &fp, int sl, int si, int ti, int par, double rho, unsigned near,
+                                             bool hook) {
+    if (near) rho = rho_near_fp64(nt, g, s, in, pt, sl, par, near) + (near == kFixNearMany ? 0.0 : rho);
+    s.rho[sl] = rho;
+    if (!hook && lattice_only(in)) {
+        int m; double p;
+        locate_d(rho, pt.inv_drho, pt.nrho, m, p);
+        const double df = der_d(pt.F_d + ti * pt.nrho, m, p);
+        s.df[sl] = df;
+        s.dfq[si] = fix_df(fp, df);
+    }
+}
 __device__ __forceinline__ void k_lat_rho_fix_site(int t, bool valid, const NeighTables &nt, const Geom &g, const Slots &s,
                                                    const Inter &in, const PotTables &pt, const FixParams &fp, bool hook, int order,
                                                    bool lists, bool full, bool wild) {
@@ -1225,15 +1419,7 @@ __device__ __forceinline__ void k_lat_rho_fix_site(int t, bool valid, const Neig
         rho = par ? rho_fix_atom<1>(nt, g, s, fp, si, ui, me, lists, full, list, live, far, near)
                   : rho_fix_atom<0>(nt, g, s, fp, si, ui, me, lists, full, list, live, far, near);
     }
-    if (near) rho = rho_near_fp64(nt, g, s, in, pt, sl, par, near) + (near == kFixNearMany ? 0.0 : rho);
-    s.rho[sl] = rho;
-    if (!hook && lattice_only(in)) {
-        int m; double p;
-        locate_d(rho, pt.inv_drho, pt.nrho, m, p);
-        const double df = der_d(pt.F_d + ti * pt.nrho, m, p);
-        s.df[sl] = df;
-        s.dfq[si] = fix_df(fp, df);
-    }
+    rho_done_fix(nt, g, s, in, pt, fp, sl, si, ti, par, rho, near, hook);
 }
 template <bool LOOP>  // LOOP: several sites per thread, one grid stride apart (no group lists)
 __global__ void __launch_bounds__(512, 2) k_lat_rho_fix(const __grid_constant__ NeighTables nt, const __grid_constant__ Geom g,
@@ -1255,6 +1441,75 @@ __global__ void __launch_bounds__(512, 2) k_lat_rho_fix(const __grid_constant__ 
     k_lat_rho_fix_site(t0, t0 < nthreads, nt, g, s, in, pt, fp, hook, order, lists && !wild, full, wild);
 }
 
+// The density pass of small boxes (see rho_mixed_split): each warp's integer sum and near pairs over a contiguous
+// share of the candidates (the near pairs keep their order), put together by the first warp (500 groups: 47 -> 19 us).
+template <int W>
+__device__ __forceinline__ void rho_fix_split(const NeighTables &nt, const float4 *cand, const Geom &g, const Slots &s, const Inter &in,
+                                              const PotTables &pt, const FixParams &fp, const SplitSite &a, bool hook, bool lists,
+                                              bool full, bool far, bool wild, SplitList &sh, i64 (*part)[32],
+                                              unsigned (*part_near)[32]) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int np = nt.npruned, end = wild ? 0 : __any_sync(0xffffffffu, far) ? nt.nfull : np;
+    double rho = 0.0;
+    unsigned near = wild ? kFixNearMany : 0u;
+    const FixRec me = a.ti >= 0 ? ld_fix_rec(s.fix + a.si) : FixRec{};
+    const i64 xb = me.x + kFixBias, yb = me.y + kFixBias, zb = me.z + kFixBias;
+    int q1;
+    for (int q0 = 0; q0 < end; q0 = q1) {
+        const bool tail = q0 >= np;
+        q1 = min(q0 + kSplitSegment, tail ? end : np);
+        const bool mine = a.ti >= 0 && (!tail || far);
+        unsigned *list = lists && !tail ? group_list(g, s, a.par, a.u) : nullptr;
+        const int n = split_list<W>(cand, s, a, mine, q0, q1, list ? fix_list_r2(g) : g.rc2_pre, full ? nullptr : list, sh);
+        if (full && list && threadIdx.x < kListWords) list[threadIdx.x] = sh.words[threadIdx.x];
+        i64 acc = 0;
+        unsigned mn = 0u;
+        if (mine) {
+            const int c1 = n * (warp + 1) / W;
+#pragma unroll 2
+            for (int c = n * warp / W; c < c1; c++)
+                rho_fix_candidate(s, fp, a.si + __float_as_int(sh.rec[c].w), xb, yb, zb, q0 + sh.num[c], acc, mn);
+        }
+        part[warp][lane] = acc;
+        part_near[warp][lane] = mn;
+        __syncthreads();
+        if (warp == 0) {
+            for (int w = 1; w < W; w++) acc += part[w][lane];
+            rho += (double) acc * fp.rho_unit;
+            for (int w = 0; w < W; w++) fix_join_near(near, part_near[w][lane]);
+        }
+    }
+    if (warp != 0 || a.sl < 0) return;
+    if (a.ti < 0) { s.rho[a.sl] = 0.0; return; }
+    rho_done_fix(nt, g, s, in, pt, fp, a.sl, a.si, a.ti, a.par, rho, near, hook);
+}
+template <int W>
+__global__ void __launch_bounds__(32 * W, 32 / W) k_lat_rho_fix_split(const __grid_constant__ NeighTables nt, const float4 *cand,
+                                                                      const __grid_constant__ Geom g, const __grid_constant__ Slots s,
+                                                                      const __grid_constant__ Inter in,
+                                                                      const __grid_constant__ PotTables pt,
+                                                                      const __grid_constant__ FixParams fp, bool hook, int u0, int u1,
+                                                                      bool lists) {
+    __shared__ SplitList sh;
+    __shared__ i64 part[W][32];
+    __shared__ unsigned part_near[W][32];
+    const bool wild = s.skin->wild != 0;
+    bool full = lists && !wild && skin_full(g, s);
+    if (lists && blockIdx.x == 0 && threadIdx.x == 0) {
+        if (wild) s.skin->dirty = 1;  // groups near a recombined atom did not rebuild their lists
+        else if (full) s.skin->rebuilt = 1;
+    }
+    const SplitSite a = split_site(g, s, u0, u1);
+    if (!__any_sync(0xffffffffu, a.ti >= 0)) {
+        if (threadIdx.x < 32 && a.sl >= 0) s.rho[a.sl] = 0.0;
+        return;
+    }
+    const bool marked = a.sl >= 0 && in.far_flag[a.sl];
+    full = full || __any_sync(0xffffffffu, marked);
+    rho_fix_split<W>(nt, cand + a.par * kMaxFull, g, s, in, pt, fp, a, hook, lists && !wild, full, marked && a.ti >= 0, wild, sh, part,
+                     part_near);
+}
+
 // atoms per thread: each thread takes rho_apt sites, one grid stride apart (the stride is a multiple
 // of 64, so warps keep their parity and thread order)
 // The passes can keep and use per-group candidate lists when every warp of both passes covers one
@@ -1264,6 +1519,39 @@ bool lists_ok(const LaunchCtx &lc, const Geom &g) {
     const bool aligned = (g.n_local_half & 31) == 0;
     return lc.nt->npruned <= 32 * kListWords && lc.rho_apt == 1 && lc.force_apt == 1 && (lc.rho_order == 1 || aligned) &&
            (lc.force_order == 1 || aligned);
+}
+// Warps per group of a split pass over n groups, 0: the whole-group pass. More warps cut the pass's latency and cost
+// instructions (the mixed form's shuffles, and each warp's own start), so their number falls as the groups fill the
+// SMs; a batch counts a member's groups once for each member. Measured on 152 SMs, us per step with 8 / 4 / 2 /
+// no split warps:
+//   mixed  500 groups 56 / 57 / 68 / 84;  1098: 80 / 65 / 73 / 86;  2048: 113 / 91 / 81 / 85;  4000: - / 130 / 127 / 100
+//   FP64   500 groups 70 / 77 / 100 / 138;  1098: 98 / 92 / 107 / 138;  2048: 139 / 129 / 126 / 149;
+//          4000: 224 / 205 / 202 / 211;  7812: 387 / 343 / 339 / 328
+static int split_groups(int u0, int u1) { return 2 * ((u1 - u0 + 31) / 32); }
+static int split_warps(const LaunchCtx &lc, bool mixed, int n) {
+    if (!mixed && !lc.fp) return 0;
+    const int64_t busy = static_cast<int64_t>(n) * lc.share / lc.num_sms;
+    if (busy < 4) return 8;
+    if (busy < (mixed ? 10 : 14)) return 4;
+    return busy < (mixed ? 14 : 28) ? 2 : 0;
+}
+template <int W>
+static void launch_rho_split_w(const LaunchCtx &lc, const Geom &g, Slots s, Inter in, PotTables t, bool mixed, bool hook, int u0, int u1,
+                               bool lists) {
+    const int n = split_groups(u0, u1);
+    if (mixed)
+        k_lat_rho_mixed_split<W><<<n, 32 * W, 0, lc.stream>>>(lc.cand, lc.nt->npruned, lc.nt->nfull, g, s, in, t, hook, u0, u1, lists);
+    else k_lat_rho_fix_split<W><<<n, 32 * W, 0, lc.stream>>>(*lc.nt, lc.cand, g, s, in, t, *lc.fp, hook, u0, u1, lists);
+}
+// the split density pass, where it serves
+static bool launch_lat_rho_split(const LaunchCtx &lc, const Geom &g, Slots s, Inter in, PotTables t, bool mixed, bool hook, int u0,
+                                 int u1, bool lists) {
+    switch (split_warps(lc, mixed, split_groups(u0, u1))) {
+        case 8: launch_rho_split_w<8>(lc, g, s, in, t, mixed, hook, u0, u1, lists); return true;
+        case 4: launch_rho_split_w<4>(lc, g, s, in, t, mixed, hook, u0, u1, lists); return true;
+        case 2: launch_rho_split_w<2>(lc, g, s, in, t, mixed, hook, u0, u1, lists); return true;
+        default: return false;
+    }
 }
 static void launch_lat_rho_threads(const LaunchCtx &lc, const Geom &g, Slots s, Inter in, PotTables t, bool mixed, bool hook,
                                    int tb, int te, bool lists = false) {
@@ -1311,7 +1599,8 @@ static bool has_lists(const LaunchCtx &lc, bool mixed) { return mixed || lc.fp; 
 void launch_lat_rho(const LaunchCtx &lc, const Geom &g, Slots s, Inter in, PotTables t, bool mixed, bool hook, bool lists) {
     const bool v = lists && has_lists(lc, mixed) && !hook && lists_ok(lc, g);
     if (!mixed) launch_fix_records(lc, g, s);
-    launch_lat_rho_threads(lc, g, s, in, t, mixed, hook, 0, gather_threads(g, lc.rho_order), v);
+    if (!launch_lat_rho_split(lc, g, s, in, t, mixed, hook, 0, g.n_local_half, v))
+        launch_lat_rho_threads(lc, g, s, in, t, mixed, hook, 0, gather_threads(g, lc.rho_order), v);
     if (v) launch_skin_advance(lc, s);
     else if (has_lists(lc, mixed)) launch_skin_dirty(lc, s);
 }
@@ -1333,7 +1622,8 @@ void launch_lat_rho_sites(const LaunchCtx &lc, const Geom &g, Slots s, Inter in,
     int tb[2], te[2], nr;
     site_threads(g, lc.rho_order, u0, u1, tb, te, nr);
     const bool v = lists && has_lists(lc, mixed) && lists_ok(lc, g);
-    for (int r = 0; r < nr; r++) launch_lat_rho_threads(lc, g, s, in, t, mixed, false, tb[r], te[r], v);
+    if (!launch_lat_rho_split(lc, g, s, in, t, mixed, false, u0, u1, v))
+        for (int r = 0; r < nr; r++) launch_lat_rho_threads(lc, g, s, in, t, mixed, false, tb[r], te[r], v);
     if (!v && has_lists(lc, mixed)) launch_skin_dirty(lc, s);  // the caller advances the skin after the last slab
 }
 
@@ -1489,10 +1779,9 @@ __device__ __noinline__ double3 force_near_fp64(const NeighTables &nt, const Geo
     }
     return make_double3(fx, fy, fz);
 }
-template <int PAR>
-__device__ __forceinline__ void force_fix_candidate(const NeighTables &nt, const Slots &s, const FixParams &fp, int si, int ti, i64 xb,
+// candidate q, at index oj
+__device__ __forceinline__ void force_fix_candidate(const Slots &s, const FixParams &fp, int oj, int ti, i64 xb,
                                                     i64 yb, i64 zb, i64 dfb, int q, FixForce &a) {
-    const int oj = si + __float_as_int(nt.cand[PAR][q].w);
     const FixRec j = ld_fix_rec(s.fix + oj);
     const FixDelta d = fix_delta(xb - j.x, yb - j.y, zb - j.z);
     const i64 r2 = fix_r2(d, fp.b0);
@@ -1530,7 +1819,7 @@ __device__ __forceinline__ void force_fix_range(const NeighTables &nt, const Geo
     for (int q = q0; q < q1; q++) {
         const float4 D = nt.cand[PAR][q];
         if (near_f32(g, uixy, ui.z, D, __ldg(s.u4 + si + __float_as_int(D.w))))
-            force_fix_candidate<PAR>(nt, s, fp, si, ti, xb, yb, zb, dfb, q, a);
+            force_fix_candidate(s, fp, si + __float_as_int(D.w), ti, xb, yb, zb, dfb, q, a);
     }
 }
 template <int PAR>
@@ -1540,8 +1829,10 @@ __device__ __forceinline__ void force_fix_atom(const NeighTables &nt, const Geom
     const int np = nt.npruned;
     if (list) {
         for (int k = 0; k * 32 < np; k++)
-            for (unsigned w = list[k]; w; w &= w - 1)
-                force_fix_candidate<PAR>(nt, s, fp, si, ti, xb, yb, zb, dfb, 32 * k + __ffs(w) - 1, a);
+            for (unsigned w = list[k]; w; w &= w - 1) {
+                const int q = 32 * k + __ffs(w) - 1;
+                force_fix_candidate(s, fp, si + __float_as_int(nt.cand[PAR][q].w), ti, xb, yb, zb, dfb, q, a);
+            }
     } else {
         force_fix_range<PAR>(nt, g, s, fp, si, ti, s.u4[si], xb, yb, zb, dfb, 0, np, a);
     }
@@ -1553,6 +1844,18 @@ __device__ __forceinline__ void force_fix_atom(const NeighTables &nt, const Geom
         f.y -= (double) a.y * fp.f_unit;
         f.z -= (double) a.z * fp.f_unit;
     }
+}
+// adds the near pairs, stores the force and takes the second half-kick where the lattice pass may
+__device__ __forceinline__ void force_done_fix(const NeighTables &nt, const Geom &g, const Slots &s, const Inter &in,
+                                               const PotTables &pt, StepParams *sp, int sl, int ti, int par, const FixForce &a,
+                                               double3 f, bool kick, bool hook) {
+    const unsigned near = a.df_hi >= kFixBadHi ? kFixNearMany : a.near;
+    if (near) {
+        const double3 n = force_near_fp64(nt, g, s, in, pt, sl, ti, par, near);
+        if (near == kFixNearMany) f = n;
+        else { f.x += n.x; f.y += n.y; f.z += n.z; }
+    }
+    force_done_fp64(s, in, sp, sl, ti, f.x, f.y, f.z, kick, hook);
 }
 __device__ __forceinline__ void k_lat_force_fix_site(int t, const NeighTables &nt, const Geom &g, const Slots &s, const Inter &in,
                                                      const PotTables &pt, const FixParams &fp, StepParams *sp, bool kick, bool hook,
@@ -1572,14 +1875,8 @@ __device__ __forceinline__ void k_lat_force_fix_site(int t, const NeighTables &n
         const bool far = in.far_flag[sl];
         if (par) force_fix_atom<1>(nt, g, s, fp, si, ti, me, list, far, a, f);
         else force_fix_atom<0>(nt, g, s, fp, si, ti, me, list, far, a, f);
-        if (a.df_hi >= kFixBadHi) a.near = kFixNearMany;
     }
-    if (a.near) {
-        const double3 n = force_near_fp64(nt, g, s, in, pt, sl, ti, par, a.near);
-        if (a.near == kFixNearMany) f = n;
-        else { f.x += n.x; f.y += n.y; f.z += n.z; }
-    }
-    force_done_fp64(s, in, sp, sl, ti, f.x, f.y, f.z, kick, hook);
+    force_done_fix(nt, g, s, in, pt, sp, sl, ti, par, a, f, kick, hook);
 }
 template <bool LOOP>  // LOOP: several sites per thread, one grid stride apart (no group lists)
 __global__ void __launch_bounds__(512, 2) k_lat_force_fix(const __grid_constant__ NeighTables nt, const __grid_constant__ Geom g,
@@ -1677,41 +1974,10 @@ __device__ __forceinline__ int local_index_of(const Geom &g, int sl, int &i, int
     return (k * g.by + j) * g.bx + i;
 }
 
-__device__ __forceinline__ void k_lat_force_mixed_site(int t, const NeighTables &nt, const Geom &g, const Slots &s, const Inter &in,
-                                                const PotTables &pt, StepParams *sp, bool kick, bool hook, int order,
-                                                bool fuse_next, bool lists) {
-    int par, u;
-    const int sl = gather_site(g, t, order, par, u);
-    if (sl < 0) return;
-    const int si = sidx(g, sl);
-    const float4 ui = s.u4[si];
-    const int ti = __float_as_int(ui.w);
-    if (ti < 0) {
-        s.fx[sl] = 0.0; s.fy[sl] = 0.0; s.fz[sl] = 0.0;
-        if (fuse_next && lattice_only(in)) {  // the next firststep's flag and record of a vacancy
-            int i, j, k;
-            in.dflag[local_index_of(g, sl, i, j, k)] = 0;
-            s.u4n[si] = vacant_u4();
-        }
-        return;
-    }
-    const float dfi = s.df32[si];
-    // compensated force sums (x and y packed, z)
-    ForceAcc acc{f2_pack(0.f, 0.f), f2_pack(0.f, 0.f), 0.f, 0.f};
-    const int np = nt.npruned;
-    if (lists) {
-        const unsigned *w = group_list(g, s, par, u);
-        if (par) force_sum_listed<1>(nt, g, s, pt, si, ti, ui, dfi, w, acc);
-        else force_sum_listed<0>(nt, g, s, pt, si, ti, ui, dfi, w, acc);
-    } else {
-        if (par) force_sum_mixed<1>(nt, g, s, pt, si, ti, ui, dfi, 0, np, acc);
-        else force_sum_mixed<0>(nt, g, s, pt, si, ti, ui, dfi, 0, np, acc);
-    }
-    if (in.far_flag[sl]) {
-        const int nf = nt.nfull;
-        if (par) force_sum_mixed<1>(nt, g, s, pt, si, ti, ui, dfi, np, nf, acc);
-        else force_sum_mixed<0>(nt, g, s, pt, si, ti, ui, dfi, np, nf, acc);
-    }
+// stores the force and takes the second half-kick where the lattice pass may; in a fused body also the next
+// body's firststep
+__device__ __forceinline__ void force_done_mixed(const Geom &g, const Slots &s, const Inter &in, StepParams *sp, int sl, int si, int ti,
+                                                 const ForceAcc &acc, bool kick, bool hook, bool fuse_next) {
     // each sum with its compensation, converted to FP64 once
     float sx, sy, mx, my;
     f2_unpack(acc.sxy, sx, sy);
@@ -1741,6 +2007,44 @@ __device__ __forceinline__ void k_lat_force_mixed_site(int t, const NeighTables 
         }
     }
 }
+// a vacant site: no force, and in a fused body the next firststep's flag and record of a vacancy
+__device__ __forceinline__ void force_vacant_mixed(const Geom &g, const Slots &s, const Inter &in, int sl, int si, bool fuse_next) {
+    s.fx[sl] = 0.0; s.fy[sl] = 0.0; s.fz[sl] = 0.0;
+    if (fuse_next && lattice_only(in)) {
+        int i, j, k;
+        in.dflag[local_index_of(g, sl, i, j, k)] = 0;
+        s.u4n[si] = vacant_u4();
+    }
+}
+__device__ __forceinline__ void k_lat_force_mixed_site(int t, const NeighTables &nt, const Geom &g, const Slots &s, const Inter &in,
+                                                const PotTables &pt, StepParams *sp, bool kick, bool hook, int order,
+                                                bool fuse_next, bool lists) {
+    int par, u;
+    const int sl = gather_site(g, t, order, par, u);
+    if (sl < 0) return;
+    const int si = sidx(g, sl);
+    const float4 ui = s.u4[si];
+    const int ti = __float_as_int(ui.w);
+    if (ti < 0) { force_vacant_mixed(g, s, in, sl, si, fuse_next); return; }
+    const float dfi = s.df32[si];
+    // compensated force sums (x and y packed, z)
+    ForceAcc acc{f2_pack(0.f, 0.f), f2_pack(0.f, 0.f), 0.f, 0.f};
+    const int np = nt.npruned;
+    if (lists) {
+        const unsigned *w = group_list(g, s, par, u);
+        if (par) force_sum_listed<1>(nt, g, s, pt, si, ti, ui, dfi, w, acc);
+        else force_sum_listed<0>(nt, g, s, pt, si, ti, ui, dfi, w, acc);
+    } else {
+        if (par) force_sum_mixed<1>(nt, g, s, pt, si, ti, ui, dfi, 0, np, acc);
+        else force_sum_mixed<0>(nt, g, s, pt, si, ti, ui, dfi, 0, np, acc);
+    }
+    if (in.far_flag[sl]) {
+        const int nf = nt.nfull;
+        if (par) force_sum_mixed<1>(nt, g, s, pt, si, ti, ui, dfi, np, nf, acc);
+        else force_sum_mixed<0>(nt, g, s, pt, si, ti, ui, dfi, np, nf, acc);
+    }
+    force_done_mixed(g, s, in, sp, sl, si, ti, acc, kick, hook, fuse_next);
+}
 template <bool LOOP>  // LOOP: several sites per thread, one grid stride apart
 __global__ void __launch_bounds__(512, 3) k_lat_force_mixed(const __grid_constant__ NeighTables nt, Geom g, Slots s, Inter in, PotTables pt,
                                                          StepParams *sp, bool kick, bool hook, int order, int tbase,
@@ -1752,6 +2056,141 @@ __global__ void __launch_bounds__(512, 3) k_lat_force_mixed(const __grid_constan
     }
     for (int t = t0; t < nthreads; t += gridDim.x * blockDim.x)
         k_lat_force_mixed_site(t, nt, g, s, in, pt, sp, kick, hook, order, fuse_next, false);
+}
+
+// ---- the force passes of small boxes and thin slabs: see rho_mixed_split (500 groups: 30 -> 16 us; FP64 form 58 ->
+// 19 us) ----
+template <int W>
+__device__ __forceinline__ void force_mixed_split(const float4 *cand, int np, int nf, const Geom &g, const Slots &s, const Inter &in,
+                                                  const PotTables &pt, StepParams *sp, const SplitSite &a, bool kick, bool hook,
+                                                  bool fuse_next, bool lists, bool far, SplitList &sh, ForceAcc *out) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int end = __any_sync(0xffffffffu, far) ? nf : np;
+    SplitLane<W> b(a);
+    constexpr int P = SplitLane<W>::P;
+    const bool b_far = __shfl_sync(0xffffffffu, far, P * warp + lane % P);
+    const float dfi = s.df32[b.si];
+    ForceAcc acc{f2_pack(0.f, 0.f), f2_pack(0.f, 0.f), 0.f, 0.f};
+    int q1;
+    for (int q0 = 0; q0 < end; q0 = q1) {
+        const bool tail = q0 >= np;
+        q1 = min(q0 + kSplitSegment, tail ? end : np);
+        const int n = split_list<W>(cand, s, a, !tail || far, q0, q1, g.rc2_h, lists && !tail ? group_list(g, s, a.par, a.u) : nullptr, sh);
+        const bool mine = !tail || b_far;
+#pragma unroll 1
+        for (int c0 = 0; c0 < n; c0 += W) {
+            const float4 D = sh.rec[min(c0 + b.stream, n - 1)];
+            const int oj = b.si + (b.in ? __float_as_int(D.w) : 0);
+            const float4 uj = __ldg(s.u4 + oj);
+            const float dfj = __ldg(s.df32 + oj);
+            f2 dxy; float dz;
+            const float r2 = pair_r2(b.uixy, b.uiz, D, uj, dxy, dz);
+            const float v = fpair_mixed(g, pt, r2, b.ti, max(__float_as_int(uj.w), 0), dfi, dfj);
+            const float t = c0 + b.stream < n && mine && r2 < g.rc2_h ? v : __uint_as_float(kSplitNone);
+            float dx, dy;
+            f2_unpack(dxy, dx, dy);
+#pragma unroll
+            for (int k = 0; k < W; k++) {
+                const int from = P * k + lane % P;
+                const float tk = __shfl_sync(0xffffffffu, t, from), xk = __shfl_sync(0xffffffffu, dx, from);
+                const float yk = __shfl_sync(0xffffffffu, dy, from), zk = __shfl_sync(0xffffffffu, dz, from);
+                if (!split_none(tk)) force_acc_add(acc, f2_pack(xk, yk), zk, tk);
+            }
+        }
+    }
+    if (b.stream == 0) out[P * warp + lane % P] = acc;
+    __syncthreads();
+    if (warp != 0 || a.sl < 0) return;
+    if (a.ti < 0) { force_vacant_mixed(g, s, in, a.sl, a.si, fuse_next); return; }
+    force_done_mixed(g, s, in, sp, a.sl, a.si, a.ti, out[lane], kick, hook, fuse_next);
+}
+template <int W>
+__global__ void __launch_bounds__(32 * W) k_lat_force_mixed_split(const float4 *cand, int np, int nf, Geom g, Slots s, Inter in,
+                                                                  PotTables pt, StepParams *sp, bool kick, bool hook, int u0, int u1,
+                                                                  bool fuse_next, bool lists) {
+    __shared__ SplitList sh;
+    __shared__ ForceAcc out[32];
+    const SplitSite a = split_site(g, s, u0, u1);
+    if (!__any_sync(0xffffffffu, a.ti >= 0)) {
+        if (threadIdx.x < 32 && a.sl >= 0) force_vacant_mixed(g, s, in, a.sl, a.si, fuse_next);
+        return;
+    }
+    const bool far = a.ti >= 0 && in.far_flag[a.sl];
+    force_mixed_split<W>(cand + a.par * kMaxFull, np, nf, g, s, in, pt, sp, a, kick, hook, fuse_next, lists, far, sh, out);
+}
+// FP64 form
+template <int W>
+struct SplitForce {
+    i64 x[W][32], y[W][32], z[W][32];
+    int df_hi[W][32];
+    unsigned near[W][32];
+};
+template <int W>
+__device__ __forceinline__ void force_fix_split(const NeighTables &nt, const float4 *cand, const Geom &g, const Slots &s,
+                                                const Inter &in, const PotTables &pt, const FixParams &fp, StepParams *sp,
+                                                const SplitSite &a, bool kick, bool hook, bool lists, bool far, bool wild,
+                                                SplitList &sh, SplitForce<W> &part) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int np = nt.npruned, end = wild ? 0 : __any_sync(0xffffffffu, far) ? nt.nfull : np;
+    FixForce tot{0, 0, 0, 0, wild ? kFixNearMany : 0u};
+    double3 f{0.0, 0.0, 0.0};
+    const FixRec me = a.ti >= 0 ? ld_fix_rec(s.fix + a.si) : FixRec{};
+    const i64 xb = me.x + kFixBias, yb = me.y + kFixBias, zb = me.z + kFixBias;
+    const i64 dfb = a.ti >= 0 ? s.dfq[a.si] + kFixBias : 0;
+    int q1;
+    for (int q0 = 0; q0 < end; q0 = q1) {
+        const bool tail = q0 >= np;
+        q1 = min(q0 + kSplitSegment, tail ? end : np);
+        const bool mine = a.ti >= 0 && (!tail || far);
+        const int n = split_list<W>(cand, s, a, mine, q0, q1, g.rc2_pre, lists && !tail ? group_list(g, s, a.par, a.u) : nullptr, sh);
+        FixForce m{0, 0, 0, 0, 0u};
+        if (mine) {
+            const int c1 = n * (warp + 1) / W;
+            for (int c = n * warp / W; c < c1; c++)
+                force_fix_candidate(s, fp, a.si + __float_as_int(sh.rec[c].w), a.ti, xb, yb, zb, dfb, q0 + sh.num[c], m);
+        }
+        part.x[warp][lane] = m.x;
+        part.y[warp][lane] = m.y;
+        part.z[warp][lane] = m.z;
+        part.df_hi[warp][lane] = m.df_hi;
+        part.near[warp][lane] = m.near;
+        __syncthreads();
+        if (warp == 0) {
+            for (int w = 1; w < W; w++) {
+                m.x += part.x[w][lane];
+                m.y += part.y[w][lane];
+                m.z += part.z[w][lane];
+            }
+            for (int w = 0; w < W; w++) {
+                tot.df_hi = max(tot.df_hi, part.df_hi[w][lane]);
+                fix_join_near(tot.near, part.near[w][lane]);
+            }
+            f.x -= (double) m.x * fp.f_unit;
+            f.y -= (double) m.y * fp.f_unit;
+            f.z -= (double) m.z * fp.f_unit;
+        }
+    }
+    if (warp != 0 || a.sl < 0) return;
+    if (a.ti < 0) { s.fx[a.sl] = 0.0; s.fy[a.sl] = 0.0; s.fz[a.sl] = 0.0; return; }
+    force_done_fix(nt, g, s, in, pt, sp, a.sl, a.ti, a.par, tot, f, kick, hook);
+}
+template <int W>
+__global__ void __launch_bounds__(32 * W, 32 / W) k_lat_force_fix_split(const __grid_constant__ NeighTables nt, const float4 *cand,
+                                                                        const __grid_constant__ Geom g, const __grid_constant__ Slots s,
+                                                                        const __grid_constant__ Inter in,
+                                                                        const __grid_constant__ PotTables pt,
+                                                                        const __grid_constant__ FixParams fp, StepParams *sp, bool kick,
+                                                                        bool hook, int u0, int u1, bool lists) {
+    __shared__ SplitList sh;
+    __shared__ SplitForce<W> part;
+    const bool wild = s.skin->wild != 0;
+    const SplitSite a = split_site(g, s, u0, u1);
+    if (!__any_sync(0xffffffffu, a.ti >= 0)) {
+        if (threadIdx.x < 32 && a.sl >= 0) { s.fx[a.sl] = 0.0; s.fy[a.sl] = 0.0; s.fz[a.sl] = 0.0; }
+        return;
+    }
+    const bool far = a.ti >= 0 && in.far_flag[a.sl];
+    force_fix_split<W>(nt, cand + a.par * kMaxFull, g, s, in, pt, fp, sp, a, kick, hook, lists && !wild, far, wild, sh, part);
 }
 
 static void launch_lat_force_threads(const LaunchCtx &lc, const Geom &g, Slots s, Inter in, PotTables t, StepParams *p,
@@ -1771,11 +2210,30 @@ static void launch_lat_force_threads(const LaunchCtx &lc, const Geom &g, Slots s
         else k_lat_force_fp64<false><<<n, b, 0, lc.stream>>>(*lc.nt, g, s, in, t, p, kick, hook, order, tb, te);
     }
 }
+template <int W>
+static void launch_force_split_w(const LaunchCtx &lc, const Geom &g, Slots s, Inter in, PotTables t, StepParams *p, bool kick, bool mixed,
+                                 bool hook, int u0, int u1, bool fuse_next, bool lists) {
+    const int n = split_groups(u0, u1);
+    if (mixed)
+        k_lat_force_mixed_split<W><<<n, 32 * W, 0, lc.stream>>>(lc.cand, lc.nt->npruned, lc.nt->nfull, g, s, in, t, p, kick, hook, u0, u1,
+                                                                fuse_next && kick && !hook, lists);
+    else k_lat_force_fix_split<W><<<n, 32 * W, 0, lc.stream>>>(*lc.nt, lc.cand, g, s, in, t, *lc.fp, p, kick, hook, u0, u1, lists);
+}
+static bool launch_lat_force_split(const LaunchCtx &lc, const Geom &g, Slots s, Inter in, PotTables t, StepParams *p, bool kick, bool mixed,
+                                   bool hook, int u0, int u1, bool fuse_next, bool lists) {
+    switch (split_warps(lc, mixed, split_groups(u0, u1))) {
+        case 8: launch_force_split_w<8>(lc, g, s, in, t, p, kick, mixed, hook, u0, u1, fuse_next, lists); return true;
+        case 4: launch_force_split_w<4>(lc, g, s, in, t, p, kick, mixed, hook, u0, u1, fuse_next, lists); return true;
+        case 2: launch_force_split_w<2>(lc, g, s, in, t, p, kick, mixed, hook, u0, u1, fuse_next, lists); return true;
+        default: return false;
+    }
+}
 void launch_lat_force(const LaunchCtx &lc, const Geom &g, Slots s, Inter in, PotTables t, StepParams *p, bool kick,
                       bool mixed, bool hook, bool fuse_next, bool lists) {
     if (hook && !mixed) launch_fix_records(lc, g, s);
-    launch_lat_force_threads(lc, g, s, in, t, p, kick, mixed, hook, 0, gather_threads(g, lc.force_order), fuse_next,
-                             lists && has_lists(lc, mixed) && !hook && lists_ok(lc, g));
+    const bool v = lists && has_lists(lc, mixed) && !hook && lists_ok(lc, g);
+    if (launch_lat_force_split(lc, g, s, in, t, p, kick, mixed, hook, 0, g.n_local_half, fuse_next, v)) return;
+    launch_lat_force_threads(lc, g, s, in, t, p, kick, mixed, hook, 0, gather_threads(g, lc.force_order), fuse_next, v);
 }
 void launch_lat_force_sites(const LaunchCtx &lc, const Geom &g, Slots s, Inter in, PotTables t, StepParams *p, bool kick,
                             bool mixed, int u0, int u1, bool lists) {
@@ -1783,6 +2241,7 @@ void launch_lat_force_sites(const LaunchCtx &lc, const Geom &g, Slots s, Inter i
     int tb[2], te[2], nr;
     site_threads(g, lc.force_order, u0, u1, tb, te, nr);
     const bool v = lists && has_lists(lc, mixed) && lists_ok(lc, g);
+    if (launch_lat_force_split(lc, g, s, in, t, p, kick, mixed, false, u0, u1, false, v)) return;
     for (int r = 0; r < nr; r++) launch_lat_force_threads(lc, g, s, in, t, p, kick, mixed, false, tb[r], te[r], false, v);
 }
 
