@@ -20,12 +20,15 @@ namespace {
 
 thread_local std::string g_create_error;
 
-constexpr int kNumTimers = 12;  // events per timed step; the kernels between consecutive events are:
-const char *kTimerNames[kNumTimers - 1] = {"firststep",  // step head and firststep
-                                           "inter_firststep",
-                                           "inter_manage",  // displaced collection, far marks and the list manager
-                                           "ghost_copy", "lat_rho", "inter_rho", "lat_df", "ghost_df", "lat_force",
-                                           "inter_force", "secondstep"};
+constexpr int kNumTimers = 10;  // events per timed step; the kernels between consecutive events are:
+const char *kTimerNames[kNumTimers - 1] = {"firststep",     // step head and firststep
+                                           "inter_manage",  // the list manager
+                                           "ghost_copy",    // and the far atoms' marks
+                                           "inter_rho",     // the FP64 form's records and the inter atoms' densities
+                                           "lat_rho",
+                                           "inter_owner",   // the density shares of lattice atoms near inter atoms
+                                           "ghost_df", "lat_force",
+                                           "inter_force"};  // and the second half-kicks near inter atoms
 
 }  // namespace
 
@@ -52,7 +55,7 @@ struct mg_context {
     OffsetTable offs;
     std::vector<int> lat_order[2];  // reordered full table (pruned entries first), linear offsets
     NeighTables nt{};               // the tables as the kernels receive them
-    float4 *d_cand = nullptr;       // nt.cand in device memory
+    NeighTables *d_nt = nullptr;    // the same in device memory
     int n_full = 0, n_pruned = 0;
     cudaStream_t stream = nullptr;
     int num_sms = 1;
@@ -107,7 +110,7 @@ struct mg_context {
         LaunchCtx l{stream, num_sms};
         l.share = share;
         l.nt = &nt;
-        l.cand = d_cand;
+        l.ntd = d_nt;
         l.fp = !mixed() && fp.on && s.fix ? &fp : nullptr;
         l.rho_order = tune[precision][0][0];
         l.rho_block = tune[precision][0][1];
@@ -192,52 +195,44 @@ void seq_firststep(mg_context *ctx, bool decide, Timer *t, bool fused = false) {
     const LaunchCtx lc = ctx->lc();
     launch_firststep(lc, ctx->g, ctx->s, ctx->in, ctx->d_sp, decide, 0, -1, fused, ctx->alt_bodies);
     if (t) t->mark(1);
-    launch_inter_firststep(lc, ctx->in, ctx->d_sp);
-    if (t) t->mark(2);
 }
 // computeEam's list work (decide, exchangeInter, borderInter, makeIndex) and the lattice ghost copy
 void seq_eam_lists(mg_context *ctx, bool with_manage_prefix, int manage_mask, Timer *t) {
     const LaunchCtx lc = ctx->lc();
     const bool mx = ctx->mixed();
     const bool decide = with_manage_prefix && (manage_mask & MANAGE_DECIDE);
-    if (decide) {
-        launch_displaced_collect(lc, ctx->g, ctx->in);  // the displaced slots of firststep, in scan order
-        launch_far_clear(lc, ctx->g, ctx->in);           // the previous far list's neighbourhood marks
-    }
     if (with_manage_prefix) launch_inter_manage(lc, ctx->g, ctx->s, ctx->in, manage_mask | MANAGE_INDEX, mx);
     else launch_inter_manage(lc, ctx->g, ctx->s, ctx->in, MANAGE_INDEX, mx);
-    if (decide) launch_far_mark(lc, ctx->g, ctx->in);   // the new far list's neighbourhoods
+    if (t) t->mark(2);
+    launch_ghost_copy(lc, ctx->g, ctx->s, ctx->in, decide);  // and the new far list's neighbourhood marks
     if (t) t->mark(3);
-    launch_ghost_copy(lc, ctx->g, ctx->s, mx);
-    if (t) t->mark(4);
 }
 // rho, dF/drho and the forward df exchange; the density pass checks or rebuilds the group lists that
 // the force pass on the same positions walks
 void seq_eam_rho(mg_context *ctx, Timer *t) {
     const LaunchCtx lc = ctx->lc();
     const bool mx = ctx->mixed();
-    launch_lat_rho(lc, ctx->g, ctx->s, ctx->in, ctx->pt, mx, false, true);
-    if (t) t->mark(5);
+    launch_fix_records(lc, ctx->g, ctx->s);
     launch_inter_rho(lc, ctx->g, ctx->s, ctx->in, ctx->pt, mx);
+    if (t) t->mark(4);
+    const bool advance = launch_lat_rho(lc, ctx->g, ctx->s, ctx->in, ctx->pt, mx, false, true);
+    if (t) t->mark(5);
+    launch_inter_rho_owners(lc, ctx->g, ctx->s, ctx->in, ctx->pt, mx);
     if (t) t->mark(6);
-    launch_lat_df(lc, ctx->g, ctx->s, ctx->in, ctx->pt, mx, false);
+    launch_ghost_df(lc, ctx->g, ctx->s, ctx->in, mx, advance);
     if (t) t->mark(7);
-    launch_ghost_df(lc, ctx->g, ctx->s, ctx->in, mx);
-    if (t) t->mark(8);
 }
-// the inter-atom force pass and the second half-kick, after the lattice force pass
+// the inter-atom force pass and the second half-kick it takes, after the lattice force pass
 void seq_eam_force_tail(mg_context *ctx, bool kick, Timer *t) {
     const LaunchCtx lc = ctx->lc();
     launch_inter_force(lc, ctx->g, ctx->s, ctx->in, ctx->pt, ctx->mixed(), ctx->d_sp, kick);
-    if (t) t->mark(10);
-    if (kick) launch_secondstep(lc, ctx->g, ctx->s, ctx->in, ctx->d_sp, false);
-    if (t) t->mark(11);
+    if (t) t->mark(9);
 }
 void seq_compute_eam(mg_context *ctx, bool kick, bool with_manage_prefix, int manage_mask, Timer *t, bool fuse_next = false) {
     seq_eam_lists(ctx, with_manage_prefix, manage_mask, t);
     seq_eam_rho(ctx, t);
     launch_lat_force(ctx->lc(), ctx->g, ctx->s, ctx->in, ctx->pt, ctx->d_sp, kick, ctx->mixed(), false, fuse_next, true);
-    if (t) t->mark(9);
+    if (t) t->mark(8);
     seq_eam_force_tail(ctx, kick, t);
 }
 // one loop body: firststep, decide, exchangeInter, borderInter, exchangeAtom, computeEam, secondstep.
@@ -251,7 +246,7 @@ void seq_step(mg_context *ctx, Timer *t, bool fused_prev = false, bool fuse_next
 }
 // steps of mg_simulate that run fused: the mixed form with a fixed dt
 bool fusable(const mg_context *ctx) { return ctx->fuse_steps >= 2 && ctx->mixed() && ctx->dx_max <= 0.0; }
-constexpr int kLaunchesPerStep = 20;
+constexpr int kLaunchesPerStep = 11;
 
 mg_status require_ready(mg_context *ctx) {
     if (!ctx->pot_ready) { ctx->err = "potential not initialised"; return MG_ERR_POTENTIAL; }
@@ -346,8 +341,8 @@ mg_status upload_tables(mg_context *ctx) {
                                         int_bits_as_float(delta));
         }
     }
-    if (!ctx->d_cand) MG_CK(dalloc(ctx, &ctx->d_cand, static_cast<size_t>(2 * kMaxFull)));
-    MG_CK(cudaMemcpy(ctx->d_cand, nt.cand, sizeof(nt.cand), cudaMemcpyHostToDevice));
+    if (!ctx->d_nt) MG_CK(dalloc(ctx, &ctx->d_nt, 1));
+    MG_CK(cudaMemcpy(ctx->d_nt, &nt, sizeof(nt), cudaMemcpyHostToDevice));
     set_mass_table(ctx->stream);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) { ctx->err = std::string("mass table: ") + cudaGetErrorString(e); return MG_ERR_CUDA; }
@@ -638,12 +633,7 @@ mg_status mg_create(const int64_t phase_space[3], double lattice_const, double r
     ALLOC(in.gtype, gcap); ALLOC(in.groot, gcap);
     ALLOC(in.gx, gcap); ALLOC(in.gy, gcap); ALLOC(in.gz, gcap); ALLOC(in.gdf, gcap);
     ALLOC(in.scratch_i, 3 * cap); ALLOC(in.scratch_d, 13 * cap); ALLOC(in.scratch_u, cap);
-    ALLOC(in.displaced, (size_t) in.dcap);
-    {
-        const size_t nblocks = (static_cast<size_t>(g.n_local) + kFirstThreads - 1) / kFirstThreads;
-        ALLOC(in.dflag, nblocks * kFirstThreads);
-        ALLOC(in.dblock, nblocks);
-    }
+    ALLOC(in.displaced, (size_t) 2 * in.dcap);
     ALLOC(in.claim, ns);
     ALLOC(in.far_list, (size_t) in.fcap);
     ALLOC(in.far_flag, ns);
@@ -669,9 +659,6 @@ mg_status mg_create(const int64_t phase_space[3], double lattice_const, double r
     if (e == cudaSuccess) e = cudaMemsetAsync(in.far_flag, 0, ns, ctx->stream);
     if (e == cudaSuccess) e = cudaMemsetAsync(in.n_bucket, 0, sizeof(int), ctx->stream);
     if (e == cudaSuccess) e = cudaMemsetAsync(in.touch_bits, 0, (ns / 32 + 1) * sizeof(unsigned), ctx->stream);
-    if (e == cudaSuccess)  // the padding past n_local is never written and must read as "not displaced"
-        e = cudaMemsetAsync(in.dflag, 0, ((static_cast<size_t>(g.n_local) + kFirstThreads - 1) / kFirstThreads) * kFirstThreads,
-                            ctx->stream);
     if (e == cudaSuccess) e = cudaMemsetAsync(s.type, 0xff, ns, ctx->stream);  // all slots INVALID
     if (e == cudaSuccess) e = cudaMemsetAsync(s.u4, 0xff, ns * sizeof(float4), ctx->stream);
     if (e == cudaSuccess) e = cudaMemsetAsync(s.u4n, 0xff, ns * sizeof(float4), ctx->stream);
@@ -804,13 +791,14 @@ static mg_status hook_download(mg_context *ctx, mg_atom_element *atoms, int fiel
 mg_status mg_eam_rho_calc(mg_context *ctx, mg_atom_element *atoms, double cutoff_radius) {
     mg_status st = hook_upload(ctx, atoms, cutoff_radius);
     if (st != MG_OK) return st;
+    launch_fix_records(ctx->lc(), ctx->g, ctx->s);
     launch_lat_rho(ctx->lc(), ctx->g, ctx->s, ctx->in, ctx->pt, ctx->mixed(), true);
     return hook_download(ctx, atoms, PACK_RHO);
 }
 mg_status mg_eam_df_calc(mg_context *ctx, mg_atom_element *atoms, double cutoff_radius) {
     mg_status st = hook_upload(ctx, atoms, cutoff_radius);
     if (st != MG_OK) return st;
-    launch_lat_df(ctx->lc(), ctx->g, ctx->s, ctx->in, ctx->pt, ctx->mixed(), true);
+    launch_lat_df(ctx->lc(), ctx->g, ctx->s, ctx->pt, ctx->mixed());
     return hook_download(ctx, atoms, PACK_DF);
 }
 mg_status mg_eam_force_calc(mg_context *ctx, mg_atom_element *atoms, double cutoff_radius) {
@@ -1056,16 +1044,15 @@ mg_status mg_phase(mg_context *ctx, int32_t phase) {
         case 0: seq_firststep(ctx, false, nullptr); break;
         case 1:
             launch_decide_scan(lc, ctx->g, ctx->s, ctx->in);
-            launch_displaced_collect(lc, ctx->g, ctx->in);
             launch_far_clear(lc, ctx->g, ctx->in);
             launch_inter_manage(lc, ctx->g, ctx->s, ctx->in, MANAGE_DECIDE | MANAGE_CLEAR_GHOST, ctx->mixed());
             launch_far_mark(lc, ctx->g, ctx->in);
             break;
         case 2: launch_inter_manage(lc, ctx->g, ctx->s, ctx->in, MANAGE_EXCHANGE, ctx->mixed()); break;
         case 3: launch_inter_manage(lc, ctx->g, ctx->s, ctx->in, MANAGE_BORDER, ctx->mixed()); break;
-        case 4: launch_ghost_copy(lc, ctx->g, ctx->s, ctx->mixed()); break;
+        case 4: launch_ghost_copy(lc, ctx->g, ctx->s, ctx->in, false); break;
         case 5: seq_compute_eam(ctx, false, false, 0, nullptr); break;
-        case 6: launch_secondstep(lc, ctx->g, ctx->s, ctx->in, ctx->d_sp, true); break;
+        case 6: launch_secondstep(lc, ctx->g, ctx->s, ctx->in, ctx->d_sp); break;
     }
     if ((st = check_launch(ctx)) != MG_OK) return st;
     uint32_t bits = 0;
@@ -1485,6 +1472,7 @@ static mg_status step_host_overlapped(mg_context *ctx, mg_atom_element *atoms, m
         if ((st = read_device_errors(ctx, &bits)) != MG_OK) return st;
         return status_from_bits(ctx, bits);
     }
+    launch_set_counts(lc, ctx->in, 0);  // the displaced list has been taken per chunk
     *n_inter = 0;
     return status_from_bits(ctx, static_cast<uint32_t>(cnt[CNT_ERRORS]));
 }
@@ -1554,6 +1542,7 @@ static mg_status step_host_pipelined(mg_context *ctx, mg_atom_element *atoms, mg
         if (k1 > k0) launch_firststep(lc, g, ctx->s, ctx->in, ctx->d_sp, true, k0 * g.by * g.bx, k1 * g.by * g.bx);
     }
     launch_inter_firststep(lc, ctx->in, ctx->d_sp);
+    launch_far_clear(lc, g, ctx->in);
     seq_eam_lists(ctx, true, MANAGE_DECIDE | MANAGE_CLEAR_GHOST | MANAGE_EXCHANGE | MANAGE_BORDER, nullptr);
     // whether decide left inter atoms: they add density and force after the lattice passes, which
     // orders the whole density pass before any force (and the slabs' early copies would be stale)
@@ -1764,6 +1753,7 @@ mg_status mg_autotune(mg_context *ctx, int32_t reps, int32_t out[6]) {
                 ctx->tune[p][kern][2] = apt;
                 const LaunchCtx lc = ctx->lc();
                 auto run = [&]() {
+                    if (kern == 0) launch_fix_records(lc, ctx->g, ctx->s);
                     if (kern == 0) launch_lat_rho(lc, ctx->g, ctx->s, ctx->in, ctx->pt, ctx->mixed(), false);
                     else launch_lat_force(lc, ctx->g, ctx->s, ctx->in, ctx->pt, ctx->d_sp, false, ctx->mixed(), false);
                 };

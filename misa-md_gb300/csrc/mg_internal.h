@@ -18,7 +18,7 @@ constexpr double kMvv2e = 1.0364269e-4;      // src/types/pre_define.h:18
 constexpr double kFtm2v = (1.0 / kMvv2e);    // src/types/pre_define.h:19
 constexpr double kNeiLatCutoff = 0.5;        // src/md_building_config.h.in:24
 constexpr int kMaxFull = 232;                // capacity of a full offset table per parity
-constexpr int kFirstThreads = 256;           // firststep block = one group of displaced flags (8 per lane)
+constexpr int kFirstThreads = 256;           // firststep block
 constexpr int kSortSmemKeys = 16384;         // bucket keys the list manager sorts in shared memory
 constexpr int kListWords = 4;                // list bits per 32-site group: pruned candidates up to 128
 constexpr int kSkinSlots = 64;               // words the per-step maximum displacement is spread over
@@ -27,13 +27,12 @@ constexpr int kSkinSlots = 64;               // words the per-step maximum displ
 constexpr uint32_t kInBox = 0, kXLow = 1u, kXHigh = 2u, kYLow = 4u, kYHigh = 8u, kZLow = 16u, kZHigh = 32u;
 
 // device counters / flags word indices
-// CNT_DISP_RAW: displaced slots counted by firststep this step (0 lets the collection kernels skip)
 // CNT_TOUCHED: lattice owners listed by an inter-atom pass for the ordered owner gather that follows;
 // CNT_TOUCH_DONE: blocks of that gather finished (the last one resets both words)
 // CNT_SPEC_VOID: the overlapped host step met a displaced atom whose decide it cannot take per chunk
 enum {
-    CNT_INTER = 0, CNT_GHOST = 1, CNT_DISPLACED = 2, CNT_ERRORS = 3, CNT_FAR = 4, CNT_DISP_RAW = 5, CNT_TOUCHED = 6,
-    CNT_TOUCH_DONE = 7, CNT_SPEC_VOID = 8, CNT_WORDS = 9
+    CNT_INTER = 0, CNT_GHOST = 1, CNT_DISPLACED = 2, CNT_ERRORS = 3, CNT_FAR = 4, CNT_TOUCHED = 5, CNT_TOUCH_DONE = 6,
+    CNT_SPEC_VOID = 7, CNT_WORDS = 8
 };
 
 inline double atom_mass(int type) {  // src/types/atom_types.h:42-53
@@ -135,11 +134,10 @@ struct Inter {
     int *scratch_i;          // 3 * cap
     double *scratch_d;       // 13 * cap
     uint64_t *scratch_u;     // cap
-    // displaced lattice slots found by the decide scan, in scan order
+    // local indices of the displaced lattice atoms found by firststep (CNT_DISPLACED of them, in any order; past dcap
+    // only counted), then dcap words for the list manager's ordered copy
     int *displaced;
     int dcap;
-    int8_t *dflag;           // per local slot (k, j, i order, padded to whole firststep blocks): 1 = displaced
-    int *dblock;             // per firststep block: displaced count, then its exclusive offset
     // per-slot claim word for recombination (INT_MAX when free)
     int *claim;
     // lattice atoms farther than 0.2 a0 from their site (only recombined atoms after decide): they
@@ -258,7 +256,7 @@ struct LaunchCtx {
     int rho_order = 0, rho_block = 256, rho_apt = 1;        // gather thread order, block size and atoms per thread
     int force_order = 0, force_block = 256, force_apt = 1;  // of the density and force passes (mg_autotune)
     const NeighTables *nt = nullptr;         // the context's offset tables
-    const float4 *cand = nullptr;            // its cand[2][kMaxFull] in device memory
+    const NeighTables *ntd = nullptr;        // the same in device memory
     const FixParams *fp = nullptr;           // FP64 form: scales and tables of the fixed-point pair arithmetic
     int share = 1;                           // contexts that step side by side (a batch's members)
 };
@@ -275,7 +273,8 @@ void launch_pack_aos(const LaunchCtx &lc, const Geom &g, mg_atom_element *aos, S
                      int s0 = 0, int s1 = -1);
 enum { PACK_ALL = 0xff, PACK_RHO = 1, PACK_DF = 2, PACK_F = 4 };
 
-// local atoms [t0, t1) in k, j, i order (t1 < 0: all)
+// local atoms [t0, t1) in k, j, i order; t1 < 0: all of them and the inter atoms, and (decide) the previous far list's
+// neighbourhood marks are cleared
 // fused: the previous force pass took this firststep already (launch_lat_force with fuse_next)
 // alt: a body of a graph whose bodies alternate their u4 buffers (the previous body's records are in
 // s.u4n)
@@ -284,20 +283,22 @@ void launch_firststep(const LaunchCtx &lc, const Geom &g, Slots s, Inter in, con
 // fill g.site_half (once per context)
 void launch_site_table(const LaunchCtx &lc, const Geom &g, double *site_half);
 void launch_decide_scan(const LaunchCtx &lc, const Geom &g, Slots s, Inter in);
-// after a deciding firststep: the displaced slots in scan order into in.displaced, count in CNT_DISPLACED
-void launch_displaced_collect(const LaunchCtx &lc, const Geom &g, Inter in);
 // FP64 form: the fixed-point records of the slots [s0, s1) (s1 < 0: to the end), after every change of a
 // position and before the density pass (the force hook: before the force pass)
 void launch_fix_records(const LaunchCtx &lc, const Geom &g, Slots s, int s0 = 0, int s1 = -1);
 // far-atom neighbourhood marks: clear those of the current far list / set them (grid-wide)
 void launch_far_clear(const LaunchCtx &lc, const Geom &g, Inter in);
 void launch_far_mark(const LaunchCtx &lc, const Geom &g, Inter in);
-void launch_ghost_copy(const LaunchCtx &lc, const Geom &g, Slots s, bool mixed);
-void launch_ghost_df(const LaunchCtx &lc, const Geom &g, Slots s, Inter in, bool mixed);
+// mark: also as launch_far_mark
+void launch_ghost_copy(const LaunchCtx &lc, const Geom &g, Slots s, Inter in, bool mark);
+// advance: also as launch_skin_advance
+void launch_ghost_df(const LaunchCtx &lc, const Geom &g, Slots s, Inter in, bool mixed, bool advance);
 // lists (mixed form): check or rebuild, per 32-site group, the list of pruned candidates that some site
 // of the group has inside rc + skin, and visit only those (when lists_ok; the force pass of the same
 // step must get the same flag)
-void launch_lat_rho(const LaunchCtx &lc, const Geom &g, Slots s, Inter in, PotTables t, bool mixed, bool hook,
+// true: the skin's advance is due. Inter atoms: after launch_inter_rho, which lists the owners whose F' the pass
+// leaves to launch_inter_rho_owners.
+bool launch_lat_rho(const LaunchCtx &lc, const Geom &g, Slots s, Inter in, PotTables t, bool mixed, bool hook,
                     bool lists = false);
 // the density pass over the sites [u0, u1) of both parities (as launch_lat_force_sites)
 void launch_lat_rho_sites(const LaunchCtx &lc, const Geom &g, Slots s, Inter in, PotTables t, bool mixed, int u0, int u1,
@@ -320,7 +321,7 @@ void launch_ghost_copy_planes(const LaunchCtx &lc, const Geom &g, Slots s, int k
 void launch_spec_decide(const LaunchCtx &lc, const Geom &g, Slots s, Inter in, int t0, int t1);
 // CNT_FAR = 0 and CNT_SPEC_VOID = 0 (after the previous far list's marks are cleared)
 void launch_spec_begin(const LaunchCtx &lc, Inter in);
-void launch_lat_df(const LaunchCtx &lc, const Geom &g, Slots s, Inter in, PotTables t, bool mixed, bool hook);
+void launch_lat_df(const LaunchCtx &lc, const Geom &g, Slots s, PotTables t, bool mixed);
 // fuse_next (mixed form, kick, fixed dt): after the second half-kick each lattice atom also takes the
 // next step's firststep (into u4n), when no inter atoms exist
 void launch_lat_force(const LaunchCtx &lc, const Geom &g, Slots s, Inter in, PotTables t, StepParams *sp, bool kick,
@@ -329,7 +330,8 @@ void launch_lat_force(const LaunchCtx &lc, const Geom &g, Slots s, Inter in, Pot
 // with u0 and u1 multiples of 32 (or u1 = n_local_half) the slabs of a split pass are disjoint warps
 void launch_lat_force_sites(const LaunchCtx &lc, const Geom &g, Slots s, Inter in, PotTables t, StepParams *sp, bool kick,
                             bool mixed, int u0, int u1, bool lists = false);
-void launch_secondstep(const LaunchCtx &lc, const Geom &g, Slots s, Inter in, StepParams *sp, bool lattice);
+// the second half-kick as a phase of its own (lattice and inter atoms)
+void launch_secondstep(const LaunchCtx &lc, const Geom &g, Slots s, Inter in, StepParams *sp);
 // step head: records the step's dt and, in variable mode, sets dt from the last kick's max |v|
 void launch_step_head(const LaunchCtx &lc, StepParams *sp, SkinState *skin);
 // out[0] = steps taken, out[1] = simulated time
@@ -343,8 +345,10 @@ void launch_energy(const LaunchCtx &lc, const Geom &g, Slots s, Inter in, PotTab
 void launch_far_rebuild(const LaunchCtx &lc, const Geom &g, Slots s, Inter in);
 void launch_inter_manage(const LaunchCtx &lc, const Geom &g, Slots s, Inter in, int steps_mask, bool mixed);
 enum { MANAGE_DECIDE = 1, MANAGE_CLEAR_GHOST = 2, MANAGE_EXCHANGE = 4, MANAGE_BORDER = 8, MANAGE_INDEX = 16 };
+// the inter atoms' own densities, listing the lattice owners near them; after the lattice density pass, the owners' shares
 void launch_inter_rho(const LaunchCtx &lc, const Geom &g, Slots s, Inter in, PotTables t, bool mixed);
-// kick: the second half-kick of the lattice owners the density pass's inter-atom sweep listed (the
+void launch_inter_rho_owners(const LaunchCtx &lc, const Geom &g, Slots s, Inter in, PotTables t, bool mixed);
+// kick: the second half-kick of the inter atoms and of the lattice owners the inter-atom density pass listed (the
 // lattice force pass kicked every other atom)
 void launch_inter_force(const LaunchCtx &lc, const Geom &g, Slots s, Inter in, PotTables t, bool mixed, StepParams *sp,
                         bool kick);

@@ -261,7 +261,9 @@ __device__ __forceinline__ bool lattice_only(const Inter &in) { return in.cnt[CN
 // atoms; with them, for every atom the density pass's inter-atom sweep did not list (no inter atom
 // within the cutoff, so no inter-atom force is added later). The listed owners are kicked by the
 // inter-atom force pass's owner gather once their force is complete.
-__device__ __forceinline__ bool kick_in_lattice_pass(const Inter &in, int sl) {
+// The same holds for F'(rho) in the density pass: the inter-atom density pass runs before it and lists
+// the owners, whose gather adds their inter-atom terms and takes their F' afterwards.
+__device__ __forceinline__ bool untouched(const Inter &in, int sl) {
     return lattice_only(in) || !((in.touch_bits[sl >> 5] >> (sl & 31)) & 1u);
 }
 // FP64 displacement test of atom::decide (src/atom.cpp:34-42) for a local slot
@@ -404,7 +406,6 @@ __global__ void k_set_counts(Inter in, int n_inter) {
     in.cnt[CNT_INTER] = n_inter;
     in.cnt[CNT_GHOST] = 0;
     in.cnt[CNT_DISPLACED] = 0;
-    in.cnt[CNT_DISP_RAW] = 0;
     *in.n_bucket = 0;
 }
 void launch_set_counts(const LaunchCtx &lc, Inter in, int n_inter) { k_set_counts<<<1, 1, 0, lc.stream>>>(in, n_inter); }
@@ -429,20 +430,17 @@ void launch_site_table(const LaunchCtx &lc, const Geom &g, double *site_half) {
     k_site_table<<<(g.n_site_half + 255) / 256, 256, 0, lc.stream>>>(g.a0, g.n_site_half, site_half);
 }
 
-// Displaced slots are recorded in scan order without a sort: firststep writes one byte per local slot
-// (byte t for local index t, in k, j, i order; 1 = displaced). A count kernel sums the bytes of each
-// group of kFirstThreads slots, a one-block scan turns the sums into offsets, and a collect kernel
-// writes the slots in order. firststep keeps its early exits and needs no warp or block collective.
-// decide's distance test (src/atom.cpp:34-42) with each operation rounded on its own; a displaced
-// atom also counts itself into CNT_DISP_RAW, so the collection kernels can skip steps without any
-// displaced atom.
-__device__ __noinline__ bool exact_displaced(double ex, double ey, double ez, double thr, int *raw_count) {
+// decide's distance test (src/atom.cpp:34-42) with each operation rounded on its own; a displaced atom
+// appends its local index to the displaced list, in any order (the list manager sorts it into the
+// reference's k, j, i scan order)
+__device__ __noinline__ void note_displaced(double ex, double ey, double ez, double thr, int t, int *count, int *list, int cap) {
     double dist = __dmul_rn(ex, ex);
     dist = __dadd_rn(dist, __dmul_rn(ey, ey));
     dist = __dadd_rn(dist, __dmul_rn(ez, ez));
-    const bool d = dist > thr;
-    if (d) atomicAdd(raw_count, 1);
-    return d;
+    if (dist > thr) {
+        const int q = atomicAdd(count, 1);
+        if (q < cap) list[q] = t;
+    }
 }
 
 // the step's largest change of a displacement record: one reduction per group of converged lanes and
@@ -456,8 +454,8 @@ __device__ __forceinline__ void skin_note(const Slots &s, float d2) {
 
 // NewtonMotion::firststep for one lattice atom (src/newton_motion.cpp:30-55) and decide's displacement
 // test (src/atom.cpp:34-42): v += c f, x += dt v (each operation rounded as the reference rounds it),
-// the displacement record u4 (written to u4_out, parity-split index) and the displaced flag of local
-// index t. MOVE = false: the test alone, on the current positions. u4_prev holds the record the last
+// the displacement record u4 (written to u4_out, parity-split index) and, where displaced, local index t
+// into the displaced list. MOVE = false: the test alone, on the current positions. u4_prev holds the record the last
 // density pass read (for the skin's displacement bound).
 template <bool MOVE, bool DECIDE>
 __device__ __forceinline__ void first_half(const Geom &g, const Slots &s, const Inter &in, const StepParams *__restrict__ p,
@@ -496,9 +494,37 @@ __device__ __forceinline__ void first_half(const Geom &g, const Slots &s, const 
     if (DECIDE) {
         // the exact FP64 test of decide runs only where the FP32 distance is not clearly below it
         // (a call, so the rare path stays a branch instead of being evaluated for every atom)
-        const bool disp = !(exf * exf + eyf * eyf + ezf * ezf < g.thr_lo_f) &&
-                          exact_displaced(ex, ey, ez, g.thr, &in.cnt[CNT_DISP_RAW]);
-        in.dflag[t] = disp ? 1 : 0;
+        if (!(exf * exf + eyf * eyf + ezf * ezf < g.thr_lo_f))
+            note_displaced(ex, ey, ez, g.thr, t, &in.cnt[CNT_DISPLACED], in.displaced, in.dcap);
+    }
+}
+
+__device__ void mark_far_neighbourhoods(const NeighTables &nt, const Geom &g, const Inter &in, int a0, int a1, int8_t v, int t0,
+                                        int stride) {
+    const int per = nt.nfull + 1;
+    const int total = (a1 - a0) * per;
+    for (int e = t0; e < total; e += stride) {
+        const int sl = in.far_list[a0 + e / per];
+        const int q = e % per;
+        const int par = (sl % g.Sx) & 1;
+        const int sj = q == nt.nfull ? sl : sl + nt.lat[par][q];
+        in.far_flag[owner_slot(g, sj)] = v;
+    }
+}
+
+// NewtonMotion::firststep for the inter atoms
+__device__ __forceinline__ void inter_firststep(const Inter &in, const StepParams *__restrict__ p, int t0, int stride) {
+    const int n = in.cnt[CNT_INTER];
+    const double dt = p->dt;
+    for (int a = t0; a < n; a += stride) {
+        const double c = dt_inv_m_of(p, in.type[a]);
+        double vx = __dadd_rn(in.vx[a], __dmul_rn(c, in.fx[a]));
+        double vy = __dadd_rn(in.vy[a], __dmul_rn(c, in.fy[a]));
+        double vz = __dadd_rn(in.vz[a], __dmul_rn(c, in.fz[a]));
+        in.vx[a] = vx; in.vy[a] = vy; in.vz[a] = vz;
+        in.x[a] = __dadd_rn(in.x[a], __dmul_rn(dt, vx));
+        in.y[a] = __dadd_rn(in.y[a], __dmul_rn(dt, vy));
+        in.z[a] = __dadd_rn(in.z[a], __dmul_rn(dt, vz));
     }
 }
 
@@ -508,18 +534,27 @@ __device__ __forceinline__ void first_half(const Geom &g, const Slots &s, const 
 // alternates between are always complete.
 // alt: inside a graph whose bodies alternate their u4 buffers, where the previous body's records are
 // in s.u4n
+// whole: the step's only firststep launch (not one of several over parts of the box). It takes the inter
+// atoms' firststep too and (deciding) clears the previous far list's neighbourhood marks, which nothing
+// reads between the previous force pass and the marks decide makes: a small box's step is a chain of
+// short kernels at 1 to 2 us each, whatever they do.
 // A grid-stride loop over a grid of a few blocks per SM: a fused body's launch, which returns at once,
 // then costs one small launch instead of a grid over every slot.
 template <bool MOVE, bool DECIDE>
-__global__ void __launch_bounds__(kFirstThreads) k_firststep(Geom g, Slots s, Inter in, const StepParams *__restrict__ p,
-                                                             int t0, int t1, bool fused, bool alt) {
+__global__ void __launch_bounds__(kFirstThreads) k_firststep(const NeighTables *nt, Geom g, Slots s, Inter in,
+                                                             const StepParams *__restrict__ p, int t0, int t1, bool fused, bool alt,
+                                                             bool whole) {
+    const int tid = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
+    if (MOVE && whole) {
+        inter_firststep(in, p, tid, stride);
+        if (DECIDE) mark_far_neighbourhoods(*nt, g, in, 0, min(in.cnt[CNT_FAR], in.fcap), 0, tid, stride);
+    }
     if (fused && lattice_only(in)) return;
-    for (int t = t0 + blockIdx.x * blockDim.x + threadIdx.x; t < t1; t += gridDim.x * blockDim.x) {
+    for (int t = t0 + tid; t < t1; t += stride) {
         int i, j, k;
         const int sl = local_slot(g, t, i, j, k);
         const int ty = s.type[sl];
         if (ty < 0) {
-            if (DECIDE) in.dflag[t] = 0;
             if (MOVE) s.u4[sidx(g, sl)] = vacant_u4();
             continue;
         }
@@ -529,17 +564,6 @@ __global__ void __launch_bounds__(kFirstThreads) k_firststep(Geom g, Slots s, In
         else
             first_half<false, DECIDE>(g, s, in, p, sl, t, i, j, k, ty, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, s.u4, s.u4);
     }
-}
-
-// one warp per group of kFirstThreads flag bytes (8 per lane, read as one 64-bit word): its count
-__global__ void k_disp_count(Inter in, int nblocks) {
-    if (in.cnt[CNT_DISP_RAW] == 0) return;  // nothing displaced this step (the usual case)
-    const int b = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    if (b >= nblocks) return;
-    const unsigned long long w = reinterpret_cast<const unsigned long long *>(in.dflag)[b * 32 + (threadIdx.x & 31)];
-    int c = __popcll(w);  // bytes are 0 or 1
-    for (int o = 16; o > 0; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
-    if ((threadIdx.x & 31) == 0) in.dblock[b] = c;
 }
 
 // one block: counts a[0..n) -> base + exclusive offsets (in place); returns base + the total (every
@@ -579,78 +603,22 @@ __device__ int block_scan_counts(int *a, int n, int base) {
     return total;
 }
 
-// one block: block counts -> exclusive offsets (in place), total -> CNT_DISPLACED (clamped to dcap)
-__global__ void __launch_bounds__(1024) k_disp_scan(Inter in, int nblocks) {
-    if (in.cnt[CNT_DISP_RAW] == 0) {  // nothing displaced this step (the usual case)
-        if (threadIdx.x == 0) in.cnt[CNT_DISPLACED] = 0;
-        return;
-    }
-    int total = block_scan_counts(in.dblock, nblocks, 0);
-    if (threadIdx.x == 0) {
-        if (total > in.dcap) { set_error(in, MG_DEVERR_DISPLACED_OVERFLOW); total = in.dcap; }
-        in.cnt[CNT_DISPLACED] = total;
-        in.cnt[CNT_DISP_RAW] = 0;
-    }
-}
-
-// one warp per group of kFirstThreads flag bytes: its displaced slots, in order, at the group's offset
-__global__ void k_disp_collect(Geom g, Inter in, int nblocks) {
-    if (in.cnt[CNT_DISPLACED] == 0) return;
-    const int b = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    if (b >= nblocks) return;
-    const int lane = threadIdx.x & 31;
-    unsigned long long w = reinterpret_cast<const unsigned long long *>(in.dflag)[b * 32 + lane];
-    const int c = __popcll(w);
-    int incl = c;  // inclusive scan over the lanes
-    for (int o = 1; o < 32; o <<= 1) {
-        const int y = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= o) incl += y;
-    }
-    if (c == 0) return;
-    int rank = in.dblock[b] + incl - c;
-    for (int byte = 0; w; byte++, w >>= 8) {
-        if ((w & 0xff) == 0) continue;
-        if (rank < in.dcap) {
-            int i, j, k;
-            in.displaced[rank] = local_slot(g, b * kFirstThreads + lane * 8 + byte, i, j, k);
-        }
-        rank++;
-    }
-}
-
 void launch_firststep(const LaunchCtx &lc, const Geom &g, Slots s, Inter in, const StepParams *p, bool decide, int t0,
                       int t1, bool fused, bool alt) {
-    if (t1 < 0) t1 = g.n_local;
+    const bool whole = t1 < 0;
+    if (whole) t1 = g.n_local;
     if (t1 <= t0) return;
     const int b = kFirstThreads, n = std::min((t1 - t0 + b - 1) / b, lc.num_sms * 8);
-    if (decide) k_firststep<true, true><<<n, b, 0, lc.stream>>>(g, s, in, p, t0, t1, fused, alt);
-    else k_firststep<true, false><<<n, b, 0, lc.stream>>>(g, s, in, p, t0, t1, fused, alt);
+    if (decide) k_firststep<true, true><<<n, b, 0, lc.stream>>>(lc.ntd, g, s, in, p, t0, t1, fused, alt, whole);
+    else k_firststep<true, false><<<n, b, 0, lc.stream>>>(lc.ntd, g, s, in, p, t0, t1, fused, alt, whole);
 }
 void launch_decide_scan(const LaunchCtx &lc, const Geom &g, Slots s, Inter in) {
     const int b = kFirstThreads, n = std::min((g.n_local + b - 1) / b, lc.num_sms * 8);
-    k_firststep<false, true><<<n, b, 0, lc.stream>>>(g, s, in, nullptr, 0, g.n_local, false, false);
+    cudaMemsetAsync(&in.cnt[CNT_DISPLACED], 0, sizeof(int), lc.stream);
+    k_firststep<false, true><<<n, b, 0, lc.stream>>>(lc.ntd, g, s, in, nullptr, 0, g.n_local, false, false, false);
 }
-void launch_displaced_collect(const LaunchCtx &lc, const Geom &g, Inter in) {
-    const int nblocks = (g.n_local + kFirstThreads - 1) / kFirstThreads;
-    const int grid = (nblocks + 7) / 8;  // 8 warps (groups) per 256-thread block
-    k_disp_count<<<grid, 256, 0, lc.stream>>>(in, nblocks);
-    k_disp_scan<<<1, 1024, 0, lc.stream>>>(in, nblocks);
-    k_disp_collect<<<grid, 256, 0, lc.stream>>>(g, in, nblocks);
-}
-
 __global__ void k_inter_firststep(Inter in, const StepParams *__restrict__ p) {
-    const int n = in.cnt[CNT_INTER];
-    const double dt = p->dt;
-    for (int a = blockIdx.x * blockDim.x + threadIdx.x; a < n; a += gridDim.x * blockDim.x) {
-        const double c = dt_inv_m_of(p, in.type[a]);
-        double vx = __dadd_rn(in.vx[a], __dmul_rn(c, in.fx[a]));
-        double vy = __dadd_rn(in.vy[a], __dmul_rn(c, in.fy[a]));
-        double vz = __dadd_rn(in.vz[a], __dmul_rn(c, in.fz[a]));
-        in.vx[a] = vx; in.vy[a] = vy; in.vz[a] = vz;
-        in.x[a] = __dadd_rn(in.x[a], __dmul_rn(dt, vx));
-        in.y[a] = __dadd_rn(in.y[a], __dmul_rn(dt, vy));
-        in.z[a] = __dadd_rn(in.z[a], __dmul_rn(dt, vz));
-    }
+    inter_firststep(in, p, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
 }
 void launch_inter_firststep(const LaunchCtx &lc, Inter in, const StepParams *p) {
     k_inter_firststep<<<lc.num_sms, 256, 0, lc.stream>>>(in, p);
@@ -702,14 +670,16 @@ __device__ __forceinline__ void ghost_copy_one(const Geom &g, const Slots &s, in
     s.z[gs] = sz ? __dadd_rn(oz, sz > 0 ? g.L[2] : -g.L[2]) : oz;
     s.u4[sidx(g, gs)] = s.u4[sidx(g, os)];
 }
-__global__ void k_ghost_copy(Geom g, Slots s) {
+// mark: after decide, also the marks of the new far list's neighbourhoods (as launch_far_mark)
+__global__ void k_ghost_copy(const NeighTables *nt, Geom g, Slots s, Inter in, bool mark) {
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (mark) mark_far_neighbourhoods(*nt, g, in, 0, min(in.cnt[CNT_FAR], in.fcap), 1, t, gridDim.x * blockDim.x);
     if (t >= g.n_ghost_slots) return;
     ghost_copy_one(g, s, ghost_slot(g, t));
 }
-void launch_ghost_copy(const LaunchCtx &lc, const Geom &g, Slots s, bool) {
+void launch_ghost_copy(const LaunchCtx &lc, const Geom &g, Slots s, Inter in, bool mark) {
     const int b = 256, n = (g.n_ghost_slots + b - 1) / b;
-    k_ghost_copy<<<n, b, 0, lc.stream>>>(g, s);
+    k_ghost_copy<<<n, b, 0, lc.stream>>>(lc.ntd, g, s, in, mark);
 }
 // The ghost slots inside the local planes [k0, k1) (y-ghost rows, then x-ghost columns of each plane;
 // their owners lie in the same plane), or (k0 < 0) the ghost planes below and above the box, whose
@@ -752,9 +722,29 @@ __device__ __forceinline__ void ghost_df_one(const Geom &g, const Slots &s, int 
         if (s.dfq) s.dfq[sidx(g, gs)] = s.dfq[sidx(g, os)];
     }
 }
+// The step's maximum change of a displacement record into the skin's sum, or a restart after a rebuild. One warp.
+__device__ __forceinline__ void skin_advance(SkinState *k) {
+    static_assert(kSkinSlots == 64, "two words per lane");
+    const int lane = threadIdx.x & 31;
+    const unsigned m = __reduce_max_sync(0xffffffffu, max(k->step_max2[lane], k->step_max2[lane + 32]));
+    k->step_max2[lane] = 0u;
+    k->step_max2[lane + 32] = 0u;
+    if (lane != 0) return;
+    if (k->rebuilt) {  // built on this step's records: the sum restarts
+        k->acc = 0.f;
+        k->dirty = 0;
+        k->rebuilt = 0;
+        k->rebuilds++;
+    } else {
+        k->acc += sqrtf(__uint_as_float(m));  // a NaN or infinity forces the next pass to rebuild
+    }
+    k->passes++;
+}
+// advance: after a density pass with the group lists (as launch_skin_advance)
 template <bool MIXED>
-__global__ void k_ghost_df(Geom g, Slots s, Inter in) {
+__global__ void k_ghost_df(Geom g, Slots s, Inter in, bool advance) {
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (advance && t < 32) skin_advance(s.skin);
     if (t < g.n_ghost_slots) {
         const int gs = ghost_slot(g, t);
         const int os = owner_slot(g, gs);
@@ -763,10 +753,10 @@ __global__ void k_ghost_df(Geom g, Slots s, Inter in) {
     const int ng = in.cnt[CNT_GHOST];
     for (int q = t; q < ng; q += gridDim.x * blockDim.x) in.gdf[q] = in.df[in.groot[q]];
 }
-void launch_ghost_df(const LaunchCtx &lc, const Geom &g, Slots s, Inter in, bool mixed) {
+void launch_ghost_df(const LaunchCtx &lc, const Geom &g, Slots s, Inter in, bool mixed, bool advance) {
     const int b = 256, n = (g.n_ghost_slots + b - 1) / b;
-    if (mixed) k_ghost_df<true><<<n, b, 0, lc.stream>>>(g, s, in);
-    else k_ghost_df<false><<<n, b, 0, lc.stream>>>(g, s, in);
+    if (mixed) k_ghost_df<true><<<n, b, 0, lc.stream>>>(g, s, in, advance);
+    else k_ghost_df<false><<<n, b, 0, lc.stream>>>(g, s, in, advance);
 }
 // the same copy for the ghost slots inside the local planes [k0, k1) (y-ghost rows, then x-ghost
 // columns of each plane; their owners lie in the same plane), or (k0 < 0) for the ghost planes below
@@ -877,7 +867,7 @@ __device__ __forceinline__ void k_lat_rho_fp64_site(int t, const NeighTables &nt
     if (ti < 0) { s.rho[sl] = 0.0; return; }
     const double acc = rho_atom_fp64(nt, g, s, in, pt, sl, par);
     s.rho[sl] = acc;
-    if (!hook && lattice_only(in)) {
+    if (!hook && untouched(in, sl)) {
         int m; double p;
         locate_d(acc, pt.inv_drho, pt.nrho, m, p);
         s.df[sl] = der_d(pt.F_d + ti * pt.nrho, m, p);
@@ -986,7 +976,7 @@ __device__ __forceinline__ void rho_done_mixed(const Slots &s, const Inter &in, 
                                                float comp, bool hook) {
     const double rho = (double) sum - (double) comp;
     s.rho[sl] = rho;
-    if (!hook && lattice_only(in)) {
+    if (!hook && untouched(in, sl)) {
         int m; float p;
         locate_f((float) rho, pt.inv_drho_f, pt.nrho, m, p);
         s.df32[si] = der_f(pt.F_dff + ti * pt.nrho, m, p);
@@ -1389,7 +1379,7 @@ __device__ __forceinline__ void rho_done_fix(const NeighTables &nt, const Geom &
                                              bool hook) {
     if (near) rho = rho_near_fp64(nt, g, s, in, pt, sl, par, near) + (near == kFixNearMany ? 0.0 : rho);
     s.rho[sl] = rho;
-    if (!hook && lattice_only(in)) {
+    if (!hook && untouched(in, sl)) {
         int m; double p;
         locate_d(rho, pt.inv_drho, pt.nrho, m, p);
         const double df = der_d(pt.F_d + ti * pt.nrho, m, p);
@@ -1540,8 +1530,8 @@ static void launch_rho_split_w(const LaunchCtx &lc, const Geom &g, Slots s, Inte
                                bool lists) {
     const int n = split_groups(u0, u1);
     if (mixed)
-        k_lat_rho_mixed_split<W><<<n, 32 * W, 0, lc.stream>>>(lc.cand, lc.nt->npruned, lc.nt->nfull, g, s, in, t, hook, u0, u1, lists);
-    else k_lat_rho_fix_split<W><<<n, 32 * W, 0, lc.stream>>>(*lc.nt, lc.cand, g, s, in, t, *lc.fp, hook, u0, u1, lists);
+        k_lat_rho_mixed_split<W><<<n, 32 * W, 0, lc.stream>>>(&lc.ntd->cand[0][0], lc.nt->npruned, lc.nt->nfull, g, s, in, t, hook, u0, u1, lists);
+    else k_lat_rho_fix_split<W><<<n, 32 * W, 0, lc.stream>>>(*lc.nt, &lc.ntd->cand[0][0], g, s, in, t, *lc.fp, hook, u0, u1, lists);
 }
 // the split density pass, where it serves
 static bool launch_lat_rho_split(const LaunchCtx &lc, const Geom &g, Slots s, Inter in, PotTables t, bool mixed, bool hook, int u0,
@@ -1568,41 +1558,20 @@ static void launch_lat_rho_threads(const LaunchCtx &lc, const Geom &g, Slots s, 
         else k_lat_rho_fp64<false><<<n, b, 0, lc.stream>>>(*lc.nt, g, s, in, t, hook, order, tb, te);
     }
 }
-// one block of kSkinSlots threads
-__global__ void __launch_bounds__(kSkinSlots) k_skin_advance(SkinState *k) {
-    __shared__ unsigned wmax[kSkinSlots / 32];
-    unsigned v = k->step_max2[threadIdx.x];
-    k->step_max2[threadIdx.x] = 0u;
-    v = __reduce_max_sync(0xffffffffu, v);
-    if ((threadIdx.x & 31) == 0) wmax[threadIdx.x >> 5] = v;
-    __syncthreads();
-    if (threadIdx.x != 0) return;
-    unsigned m = 0u;
-    for (int w = 0; w < kSkinSlots / 32; w++) m = max(m, wmax[w]);
-    if (k->rebuilt) {  // built on this step's records: the sum restarts
-        k->acc = 0.f;
-        k->dirty = 0;
-        k->rebuilt = 0;
-        k->rebuilds++;
-    } else {
-        k->acc += sqrtf(__uint_as_float(m));  // a NaN or infinity forces the next pass to rebuild
-    }
-    k->passes++;
-}
-void launch_skin_advance(const LaunchCtx &lc, Slots s) { k_skin_advance<<<1, kSkinSlots, 0, lc.stream>>>(s.skin); }
+__global__ void __launch_bounds__(32) k_skin_advance(SkinState *k) { skin_advance(k); }
+void launch_skin_advance(const LaunchCtx &lc, Slots s) { k_skin_advance<<<1, 32, 0, lc.stream>>>(s.skin); }
 void launch_skin_dirty(const LaunchCtx &lc, Slots s) { cudaMemsetAsync(&s.skin->dirty, 1, 1, lc.stream); }
 
 // whether a pass can use the group lists: the mixed form, and the FP64 form's fixed-point passes
 static bool has_lists(const LaunchCtx &lc, bool mixed) { return mixed || lc.fp; }
-// A pass with the group lists is followed by the skin's advance. A pass without them leaves the lists
-// behind the positions, so the next pass with them rebuilds them.
-void launch_lat_rho(const LaunchCtx &lc, const Geom &g, Slots s, Inter in, PotTables t, bool mixed, bool hook, bool lists) {
+// A pass with the group lists is followed by the skin's advance, which the caller launches (true: it is due). A
+// pass without them leaves the lists behind the positions, so the next pass with them rebuilds them.
+bool launch_lat_rho(const LaunchCtx &lc, const Geom &g, Slots s, Inter in, PotTables t, bool mixed, bool hook, bool lists) {
     const bool v = lists && has_lists(lc, mixed) && !hook && lists_ok(lc, g);
-    if (!mixed) launch_fix_records(lc, g, s);
     if (!launch_lat_rho_split(lc, g, s, in, t, mixed, hook, 0, g.n_local_half, v))
         launch_lat_rho_threads(lc, g, s, in, t, mixed, hook, 0, gather_threads(g, lc.rho_order), v);
-    if (v) launch_skin_advance(lc, s);
-    else if (has_lists(lc, mixed)) launch_skin_dirty(lc, s);
+    if (!v && has_lists(lc, mixed)) launch_skin_dirty(lc, s);
+    return v;
 }
 // thread range of the sites [u0, u1) of both parities (u0, u1 multiples of 32, or u1 = n_local_half)
 static void site_threads(const Geom &g, int order, int u0, int u1, int tb[2], int te[2], int &nr) {
@@ -1627,33 +1596,36 @@ void launch_lat_rho_sites(const LaunchCtx &lc, const Geom &g, Slots s, Inter in,
     if (!v && has_lists(lc, mixed)) launch_skin_dirty(lc, s);  // the caller advances the skin after the last slab
 }
 
-// dF/drho when inter atoms added density after the lattice pass (or for the df hook)
+// dF/drho of a lattice slot from its density
 template <bool MIXED>
-__global__ void k_lat_df(Geom g, Slots s, Inter in, PotTables pt, bool hook, FixParams fp) {
-    if (!hook && lattice_only(in)) return;  // already fused into the density pass
-    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < g.n_local; t += gridDim.x * blockDim.x) {
-        int i, j, k;
-        const int sl = local_slot(g, t, i, j, k);
-        const int ti = s.type[sl];
-        if (ti < 0) continue;
-        if (MIXED) {
-            int m; float p;
-            locate_f((float) s.rho[sl], pt.inv_drho_f, pt.nrho, m, p);
-            s.df32[sidx(g, sl)] = der_f(pt.F_dff + ti * pt.nrho, m, p);
-        } else {
-            int m; double p;
-            locate_d(s.rho[sl], pt.inv_drho, pt.nrho, m, p);
-            const double df = der_d(pt.F_d + ti * pt.nrho, m, p);
-            s.df[sl] = df;
-            if (fp.on) s.dfq[sidx(g, sl)] = fix_df(fp, df);
-        }
+__device__ __forceinline__ void lat_df_one(const Geom &g, const Slots &s, const PotTables &pt, const FixParams &fp, int sl, int ti,
+                                           double rho) {
+    if (MIXED) {
+        int m; float p;
+        locate_f((float) rho, pt.inv_drho_f, pt.nrho, m, p);
+        s.df32[sidx(g, sl)] = der_f(pt.F_dff + ti * pt.nrho, m, p);
+    } else {
+        int m; double p;
+        locate_d(rho, pt.inv_drho, pt.nrho, m, p);
+        const double df = der_d(pt.F_d + ti * pt.nrho, m, p);
+        s.df[sl] = df;
+        if (fp.on) s.dfq[sidx(g, sl)] = fix_df(fp, df);
     }
 }
-void launch_lat_df(const LaunchCtx &lc, const Geom &g, Slots s, Inter in, PotTables t, bool mixed, bool hook) {
-    const int b = 256;
-    const int n = hook ? (g.n_local + b - 1) / b : std::max(1, std::min(lc.num_sms * 8, (g.n_local + b - 1) / b));
-    if (mixed) k_lat_df<true><<<n, b, 0, lc.stream>>>(g, s, in, t, hook, FixParams{});
-    else k_lat_df<false><<<n, b, 0, lc.stream>>>(g, s, in, t, hook, fix_params(lc));
+// the df hook: every lattice slot
+template <bool MIXED>
+__global__ void k_lat_df(Geom g, Slots s, PotTables pt, FixParams fp) {
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= g.n_local) return;
+    int i, j, k;
+    const int sl = local_slot(g, t, i, j, k);
+    const int ti = s.type[sl];
+    if (ti >= 0) lat_df_one<MIXED>(g, s, pt, fp, sl, ti, s.rho[sl]);
+}
+void launch_lat_df(const LaunchCtx &lc, const Geom &g, Slots s, PotTables t, bool mixed) {
+    const int b = 256, n = (g.n_local + b - 1) / b;
+    if (mixed) k_lat_df<true><<<n, b, 0, lc.stream>>>(g, s, t, FixParams{});
+    else k_lat_df<false><<<n, b, 0, lc.stream>>>(g, s, t, fix_params(lc));
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -1722,7 +1694,7 @@ __device__ __forceinline__ void force_atom_fp64(const NeighTables &nt, const Geo
 __device__ __forceinline__ void force_done_fp64(const Slots &s, const Inter &in, StepParams *sp, int sl, int ti, double fx,
                                                 double fy, double fz, bool kick, bool hook) {
     s.fx[sl] = fx; s.fy[sl] = fy; s.fz[sl] = fz;
-    if (kick && !hook && kick_in_lattice_pass(in, sl)) {
+    if (kick && !hook && untouched(in, sl)) {
         const double c = dt_inv_m_of(sp, ti);
         const double vx = __dadd_rn(s.vx[sl], __dmul_rn(c, fx));
         const double vy = __dadd_rn(s.vy[sl], __dmul_rn(c, fy));
@@ -1990,7 +1962,7 @@ __device__ __forceinline__ void force_done_mixed(const Geom &g, const Slots &s, 
     // a fused body's forces are used only in registers: the next body's firststep is taken here, and
     // the last body of a graph (never fused) stores the forces the state keeps between launches
     if (!fused) { s.fx[sl] = fx; s.fy[sl] = fy; s.fz[sl] = fz; }
-    if (kick && !hook && kick_in_lattice_pass(in, sl)) {
+    if (kick && !hook && untouched(in, sl)) {
         const double c = dt_inv_m_of(sp, ti);
         const double vx = __dadd_rn(s.vx[sl], __dmul_rn(c, fx));
         const double vy = __dadd_rn(s.vy[sl], __dmul_rn(c, fy));
@@ -2007,14 +1979,10 @@ __device__ __forceinline__ void force_done_mixed(const Geom &g, const Slots &s, 
         }
     }
 }
-// a vacant site: no force, and in a fused body the next firststep's flag and record of a vacancy
+// a vacant site: no force, and in a fused body the next firststep's record of a vacancy
 __device__ __forceinline__ void force_vacant_mixed(const Geom &g, const Slots &s, const Inter &in, int sl, int si, bool fuse_next) {
     s.fx[sl] = 0.0; s.fy[sl] = 0.0; s.fz[sl] = 0.0;
-    if (fuse_next && lattice_only(in)) {
-        int i, j, k;
-        in.dflag[local_index_of(g, sl, i, j, k)] = 0;
-        s.u4n[si] = vacant_u4();
-    }
+    if (fuse_next && lattice_only(in)) s.u4n[si] = vacant_u4();
 }
 __device__ __forceinline__ void k_lat_force_mixed_site(int t, const NeighTables &nt, const Geom &g, const Slots &s, const Inter &in,
                                                 const PotTables &pt, StepParams *sp, bool kick, bool hook, int order,
@@ -2215,9 +2183,9 @@ static void launch_force_split_w(const LaunchCtx &lc, const Geom &g, Slots s, In
                                  bool hook, int u0, int u1, bool fuse_next, bool lists) {
     const int n = split_groups(u0, u1);
     if (mixed)
-        k_lat_force_mixed_split<W><<<n, 32 * W, 0, lc.stream>>>(lc.cand, lc.nt->npruned, lc.nt->nfull, g, s, in, t, p, kick, hook, u0, u1,
+        k_lat_force_mixed_split<W><<<n, 32 * W, 0, lc.stream>>>(&lc.ntd->cand[0][0], lc.nt->npruned, lc.nt->nfull, g, s, in, t, p, kick, hook, u0, u1,
                                                                 fuse_next && kick && !hook, lists);
-    else k_lat_force_fix_split<W><<<n, 32 * W, 0, lc.stream>>>(*lc.nt, lc.cand, g, s, in, t, *lc.fp, p, kick, hook, u0, u1, lists);
+    else k_lat_force_fix_split<W><<<n, 32 * W, 0, lc.stream>>>(*lc.nt, &lc.ntd->cand[0][0], g, s, in, t, *lc.fp, p, kick, hook, u0, u1, lists);
 }
 static bool launch_lat_force_split(const LaunchCtx &lc, const Geom &g, Slots s, Inter in, PotTables t, StepParams *p, bool kick, bool mixed,
                                    bool hook, int u0, int u1, bool fuse_next, bool lists) {
@@ -2245,30 +2213,10 @@ void launch_lat_force_sites(const LaunchCtx &lc, const Geom &g, Slots s, Inter i
     for (int r = 0; r < nr; r++) launch_lat_force_threads(lc, g, s, in, t, p, kick, mixed, false, tb[r], te[r], false, v);
 }
 
-// second half-kick for lattice slots (only when inter atoms prevented fusion, or always) and for
-// inter atoms (src/newton_motion.cpp:57-74)
-__global__ void k_secondstep(Geom g, Slots s, Inter in, StepParams *p, int lattice_mode) {
+// NewtonMotion::secondstep for the inter atoms (src/newton_motion.cpp:57-74)
+__device__ __forceinline__ void inter_secondstep(const Inter &in, StepParams *p, int t0, int stride) {
     const int n_inter = in.cnt[CNT_INTER];
-    // mode 2 (after a kicking force pass): the lattice atoms were kicked by the lattice force pass or,
-    // for the owners of inter-atom pairs, by the owner gather; inter atoms only
-    const bool lattice = lattice_mode == 1;
-    const int stride = gridDim.x * blockDim.x;
-    const int t0 = blockIdx.x * blockDim.x + threadIdx.x;
     double v2max = 0.0;
-    if (lattice) {
-        for (int t = t0; t < g.n_local; t += stride) {
-            int i, j, k;
-            const int sl = local_slot(g, t, i, j, k);
-            const int ty = s.type[sl];
-            if (ty < 0) continue;
-            const double c = dt_inv_m_of(p, ty);
-            const double vx = __dadd_rn(s.vx[sl], __dmul_rn(c, s.fx[sl]));
-            const double vy = __dadd_rn(s.vy[sl], __dmul_rn(c, s.fy[sl]));
-            const double vz = __dadd_rn(s.vz[sl], __dmul_rn(c, s.fz[sl]));
-            s.vx[sl] = vx; s.vy[sl] = vy; s.vz[sl] = vz;
-            v2max = fmax(v2max, speed2(vx, vy, vz));
-        }
-    }
     for (int a = t0; a < n_inter; a += stride) {
         const double c = dt_inv_m_of(p, in.type[a]);
         const double vx = __dadd_rn(in.vx[a], __dmul_rn(c, in.fx[a]));
@@ -2279,13 +2227,34 @@ __global__ void k_secondstep(Geom g, Slots s, Inter in, StepParams *p, int latti
     }
     if (v2max > 0.0) note_vmax2(p, v2max);
 }
+// the second half-kick as a phase of its own: lattice atoms and inter atoms (after a kicking force pass, that pass
+// and the owner gather have taken it)
+__global__ void k_secondstep(Geom g, Slots s, Inter in, StepParams *p) {
+    const int stride = gridDim.x * blockDim.x;
+    const int t0 = blockIdx.x * blockDim.x + threadIdx.x;
+    double v2max = 0.0;
+    for (int t = t0; t < g.n_local; t += stride) {
+        int i, j, k;
+        const int sl = local_slot(g, t, i, j, k);
+        const int ty = s.type[sl];
+        if (ty < 0) continue;
+        const double c = dt_inv_m_of(p, ty);
+        const double vx = __dadd_rn(s.vx[sl], __dmul_rn(c, s.fx[sl]));
+        const double vy = __dadd_rn(s.vy[sl], __dmul_rn(c, s.fy[sl]));
+        const double vz = __dadd_rn(s.vz[sl], __dmul_rn(c, s.fz[sl]));
+        s.vx[sl] = vx; s.vy[sl] = vy; s.vz[sl] = vz;
+        v2max = fmax(v2max, speed2(vx, vy, vz));
+    }
+    if (v2max > 0.0) note_vmax2(p, v2max);
+    inter_secondstep(in, p, t0, stride);
+}
 // grid-stride kernels that often have nothing to do: a grid no larger than the box needs, so a
 // small box does not schedule a thousand idle blocks every step
 inline int box_grid(const LaunchCtx &lc, const Geom &g, int per_sm, int threads) {
     return std::max(1, std::min(lc.num_sms * per_sm, (g.n_local + threads - 1) / threads));
 }
-void launch_secondstep(const LaunchCtx &lc, const Geom &g, Slots s, Inter in, StepParams *p, bool lattice) {
-    k_secondstep<<<box_grid(lc, g, 8, 256), 256, 0, lc.stream>>>(g, s, in, p, lattice ? 1 : 2);
+void launch_secondstep(const LaunchCtx &lc, const Geom &g, Slots s, Inter in, StepParams *p) {
+    k_secondstep<<<box_grid(lc, g, 8, 256), 256, 0, lc.stream>>>(g, s, in, p);
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -2452,18 +2421,6 @@ void launch_energy(const LaunchCtx &lc, const Geom &g, Slots s, Inter in, PotTab
 // owner of a ghost slot in i's neighbourhood, so it is marked too.) Clearing writes 0 over the same
 // slots of the old list. Work item e of a flat loop covers (far atom e / (nfull + 1), entry).
 // ------------------------------------------------------------------------------------------------
-__device__ void mark_far_neighbourhoods(const NeighTables &nt, const Geom &g, const Inter &in, int a0, int a1, int8_t v, int t0,
-                                        int stride) {
-    const int per = nt.nfull + 1;
-    const int total = (a1 - a0) * per;
-    for (int e = t0; e < total; e += stride) {
-        const int sl = in.far_list[a0 + e / per];
-        const int q = e % per;
-        const int par = (sl % g.Sx) & 1;
-        const int sj = q == nt.nfull ? sl : sl + (par ? nt.lat[1][q] : nt.lat[0][q]);
-        in.far_flag[owner_slot(g, sj)] = v;
-    }
-}
 
 // ------------------------------------------------------------------------------------------------
 // Inter-atom list management: one block, so the reference's list order is kept exactly.
@@ -2543,6 +2500,66 @@ __device__ void block_bitonic_sort_smem(long long *buf, int n, long long *sm) {
     __syncthreads();
 }
 
+// The displaced list's local indices in increasing order (the second half of in.displaced), n of them. Up to
+// 1024: each thread counts the smaller ones. More: kDispBuckets equal ranges of the local indices, each entry
+// counts the smaller ones of its range; a range holds a handful (a cascade's displaced atoms spread over its
+// rows). sm: kDispBuckets + 1024 ints.
+constexpr int kDispBuckets = 4096;
+__device__ const int *block_sort_displaced(const Geom &g, const Inter &in, int n, int *sm) {
+    int *out = in.displaced + in.dcap;
+    const int tid = threadIdx.x, nthr = blockDim.x;
+    if (n <= 1024) {
+        for (int e = tid; e < n; e += nthr) sm[e] = in.displaced[e];
+        __syncthreads();
+        for (int e = tid; e < n; e += nthr) {
+            const int t = sm[e];
+            int r = 0;
+            for (int q = 0; q < n; q++) r += sm[q] < t;
+            out[r] = t;
+        }
+        __syncthreads();
+        return out;
+    }
+    int *first = sm, *tot = sm + kDispBuckets;  // first entry of each bucket; the threads' sums
+    const int per = g.n_local / kDispBuckets + 1, own = kDispBuckets / nthr;  // own buckets a thread scans
+    for (int b = tid; b < kDispBuckets; b += nthr) first[b] = 0;
+    __syncthreads();
+    for (int e = tid; e < n; e += nthr) atomicAdd(&first[in.displaced[e] / per], 1);
+    __syncthreads();
+    int v = 0;
+    for (int b = own * tid; b < own * tid + own; b++) v += first[b];
+    tot[tid] = v;
+    __syncthreads();
+    for (int o = 1; o < nthr; o <<= 1) {
+        const int y = tid >= o ? tot[tid - o] : 0;
+        __syncthreads();
+        tot[tid] += y;
+        __syncthreads();
+    }
+    int run = tot[tid] - v;
+    for (int b = own * tid; b < own * tid + own; b++) {
+        const int c = first[b];
+        first[b] = run;
+        run += c;
+    }
+    __syncthreads();
+    // into the buckets, leaving each one's end in first (the bucket index is made after decide, so its keys are free)
+    int *part = reinterpret_cast<int *>(in.bucket);
+    for (int e = tid; e < n; e += nthr) {
+        const int t = in.displaced[e];
+        part[atomicAdd(&first[t / per], 1)] = t;
+    }
+    __syncthreads();
+    for (int e = tid; e < n; e += nthr) {
+        const int t = part[e], b = t / per, b0 = b ? first[b - 1] : 0, b1 = first[b];
+        int r = b0;
+        for (int q = b0; q < b1; q++) r += part[q] < t;
+        out[r] = t;
+    }
+    __syncthreads();
+    return out;
+}
+
 // inter record move helpers (scratch layout: 13 doubles per record)
 __device__ __forceinline__ void inter_save(const Inter &in, int a, int dst) {
     double *d = in.scratch_d + 13 * dst;
@@ -2609,7 +2626,8 @@ __device__ __forceinline__ void border_put(Inter &in, int q, const double p3[3],
     in.gdf[q] = 0.0;
 }
 
-__global__ void __launch_bounds__(kManageThreads) k_inter_manage(const __grid_constant__ NeighTables nt, Geom g, Slots s, Inter in, int mask, bool mixed) {
+__global__ void __launch_bounds__(kManageThreads) k_inter_manage(Geom g, Slots s, Inter in, int mask, bool mixed) {
+    extern __shared__ long long sm_keys[];
     const int tid = threadIdx.x, nthr = blockDim.x;
 
     // The list counts are read once, by all threads before any is written, and then followed in
@@ -2640,15 +2658,17 @@ __global__ void __launch_bounds__(kManageThreads) k_inter_manage(const __grid_co
         // the far list of the previous step is void (its marks were cleared before this kernel)
         if (tid == 0) in.cnt[CNT_FAR] = 0;
         __syncthreads();
-        // (i) displaced lattice atoms join the list in scan order (the collected list is ordered)
+        // (i) displaced lattice atoms join the list in scan order
         int nd = n_disp;
-        if (nd > in.dcap) nd = in.dcap;
+        if (nd > in.dcap) { if (tid == 0) set_error(in, MG_DEVERR_DISPLACED_OVERFLOW); nd = in.dcap; }
+        const int *order = block_sort_displaced(g, in, nd, reinterpret_cast<int *>(sm_keys));
         const int n0 = n_inter;
         if (nd > 0) {
             int room = in.cap - n0;
             if (nd > room) { if (tid == 0) set_error(in, MG_DEVERR_INTER_OVERFLOW); nd = room; }
             for (int q = tid; q < nd; q += nthr) {
-                const int sl = in.displaced[q];
+                int i, j, k;
+                const int sl = local_slot(g, order[q], i, j, k);
                 const int a = n0 + q;
                 in.id[a] = s.id[sl];
                 in.type[a] = s.type[sl];
@@ -2869,7 +2889,6 @@ __global__ void __launch_bounds__(kManageThreads) k_inter_manage(const __grid_co
             in.bucket[e] = (key << 32) | (long long) ref;
         }
         __syncthreads();
-        extern __shared__ long long sm_keys[];
         if (total <= kSortSmemKeys) block_bitonic_sort_smem(in.bucket, total, sm_keys);
         else block_bitonic_sort(in.bucket, total);
         if (tid == 0) *in.n_bucket = total;
@@ -2882,7 +2901,7 @@ void configure_manage_kernel() {
                          static_cast<int>(kSortSmemKeys * sizeof(long long)));
 }
 void launch_inter_manage(const LaunchCtx &lc, const Geom &g, Slots s, Inter in, int mask, bool mixed) {
-    k_inter_manage<<<1, kManageThreads, kSortSmemKeys * sizeof(long long), lc.stream>>>(*lc.nt, g, s, in, mask, mixed);
+    k_inter_manage<<<1, kManageThreads, kSortSmemKeys * sizeof(long long), lc.stream>>>(g, s, in, mask, mixed);
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -2972,7 +2991,7 @@ __device__ __forceinline__ bool is_local_slot(const Geom &g, int sl) {
     return X >= g.gx && X < g.gx + g.bx && Y >= g.gy && Y < g.gy + g.by && Z >= g.gz && Z < g.gz + g.bz;
 }
 template <int KIND>
-__global__ void __launch_bounds__(kInterThreads) k_inter_eam(const __grid_constant__ NeighTables nt, Geom g, Slots s, Inter in, PotTables pt, bool mixed) {
+__global__ void __launch_bounds__(kInterThreads) k_inter_eam(const NeighTables *__restrict__ ntd, Geom g, Slots s, Inter in, PotTables pt, bool mixed) {
     const int n = in.cnt[CNT_INTER];
     const int nb = *in.n_bucket;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -2987,9 +3006,9 @@ __global__ void __launch_bounds__(kInterThreads) k_inter_eam(const __grid_consta
         double acc = 0.0, fx = 0.0, fy = 0.0, fz = 0.0;
         // lattice partners: the nearest site's atom, then the full offsets of that site
         const int par = (near % g.Sx) & 1;
-        const int nf = nt.nfull;
+        const int nf = ntd->nfull;
         for (int q = (int) threadIdx.x - 1; q < nf; q += kInterThreads) {
-            const int sj = q < 0 ? near : near + (par ? nt.full[1][q] : nt.full[0][q]);
+            const int sj = q < 0 ? near : near + ntd->full[par][q];
             if (sj < 0 || sj >= g.n_slots) { set_error(in, MG_DEVERR_OUT_OF_GRID); continue; }
             const int tj = s.type[sj];
             if (tj < 0) continue;
@@ -3008,7 +3027,7 @@ __global__ void __launch_bounds__(kInterThreads) k_inter_eam(const __grid_consta
         }
         // inter partners: same-site bucket (not itself), then the buckets of the full offsets
         for (int q = (int) threadIdx.x - 1; q < nf; q += kInterThreads) {
-            const int key = q < 0 ? near : near + (par ? nt.full[1][q] : nt.full[0][q]);
+            const int key = q < 0 ? near : near + ntd->full[par][q];
             for (int b = bucket_begin(in, nb, key); b < nb && (int) (in.bucket[b] >> 32) == key; b++) {
                 const InterRef o = inter_ref(in, (int) (in.bucket[b] & 0xffffffffLL));
                 if (q < 0 && o.id == ida) continue;
@@ -3070,8 +3089,9 @@ __global__ void __launch_bounds__(kInterThreads) k_inter_eam(const __grid_consta
 // inter-atom pass. The last block to finish resets the list for the next pass; the bits are clear by
 // then.
 template <int KIND>
-__global__ void __launch_bounds__(128) k_inter_owner(const __grid_constant__ NeighTables nt, Geom g, Slots s, Inter in, PotTables pt, bool mixed,
-                                                     StepParams *sp, bool kick) {
+__global__ void __launch_bounds__(128) k_inter_owner(const NeighTables *__restrict__ ntd, Geom g, Slots s, Inter in, PotTables pt, bool mixed,
+                                                     FixParams fp, StepParams *sp, bool kick) {
+    if (KIND == 1 && kick) inter_secondstep(in, sp, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
     const int n = min(in.cnt[CNT_TOUCHED], in.tcap);
     if (n == 0) return;  // nothing listed: no block writes, so no reset is due
     const int nb = *in.n_bucket;
@@ -3083,11 +3103,11 @@ __global__ void __launch_bounds__(128) k_inter_owner(const __grid_constant__ Nei
         const double xj = s.x[j], yj = s.y[j], zj = s.z[j];
         const double dfj = KIND == 1 ? lat_df(g, s, j, mixed) : 0.0;
         const int par = (j % g.Sx) & 1;
-        const int nf = nt.nfull;
+        const int nf = ntd->nfull;
         double acc = 0.0, fx = 0.0, fy = 0.0, fz = 0.0;
         if (tj >= 0) {
             for (int q = lane - 1; q < nf; q += 32) {
-                const int key = q < 0 ? j : j + (par ? nt.full[1][q] : nt.full[0][q]);
+                const int key = q < 0 ? j : j + ntd->full[par][q];
                 for (int b = bucket_begin(in, nb, key); b < nb && (int) (in.bucket[b] >> 32) == key; b++) {
                     const int ref = (int) (in.bucket[b] & 0xffffffffLL);
                     if (ref < in.cap && !is_local_slot(g, key)) continue;
@@ -3115,8 +3135,12 @@ __global__ void __launch_bounds__(128) k_inter_owner(const __grid_constant__ Nei
         }
         if (lane == 0) {
             if (tj >= 0) {
-                if (KIND == 0) s.rho[j] += acc;
-                else if (KIND == 1) {
+                if (KIND == 0) {  // and the F' that the density pass left to this owner
+                    const double rho = s.rho[j] + acc;
+                    s.rho[j] = rho;
+                    if (mixed) lat_df_one<true>(g, s, pt, fp, j, tj, rho);
+                    else lat_df_one<false>(g, s, pt, fp, j, tj, rho);
+                } else if (KIND == 1) {
                     const double f0 = s.fx[j] + fx, f1 = s.fy[j] + fy, f2v = s.fz[j] + fz;
                     s.fx[j] = f0; s.fy[j] = f1; s.fz[j] = f2v;
                     if (kick) {  // the second half-kick the lattice force pass left to this owner
@@ -3147,28 +3171,36 @@ __global__ void __launch_bounds__(128) k_inter_owner(const __grid_constant__ Nei
     }
 }
 template <int KIND>
-void launch_inter_kind(const LaunchCtx &lc, const Geom &g, Slots s, Inter in, PotTables t, bool mixed, StepParams *sp = nullptr,
-                       bool kick = false) {
-    k_inter_eam<KIND><<<lc.num_sms * 4, kInterThreads, 0, lc.stream>>>(*lc.nt, g, s, in, t, mixed);
-    k_inter_owner<KIND><<<lc.num_sms * 4, 128, 0, lc.stream>>>(*lc.nt, g, s, in, t, mixed, sp, kick);
+void launch_inter_eam(const LaunchCtx &lc, const Geom &g, Slots s, Inter in, PotTables t, bool mixed) {
+    k_inter_eam<KIND><<<lc.num_sms * 4, kInterThreads, 0, lc.stream>>>(lc.ntd, g, s, in, t, mixed);
+}
+template <int KIND>
+void launch_inter_owner(const LaunchCtx &lc, const Geom &g, Slots s, Inter in, PotTables t, bool mixed, StepParams *sp = nullptr,
+                        bool kick = false) {
+    k_inter_owner<KIND><<<lc.num_sms * 4, 128, 0, lc.stream>>>(lc.ntd, g, s, in, t, mixed, fix_params(lc), sp, kick);
 }
 void launch_inter_rho(const LaunchCtx &lc, const Geom &g, Slots s, Inter in, PotTables t, bool mixed) {
-    launch_inter_kind<0>(lc, g, s, in, t, mixed);
+    launch_inter_eam<0>(lc, g, s, in, t, mixed);
+}
+void launch_inter_rho_owners(const LaunchCtx &lc, const Geom &g, Slots s, Inter in, PotTables t, bool mixed) {
+    launch_inter_owner<0>(lc, g, s, in, t, mixed);
 }
 void launch_inter_force(const LaunchCtx &lc, const Geom &g, Slots s, Inter in, PotTables t, bool mixed, StepParams *sp, bool kick) {
-    launch_inter_kind<1>(lc, g, s, in, t, mixed, sp, kick);
+    launch_inter_eam<1>(lc, g, s, in, t, mixed);
+    launch_inter_owner<1>(lc, g, s, in, t, mixed, sp, kick);
 }
 void launch_inter_energy(const LaunchCtx &lc, const Geom &g, Slots s, Inter in, PotTables t, bool mixed) {
-    launch_inter_kind<2>(lc, g, s, in, t, mixed);
+    launch_inter_eam<2>(lc, g, s, in, t, mixed);
+    launch_inter_owner<2>(lc, g, s, in, t, mixed);
 }
 
 // ------------------------------------------------------------------------------------------------
 // far lattice atoms (farther than 0.2 a0 from their site). Rebuild from positions for states that did
 // not come through atom::decide (uploads, the per-phase hooks).
 // ------------------------------------------------------------------------------------------------
-__global__ void k_far_clear(const __grid_constant__ NeighTables nt, Geom g, Inter in) {
+__global__ void k_far_clear(const NeighTables *nt, Geom g, Inter in) {
     const int nf = min(in.cnt[CNT_FAR], in.fcap);
-    mark_far_neighbourhoods(nt, g, in, 0, nf, 0, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
+    mark_far_neighbourhoods(*nt, g, in, 0, nf, 0, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
 }
 __global__ void k_far_count_reset(Inter in) { in.cnt[CNT_FAR] = 0; }
 __global__ void k_far_scan(Geom g, Slots s, Inter in) {
@@ -3183,15 +3215,15 @@ __global__ void k_far_scan(Geom g, Slots s, Inter in) {
         else set_error(in, MG_DEVERR_DISPLACED_OVERFLOW);
     }
 }
-__global__ void k_far_mark(const __grid_constant__ NeighTables nt, Geom g, Inter in) {
+__global__ void k_far_mark(const NeighTables *nt, Geom g, Inter in) {
     const int nf = min(in.cnt[CNT_FAR], in.fcap);
-    mark_far_neighbourhoods(nt, g, in, 0, nf, 1, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
+    mark_far_neighbourhoods(*nt, g, in, 0, nf, 1, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
 }
 void launch_far_clear(const LaunchCtx &lc, const Geom &g, Inter in) {
-    k_far_clear<<<lc.num_sms * 4, 256, 0, lc.stream>>>(*lc.nt, g, in);
+    k_far_clear<<<lc.num_sms * 4, 256, 0, lc.stream>>>(lc.ntd, g, in);
 }
 void launch_far_mark(const LaunchCtx &lc, const Geom &g, Inter in) {
-    k_far_mark<<<lc.num_sms * 4, 256, 0, lc.stream>>>(*lc.nt, g, in);
+    k_far_mark<<<lc.num_sms * 4, 256, 0, lc.stream>>>(lc.ntd, g, in);
 }
 void launch_far_rebuild(const LaunchCtx &lc, const Geom &g, Slots s, Inter in) {
     launch_far_clear(lc, g, in);
@@ -3219,10 +3251,15 @@ __global__ void k_spec_begin(Inter in) {
 }
 void launch_spec_begin(const LaunchCtx &lc, Inter in) { k_spec_begin<<<1, 1, 0, lc.stream>>>(in); }
 
-__global__ void k_spec_decide(const __grid_constant__ NeighTables nt, Geom g, Slots s, Inter in, int t0, int t1) {
-    if (in.cnt[CNT_DISP_RAW] == 0) return;  // nothing displaced so far this step
-    for (int t = t0 + blockIdx.x * blockDim.x + threadIdx.x; t < t1; t += gridDim.x * blockDim.x) {
-        if (!in.dflag[t]) continue;
+__global__ void k_spec_decide(const NeighTables *nt, Geom g, Slots s, Inter in, int t0, int t1) {
+    const int n = in.cnt[CNT_DISPLACED];  // displaced so far this step (usually none)
+    if (n > in.dcap) {
+        in.cnt[CNT_SPEC_VOID] = 1;
+        return;
+    }
+    for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < n; e += gridDim.x * blockDim.x) {
+        const int t = in.displaced[e];
+        if (t < t0 || t >= t1) continue;  // an earlier chunk's
         int i, j, k;
         const int sl = local_slot(g, t, i, j, k);
         const double x = s.x[sl], y = s.y[sl], z = s.z[sl];
@@ -3239,13 +3276,12 @@ __global__ void k_spec_decide(const __grid_constant__ NeighTables nt, Geom g, Sl
         site_of(g, i + g.gx, j + g.gy, k + g.gz, xs, ys, zs);
         s.u4[sidx(g, sl)] = make_u4(g, x, y, z, xs, ys, zs, s.type[sl]);
         in.far_list[q] = sl;
-        mark_far_neighbourhoods(nt, g, in, q, q + 1, 1, 0, 1);
+        mark_far_neighbourhoods(*nt, g, in, q, q + 1, 1, 0, 1);
     }
 }
 void launch_spec_decide(const LaunchCtx &lc, const Geom &g, Slots s, Inter in, int t0, int t1) {
     if (t1 <= t0) return;
-    const int b = 256, n = std::min((t1 - t0 + b - 1) / b, lc.num_sms * 4);
-    k_spec_decide<<<n, b, 0, lc.stream>>>(*lc.nt, g, s, in, t0, t1);
+    k_spec_decide<<<8, 256, 0, lc.stream>>>(lc.ntd, g, s, in, t0, t1);
 }
 
 
