@@ -1060,6 +1060,7 @@ __global__ void __launch_bounds__(512, 4) k_lat_rho_mixed(const __grid_constant_
 // goes through memory.
 // ------------------------------------------------------------------------------------------------
 constexpr int kSplitSegment = 32 * kListWords;  // candidates listed at a time
+constexpr int kSplitAhead = 2;                  // candidates of a stream whose loads are in flight together
 struct SplitList {
     unsigned words[kListWords];
     float4 rec[kSplitSegment];                  // the listed candidates' records, in candidate order
@@ -1152,7 +1153,7 @@ struct SplitLane {
     }
 };
 
-// Density, mixed form (500 groups: 26 -> 12 us).
+// Density, mixed form (500 groups: 26 -> 9 us).
 template <int W>
 __device__ __forceinline__ void rho_mixed_split(const float4 *cand, int np, int nf, const Geom &g, const Slots &s, const Inter &in,
                                                 const PotTables &pt, const SplitSite &a, bool hook, bool lists, bool full, bool far,
@@ -1171,19 +1172,29 @@ __device__ __forceinline__ void rho_mixed_split(const float4 *cand, int np, int 
         const int n = split_list<W>(cand, s, a, !tail || far, q0, q1, list ? g.rcs2_h : g.rc2_h, full ? nullptr : list, sh);
         if (full && list && threadIdx.x < kListWords) list[threadIdx.x] = sh.words[threadIdx.x];
         const bool mine = !tail || b_far;
-#pragma unroll 2
-        for (int c0 = 0; c0 < n; c0 += W) {
-            const float4 D = sh.rec[min(c0 + b.stream, n - 1)];
-            const float4 uj = __ldg(s.u4 + b.si + (b.in ? __float_as_int(D.w) : 0));
-            f2 dxy; float dz;
-            const float r2 = pair_r2(b.uixy, b.uiz, D, uj, dxy, dz);
-            // outside the cutoff the knot stays on the table, and its value is not used
-            const float v = rho_term_mixed(pt, r2, max(__float_as_int(uj.w), 0));
-            const float t = c0 + b.stream < n && mine && r2 < g.rc2_h ? v : __uint_as_float(kSplitNone);
+        for (int c0 = 0; c0 < n; c0 += kSplitAhead * W) {
+            float r2[kSplitAhead], t[kSplitAhead];
+            int tj[kSplitAhead];
 #pragma unroll
-            for (int k = 0; k < W; k++) {
-                const float tk = __shfl_sync(0xffffffffu, t, P * k + lane % P);
-                if (!split_none(tk)) kahan(sum, comp, tk);
+            for (int u = 0; u < kSplitAhead; u++) {
+                const float4 D = sh.rec[min(c0 + u * W + b.stream, n - 1)];
+                const float4 uj = __ldg(s.u4 + b.si + (b.in ? __float_as_int(D.w) : 0));
+                f2 dxy; float dz;
+                r2[u] = pair_r2(b.uixy, b.uiz, D, uj, dxy, dz);
+                tj[u] = max(__float_as_int(uj.w), 0);
+            }
+            // outside the cutoff the knot stays on the table, and the value is not used
+#pragma unroll
+            for (int u = 0; u < kSplitAhead; u++) t[u] = rho_term_mixed(pt, r2[u], tj[u]);
+#pragma unroll
+            for (int u = 0; u < kSplitAhead; u++) {
+                if (c0 + u * W >= n) break;
+                const float v = c0 + u * W + b.stream < n && mine && r2[u] < g.rc2_h ? t[u] : __uint_as_float(kSplitNone);
+#pragma unroll
+                for (int k = 0; k < W; k++) {
+                    const float tk = __shfl_sync(0xffffffffu, v, P * k + lane % P);
+                    if (!split_none(tk)) kahan(sum, comp, tk);
+                }
             }
         }
     }
@@ -1514,16 +1525,17 @@ bool lists_ok(const LaunchCtx &lc, const Geom &g) {
 // instructions (the mixed form's shuffles, and each warp's own start), so their number falls as the groups fill the
 // SMs; a batch counts a member's groups once for each member. Measured on 152 SMs, us per step with 8 / 4 / 2 /
 // no split warps:
-//   mixed  500 groups 56 / 57 / 68 / 84;  1098: 80 / 65 / 73 / 86;  2048: 113 / 91 / 81 / 85;  4000: - / 130 / 127 / 100
-//   FP64   500 groups 70 / 77 / 100 / 138;  1098: 98 / 92 / 107 / 138;  2048: 139 / 129 / 126 / 149;
-//          4000: 224 / 205 / 202 / 211;  7812: 387 / 343 / 339 / 328
+//   mixed  62 groups 37 / 42 / 52 / 70;  364: 51 / 44 / 53 / 73;  1098: 81 / 53 / 56 / 75;
+//          2048: 122 / 75 / 65 / 74;  2916: 164 / 99 / 99 / 80
+//   FP64   62 groups 52 / 63 / 88 / 123;  500: 60 / 67 / 90 / 126;  1098: 88 / 82 / 97 / 129;
+//          2916: 169 / 156 / 172 / 167;  5695: 285 / 254 / 254 / 267;  7812: 377 / 334 / 329 / 319
 static int split_groups(int u0, int u1) { return 2 * ((u1 - u0 + 31) / 32); }
 static int split_warps(const LaunchCtx &lc, bool mixed, int n) {
     if (!mixed && !lc.fp) return 0;
     const int64_t busy = static_cast<int64_t>(n) * lc.share / lc.num_sms;
-    if (busy < 4) return 8;
-    if (busy < (mixed ? 10 : 14)) return 4;
-    return busy < (mixed ? 14 : 28) ? 2 : 0;
+    if (busy < (mixed ? 2 : 4)) return 8;
+    if (busy < (mixed ? 8 : 22)) return 4;
+    return busy < (mixed ? 14 : 40) ? 2 : 0;
 }
 template <int W>
 static void launch_rho_split_w(const LaunchCtx &lc, const Geom &g, Slots s, Inter in, PotTables t, bool mixed, bool hook, int u0, int u1,
@@ -1886,22 +1898,32 @@ __device__ __forceinline__ void force_acc_add(ForceAcc &a, f2 dxy, float dz, flo
     a.sz = tz;
 }
 
-// fpair of one pair inside the cutoff (types ti and tj, F' dfi and dfj). Every rounding is spelled out, so
-// that each kernel that evaluates it gets the same bits.
-__device__ __forceinline__ float fpair_mixed(const Geom &g, const PotTables &pt, float r2, int ti, int tj, float dfi, float dfj) {
-    const PairKnot k = pair_knot(pt, r2);
-    // record {c0, d0, c1, d1, c2, d2, c3, 3 c3}: r*phi = c(p), rho_tj' = d(p), the last two steps of both in
-    // one packed Horner
-    float z[8];
-    ld_nc_v8(pt.zr8 + 8 * ((ti * 3 + tj) * pt.nr + k.m - kKnotBias), z);
-    const f2 pp = f2_pack(k.p, k.p);
-    f2 h = f2_fma(f2_pack(__fmaf_rn(z[6], k.p, z[4]), z[5]), pp, f2_pack(z[2], z[3]));
+// fpair of one pair inside the cutoff (types ti and tj, F' dfi and dfj): its table records, and its value
+// from them. Every rounding is spelled out, so that each kernel that evaluates it gets the same bits.
+struct PairRecord {
+    PairKnot k;
+    float z[8];  // {c0, d0, c1, d1, c2, d2, c3, 3 c3}: r*phi = c(p), rho_tj' = d(p)
+    float4 d;    // rho_ti' where the types differ
+};
+__device__ __forceinline__ PairRecord pair_record(const PotTables &pt, float r2, int ti, int tj) {
+    PairRecord r;
+    r.k = pair_knot(pt, r2);
+    ld_nc_v8(pt.zr8 + 8 * ((ti * 3 + tj) * pt.nr + r.k.m - kKnotBias), r.z);
+    if (tj != ti) r.d = __ldg(pt.rho_dff + ti * pt.nr + r.k.m - kKnotBias);
+    return r;
+}
+__device__ __forceinline__ float fpair_mixed(const Geom &g, const PotTables &pt, const PairRecord &r, int ti, int tj, float dfi,
+                                             float dfj) {
+    const float *z = r.z, p = r.k.p;
+    // the last two steps of both polynomials in one packed Horner
+    const f2 pp = f2_pack(p, p);
+    f2 h = f2_fma(f2_pack(__fmaf_rn(z[6], p, z[4]), z[5]), pp, f2_pack(z[2], z[3]));
     h = f2_fma(h, pp, f2_pack(z[0], z[1]));
     float zv, rhojp;
     f2_unpack(h, zv, rhojp);
-    const float zd = __fmaf_rn(__fmaf_rn(z[7], k.p, __fadd_rn(z[4], z[4])), k.p, z[2]);
-    const float rhoip = (tj == ti) ? rhojp : der_f(pt.rho_dff, ti * pt.nr + k.m - kKnotBias, k.p);
-    const float rinv = __fmul_rn(k.rinv, g.inv_h_f);
+    const float zd = __fmaf_rn(__fmaf_rn(z[7], p, __fadd_rn(z[4], z[4])), p, z[2]);
+    const float rhoip = (tj == ti) ? rhojp : __fmaf_rn(__fmaf_rn(r.d.z, p, r.d.y), p, r.d.x);
+    const float rinv = __fmul_rn(r.k.rinv, g.inv_h_f);
     const float dphi = __fmaf_rn(zd, pt.inv_dr_f, -__fmul_rn(zv, rinv));  // phi' r
     const float psip = __fmaf_rn(dphi, rinv, __fmaf_rn(dfi, rhojp, __fmul_rn(dfj, rhoip)));
     return __fmul_rn(-psip, rinv);
@@ -1915,7 +1937,10 @@ __device__ __forceinline__ void force_candidate(const NeighTables &nt, const Geo
     const float4 uj = __ldg(s.u4 + oj);
     f2 dxy; float dz;
     const float r2 = pair_r2(uixy, uiz, D, uj, dxy, dz);
-    if (r2 < g.rc2_h) force_acc_add(acc, dxy, dz, fpair_mixed(g, pt, r2, ti, __float_as_int(uj.w), dfi, __ldg(s.df32 + oj)));
+    if (r2 < g.rc2_h) {
+        const int tj = __float_as_int(uj.w);
+        force_acc_add(acc, dxy, dz, fpair_mixed(g, pt, pair_record(pt, r2, ti, tj), ti, tj, dfi, __ldg(s.df32 + oj)));
+    }
 }
 template <int PAR>
 __device__ __forceinline__ void force_sum_mixed(const NeighTables &nt, const Geom &g, const Slots &s, const PotTables &pt, int si, int ti,
@@ -2026,7 +2051,7 @@ __global__ void __launch_bounds__(512, 3) k_lat_force_mixed(const __grid_constan
         k_lat_force_mixed_site(t, nt, g, s, in, pt, sp, kick, hook, order, fuse_next, false);
 }
 
-// ---- the force passes of small boxes and thin slabs: see rho_mixed_split (500 groups: 30 -> 16 us; FP64 form 58 ->
+// ---- the force passes of small boxes and thin slabs: see rho_mixed_split (500 groups: 30 -> 14 us; FP64 form 58 ->
 // 19 us) ----
 template <int W>
 __device__ __forceinline__ void force_mixed_split(const float4 *cand, int np, int nf, const Geom &g, const Slots &s, const Inter &in,
@@ -2045,24 +2070,36 @@ __device__ __forceinline__ void force_mixed_split(const float4 *cand, int np, in
         q1 = min(q0 + kSplitSegment, tail ? end : np);
         const int n = split_list<W>(cand, s, a, !tail || far, q0, q1, g.rc2_h, lists && !tail ? group_list(g, s, a.par, a.u) : nullptr, sh);
         const bool mine = !tail || b_far;
-#pragma unroll 1
-        for (int c0 = 0; c0 < n; c0 += W) {
-            const float4 D = sh.rec[min(c0 + b.stream, n - 1)];
-            const int oj = b.si + (b.in ? __float_as_int(D.w) : 0);
-            const float4 uj = __ldg(s.u4 + oj);
-            const float dfj = __ldg(s.df32 + oj);
-            f2 dxy; float dz;
-            const float r2 = pair_r2(b.uixy, b.uiz, D, uj, dxy, dz);
-            const float v = fpair_mixed(g, pt, r2, b.ti, max(__float_as_int(uj.w), 0), dfi, dfj);
-            const float t = c0 + b.stream < n && mine && r2 < g.rc2_h ? v : __uint_as_float(kSplitNone);
-            float dx, dy;
-            f2_unpack(dxy, dx, dy);
+        for (int c0 = 0; c0 < n; c0 += kSplitAhead * W) {
+            float r2[kSplitAhead], dx[kSplitAhead], dy[kSplitAhead], dz[kSplitAhead], dfj[kSplitAhead], t[kSplitAhead];
+            int tj[kSplitAhead];
 #pragma unroll
-            for (int k = 0; k < W; k++) {
-                const int from = P * k + lane % P;
-                const float tk = __shfl_sync(0xffffffffu, t, from), xk = __shfl_sync(0xffffffffu, dx, from);
-                const float yk = __shfl_sync(0xffffffffu, dy, from), zk = __shfl_sync(0xffffffffu, dz, from);
-                if (!split_none(tk)) force_acc_add(acc, f2_pack(xk, yk), zk, tk);
+            for (int u = 0; u < kSplitAhead; u++) {
+                const float4 D = sh.rec[min(c0 + u * W + b.stream, n - 1)];
+                const int oj = b.si + (b.in ? __float_as_int(D.w) : 0);
+                const float4 uj = __ldg(s.u4 + oj);
+                dfj[u] = __ldg(s.df32 + oj);
+                f2 dxy;
+                r2[u] = pair_r2(b.uixy, b.uiz, D, uj, dxy, dz[u]);
+                f2_unpack(dxy, dx[u], dy[u]);
+                tj[u] = max(__float_as_int(uj.w), 0);
+            }
+            PairRecord r[kSplitAhead];
+#pragma unroll
+            for (int u = 0; u < kSplitAhead; u++) r[u] = pair_record(pt, r2[u], b.ti, tj[u]);
+#pragma unroll
+            for (int u = 0; u < kSplitAhead; u++) t[u] = fpair_mixed(g, pt, r[u], b.ti, tj[u], dfi, dfj[u]);
+#pragma unroll
+            for (int u = 0; u < kSplitAhead; u++) {
+                if (c0 + u * W >= n) break;
+                const float v = c0 + u * W + b.stream < n && mine && r2[u] < g.rc2_h ? t[u] : __uint_as_float(kSplitNone);
+#pragma unroll
+                for (int k = 0; k < W; k++) {
+                    const int from = P * k + lane % P;
+                    const float tk = __shfl_sync(0xffffffffu, v, from), xk = __shfl_sync(0xffffffffu, dx[u], from);
+                    const float yk = __shfl_sync(0xffffffffu, dy[u], from), zk = __shfl_sync(0xffffffffu, dz[u], from);
+                    if (!split_none(tk)) force_acc_add(acc, f2_pack(xk, yk), zk, tk);
+                }
             }
         }
     }

@@ -24,11 +24,11 @@ def _ctx(pkg, pot, cells, atoms, prec, kick=None):
     return ctx
 
 
-# 13x17x31: 430 groups of 32 sites, the last of each parity a short one; 24x25x27: 1014. On 152 SMs the members
-# make them run with 8, 4 and no split warps, and with 4, 2 (mixed) and no split warps.
+# 13x17x31: 430 groups of 32 sites, the last of each parity a short one; 9x10x14: 80; 24x25x27: 1014. On 152 SMs the
+# members make them run with every number of split warps and with none.
 @pytest.mark.parametrize("prec", ["fp64", "mixed"])
-@pytest.mark.parametrize("cells,members,kick", [((13, 17, 31), (3, 24), None), ((13, 17, 31), (3, 24), 400.0),
-                                                ((24, 25, 27), (2, 5), 800.0)])
+@pytest.mark.parametrize("cells,members,kick", [((9, 10, 14), (10,), None), ((13, 17, 31), (2, 4, 10, 24), None),
+                                                ((13, 17, 31), (4, 10, 24), 400.0), ((24, 25, 27), (2, 5, 7), 800.0)])
 def test_every_split_gives_the_same_bits(pkg, wl, potentials, gpu_lib, prec, cells, members, kick):
     pot = potentials["fecuni"]
     atoms = wl.build_state(cells, A0, RCF, temperature=600.0, seed=31, cu_frac=0.06, ni_frac=0.04)
