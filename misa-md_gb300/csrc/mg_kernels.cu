@@ -1312,6 +1312,35 @@ __device__ __noinline__ double rho_near_fp64(const NeighTables &nt, const Geom &
     return acc;
 }
 
+// U candidates (numbers q, at indices oj; those without `use` do not count) of the atom at (xb, yb, zb) (biased).
+// The pass waits for its loads and its chains of products, so U candidates go through each stage side by side,
+// and no branch stands between the stages: outside the cutoff the last interval is evaluated and nothing added.
+// For the split passes (us per step, one at a time -> two: 62 groups 50 -> 46, 5695 groups 255 -> 238); the
+// whole-group passes fill the SMs with warps and gain nothing (2M atoms: 2037 -> 2050).
+template <int U>
+__device__ __forceinline__ void rho_fix_pairs(const Slots &s, const FixParams &fp, const int (&oj)[U], const bool (&use)[U],
+                                              const int (&q)[U], i64 xb, i64 yb, i64 zb, i64 &acc, unsigned &near) {
+    FixRec j[U];
+    FixPoly rec[U];
+    FixCoord t[U];
+    bool in[U];
+#pragma unroll
+    for (int u = 0; u < U; u++) j[u] = ld_fix_rec(s.fix + oj[u]);
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+        const i64 r2 = fix_r2(fix_delta(xb - j[u].x, yb - j[u].y, zb - j[u].z), fp.b0);
+        in[u] = use[u] && (unsigned long long) (r2 - fp.lo) < (unsigned long long) (fp.rc2 - fp.lo);
+        if (use[u] && (unsigned long long) r2 < (unsigned long long) fp.lo) fix_note_near(near, q[u]);
+        int m;
+        t[u] = fix_locate(fp, in[u] ? r2 : fp.rc2 - 1, m);
+        rec[u] = ld_fix_poly(fp.rho + (in[u] ? (int) j[u].type : 0) * fp.nr1 + m);
+    }
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+        const i64 v = fix_poly(rec[u], t[u], fp.e3_rho);
+        acc += in[u] ? v : 0;
+    }
+}
 // candidate q, at index oj, of the atom at (xb, yb, zb) (biased)
 __device__ __forceinline__ void rho_fix_candidate(const Slots &s, const FixParams &fp, int oj, i64 xb, i64 yb,
                                                   i64 zb, int q, i64 &acc, unsigned &near) {
@@ -1325,6 +1354,7 @@ __device__ __forceinline__ void rho_fix_candidate(const Slots &s, const FixParam
         fix_note_near(near, q);
     }
 }
+constexpr int kFixRhoAhead = 2, kFixForceAhead = 2;  // candidates side by side
 // within this the FP64 form's lists hold a pair: rc + skin, and (skin 0) whatever the single-precision test lets by
 __device__ __forceinline__ float fix_list_r2(const Geom &g) { return fmaxf(g.rcs2_h, g.rc2_pre); }
 // the candidates [q0, q1) after the single-precision test; NOTED: bit j of the result marks candidate
@@ -1442,6 +1472,17 @@ __global__ void __launch_bounds__(512, 2) k_lat_rho_fix(const __grid_constant__ 
     k_lat_rho_fix_site(t0, t0 < nthreads, nt, g, s, in, pt, fp, hook, order, lists && !wild, full, wild);
 }
 
+// the list's next U candidates from c on, those below c1 in use
+template <int U>
+__device__ __forceinline__ void split_next(const SplitList &sh, int si, int q0, int c, int c1, int (&oj)[U], bool (&use)[U], int (&q)[U]) {
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+        const int e = min(c + u, c1 - 1);
+        use[u] = c + u < c1;
+        oj[u] = si + __float_as_int(sh.rec[e].w);
+        q[u] = q0 + sh.num[e];
+    }
+}
 // The density pass of small boxes (see rho_mixed_split): each warp's integer sum and near pairs over a contiguous
 // share of the candidates (the near pairs keep their order), put together by the first warp (500 groups: 47 -> 19 us).
 template <int W>
@@ -1467,9 +1508,12 @@ __device__ __forceinline__ void rho_fix_split(const NeighTables &nt, const float
         unsigned mn = 0u;
         if (mine) {
             const int c1 = n * (warp + 1) / W;
-#pragma unroll 2
-            for (int c = n * warp / W; c < c1; c++)
-                rho_fix_candidate(s, fp, a.si + __float_as_int(sh.rec[c].w), xb, yb, zb, q0 + sh.num[c], acc, mn);
+            for (int c = n * warp / W; c < c1; c += kFixRhoAhead) {
+                int oj[kFixRhoAhead], q[kFixRhoAhead];
+                bool use[kFixRhoAhead];
+                split_next<kFixRhoAhead>(sh, a.si, q0, c, c1, oj, use, q);
+                rho_fix_pairs<kFixRhoAhead>(s, fp, oj, use, q, xb, yb, zb, acc, mn);
+            }
         }
         part[warp][lane] = acc;
         part_near[warp][lane] = mn;
@@ -1528,14 +1572,14 @@ bool lists_ok(const LaunchCtx &lc, const Geom &g) {
 //   mixed  62 groups 37 / 42 / 52 / 70;  364: 51 / 44 / 53 / 73;  1098: 81 / 53 / 56 / 75;
 //          2048: 122 / 75 / 65 / 74;  2916: 164 / 99 / 99 / 80
 //   FP64   62 groups 52 / 63 / 88 / 123;  500: 60 / 67 / 90 / 126;  1098: 88 / 82 / 97 / 129;
-//          2916: 169 / 156 / 172 / 167;  5695: 285 / 254 / 254 / 267;  7812: 377 / 334 / 329 / 319
+//          2916: 169 / 156 / 172 / 167;  5695: 285 / 254 / 238 / 267;  7812: 377 / 334 / 313 / 319
 static int split_groups(int u0, int u1) { return 2 * ((u1 - u0 + 31) / 32); }
 static int split_warps(const LaunchCtx &lc, bool mixed, int n) {
     if (!mixed && !lc.fp) return 0;
     const int64_t busy = static_cast<int64_t>(n) * lc.share / lc.num_sms;
     if (busy < (mixed ? 2 : 4)) return 8;
     if (busy < (mixed ? 8 : 22)) return 4;
-    return busy < (mixed ? 14 : 40) ? 2 : 0;
+    return busy < (mixed ? 14 : 52) ? 2 : 0;
 }
 template <int W>
 static void launch_rho_split_w(const LaunchCtx &lc, const Geom &g, Slots s, Inter in, PotTables t, bool mixed, bool hook, int u0, int u1,
@@ -1762,6 +1806,55 @@ __device__ __noinline__ double3 force_near_fp64(const NeighTables &nt, const Geo
         }
     }
     return make_double3(fx, fy, fz);
+}
+// U candidates, as rho_fix_pairs
+template <int U>
+__device__ __forceinline__ void force_fix_pairs(const Slots &s, const FixParams &fp, const int (&oj)[U], const bool (&use)[U],
+                                                const int (&q)[U], int ti, i64 xb, i64 yb, i64 zb, i64 dfb, FixForce &a) {
+    FixRec j[U];
+    i64 dfj[U];
+    FixDelta d[U];
+    FixCoord t[U];
+    FixPoly pg[U], ph[U];
+    bool in[U];
+    int tj[U], m[U];
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+        j[u] = ld_fix_rec(s.fix + oj[u]);
+        dfj[u] = __ldg(s.dfq + oj[u]);
+    }
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+        d[u] = fix_delta(xb - j[u].x, yb - j[u].y, zb - j[u].z);
+        const i64 r2 = fix_r2(d[u], fp.b0);
+        in[u] = use[u] && (unsigned long long) (r2 - fp.lo) < (unsigned long long) (fp.rc2 - fp.lo);
+        if (use[u] && (unsigned long long) r2 < (unsigned long long) fp.lo) fix_note_near(a.near, q[u]);
+        t[u] = fix_locate(fp, in[u] ? r2 : fp.rc2 - 1, m[u]);
+        tj[u] = in[u] ? (int) j[u].type : ti;
+        const FixPoly *rec = fp.zg + 2 * ((ti * 3 + tj[u]) * fp.nr1 + m[u]);
+        pg[u] = ld_fix_poly(rec);
+        ph[u] = ld_fix_poly(rec + 1);
+    }
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+        const i64 gj = fix_poly(pg[u], t[u], fp.e3_g);
+        i64 f = fix_poly(ph[u], t[u], fp.e3_h);
+        const i64 both = dfb + dfj[u];  // biased
+        if (in[u]) a.df_hi = max(a.df_hi, fix_hi(both));
+        if (tj[u] == ti) {
+            f = fix_mul_add(fix_hi(both), fix_lo(both), fix_hi(gj), fix_lo(gj), f);
+        } else {
+            const i64 gi = fix_poly(ld_fix_poly(fp.zg + 2 * ((tj[u] * 3 + ti) * fp.nr1 + m[u])), t[u], fp.e3_g);
+            const i64 djb = dfj[u] + kFixBias;
+            f = fix_mul_add(fix_hi(dfb), fix_lo(dfb), fix_hi(gj), fix_lo(gj), f);
+            f = fix_mul_add(fix_hi(djb), fix_lo(djb), fix_hi(gi), fix_lo(gi), f);
+        }
+        if (!in[u]) f = kFixBias;  // zero as a factor
+        const int fh = fix_hi(f), fl = fix_lo(f);
+        a.x = fix_mul_add(d[u].xh, d[u].xl, fh, fl, a.x);
+        a.y = fix_mul_add(d[u].yh, d[u].yl, fh, fl, a.y);
+        a.z = fix_mul_add(d[u].zh, d[u].zl, fh, fl, a.z);
+    }
 }
 // candidate q, at index oj
 __device__ __forceinline__ void force_fix_candidate(const Slots &s, const FixParams &fp, int oj, int ti, i64 xb,
@@ -2151,8 +2244,12 @@ __device__ __forceinline__ void force_fix_split(const NeighTables &nt, const flo
         FixForce m{0, 0, 0, 0, 0u};
         if (mine) {
             const int c1 = n * (warp + 1) / W;
-            for (int c = n * warp / W; c < c1; c++)
-                force_fix_candidate(s, fp, a.si + __float_as_int(sh.rec[c].w), a.ti, xb, yb, zb, dfb, q0 + sh.num[c], m);
+            for (int c = n * warp / W; c < c1; c += kFixForceAhead) {
+                int oj[kFixForceAhead], q[kFixForceAhead];
+                bool use[kFixForceAhead];
+                split_next<kFixForceAhead>(sh, a.si, q0, c, c1, oj, use, q);
+                force_fix_pairs<kFixForceAhead>(s, fp, oj, use, q, a.ti, xb, yb, zb, dfb, m);
+            }
         }
         part.x[warp][lane] = m.x;
         part.y[warp][lane] = m.y;
@@ -2180,7 +2277,7 @@ __device__ __forceinline__ void force_fix_split(const NeighTables &nt, const flo
     force_done_fix(nt, g, s, in, pt, sp, a.sl, a.ti, a.par, tot, f, kick, hook);
 }
 template <int W>
-__global__ void __launch_bounds__(32 * W, 32 / W) k_lat_force_fix_split(const __grid_constant__ NeighTables nt, const float4 *cand,
+__global__ void __launch_bounds__(32 * W, 20 / W) k_lat_force_fix_split(const __grid_constant__ NeighTables nt, const float4 *cand,
                                                                         const __grid_constant__ Geom g, const __grid_constant__ Slots s,
                                                                         const __grid_constant__ Inter in,
                                                                         const __grid_constant__ PotTables pt,
