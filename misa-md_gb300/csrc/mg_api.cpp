@@ -92,9 +92,10 @@ struct mg_context {
     std::vector<double> timer_ms;      // accumulated per kernel
     int64_t timed_steps = 0;
     bool energy_valid = false;
-    // mg_step_host pipeline: z-slab chunks (< 2: off), its copy streams and events
-    int host_chunks = 16;
-    cudaStream_t copy_in = nullptr, copy_out = nullptr;
+    // mg_step_host pipeline: z-slab chunks (< 2: off; negative: by the box's size), its copy streams, the stream of
+    // its force slabs, and events
+    int host_chunks = -1;
+    cudaStream_t copy_in = nullptr, copy_out = nullptr, side = nullptr;
     std::vector<cudaEvent_t> pipe_ev;
     // stage-machine dumps (mg_set_stage_output)
     mg_dump *stage_dump = nullptr;
@@ -682,6 +683,7 @@ mg_status mg_destroy(mg_context *ctx) {
     for (cudaEvent_t e : ctx->pipe_ev) cudaEventDestroy(e);
     if (ctx->copy_in) cudaStreamDestroy(ctx->copy_in);
     if (ctx->copy_out) cudaStreamDestroy(ctx->copy_out);
+    if (ctx->side) cudaStreamDestroy(ctx->side);
     for (void *p : ctx->dev_allocs) cudaFree(p);
     if (ctx->pot_mem) cudaFree(ctx->pot_mem);
     if (ctx->fix_mem) cudaFree(ctx->fix_mem);
@@ -1317,7 +1319,9 @@ mg_status mg_clear_errors(mg_context *ctx) {
 // top into a kept input buffer. Each is unpacked and takes its firststep, decide's own-site case
 // (launch_spec_decide) and its in-plane ghost copy. A density slab runs once every plane within 3 of it
 // has arrived, a force slab once the density slabs beside it have run, and its finished planes are packed
-// and copied out at once while later chunks are still coming in. The thin slabs at the periodic z seam
+// and copied out at once while later chunks are still coming in. The force slabs and the packs go on a
+// stream of their own: a thin slab does not fill the SMs, and the density slabs ahead run beside it (2M atoms:
+// 2.69 -> 2.44 ms). The thin slabs at the periodic z seam
 // (two of 4 planes at each end) wait for the ghost planes, copied after the last chunk. Per atom the
 // kernels and their order are those of the unpipelined path, so the result is bit-identical to it. If a
 // chunk's decide met a displaced atom that does not go straight back to its own site, the step is void:
@@ -1328,7 +1332,8 @@ static mg_status step_host_overlapped(mg_context *ctx, mg_atom_element *atoms, m
     const Geom &g = ctx->g;
     if (!ctx->copy_in) MG_CK(cudaStreamCreateWithFlags(&ctx->copy_in, cudaStreamNonBlocking));
     if (!ctx->copy_out) MG_CK(cudaStreamCreateWithFlags(&ctx->copy_out, cudaStreamNonBlocking));
-    const size_t n_ev = static_cast<size_t>(S + SS + 8);
+    if (!ctx->side) MG_CK(cudaStreamCreateWithFlags(&ctx->side, cudaStreamNonBlocking));
+    const size_t n_ev = static_cast<size_t>(S + 2 * SS + 12);
     while (ctx->pipe_ev.size() < n_ev) {
         cudaEvent_t e;
         MG_CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
@@ -1338,6 +1343,8 @@ static mg_status step_host_overlapped(mg_context *ctx, mg_atom_element *atoms, m
     if ((st = ensure_aos(ctx)) != MG_OK) return st;
     if (!ctx->d_aos_in) MG_CK(dalloc(ctx, &ctx->d_aos_in, static_cast<size_t>(g.n_slots)));
     const LaunchCtx lc = ctx->lc();
+    LaunchCtx lf = lc;  // force slabs and packs
+    lf.stream = ctx->side;
     const bool mx = ctx->mixed();
     const int K = g.bz;
     const int64_t plane = static_cast<int64_t>(g.Sx) * g.Sy;  // slots per z plane
@@ -1388,8 +1395,8 @@ static mg_status step_host_overlapped(mg_context *ctx, mg_atom_element *atoms, m
     auto flush = [&](int z0, int z1) -> mg_status {
         if (z1 <= z0) return MG_OK;
         const int64_t s0 = z0 * plane, s1 = z1 * plane;
-        launch_pack_aos(lc, g, ctx->d_aos, ctx->s, PACK_ALL, mx, static_cast<int>(s0), static_cast<int>(s1));
-        MG_CK(cudaEventRecord(ctx->pipe_ev[ev], ctx->stream));
+        launch_pack_aos(lf, g, ctx->d_aos, ctx->s, PACK_ALL, mx, static_cast<int>(s0), static_cast<int>(s1));
+        MG_CK(cudaEventRecord(ctx->pipe_ev[ev], ctx->side));
         MG_CK(cudaStreamWaitEvent(ctx->copy_out, ctx->pipe_ev[ev++], 0));
         MG_CK(cudaMemcpyAsync(atoms + s0, ctx->d_aos + s0, static_cast<size_t>(s1 - s0) * rec, cudaMemcpyDeviceToHost,
                               ctx->copy_out));
@@ -1397,7 +1404,13 @@ static mg_status step_host_overlapped(mg_context *ctx, mg_atom_element *atoms, m
     };
     auto rho_slab = [&](int c) { launch_lat_rho_sites(lc, g, ctx->s, ctx->in, ctx->pt, mx, u[c], u[c + 1], true); };
     auto force_slab = [&](int c) {
-        launch_lat_force_sites(lc, g, ctx->s, ctx->in, ctx->pt, ctx->d_sp, true, mx, u[c], u[c + 1], true);
+        launch_lat_force_sites(lf, g, ctx->s, ctx->in, ctx->pt, ctx->d_sp, true, mx, u[c], u[c + 1], true);
+    };
+    // the side stream waits for what the library stream has done so far
+    auto side_follows = [&]() -> mg_status {
+        MG_CK(cudaEventRecord(ctx->pipe_ev[ev], ctx->stream));
+        MG_CK(cudaStreamWaitEvent(ctx->side, ctx->pipe_ev[ev++], 0));
+        return MG_OK;
     };
     int next_rho = 1, next_force = 2;
     int df_hi = planes_from(1);                 // in-plane ghosts of planes [planes_from(1), df_hi) have their df
@@ -1421,6 +1434,7 @@ static mg_status step_host_overlapped(mg_context *ctx, mg_atom_element *atoms, m
             launch_ghost_df_planes(lc, g, ctx->s, ctx->in, mx, df_hi, hi);
             df_hi = std::max(df_hi, hi);
             next_rho++;
+            if ((st = side_follows()) != MG_OK) return st;
             while (next_force <= SS - 3 && next_force + 1 < next_rho) {
                 force_slab(next_force);
                 const int z_to = g.gz + planes_below(next_force + 1);
@@ -1444,12 +1458,15 @@ static mg_status step_host_overlapped(mg_context *ctx, mg_atom_element *atoms, m
     launch_ghost_df_planes(lc, g, ctx->s, ctx->in, mx, df_hi, K);
     launch_ghost_df_planes(lc, g, ctx->s, ctx->in, mx, -1, -1);
     if (mx || lc.fp) launch_skin_advance(lc, ctx->s);  // after the last density slab
+    if ((st = side_follows()) != MG_OK) return st;
     force_slab(1);
     force_slab(0);
     if ((st = flush(0, out_lo)) != MG_OK) return st;
     force_slab(SS - 2);
     force_slab(SS - 1);
     if ((st = flush(out_hi, g.Sz)) != MG_OK) return st;
+    MG_CK(cudaEventRecord(ctx->pipe_ev[ev], ctx->side));
+    MG_CK(cudaStreamWaitEvent(ctx->stream, ctx->pipe_ev[ev++], 0));
     seq_eam_force_tail(ctx, true, nullptr);
     if ((st = check_launch(ctx)) != MG_OK) return st;
 
@@ -1477,6 +1494,17 @@ static mg_status step_host_overlapped(mg_context *ctx, mg_atom_element *atoms, m
     return status_from_bits(ctx, static_cast<uint32_t>(cnt[CNT_ERRORS]));
 }
 
+// Chunks of a host step (< 2: one upload, one step, one download). More of them start the slabs and the copies out
+// earlier and cost launches, each slab's latency and the link's rate. Measured, ms per step of the mixed form with
+// 1 / 4 / 6 / 8 / 12 / 16 chunks: 10 MB of slots 0.27 / 0.38 / 0.46 / 0.51 / 0.59 / 0.68;
+// 60 MB 1.03 / 0.96 / 1.00 / 1.05 / 1.14 / 1.19;  132 MB 2.15 / 1.84 / 1.52 / 1.62 / 1.86 / 1.97;
+// 248 MB 3.9 / 3.14 / 2.64 / 2.44 / 2.51 / 2.62;  647 MB 9.9 / 8.1 / 6.7 / 6.1 / 5.8 / 5.9;  1818 MB: 15.9 with 16.
+static int host_chunks(const mg_context *ctx) {
+    if (ctx->host_chunks >= 0) return ctx->host_chunks;
+    const double mb = 1e-6 * sizeof(mg_atom_element) * ctx->g.n_slots;
+    return std::min(16, static_cast<int>(std::sqrt(mb / 3.6)));
+}
+
 // One loop body from and to the host slot array with the copies overlapped by the step (fixed dt, no
 // inter atoms in), for boxes too thin for the overlapped path above. The slot grid is cut into z-slabs
 // of whole planes:
@@ -1490,7 +1518,7 @@ static mg_status step_host_overlapped(mg_context *ctx, mg_atom_element *atoms, m
 static mg_status step_host_pipelined(mg_context *ctx, mg_atom_element *atoms, mg_atom_element *inter, int64_t inter_cap,
                                      int64_t *n_inter) {
     const Geom &g = ctx->g;
-    const int S = std::min(ctx->host_chunks, g.bz);
+    const int S = std::min(host_chunks(ctx), g.bz);
     {
         // density slabs about twice as many as the chunks: thinner slabs keep the copies out close
         // behind the copies in
@@ -1676,7 +1704,7 @@ mg_status mg_set_host_pipeline(mg_context *ctx, int32_t chunks) {
 mg_status mg_step_host(mg_context *ctx, mg_atom_element *atoms, int64_t n_slots, mg_atom_element *inter,
                        int64_t inter_cap, int64_t *n_inter, int64_t nsteps) {
     if (!ctx || !atoms || !n_inter) return MG_ERR_ARG;
-    if (nsteps == 1 && *n_inter == 0 && n_slots == ctx->g.n_slots && ctx->host_chunks >= 2 && ctx->dx_max <= 0.0 &&
+    if (nsteps == 1 && *n_inter == 0 && n_slots == ctx->g.n_slots && host_chunks(ctx) >= 2 && ctx->dx_max <= 0.0 &&
         !ctx->timing && ctx->pot_ready)
         return step_host_pipelined(ctx, atoms, inter, inter_cap, n_inter);
     mg_status st = mg_upload(ctx, atoms, n_slots, inter, std::min<int64_t>(*n_inter, inter_cap));
