@@ -265,18 +265,18 @@ void ensure_fix(mg_context *ctx) {
     for (int t = 0; t < 3; t++) ele_of_type[t] = std::max(0, hp.ele(type_key(t)));
     FixParams fp;
     FixTables ft;
-    if (!build_fixed(hp, ele_of_type, ctx->g.a0, ctx->g.rc / ctx->g.a0, std::max(ctx->n_pruned, ctx->n_full - ctx->n_pruned), fp, ft)) return;
+    if (!build_fixed(hp, ele_of_type, ctx->g.a0, ctx->g.rc / ctx->g.a0, std::max(ctx->n_pruned, ctx->n_full - ctx->n_pruned), fp, ft, false)) return;
     Slots &s = ctx->s;
     const size_t ns = static_cast<size_t>(ctx->g.n_slots);
-    const size_t n[3] = {ft.rho.size(), ft.zg.size(), ft.phi.size()};
+    const size_t n[2] = {ft.rho.size(), ft.zg.size()};
     void *tab = nullptr, *rec = s.fix, *df = s.dfq;
-    cudaError_t e = cudaMalloc(&tab, (n[0] + n[1] + n[2]) * sizeof(FixPoly));
+    cudaError_t e = cudaMalloc(&tab, (n[0] + n[1]) * sizeof(FixPoly));
     if (e == cudaSuccess && !rec) e = cudaMalloc(&rec, ns * sizeof(FixRec));
     if (e == cudaSuccess && !df) e = cudaMalloc(&df, ns * sizeof(i64));
     FixPoly *d = static_cast<FixPoly *>(tab);
-    const FixPoly *src[3] = {ft.rho.data(), ft.zg.data(), ft.phi.data()};
-    const FixPoly *at[3];
-    for (int k = 0; k < 3; k++) {
+    const FixPoly *src[2] = {ft.rho.data(), ft.zg.data()};
+    const FixPoly *at[2];
+    for (int k = 0; k < 2; k++) {
         at[k] = d;
         if (e == cudaSuccess) e = cudaMemcpy(d, src[k], n[k] * sizeof(FixPoly), cudaMemcpyHostToDevice);
         if (d) d += n[k];
@@ -296,7 +296,6 @@ void ensure_fix(mg_context *ctx) {
     ctx->fix_mem = tab;
     fp.rho = at[0];
     fp.zg = at[1];
-    fp.phi = at[2];
     ctx->fp = fp;
     launch_skin_dirty(ctx->lc(), s);  // FP64 passes before this kept no lists
     ctx->graph_stale = true;  // graphs captured without them

@@ -142,11 +142,41 @@ int exponent_for(double bound, int bits) {
     return bits - e;
 }
 
+// the largest values of the functions from a knot on to the cutoff, over elements and pairs
+struct Largest {
+    double rho, g, h, phi, rg, rh, f_typ;
+};
+// at[m]: from knot m on (m_from <= m <= nr - 2); one pass serves every inner end that is tried
+std::vector<Largest> largest_from(const HostPotential &hp, int m_from, double nn) {
+    std::vector<Largest> at(hp.nr - 1, Largest{});
+    Largest v{};
+    for (int m = hp.nr - 2; m >= m_from; m--) {
+        const double r = m * hp.dr;
+        for (int a = 0; a < hp.n_ele; a++) {
+            const double g = std::fabs(hp.rho[a].d0[m]) / r;
+            v.rho = std::max(v.rho, std::fabs(hp.rho[a].c0[m]));
+            v.g = std::max(v.g, g);
+            v.rg = std::max(v.rg, r * g);
+            for (int b = 0; b <= a; b++) {
+                const HostSpline &z = hp.z2[HostPotential::pair_index(a, b)];
+                const double phi = z.c0[m] / r, h = std::fabs((z.d0[m] - phi) / (r * r));
+                v.phi = std::max(v.phi, std::fabs(phi));
+                v.h = std::max(v.h, h);
+                v.rh = std::max(v.rh, r * h);
+                if (r >= 0.97 * nn) v.f_typ = std::max(v.f_typ, r * h);
+            }
+        }
+        at[m] = v;
+    }
+    return at;
+}
+int first_knot(double r_lo, double dr) { return std::max(1, (int) (r_lo / dr) - 1); }
+
 }  // namespace
 
 // build_fixed for one inner end r_lo of the tables' range; tab null: the scales only
 static bool build_from(const HostPotential &hp, const int ele_of_type[3], double a0, double rcf, int n_part, double r_lo,
-                       FixParams &fp, FixTables *tab) {
+                       const std::vector<Largest> &largest, FixParams &fp, FixTables *tab, bool want_phi) {
     fp = FixParams{};
     const double rc = a0 * rcf, dr = hp.dr;
     const int nr = hp.nr;
@@ -176,29 +206,13 @@ static bool build_from(const HostPotential &hp, const int ele_of_type[3], double
     fp.quarter = (float) std::ldexp(kc, fp.ks + fp.sh - 32);
 
     // the range of the tables: pairs closer than r_lo take the FP64 loops
-    const double nn = 0.5 * std::sqrt(3.0) * a0;
-    const int m_lo = std::max(1, (int) (r_lo / dr) - 1);
+    const int m_lo = first_knot(r_lo, dr);
     const int m_hi = nr - 2;
     if (m_lo + 8 > m_hi || !((m_lo + 1) * dr < rc)) return false;
-    double rho_max = 0, g_max = 0, h_max = 0, phi_max = 0, rg_max = 0, rh_max = 0, f_typ = 0;
     const double inv_dr = hp.rho[0].inv_delta;
-    for (int m = m_lo; m <= m_hi; m++) {
-        const double r = m * dr;
-        for (int a = 0; a < hp.n_ele; a++) {
-            const double g = std::fabs(hp.rho[a].d0[m]) / r;
-            rho_max = std::max(rho_max, std::fabs(hp.rho[a].c0[m]));
-            g_max = std::max(g_max, g);
-            rg_max = std::max(rg_max, r * g);
-            for (int b = 0; b <= a; b++) {
-                const HostSpline &z = hp.z2[HostPotential::pair_index(a, b)];
-                const double phi = z.c0[m] / r, h = std::fabs((z.d0[m] - phi) / (r * r));
-                phi_max = std::max(phi_max, std::fabs(phi));
-                h_max = std::max(h_max, h);
-                rh_max = std::max(rh_max, r * h);
-                if (r >= 0.97 * nn) f_typ = std::max(f_typ, r * h);
-            }
-        }
-    }
+    const Largest &top = largest[m_lo];
+    const double rho_max = top.rho, g_max = top.g, h_max = top.h, phi_max = top.phi, rg_max = top.rg, rh_max = top.rh;
+    const double f_typ = top.f_typ;
     if (!(rho_max > 0) || !(g_max > 0) || !(h_max > 0) || !(f_typ > 0) || !std::isfinite(rho_max + g_max + h_max + phi_max))
         return false;
     const double room = 1.01;  // values between the knots
@@ -268,7 +282,7 @@ static bool build_from(const HostPotential &hp, const int ele_of_type[3], double
         return (int) tables.size() - (pairs ? n_pair : hp.n_ele);
     };
     const int first[4] = {add(FN_RHO, krho, false, rho_max), add(FN_G, kg, true, g_max), add(FN_H, kf, true, h_max),
-                          add(FN_PHI, kphi, false, phi_max)};
+                          want_phi ? add(FN_PHI, kphi, false, phi_max) : 0};
     auto expand = [&](Table &t) {
         t.w.resize(fp.nr1);
         t.out.assign(fp.nr1, FixPoly{});
@@ -346,12 +360,12 @@ static bool build_from(const HostPotential &hp, const int ele_of_type[3], double
     fp.e3_phi = e3[FN_PHI];
     tab->rho.assign((size_t) 3 * fp.nr1, FixPoly{});
     tab->zg.assign((size_t) 18 * fp.nr1, FixPoly{});
-    tab->phi.assign((size_t) 9 * fp.nr1, FixPoly{});
+    tab->phi.assign(want_phi ? (size_t) 9 * fp.nr1 : 0, FixPoly{});
     for (int a = 0; a < 3; a++) {
         std::copy_n(tables[first[FN_RHO] + ele_of_type[a]].out.data(), fp.nr1, &tab->rho[(size_t) a * fp.nr1]);
         for (int b = 0; b < 3; b++) {
             const int pi = HostPotential::pair_index(ele_of_type[a], ele_of_type[b]);
-            std::copy_n(tables[first[FN_PHI] + pi].out.data(), fp.nr1, &tab->phi[(size_t) (a * 3 + b) * fp.nr1]);
+            if (want_phi) std::copy_n(tables[first[FN_PHI] + pi].out.data(), fp.nr1, &tab->phi[(size_t) (a * 3 + b) * fp.nr1]);
             const FixPoly *pg = tables[first[FN_G] + ele_of_type[b]].out.data(), *ph = tables[first[FN_H] + pi].out.data();
             for (int m = 0; m < fp.nr1; m++) {
                 FixPoly *r = &tab->zg[2 * ((size_t) (a * 3 + b) * fp.nr1 + m)];
@@ -369,15 +383,20 @@ static bool build_from(const HostPotential &hp, const int ele_of_type[3], double
 // bound admits. The closer it is, the fewer pairs of a hot crystal take the FP64 terms; at 320 K about one
 // pair in 1e5 is closer than 0.82.
 bool build_fixed(const HostPotential &hp, const int ele_of_type[3], double a0, double rcf, int n_part, FixParams &fp,
-                 FixTables &tab) {
-    const double percent = 0.01 * 0.5 * std::sqrt(3.0) * a0;
+                 FixTables &tab, bool want_phi) {
+    fp = FixParams{};
+    if (hp.nr < 64 || hp.nr > 20000) return false;
+    const double nn = 0.5 * std::sqrt(3.0) * a0, percent = 0.01 * nn;
+    const int m_from = std::min(first_knot(70 * percent, hp.dr), hp.nr - 1);
+    const std::vector<Largest> largest = largest_from(hp, m_from, nn);
     double finest = 0.0;
     for (int f = 70; f <= 86; f += 2)
-        if (build_from(hp, ele_of_type, a0, rcf, n_part, f * percent, fp, nullptr) && (finest == 0.0 || fp.f_unit < finest))
+        if (build_from(hp, ele_of_type, a0, rcf, n_part, f * percent, largest, fp, nullptr, want_phi) &&
+            (finest == 0.0 || fp.f_unit < finest))
             finest = fp.f_unit;
     for (int f = 70; f <= 86 && finest > 0.0; f += 2)
-        if (build_from(hp, ele_of_type, a0, rcf, n_part, f * percent, fp, nullptr) && fp.f_unit == finest &&
-            build_from(hp, ele_of_type, a0, rcf, n_part, f * percent, fp, &tab))
+        if (build_from(hp, ele_of_type, a0, rcf, n_part, f * percent, largest, fp, nullptr, want_phi) && fp.f_unit == finest &&
+            build_from(hp, ele_of_type, a0, rcf, n_part, f * percent, largest, fp, &tab, want_phi))
             return true;
     fp = FixParams{};
     return false;

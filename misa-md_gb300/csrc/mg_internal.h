@@ -222,11 +222,12 @@ bool build_potential(int n_ele, const int32_t *zs, int nrho, double drho, int nr
 
 // Scales and tables of the fixed-point pair arithmetic for a lattice (a0, cutoff factor, the most candidates
 // summed at a time) and a potential; false when the tables do not suit it (mg_fixed.cpp states the bounds).
+// want_phi: phi as well, which the force passes do not need.
 struct FixTables {
     std::vector<FixPoly> rho, zg, phi;
 };
 bool build_fixed(const HostPotential &hp, const int ele_of_type[3], double a0, double rcf, int n_part, FixParams &fp,
-                 FixTables &tab);
+                 FixTables &tab, bool want_phi = true);
 
 // Offset tables (restatement of NeighbourIndex::make, src/atom/neighbour_index.inl:13-76) plus the
 // real-space site vector (in units of a0) of every entry.
