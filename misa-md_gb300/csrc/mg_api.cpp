@@ -104,8 +104,9 @@ struct mg_context {
 
     // [precision][rho, force] = {thread order, block size, atoms per thread}. Order 1 until an autotune: its
     // warps cover whole 32-site groups in every box, so the group lists serve boxes with an odd number of sites
-    // of a parity as well (order 0 visits all 112 candidates there).
-    int tune[2][2][3] = {{{1, 256, 1}, {1, 256, 1}}, {{1, 256, 1}, {1, 256, 1}}};
+    // of a parity as well (order 0 visits all 112 candidates there). Blocks of 256; the FP64 density pass, at 56
+    // registers, fills the SMs better with 128 (2M atoms: 720 -> 682 us).
+    int tune[2][2][3] = {{{1, 128, 1}, {1, 256, 1}}, {{1, 256, 1}, {1, 256, 1}}};
     int share = 1;                  // contexts stepping side by side (while a batch captures)
     LaunchCtx lc() const {
         LaunchCtx l{stream, num_sms};
