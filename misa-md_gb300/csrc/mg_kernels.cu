@@ -1573,11 +1573,14 @@ bool lists_ok(const LaunchCtx &lc, const Geom &g) {
 //          2048: 122 / 75 / 65 / 74;  2916: 164 / 99 / 99 / 80
 //   FP64   62 groups 52 / 63 / 88 / 123;  500: 60 / 67 / 90 / 126;  1098: 88 / 82 / 97 / 129;
 //          2916: 169 / 156 / 172 / 167;  5695: 285 / 254 / 238 / 267;  7812: 377 / 334 / 313 / 319
+// A pass without lists (the hooks) searches all candidates first, which the warps share less well; ms for the three
+// hooks: FP64 500 groups - / 0.39 / 0.42 / 0.47;  2048: 0.76 / 0.72 / 0.75 / 0.73;  7812: 2.00 / 1.92 / 1.91 / 1.83.
 static int split_groups(int u0, int u1) { return 2 * ((u1 - u0 + 31) / 32); }
-static int split_warps(const LaunchCtx &lc, bool mixed, int n) {
+static int split_warps(const LaunchCtx &lc, bool mixed, bool lists, int n) {
     if (!mixed && !lc.fp) return 0;
     const int64_t busy = static_cast<int64_t>(n) * lc.share / lc.num_sms;
-    if (busy < (mixed ? 2 : 4)) return 8;
+    if (busy < (mixed || !lists ? 2 : 4)) return 8;
+    if (!lists) return busy < (mixed ? 8 : 14) ? 4 : 0;
     if (busy < (mixed ? 8 : 22)) return 4;
     return busy < (mixed ? 14 : 52) ? 2 : 0;
 }
@@ -1592,7 +1595,7 @@ static void launch_rho_split_w(const LaunchCtx &lc, const Geom &g, Slots s, Inte
 // the split density pass, where it serves
 static bool launch_lat_rho_split(const LaunchCtx &lc, const Geom &g, Slots s, Inter in, PotTables t, bool mixed, bool hook, int u0,
                                  int u1, bool lists) {
-    switch (split_warps(lc, mixed, split_groups(u0, u1))) {
+    switch (split_warps(lc, mixed, lists, split_groups(u0, u1))) {
         case 8: launch_rho_split_w<8>(lc, g, s, in, t, mixed, hook, u0, u1, lists); return true;
         case 4: launch_rho_split_w<4>(lc, g, s, in, t, mixed, hook, u0, u1, lists); return true;
         case 2: launch_rho_split_w<2>(lc, g, s, in, t, mixed, hook, u0, u1, lists); return true;
@@ -2323,7 +2326,7 @@ static void launch_force_split_w(const LaunchCtx &lc, const Geom &g, Slots s, In
 }
 static bool launch_lat_force_split(const LaunchCtx &lc, const Geom &g, Slots s, Inter in, PotTables t, StepParams *p, bool kick, bool mixed,
                                    bool hook, int u0, int u1, bool fuse_next, bool lists) {
-    switch (split_warps(lc, mixed, split_groups(u0, u1))) {
+    switch (split_warps(lc, mixed, lists, split_groups(u0, u1))) {
         case 8: launch_force_split_w<8>(lc, g, s, in, t, p, kick, mixed, hook, u0, u1, fuse_next, lists); return true;
         case 4: launch_force_split_w<4>(lc, g, s, in, t, p, kick, mixed, hook, u0, u1, fuse_next, lists); return true;
         case 2: launch_force_split_w<2>(lc, g, s, in, t, p, kick, mixed, hook, u0, u1, fuse_next, lists); return true;
