@@ -21,14 +21,15 @@ namespace {
 thread_local std::string g_create_error;
 
 constexpr int kNumTimers = 10;  // events per timed step; the kernels between consecutive events are:
-const char *kTimerNames[kNumTimers - 1] = {"firststep",     // step head and firststep
+const char *kTimerNames[kNumTimers - 1] = {"firststep",     // the step head (variable dt) and firststep
                                            "inter_manage",  // the list manager
-                                           "ghost_copy",    // and the far atoms' marks
-                                           "inter_rho",     // the FP64 form's records and the inter atoms' densities
+                                           "ghost_copy",    // and the far atoms' marks and the inter atoms' densities
+                                           "fix_records",   // the FP64 form's records
                                            "lat_rho",
-                                           "inter_owner",   // the density shares of lattice atoms near inter atoms
-                                           "ghost_df", "lat_force",
-                                           "inter_force"};  // and the second half-kicks near inter atoms
+                                           "inter_rho",     // the density shares of lattice atoms near inter atoms
+                                           "ghost_df",      // and the forces on the inter atoms
+                                           "lat_force",
+                                           "inter_force"};  // the force shares of those atoms, and their half-kicks
 
 }  // namespace
 
@@ -176,6 +177,10 @@ mg_status check_launch(mg_context *ctx) {
 // record; dx_max > 0 switches to the variable rule, which the step head applies from the next step
 void set_dt(mg_context *ctx, double dt, double dx_max = 0.0, double dt_min = 0.0, double dt_max = 0.0) {
     ctx->dt = dt;
+    if ((dx_max > 0.0) != (ctx->dx_max > 0.0)) {  // steps captured under the other rule
+        ctx->graph_stale = true;
+        ctx->gen++;
+    }
     ctx->dx_max = dx_max;
     ctx->dt_min = dt_min;
     ctx->dt_max = dt_max;
@@ -203,10 +208,10 @@ void seq_eam_lists(mg_context *ctx, bool with_manage_prefix, int manage_mask, Ti
     const LaunchCtx lc = ctx->lc();
     const bool mx = ctx->mixed();
     const bool decide = with_manage_prefix && (manage_mask & MANAGE_DECIDE);
-    if (with_manage_prefix) launch_inter_manage(lc, ctx->g, ctx->s, ctx->in, manage_mask | MANAGE_INDEX, mx);
-    else launch_inter_manage(lc, ctx->g, ctx->s, ctx->in, MANAGE_INDEX, mx);
+    launch_inter_manage(lc, ctx->g, ctx->s, ctx->in, (with_manage_prefix ? manage_mask : 0) | MANAGE_INDEX, mx, ctx->d_sp);
     if (t) t->mark(2);
-    launch_ghost_copy(lc, ctx->g, ctx->s, ctx->in, decide);  // and the new far list's neighbourhood marks
+    // and the new far list's neighbourhood marks, and the inter atoms' own densities
+    launch_ghost_copy(lc, ctx->g, ctx->s, ctx->in, ctx->pt, mx, decide, true);
     if (t) t->mark(3);
 }
 // rho, dF/drho and the forward df exchange; the density pass checks or rebuilds the group lists that
@@ -215,19 +220,18 @@ void seq_eam_rho(mg_context *ctx, Timer *t) {
     const LaunchCtx lc = ctx->lc();
     const bool mx = ctx->mixed();
     launch_fix_records(lc, ctx->g, ctx->s);
-    launch_inter_rho(lc, ctx->g, ctx->s, ctx->in, ctx->pt, mx);
     if (t) t->mark(4);
     const bool advance = launch_lat_rho(lc, ctx->g, ctx->s, ctx->in, ctx->pt, mx, false, true);
     if (t) t->mark(5);
     launch_inter_rho_owners(lc, ctx->g, ctx->s, ctx->in, ctx->pt, mx);
     if (t) t->mark(6);
-    launch_ghost_df(lc, ctx->g, ctx->s, ctx->in, mx, advance);
+    launch_ghost_df(lc, ctx->g, ctx->s, ctx->in, ctx->pt, mx, advance);  // and the forces on the inter atoms
     if (t) t->mark(7);
 }
-// the inter-atom force pass and the second half-kick it takes, after the lattice force pass
+// the owners' shares of the inter atoms' forces and the second half-kicks left to them, after the lattice force pass
 void seq_eam_force_tail(mg_context *ctx, bool kick, Timer *t) {
     const LaunchCtx lc = ctx->lc();
-    launch_inter_force(lc, ctx->g, ctx->s, ctx->in, ctx->pt, ctx->mixed(), ctx->d_sp, kick);
+    launch_inter_force_owners(lc, ctx->g, ctx->s, ctx->in, ctx->pt, ctx->mixed(), ctx->d_sp, kick);
     if (t) t->mark(9);
 }
 void seq_compute_eam(mg_context *ctx, bool kick, bool with_manage_prefix, int manage_mask, Timer *t, bool fuse_next = false) {
@@ -242,13 +246,16 @@ void seq_compute_eam(mg_context *ctx, bool kick, bool with_manage_prefix, int ma
 // next one (both only act when no inter atoms exist, which the kernels check on the device)
 void seq_step(mg_context *ctx, Timer *t, bool fused_prev = false, bool fuse_next = false) {
     if (t) t->mark(0);
-    launch_step_head(ctx->lc(), ctx->d_sp, ctx->s.skin);
+    // a fixed dt needs no head: the list manager keeps the clock
+    const bool variable = ctx->dx_max > 0.0;
+    if (variable) launch_step_head(ctx->lc(), ctx->d_sp, ctx->s.skin);
     seq_firststep(ctx, true, t, fused_prev);
-    seq_compute_eam(ctx, true, true, MANAGE_DECIDE | MANAGE_CLEAR_GHOST | MANAGE_EXCHANGE | MANAGE_BORDER, t, fuse_next);
+    seq_compute_eam(ctx, true, true, MANAGE_DECIDE | MANAGE_CLEAR_GHOST | MANAGE_EXCHANGE | MANAGE_BORDER | (variable ? 0 : MANAGE_CLOCK), t,
+                    fuse_next);
 }
 // steps of mg_simulate that run fused: the mixed form with a fixed dt
 bool fusable(const mg_context *ctx) { return ctx->fuse_steps >= 2 && ctx->mixed() && ctx->dx_max <= 0.0; }
-constexpr int kLaunchesPerStep = 11;
+constexpr int kLaunchesPerStep = 8;
 
 mg_status require_ready(mg_context *ctx) {
     if (!ctx->pot_ready) { ctx->err = "potential not initialised"; return MG_ERR_POTENTIAL; }
@@ -1052,7 +1059,7 @@ mg_status mg_phase(mg_context *ctx, int32_t phase) {
             break;
         case 2: launch_inter_manage(lc, ctx->g, ctx->s, ctx->in, MANAGE_EXCHANGE, ctx->mixed()); break;
         case 3: launch_inter_manage(lc, ctx->g, ctx->s, ctx->in, MANAGE_BORDER, ctx->mixed()); break;
-        case 4: launch_ghost_copy(lc, ctx->g, ctx->s, ctx->in, false); break;
+        case 4: launch_ghost_copy(lc, ctx->g, ctx->s, ctx->in, ctx->pt, ctx->mixed(), false, false); break;
         case 5: seq_compute_eam(ctx, false, false, 0, nullptr); break;
         case 6: launch_secondstep(lc, ctx->g, ctx->s, ctx->in, ctx->d_sp); break;
     }

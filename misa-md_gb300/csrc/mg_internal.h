@@ -290,14 +290,14 @@ void launch_fix_records(const LaunchCtx &lc, const Geom &g, Slots s, int s0 = 0,
 // far-atom neighbourhood marks: clear those of the current far list / set them (grid-wide)
 void launch_far_clear(const LaunchCtx &lc, const Geom &g, Inter in);
 void launch_far_mark(const LaunchCtx &lc, const Geom &g, Inter in);
-// mark: also as launch_far_mark
-void launch_ghost_copy(const LaunchCtx &lc, const Geom &g, Slots s, Inter in, bool mark);
-// advance: also as launch_skin_advance
-void launch_ghost_df(const LaunchCtx &lc, const Geom &g, Slots s, Inter in, bool mixed, bool advance);
+// mark: also as launch_far_mark; inter: also the inter atoms' own densities, listing the lattice owners near them
+void launch_ghost_copy(const LaunchCtx &lc, const Geom &g, Slots s, Inter in, PotTables t, bool mixed, bool mark, bool inter);
+// also the forces on the inter atoms; advance: also as launch_skin_advance
+void launch_ghost_df(const LaunchCtx &lc, const Geom &g, Slots s, Inter in, PotTables t, bool mixed, bool advance);
 // lists (mixed form): check or rebuild, per 32-site group, the list of pruned candidates that some site
 // of the group has inside rc + skin, and visit only those (when lists_ok; the force pass of the same
 // step must get the same flag)
-// true: the skin's advance is due. Inter atoms: after launch_inter_rho, which lists the owners whose F' the pass
+// true: the skin's advance is due. Inter atoms: after launch_ghost_copy, which lists the owners whose F' the pass
 // leaves to launch_inter_rho_owners.
 bool launch_lat_rho(const LaunchCtx &lc, const Geom &g, Slots s, Inter in, PotTables t, bool mixed, bool hook,
                     bool lists = false);
@@ -344,15 +344,15 @@ void launch_vmax_full(const LaunchCtx &lc, const Geom &g, Slots s, Inter in, Ste
 void launch_energy(const LaunchCtx &lc, const Geom &g, Slots s, Inter in, PotTables t, bool mixed);
 // far atoms: rebuild the list and its neighbourhood marks from positions (uploads, hooks)
 void launch_far_rebuild(const LaunchCtx &lc, const Geom &g, Slots s, Inter in);
-void launch_inter_manage(const LaunchCtx &lc, const Geom &g, Slots s, Inter in, int steps_mask, bool mixed);
-enum { MANAGE_DECIDE = 1, MANAGE_CLEAR_GHOST = 2, MANAGE_EXCHANGE = 4, MANAGE_BORDER = 8, MANAGE_INDEX = 16 };
-// the inter atoms' own densities, listing the lattice owners near them; after the lattice density pass, the owners' shares
-void launch_inter_rho(const LaunchCtx &lc, const Geom &g, Slots s, Inter in, PotTables t, bool mixed);
+// MANAGE_CLOCK (fixed dt): also records the step's dt and advances the clock, as the step head does
+void launch_inter_manage(const LaunchCtx &lc, const Geom &g, Slots s, Inter in, int steps_mask, bool mixed, StepParams *sp = nullptr);
+enum { MANAGE_DECIDE = 1, MANAGE_CLEAR_GHOST = 2, MANAGE_EXCHANGE = 4, MANAGE_BORDER = 8, MANAGE_INDEX = 16, MANAGE_CLOCK = 32 };
+// after the lattice density pass: the shares of the lattice owners near inter atoms
 void launch_inter_rho_owners(const LaunchCtx &lc, const Geom &g, Slots s, Inter in, PotTables t, bool mixed);
-// kick: the second half-kick of the inter atoms and of the lattice owners the inter-atom density pass listed (the
-// lattice force pass kicked every other atom)
-void launch_inter_force(const LaunchCtx &lc, const Geom &g, Slots s, Inter in, PotTables t, bool mixed, StepParams *sp,
-                        bool kick);
+// after the lattice force pass: their shares of the forces; kick: the second half-kick of the inter atoms and of those
+// owners (the lattice force pass kicked every other atom)
+void launch_inter_force_owners(const LaunchCtx &lc, const Geom &g, Slots s, Inter in, PotTables t, bool mixed, StepParams *sp,
+                               bool kick);
 void launch_inter_energy(const LaunchCtx &lc, const Geom &g, Slots s, Inter in, PotTables t, bool mixed);
 void launch_inter_firststep(const LaunchCtx &lc, Inter in, const StepParams *sp);
 void launch_setv(const LaunchCtx &lc, const Geom &g, Slots s, int64_t slot, const double dir[3], double energy);

@@ -659,27 +659,17 @@ __device__ __forceinline__ int ghost_slot(const Geom &g, int t) {
     return lin(g, X, Y, Z);
 }
 
+// the coordinate of a periodic image (sgn: the side it lies on)
+__device__ __forceinline__ double shifted(double x, int sgn, double L) { return sgn ? __dadd_rn(x, sgn > 0 ? L : -L) : x; }
 __device__ __forceinline__ void ghost_copy_one(const Geom &g, const Slots &s, int gs) {
     const int X = gs % g.Sx, r = gs / g.Sx, Y = r % g.Sy, Z = r / g.Sy;
     int sx, sy, sz;
     const int os = lin(g, wrap_axis(X, g.gx, g.bx, sx), wrap_axis(Y, g.gy, g.by, sy), wrap_axis(Z, g.gz, g.bz, sz));
     s.type[gs] = s.type[os];
-    const double ox = s.x[os], oy = s.y[os], oz = s.z[os];
-    s.x[gs] = sx ? __dadd_rn(ox, sx > 0 ? g.L[0] : -g.L[0]) : ox;
-    s.y[gs] = sy ? __dadd_rn(oy, sy > 0 ? g.L[1] : -g.L[1]) : oy;
-    s.z[gs] = sz ? __dadd_rn(oz, sz > 0 ? g.L[2] : -g.L[2]) : oz;
+    s.x[gs] = shifted(s.x[os], sx, g.L[0]);
+    s.y[gs] = shifted(s.y[os], sy, g.L[1]);
+    s.z[gs] = shifted(s.z[os], sz, g.L[2]);
     s.u4[sidx(g, gs)] = s.u4[sidx(g, os)];
-}
-// mark: after decide, also the marks of the new far list's neighbourhoods (as launch_far_mark)
-__global__ void k_ghost_copy(const NeighTables *nt, Geom g, Slots s, Inter in, bool mark) {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (mark) mark_far_neighbourhoods(*nt, g, in, 0, min(in.cnt[CNT_FAR], in.fcap), 1, t, gridDim.x * blockDim.x);
-    if (t >= g.n_ghost_slots) return;
-    ghost_copy_one(g, s, ghost_slot(g, t));
-}
-void launch_ghost_copy(const LaunchCtx &lc, const Geom &g, Slots s, Inter in, bool mark) {
-    const int b = 256, n = (g.n_ghost_slots + b - 1) / b;
-    k_ghost_copy<<<n, b, 0, lc.stream>>>(lc.ntd, g, s, in, mark);
 }
 // The ghost slots inside the local planes [k0, k1) (y-ghost rows, then x-ghost columns of each plane;
 // their owners lie in the same plane), or (k0 < 0) the ghost planes below and above the box, whose
@@ -739,24 +729,6 @@ __device__ __forceinline__ void skin_advance(SkinState *k) {
         k->acc += sqrtf(__uint_as_float(m));  // a NaN or infinity forces the next pass to rebuild
     }
     k->passes++;
-}
-// advance: after a density pass with the group lists (as launch_skin_advance)
-template <bool MIXED>
-__global__ void k_ghost_df(Geom g, Slots s, Inter in, bool advance) {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (advance && t < 32) skin_advance(s.skin);
-    if (t < g.n_ghost_slots) {
-        const int gs = ghost_slot(g, t);
-        const int os = owner_slot(g, gs);
-        ghost_df_one<MIXED>(g, s, gs, os);
-    }
-    const int ng = in.cnt[CNT_GHOST];
-    for (int q = t; q < ng; q += gridDim.x * blockDim.x) in.gdf[q] = in.df[in.groot[q]];
-}
-void launch_ghost_df(const LaunchCtx &lc, const Geom &g, Slots s, Inter in, bool mixed, bool advance) {
-    const int b = 256, n = (g.n_ghost_slots + b - 1) / b;
-    if (mixed) k_ghost_df<true><<<n, b, 0, lc.stream>>>(g, s, in, advance);
-    else k_ghost_df<false><<<n, b, 0, lc.stream>>>(g, s, in, advance);
 }
 // the same copy for the ghost slots inside the local planes [k0, k1) (y-ghost rows, then x-ghost
 // columns of each plane; their owners lie in the same plane), or (k0 < 0) for the ghost planes below
@@ -2412,7 +2384,16 @@ __global__ void k_set_step(StepParams *p, double dt, double dx_max, double dt_mi
 void launch_set_step(const LaunchCtx &lc, StepParams *sp, double dt, double dx_max, double dt_min, double dt_max) {
     k_set_step<<<1, 1, 0, lc.stream>>>(sp, dt, dx_max, dt_min, dt_max);
 }
-// One block of kVmaxSlots threads: reduce and clear the max words, then (variable mode)
+// The timestep taken into the history and the clock; one thread, once a step.
+__device__ __forceinline__ void step_record(StepParams *p, SkinState *skin) {
+    skin->wild = 0;  // the step's records find out again
+    const long long k = p->steps;
+    p->hist[k % kDtHistory] = p->dt;
+    p->time = __dadd_rn(p->time, p->dt);
+    p->steps = k + 1;
+}
+
+// One block of kVmaxSlots threads, ahead of a step: reduce and clear the max words, then (variable mode)
 // dt = clamp(dx_max / sqrt(max |v|^2), dt_min, dt_max); record dt and advance the clock.
 __global__ void __launch_bounds__(kVmaxSlots) k_step_head(StepParams *p, SkinState *skin) {
     __shared__ unsigned long long part[kVmaxSlots / 32];
@@ -2424,7 +2405,6 @@ __global__ void __launch_bounds__(kVmaxSlots) k_step_head(StepParams *p, SkinSta
     if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = ((unsigned long long) mhi << 32) | mlo;
     __syncthreads();
     if (threadIdx.x != 0) return;
-    skin->wild = 0;  // the step's records find out again
     unsigned long long m = 0ull;
     for (int w = 0; w < kVmaxSlots / 32; w++) m = part[w] > m ? part[w] : m;
     if (p->dx_max > 0.0) {
@@ -2434,10 +2414,7 @@ __global__ void __launch_bounds__(kVmaxSlots) k_step_head(StepParams *p, SkinSta
         if (dt > p->dt_max) dt = p->dt_max;
         set_dt_dev(p, dt);
     }
-    const long long k = p->steps;
-    p->hist[k % kDtHistory] = p->dt;
-    p->time = __dadd_rn(p->time, p->dt);
-    p->steps = k + 1;
+    step_record(p, skin);
 }
 void launch_step_head(const LaunchCtx &lc, StepParams *sp, SkinState *skin) {
     k_step_head<<<1, kVmaxSlots, 0, lc.stream>>>(sp, skin);
@@ -2763,9 +2740,10 @@ __device__ __forceinline__ void border_put(Inter &in, int q, const double p3[3],
     in.gdf[q] = 0.0;
 }
 
-__global__ void __launch_bounds__(kManageThreads) k_inter_manage(Geom g, Slots s, Inter in, int mask, bool mixed) {
+__global__ void __launch_bounds__(kManageThreads) k_inter_manage(Geom g, Slots s, Inter in, int mask, bool mixed, StepParams *sp) {
     extern __shared__ long long sm_keys[];
     const int tid = threadIdx.x, nthr = blockDim.x;
+    if ((mask & MANAGE_CLOCK) && tid == 0) step_record(sp, s.skin);
 
     // The list counts are read once, by all threads before any is written, and then followed in
     // registers: every change to them is block-uniform (scan totals), and one global round trip
@@ -3037,8 +3015,8 @@ void configure_manage_kernel() {
     cudaFuncSetAttribute(k_inter_manage, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          static_cast<int>(kSortSmemKeys * sizeof(long long)));
 }
-void launch_inter_manage(const LaunchCtx &lc, const Geom &g, Slots s, Inter in, int mask, bool mixed) {
-    k_inter_manage<<<1, kManageThreads, kSortSmemKeys * sizeof(long long), lc.stream>>>(g, s, in, mask, mixed);
+void launch_inter_manage(const LaunchCtx &lc, const Geom &g, Slots s, Inter in, int mask, bool mixed, StepParams *sp) {
+    k_inter_manage<<<1, kManageThreads, kSortSmemKeys * sizeof(long long), lc.stream>>>(g, s, in, mask, mixed, sp);
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -3068,7 +3046,7 @@ __device__ __forceinline__ InterRef inter_ref(const Inter &in, int ref) {
     if (ref < in.cap) { r.x = in.x[ref]; r.y = in.y[ref]; r.z = in.z[ref]; r.type = in.type[ref]; r.id = in.id[ref]; r.df = in.df[ref]; }
     else {
         const int q = ref - in.cap;
-        r.x = in.gx[q]; r.y = in.gy[q]; r.z = in.gz[q]; r.type = in.gtype[q]; r.id = 0; r.df = in.gdf[q];
+        r.x = in.gx[q]; r.y = in.gy[q]; r.z = in.gz[q]; r.type = in.gtype[q]; r.id = 0; r.df = in.df[in.groot[q]];
     }
     return r;
 }
@@ -3128,12 +3106,13 @@ __device__ __forceinline__ bool is_local_slot(const Geom &g, int sl) {
     return X >= g.gx && X < g.gx + g.bx && Y >= g.gy && Y < g.gy + g.by && Z >= g.gz && Z < g.gz + g.bz;
 }
 template <int KIND>
-__global__ void __launch_bounds__(kInterThreads) k_inter_eam(const NeighTables *__restrict__ ntd, Geom g, Slots s, Inter in, PotTables pt, bool mixed) {
+__device__ __forceinline__ void inter_eam(const NeighTables &nt, const Geom &g, const Slots &s, Inter &in, const PotTables &pt, bool mixed,
+                                          int block, int blocks) {
     const int n = in.cnt[CNT_INTER];
     const int nb = *in.n_bucket;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     __shared__ double red[3][kInterThreads / 32];
-    for (int a = blockIdx.x; a < n; a += gridDim.x) {  // block-uniform
+    for (int a = block; a < n; a += blocks) {  // block-uniform
         const double xa = in.x[a], ya = in.y[a], za = in.z[a];
         const int ta = in.type[a];
         const uint64_t ida = in.id[a];
@@ -3143,20 +3122,29 @@ __global__ void __launch_bounds__(kInterThreads) k_inter_eam(const NeighTables *
         double acc = 0.0, fx = 0.0, fy = 0.0, fz = 0.0;
         // lattice partners: the nearest site's atom, then the full offsets of that site
         const int par = (near % g.Sx) & 1;
-        const int nf = ntd->nfull;
+        const int nf = nt.nfull;
         for (int q = (int) threadIdx.x - 1; q < nf; q += kInterThreads) {
-            const int sj = q < 0 ? near : near + ntd->full[par][q];
+            const int sj = q < 0 ? near : near + nt.full[par][q];
             if (sj < 0 || sj >= g.n_slots) { set_error(in, MG_DEVERR_OUT_OF_GRID); continue; }
-            const int tj = s.type[sj];
+            // a ghost slot's record from its owner, shifted as the ghost copy shifts it, so that the pass need
+            // not wait for that copy (or for the copy of F'); the energies follow both and read the slot itself
+            int wx, wy, wz;
+            const int X = sj % g.Sx, r = sj / g.Sx, Y = r % g.Sy, Z = r / g.Sy;
+            const int own = lin(g, wrap_axis(X, g.gx, g.bx, wx), wrap_axis(Y, g.gy, g.by, wy), wrap_axis(Z, g.gz, g.bz, wz));
+            const int at = KIND == 2 ? sj : own;
+            const int tj = s.type[at];
             if (tj < 0) continue;
-            const double dx = xa - s.x[sj], dy = ya - s.y[sj], dz = za - s.z[sj];
+            const double xj = KIND == 2 ? s.x[at] : shifted(s.x[at], wx, g.L[0]);
+            const double yj = KIND == 2 ? s.y[at] : shifted(s.y[at], wy, g.L[1]);
+            const double zj = KIND == 2 ? s.z[at] : shifted(s.z[at], wz, g.L[2]);
+            const double dx = xa - xj, dy = ya - yj, dz = za - zj;
             const double r2 = dx * dx + dy * dy + dz * dz;
             if (!(r2 < g.rc2)) continue;
-            touch_owner(in, owner_slot(g, sj));
+            touch_owner(in, own);
             if (KIND == 0) {
                 acc += rho_fn(pt, tj, r2);
             } else if (KIND == 1) {
-                const double fp = to_force(pt, ta, tj, r2, dfa, lat_df(g, s, sj, mixed));
+                const double fp = to_force(pt, ta, tj, r2, dfa, lat_df(g, s, own, mixed));
                 fx += dx * fp; fy += dy * fp; fz += dz * fp;
             } else {
                 acc += 0.5 * pair_fn(pt, ta, tj, r2);
@@ -3164,7 +3152,7 @@ __global__ void __launch_bounds__(kInterThreads) k_inter_eam(const NeighTables *
         }
         // inter partners: same-site bucket (not itself), then the buckets of the full offsets
         for (int q = (int) threadIdx.x - 1; q < nf; q += kInterThreads) {
-            const int key = q < 0 ? near : near + ntd->full[par][q];
+            const int key = q < 0 ? near : near + nt.full[par][q];
             for (int b = bucket_begin(in, nb, key); b < nb && (int) (in.bucket[b] >> 32) == key; b++) {
                 const InterRef o = inter_ref(in, (int) (in.bucket[b] & 0xffffffffLL));
                 if (q < 0 && o.id == ida) continue;
@@ -3214,6 +3202,57 @@ __global__ void __launch_bounds__(kInterThreads) k_inter_eam(const NeighTables *
             in.e[a] = val_d(pt.F_v + ta * pt.nrho, m, p) + acc;
         }
     }
+}
+template <int KIND>
+__global__ void __launch_bounds__(kInterThreads) k_inter_eam(const NeighTables *nt, Geom g, Slots s, Inter in, PotTables pt, bool mixed) {
+    inter_eam<KIND>(*nt, g, s, in, pt, mixed, blockIdx.x, gridDim.x);
+}
+// blocks of the inter-atom pass beside a kernel over the ghost slots
+inline int inter_blocks(const LaunchCtx &lc, const Geom &g) {
+    return std::max(1, std::min(lc.num_sms * 4, (g.n_local + kInterThreads - 1) / kInterThreads));
+}
+// The ghost copy and what only needs the lists: (mark) after decide, the marks of the new far list's
+// neighbourhoods, as launch_far_mark; (inter_n blocks past the ghost slots') the inter atoms' own densities.
+__global__ void __launch_bounds__(kInterThreads) k_ghost_copy(const NeighTables *nt, Geom g, Slots s, Inter in, PotTables pt, bool mixed,
+                                                              bool mark, int inter_n) {
+    const int blocks = gridDim.x - inter_n;
+    if ((int) blockIdx.x >= blocks) {
+        inter_eam<0>(*nt, g, s, in, pt, mixed, blockIdx.x - blocks, inter_n);
+        return;
+    }
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (mark) mark_far_neighbourhoods(*nt, g, in, 0, min(in.cnt[CNT_FAR], in.fcap), 1, t, blocks * blockDim.x);
+    if (t >= g.n_ghost_slots) return;
+    ghost_copy_one(g, s, ghost_slot(g, t));
+}
+void launch_ghost_copy(const LaunchCtx &lc, const Geom &g, Slots s, Inter in, PotTables t, bool mixed, bool mark, bool inter) {
+    const int n = (g.n_ghost_slots + kInterThreads - 1) / kInterThreads, e = inter ? inter_blocks(lc, g) : 0;
+    k_ghost_copy<<<n + e, kInterThreads, 0, lc.stream>>>(lc.ntd, g, s, in, t, mixed, mark, e);
+}
+// The copy of F' and what only needs F' of the box's own atoms: (advance) after a density pass with the group lists,
+// as launch_skin_advance; (inter_n blocks past the ghost slots') the forces on the inter atoms.
+template <bool MIXED>
+__global__ void __launch_bounds__(kInterThreads) k_ghost_df(const NeighTables *nt, Geom g, Slots s, Inter in, PotTables pt, bool advance,
+                                                            int inter_n) {
+    const int blocks = gridDim.x - inter_n;
+    if ((int) blockIdx.x >= blocks) {
+        inter_eam<1>(*nt, g, s, in, pt, MIXED, blockIdx.x - blocks, inter_n);
+        return;
+    }
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (advance && t < 32) skin_advance(s.skin);
+    if (t < g.n_ghost_slots) {
+        const int gs = ghost_slot(g, t);
+        const int os = owner_slot(g, gs);
+        ghost_df_one<MIXED>(g, s, gs, os);
+    }
+    const int ng = in.cnt[CNT_GHOST];
+    for (int q = t; q < ng; q += blocks * blockDim.x) in.gdf[q] = in.df[in.groot[q]];
+}
+void launch_ghost_df(const LaunchCtx &lc, const Geom &g, Slots s, Inter in, PotTables t, bool mixed, bool advance) {
+    const int n = (g.n_ghost_slots + kInterThreads - 1) / kInterThreads, e = inter_blocks(lc, g);
+    if (mixed) k_ghost_df<true><<<n + e, kInterThreads, 0, lc.stream>>>(lc.ntd, g, s, in, t, advance, e);
+    else k_ghost_df<false><<<n + e, kInterThreads, 0, lc.stream>>>(lc.ntd, g, s, in, t, advance, e);
 }
 // The lattice owners' side of the inter-atom pairs. One warp per owner listed by k_inter_eam: the
 // lanes walk the owner's site and its full offsets (reference order) and, per site, the bucket of
@@ -3308,26 +3347,18 @@ __global__ void __launch_bounds__(128) k_inter_owner(const NeighTables *__restri
     }
 }
 template <int KIND>
-void launch_inter_eam(const LaunchCtx &lc, const Geom &g, Slots s, Inter in, PotTables t, bool mixed) {
-    k_inter_eam<KIND><<<lc.num_sms * 4, kInterThreads, 0, lc.stream>>>(lc.ntd, g, s, in, t, mixed);
-}
-template <int KIND>
 void launch_inter_owner(const LaunchCtx &lc, const Geom &g, Slots s, Inter in, PotTables t, bool mixed, StepParams *sp = nullptr,
                         bool kick = false) {
     k_inter_owner<KIND><<<lc.num_sms * 4, 128, 0, lc.stream>>>(lc.ntd, g, s, in, t, mixed, fix_params(lc), sp, kick);
 }
-void launch_inter_rho(const LaunchCtx &lc, const Geom &g, Slots s, Inter in, PotTables t, bool mixed) {
-    launch_inter_eam<0>(lc, g, s, in, t, mixed);
-}
 void launch_inter_rho_owners(const LaunchCtx &lc, const Geom &g, Slots s, Inter in, PotTables t, bool mixed) {
     launch_inter_owner<0>(lc, g, s, in, t, mixed);
 }
-void launch_inter_force(const LaunchCtx &lc, const Geom &g, Slots s, Inter in, PotTables t, bool mixed, StepParams *sp, bool kick) {
-    launch_inter_eam<1>(lc, g, s, in, t, mixed);
+void launch_inter_force_owners(const LaunchCtx &lc, const Geom &g, Slots s, Inter in, PotTables t, bool mixed, StepParams *sp, bool kick) {
     launch_inter_owner<1>(lc, g, s, in, t, mixed, sp, kick);
 }
 void launch_inter_energy(const LaunchCtx &lc, const Geom &g, Slots s, Inter in, PotTables t, bool mixed) {
-    launch_inter_eam<2>(lc, g, s, in, t, mixed);
+    k_inter_eam<2><<<lc.num_sms * 4, kInterThreads, 0, lc.stream>>>(lc.ntd, g, s, in, t, mixed);
     launch_inter_owner<2>(lc, g, s, in, t, mixed);
 }
 
