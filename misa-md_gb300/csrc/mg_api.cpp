@@ -20,11 +20,10 @@ namespace {
 
 thread_local std::string g_create_error;
 
-constexpr int kNumTimers = 10;  // events per timed step; the kernels between consecutive events are:
+constexpr int kNumTimers = 9;  // events per timed step; the kernels between consecutive events are:
 const char *kTimerNames[kNumTimers - 1] = {"firststep",     // the step head (variable dt) and firststep
                                            "inter_manage",  // the list manager
                                            "ghost_copy",    // and the far atoms' marks and the inter atoms' densities
-                                           "fix_records",   // the FP64 form's records
                                            "lat_rho",
                                            "inter_rho",     // the density shares of lattice atoms near inter atoms
                                            "ghost_df",      // and the forces on the inter atoms
@@ -219,26 +218,24 @@ void seq_eam_lists(mg_context *ctx, bool with_manage_prefix, int manage_mask, Ti
 void seq_eam_rho(mg_context *ctx, Timer *t) {
     const LaunchCtx lc = ctx->lc();
     const bool mx = ctx->mixed();
-    launch_fix_records(lc, ctx->g, ctx->s);
-    if (t) t->mark(4);
     const bool advance = launch_lat_rho(lc, ctx->g, ctx->s, ctx->in, ctx->pt, mx, false, true);
-    if (t) t->mark(5);
+    if (t) t->mark(4);
     launch_inter_rho_owners(lc, ctx->g, ctx->s, ctx->in, ctx->pt, mx);
-    if (t) t->mark(6);
+    if (t) t->mark(5);
     launch_ghost_df(lc, ctx->g, ctx->s, ctx->in, ctx->pt, mx, advance);  // and the forces on the inter atoms
-    if (t) t->mark(7);
+    if (t) t->mark(6);
 }
 // the owners' shares of the inter atoms' forces and the second half-kicks left to them, after the lattice force pass
 void seq_eam_force_tail(mg_context *ctx, bool kick, Timer *t) {
     const LaunchCtx lc = ctx->lc();
     launch_inter_force_owners(lc, ctx->g, ctx->s, ctx->in, ctx->pt, ctx->mixed(), ctx->d_sp, kick);
-    if (t) t->mark(9);
+    if (t) t->mark(8);
 }
 void seq_compute_eam(mg_context *ctx, bool kick, bool with_manage_prefix, int manage_mask, Timer *t, bool fuse_next = false) {
     seq_eam_lists(ctx, with_manage_prefix, manage_mask, t);
     seq_eam_rho(ctx, t);
     launch_lat_force(ctx->lc(), ctx->g, ctx->s, ctx->in, ctx->pt, ctx->d_sp, kick, ctx->mixed(), false, fuse_next, true);
-    if (t) t->mark(8);
+    if (t) t->mark(7);
     seq_eam_force_tail(ctx, kick, t);
 }
 // one loop body: firststep, decide, exchangeInter, borderInter, exchangeAtom, computeEam, secondstep.
@@ -248,7 +245,7 @@ void seq_step(mg_context *ctx, Timer *t, bool fused_prev = false, bool fuse_next
     if (t) t->mark(0);
     // a fixed dt needs no head: the list manager keeps the clock
     const bool variable = ctx->dx_max > 0.0;
-    if (variable) launch_step_head(ctx->lc(), ctx->d_sp, ctx->s.skin);
+    if (variable) launch_step_head(ctx->lc(), ctx->d_sp);
     seq_firststep(ctx, true, t, fused_prev);
     seq_compute_eam(ctx, true, true, MANAGE_DECIDE | MANAGE_CLEAR_GHOST | MANAGE_EXCHANGE | MANAGE_BORDER | (variable ? 0 : MANAGE_CLOCK), t,
                     fuse_next);
@@ -314,6 +311,7 @@ void ensure_fix(mg_context *ctx) {
     fp.rho = at[0];
     fp.zg = at[1];
     ctx->fp = fp;
+    launch_fix_records(ctx->lc(), ctx->g, s);
     launch_skin_dirty(ctx->lc(), s);  // FP64 passes before this kept no lists
     ctx->graph_stale = true;  // graphs captured without them
     ctx->gen++;
@@ -724,6 +722,7 @@ mg_status mg_set_precision(mg_context *ctx, int32_t precision) {
     ctx->precision = precision;
     ctx->prepared = false;  // derived arrays (u4, df32) must be rebuilt by an upload
     ctx->gen++;
+    launch_fix_records(ctx->lc(), ctx->g, ctx->s);  // the mixed form does not keep them
     return MG_OK;
 }
 
@@ -813,7 +812,6 @@ static mg_status hook_download(mg_context *ctx, mg_atom_element *atoms, int fiel
 mg_status mg_eam_rho_calc(mg_context *ctx, mg_atom_element *atoms, double cutoff_radius) {
     mg_status st = hook_upload(ctx, atoms, cutoff_radius);
     if (st != MG_OK) return st;
-    launch_fix_records(ctx->lc(), ctx->g, ctx->s);
     launch_lat_rho(ctx->lc(), ctx->g, ctx->s, ctx->in, ctx->pt, ctx->mixed(), true);
     return hook_download(ctx, atoms, PACK_RHO);
 }
@@ -1398,7 +1396,7 @@ static mg_status step_host_overlapped(mg_context *ctx, mg_atom_element *atoms, m
     MG_CK(cudaEventRecord(ctx->pipe_ev[ev], ctx->stream));
     MG_CK(cudaStreamWaitEvent(ctx->copy_in, ctx->pipe_ev[ev++], 0));
     launch_set_counts(lc, ctx->in, 0);
-    launch_step_head(lc, ctx->d_sp, ctx->s.skin);
+    launch_step_head(lc, ctx->d_sp);
     launch_far_clear(lc, g, ctx->in);  // the previous far list's marks, which decide clears
     launch_spec_begin(lc, ctx->in);
     std::vector<size_t> in_ev(S);
@@ -1447,7 +1445,6 @@ static mg_status step_host_overlapped(mg_context *ctx, mg_atom_element *atoms, m
         launch_firststep(lc, g, ctx->s, ctx->in, ctx->d_sp, true, t0, t1);
         launch_spec_decide(lc, g, ctx->s, ctx->in, t0, t1);
         launch_ghost_copy_planes(lc, g, ctx->s, k0, k1);
-        launch_fix_records(lc, g, ctx->s, static_cast<int>((g.gz + k0) * plane), static_cast<int>((g.gz + k1) * plane));
         // slabs 1 .. SS - 2 in order once the planes within 3 of them are in; then the forces of slabs
         // 2 .. SS - 3 whose neighbour slabs have their density, and their finished planes go out
         while (next_rho <= SS - 2 && last_plane(next_rho) + 3 < k1) {
@@ -1472,8 +1469,6 @@ static mg_status step_host_overlapped(mg_context *ctx, mg_atom_element *atoms, m
     }
     // the seam: ghost planes, the end slabs' density and ghost df, then their forces
     launch_ghost_copy_planes(lc, g, ctx->s, -1, -1);
-    launch_fix_records(lc, g, ctx->s, 0, static_cast<int>(g.gz * plane));
-    launch_fix_records(lc, g, ctx->s, static_cast<int>((g.gz + K) * plane), g.n_slots);
     rho_slab(0);
     rho_slab(SS - 1);
     launch_ghost_df_planes(lc, g, ctx->s, ctx->in, mx, 0, planes_from(1));
@@ -1577,7 +1572,7 @@ static mg_status step_host_pipelined(mg_context *ctx, mg_atom_element *atoms, mg
     MG_CK(cudaEventRecord(ctx->pipe_ev[ev], ctx->stream));
     MG_CK(cudaStreamWaitEvent(ctx->copy_in, ctx->pipe_ev[ev++], 0));
     launch_set_counts(lc, ctx->in, 0);
-    launch_step_head(lc, ctx->d_sp, ctx->s.skin);
+    launch_step_head(lc, ctx->d_sp);
     for (int c = 0; c < S; c++) {
         const int z0 = c == 0 ? 0 : g.gz + local_plane_bound(c);
         const int z1 = c == S - 1 ? g.Sz : g.gz + local_plane_bound(c + 1);
@@ -1656,7 +1651,6 @@ static mg_status step_host_pipelined(mg_context *ctx, mg_atom_element *atoms, mg
             launch_ghost_df_planes(lc, g, ctx->s, ctx->in, mx, df_done, k);
             df_done = k;
         };
-        launch_fix_records(lc, g, ctx->s);
         rho_slab(0);
         rho_slab(1);
         // planes of slabs 1 .. S - 2 go out after their force; the plane cut by u[1] waits for slab 0
@@ -1803,7 +1797,6 @@ mg_status mg_autotune(mg_context *ctx, int32_t reps, int32_t out[6]) {
                 ctx->tune[p][kern][2] = apt;
                 const LaunchCtx lc = ctx->lc();
                 auto run = [&]() {
-                    if (kern == 0) launch_fix_records(lc, ctx->g, ctx->s);
                     if (kern == 0) launch_lat_rho(lc, ctx->g, ctx->s, ctx->in, ctx->pt, ctx->mixed(), false);
                     else launch_lat_force(lc, ctx->g, ctx->s, ctx->in, ctx->pt, ctx->d_sp, false, ctx->mixed(), false);
                 };

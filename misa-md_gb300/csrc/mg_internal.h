@@ -95,6 +95,7 @@ struct SkinState {
     int dirty;                       // a record changed outside firststep: the next pass rebuilds
     int rebuilt;                     // the last density pass rebuilt every group's list
     int wild;                        // FP64 form: an atom is too far from its site for the fixed-point records
+    int wild_next;                   // the same of the positions of the firststep just taken, until decide
     unsigned long long rebuilds;     // density passes that rebuilt every group's list
     unsigned long long passes;       // density passes with the group lists
 };
@@ -116,7 +117,9 @@ struct Slots {
     SkinState *skin;
     float *df32;             // F'(rho) in float
     // FP64 form, the same layout (null: the passes run in FP64 throughout):
-    FixRec *fix;             // fixed-point coordinates and type of the positions the density pass is about to read
+    FixRec *fix;             // fixed-point coordinates and type
+    int kx;                  // of a launch that keeps them: their unit's exponent (0: not kept)
+    int wild_now;            // of a firststep over part of the box: SkinState::wild holds at once
     i64 *dfq;                // F'(rho) in fixed point, written wherever df is
 };
 
@@ -284,9 +287,8 @@ void launch_firststep(const LaunchCtx &lc, const Geom &g, Slots s, Inter in, con
 // fill g.site_half (once per context)
 void launch_site_table(const LaunchCtx &lc, const Geom &g, double *site_half);
 void launch_decide_scan(const LaunchCtx &lc, const Geom &g, Slots s, Inter in);
-// FP64 form: the fixed-point records of the slots [s0, s1) (s1 < 0: to the end), after every change of a
-// position and before the density pass (the force hook: before the force pass)
-void launch_fix_records(const LaunchCtx &lc, const Geom &g, Slots s, int s0 = 0, int s1 = -1);
+// FP64 form: the fixed-point records of every slot, when their tables are made after the state came in
+void launch_fix_records(const LaunchCtx &lc, const Geom &g, Slots s);
 // far-atom neighbourhood marks: clear those of the current far list / set them (grid-wide)
 void launch_far_clear(const LaunchCtx &lc, const Geom &g, Inter in);
 void launch_far_mark(const LaunchCtx &lc, const Geom &g, Inter in);
@@ -334,7 +336,7 @@ void launch_lat_force_sites(const LaunchCtx &lc, const Geom &g, Slots s, Inter i
 // the second half-kick as a phase of its own (lattice and inter atoms)
 void launch_secondstep(const LaunchCtx &lc, const Geom &g, Slots s, Inter in, StepParams *sp);
 // step head: records the step's dt and, in variable mode, sets dt from the last kick's max |v|
-void launch_step_head(const LaunchCtx &lc, StepParams *sp, SkinState *skin);
+void launch_step_head(const LaunchCtx &lc, StepParams *sp);
 // out[0] = steps taken, out[1] = simulated time
 void launch_clock_sample(const LaunchCtx &lc, const StepParams *sp, double *out);
 // set the timestep rule and dt / dt/(2m) (dx_max <= 0: fixed dt)

@@ -343,6 +343,41 @@ __device__ __forceinline__ void kahan(float &sum, float &comp, float term) {
 }
 
 // ------------------------------------------------------------------------------------------------
+// Fixed-point records of the FP64 form (mg_fixed.h), kept beside the positions where s.kx is set: whoever changes a
+// position writes its slot's record. A candidate then costs one 32-byte load instead of three 8-byte loads and three
+// conversions per pair, and no pass over the slots makes the records (35 us of a step of 2.0 ms at 2M atoms, 4 us of
+// 55 at 16k).
+// ------------------------------------------------------------------------------------------------
+__device__ __forceinline__ void fix_store(FixRec *to, i64 x, i64 y, i64 z, i64 type) {
+    longlong2 *o = reinterpret_cast<longlong2 *>(to);
+    o[0] = make_longlong2(x, y);
+    o[1] = make_longlong2(z, type);
+}
+__device__ __forceinline__ void fix_put(FixRec *to, int kx, double x, double y, double z, int type) {
+    fix_store(to, fix_coord(x, kx), fix_coord(y, kx), fix_coord(z, kx), type);
+}
+// a vacant slot's: half a period away from its site
+__device__ __forceinline__ void fix_put_vacant(const Geom &g, FixRec *to, int kx, int sl) {
+    const int X = sl % g.Sx, q = sl / g.Sx, Y = q % g.Sy, Z = q / g.Sy;
+    double xs, ys, zs;
+    site_of(g, X, Y, Z, xs, ys, zs);
+    const unsigned long long away = 1ull << 63;
+    fix_store(to, (i64) ((unsigned long long) fix_coord(xs, kx) ^ away), (i64) ((unsigned long long) fix_coord(ys, kx) ^ away),
+              (i64) ((unsigned long long) fix_coord(zs, kx) ^ away), kInvalid);
+}
+// too far from its site for the wrapped coordinates: 1.2 half-lattice units (recombined atoms sit up to
+// sqrt(5) / 2 of them from their site)
+__device__ __forceinline__ bool fix_wild(float4 u) {
+    return !(fmaxf(fmaxf(fabsf(u.x), fabsf(u.y)), fabsf(u.z)) <= 1.2f) || u.x != u.x || u.y != u.y || u.z != u.z;
+}
+// with the FP64 form's records (off when the launch's form keeps none)
+inline Slots with_records(const LaunchCtx &lc, Slots s) {
+    s.kx = lc.fp ? lc.fp->kx : 0;
+    s.wild_now = 0;
+    return s;
+}
+
+// ------------------------------------------------------------------------------------------------
 // AoS <-> SoA (the reference's AtomElement array crosses the boundary as raw records)
 // ------------------------------------------------------------------------------------------------
 __global__ void k_unpack_aos(Geom g, const mg_atom_element *aos, Slots s, Inter in, int types_ok_mask, bool mixed, int s0,
@@ -364,7 +399,14 @@ __global__ void k_unpack_aos(Geom g, const mg_atom_element *aos, Slots s, Inter 
         const int X = t % g.Sx, r = t / g.Sx, Y = r % g.Sy, Z = r / g.Sy;
         double xs, ys, zs;
         site_of(g, X, Y, Z, xs, ys, zs);
-        s.u4[sidx(g, t)] = a.type < 0 ? vacant_u4() : make_u4(g, a.x[0], a.x[1], a.x[2], xs, ys, zs, a.type);
+        const float4 u = a.type < 0 ? vacant_u4() : make_u4(g, a.x[0], a.x[1], a.x[2], xs, ys, zs, a.type);
+        const int si = sidx(g, t);
+        s.u4[si] = u;
+        if (s.kx && a.type < 0) fix_put_vacant(g, s.fix + si, s.kx, t);
+        else if (s.kx) {
+            fix_put(s.fix + si, s.kx, a.x[0], a.x[1], a.x[2], a.type);
+            if (fix_wild(u)) s.skin->wild = 1;
+        }
     }
     if (mixed) s.df32[sidx(g, t)] = (float) a.df;
     else if (fp.on) s.dfq[sidx(g, t)] = fix_df(fp, a.df);
@@ -398,9 +440,9 @@ void launch_unpack_aos(const LaunchCtx &lc, const Geom &g, const mg_atom_element
     if (s1 < 0) s1 = g.n_slots;
     if (s1 <= s0) return;
     const int b = 256;
-    k_unpack_aos<<<(s1 - s0 + b - 1) / b, b, 0, lc.stream>>>(g, aos, s, in, types_ok_mask, mixed, s0, s1, fix_params(lc));
+    if (lc.fp && s0 == 0) cudaMemsetAsync(&s.skin->wild, 0, 2 * sizeof(int), lc.stream);  // a state's first part
+    k_unpack_aos<<<(s1 - s0 + b - 1) / b, b, 0, lc.stream>>>(g, aos, with_records(lc, s), in, types_ok_mask, mixed, s0, s1, fix_params(lc));
     launch_skin_dirty(lc, s);
-    if (lc.fp) cudaMemsetAsync(&s.skin->wild, 0, sizeof(int), lc.stream);
 }
 __global__ void k_set_counts(Inter in, int n_inter) {
     in.cnt[CNT_INTER] = n_inter;
@@ -490,6 +532,13 @@ __device__ __forceinline__ void first_half(const Geom &g, const Slots &s, const 
             skin_note(s, dx * dx + dy * dy + dz * dz);
         }
         u4_out[si] = nu;
+        if (s.kx) {
+            fix_put(s.fix + si, s.kx, x, y, z, ty);
+            if (fix_wild(nu)) {
+                s.skin->wild_next = 1;
+                if (s.wild_now) s.skin->wild = 1;
+            }
+        }
     }
     if (DECIDE) {
         // the exact FP64 test of decide runs only where the FP32 distance is not clearly below it
@@ -556,6 +605,7 @@ __global__ void __launch_bounds__(kFirstThreads) k_firststep(const NeighTables *
         const int ty = s.type[sl];
         if (ty < 0) {
             if (MOVE) s.u4[sidx(g, sl)] = vacant_u4();
+            if (MOVE && s.kx) fix_put_vacant(g, s.fix + sidx(g, sl), s.kx, sl);
             continue;
         }
         if (MOVE)
@@ -609,6 +659,8 @@ void launch_firststep(const LaunchCtx &lc, const Geom &g, Slots s, Inter in, con
     if (whole) t1 = g.n_local;
     if (t1 <= t0) return;
     const int b = kFirstThreads, n = std::min((t1 - t0 + b - 1) / b, lc.num_sms * 8);
+    s = with_records(lc, s);
+    s.wild_now = !whole;  // a part's passes may come before the list manager
     if (decide) k_firststep<true, true><<<n, b, 0, lc.stream>>>(lc.ntd, g, s, in, p, t0, t1, fused, alt, whole);
     else k_firststep<true, false><<<n, b, 0, lc.stream>>>(lc.ntd, g, s, in, p, t0, t1, fused, alt, whole);
 }
@@ -665,11 +717,16 @@ __device__ __forceinline__ void ghost_copy_one(const Geom &g, const Slots &s, in
     const int X = gs % g.Sx, r = gs / g.Sx, Y = r % g.Sy, Z = r / g.Sy;
     int sx, sy, sz;
     const int os = lin(g, wrap_axis(X, g.gx, g.bx, sx), wrap_axis(Y, g.gy, g.by, sy), wrap_axis(Z, g.gz, g.bz, sz));
-    s.type[gs] = s.type[os];
-    s.x[gs] = shifted(s.x[os], sx, g.L[0]);
-    s.y[gs] = shifted(s.y[os], sy, g.L[1]);
-    s.z[gs] = shifted(s.z[os], sz, g.L[2]);
-    s.u4[sidx(g, gs)] = s.u4[sidx(g, os)];
+    const int type = s.type[os];
+    const double x = shifted(s.x[os], sx, g.L[0]), y = shifted(s.y[os], sy, g.L[1]), z = shifted(s.z[os], sz, g.L[2]);
+    s.type[gs] = (int8_t) type;
+    s.x[gs] = x;
+    s.y[gs] = y;
+    s.z[gs] = z;
+    const int si = sidx(g, gs);
+    s.u4[si] = s.u4[sidx(g, os)];
+    if (s.kx && type < 0) fix_put_vacant(g, s.fix + si, s.kx, gs);
+    else if (s.kx) fix_put(s.fix + si, s.kx, x, y, z, type);
 }
 // The ghost slots inside the local planes [k0, k1) (y-ghost rows, then x-ghost columns of each plane;
 // their owners lie in the same plane), or (k0 < 0) the ghost planes below and above the box, whose
@@ -699,7 +756,7 @@ void launch_ghost_copy_planes(const LaunchCtx &lc, const Geom &g, Slots s, int k
     const int b = 256;
     const int work = k0 < 0 ? 2 * g.gz * g.Sy * g.Sx : (k1 - k0) * (2 * g.gy * g.Sx + 2 * g.gx * g.by);
     if (work <= 0) return;
-    k_ghost_copy_planes<<<(work + b - 1) / b, b, 0, lc.stream>>>(g, s, k0, k1);
+    k_ghost_copy_planes<<<(work + b - 1) / b, b, 0, lc.stream>>>(g, with_records(lc, s), k0, k1);
 }
 
 // forward df (DfEmbedPacker, src/pack/df_embed_packer.cpp): lattice ghosts and ghost inter atoms
@@ -1207,41 +1264,22 @@ __global__ void __launch_bounds__(32 * W) k_lat_rho_mixed_split(const float4 *ca
 // range, is done in FP64 altogether, and so is every atom of a pass while some atom is too far from its
 // site for the wrapped coordinates (an uploaded state before its first decide).
 // ------------------------------------------------------------------------------------------------
-// The records of the slots [s0, s1): 25 bytes read and 32 written per slot, bound by HBM (0.2 ms at 16M
-// atoms of a 10 ms step), so that a candidate costs one 32-byte load instead of three 8-byte loads and
-// three conversions per pair.
-__global__ void k_fix_records(Geom g, Slots s, FixParams fp, int s0, int s1) {
-    const int t = s0 + blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= s1) return;
-    const int si = sidx(g, t);
-    const float4 u = s.u4[si];
-    const int ty = __float_as_int(u.w);
-    FixRec r;
-    r.type = ty;
-    if (ty >= 0) {
-        r.x = fix_coord(s.x[t], fp.kx);
-        r.y = fix_coord(s.y[t], fp.kx);
-        r.z = fix_coord(s.z[t], fp.kx);
-        // 1.2 half-lattice units: recombined atoms sit up to sqrt(5) / 2 of them from their site
-        if (!(fmaxf(fmaxf(fabsf(u.x), fabsf(u.y)), fabsf(u.z)) <= 1.2f) || u.x != u.x || u.y != u.y || u.z != u.z) s.skin->wild = 1;
-    } else {
-        const int X = t % g.Sx, q = t / g.Sx, Y = q % g.Sy, Z = q / g.Sy;
-        double xs, ys, zs;
-        site_of(g, X, Y, Z, xs, ys, zs);
-        const unsigned long long away = 1ull << 63;
-        r.x = (i64) ((unsigned long long) fix_coord(xs, fp.kx) ^ away);
-        r.y = (i64) ((unsigned long long) fix_coord(ys, fp.kx) ^ away);
-        r.z = (i64) ((unsigned long long) fix_coord(zs, fp.kx) ^ away);
+// the records of every slot, for tables made after the state came in
+__global__ void k_fix_records(Geom g, Slots s) {
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= g.n_slots) return;
+    const int si = sidx(g, t), ty = s.type[t];
+    if (ty < 0) {
+        fix_put_vacant(g, s.fix + si, s.kx, t);
+        return;
     }
-    longlong2 *o = reinterpret_cast<longlong2 *>(s.fix + si);
-    o[0] = make_longlong2(r.x, r.y);
-    o[1] = make_longlong2(r.z, r.type);
+    fix_put(s.fix + si, s.kx, s.x[t], s.y[t], s.z[t], ty);
+    if (fix_wild(s.u4[si])) s.skin->wild = 1;
 }
-void launch_fix_records(const LaunchCtx &lc, const Geom &g, Slots s, int s0, int s1) {
+void launch_fix_records(const LaunchCtx &lc, const Geom &g, Slots s) {
     if (!lc.fp) return;
-    if (s1 < 0) s1 = g.n_slots;
-    if (s1 <= s0) return;
-    k_fix_records<<<(s1 - s0 + 255) / 256, 256, 0, lc.stream>>>(g, s, *lc.fp, s0, s1);
+    cudaMemsetAsync(&s.skin->wild, 0, 2 * sizeof(int), lc.stream);
+    k_fix_records<<<(g.n_slots + 255) / 256, 256, 0, lc.stream>>>(g, with_records(lc, s));
 }
 
 // one 32-byte read-only load each
@@ -2307,7 +2345,6 @@ static bool launch_lat_force_split(const LaunchCtx &lc, const Geom &g, Slots s, 
 }
 void launch_lat_force(const LaunchCtx &lc, const Geom &g, Slots s, Inter in, PotTables t, StepParams *p, bool kick,
                       bool mixed, bool hook, bool fuse_next, bool lists) {
-    if (hook && !mixed) launch_fix_records(lc, g, s);
     const bool v = lists && has_lists(lc, mixed) && !hook && lists_ok(lc, g);
     if (launch_lat_force_split(lc, g, s, in, t, p, kick, mixed, hook, 0, g.n_local_half, fuse_next, v)) return;
     launch_lat_force_threads(lc, g, s, in, t, p, kick, mixed, hook, 0, gather_threads(g, lc.force_order), fuse_next, v);
@@ -2385,8 +2422,7 @@ void launch_set_step(const LaunchCtx &lc, StepParams *sp, double dt, double dx_m
     k_set_step<<<1, 1, 0, lc.stream>>>(sp, dt, dx_max, dt_min, dt_max);
 }
 // The timestep taken into the history and the clock; one thread, once a step.
-__device__ __forceinline__ void step_record(StepParams *p, SkinState *skin) {
-    skin->wild = 0;  // the step's records find out again
+__device__ __forceinline__ void step_record(StepParams *p) {
     const long long k = p->steps;
     p->hist[k % kDtHistory] = p->dt;
     p->time = __dadd_rn(p->time, p->dt);
@@ -2395,7 +2431,7 @@ __device__ __forceinline__ void step_record(StepParams *p, SkinState *skin) {
 
 // One block of kVmaxSlots threads, ahead of a step: reduce and clear the max words, then (variable mode)
 // dt = clamp(dx_max / sqrt(max |v|^2), dt_min, dt_max); record dt and advance the clock.
-__global__ void __launch_bounds__(kVmaxSlots) k_step_head(StepParams *p, SkinState *skin) {
+__global__ void __launch_bounds__(kVmaxSlots) k_step_head(StepParams *p) {
     __shared__ unsigned long long part[kVmaxSlots / 32];
     const unsigned long long b = p->vmax2[threadIdx.x];
     p->vmax2[threadIdx.x] = 0ull;
@@ -2414,10 +2450,10 @@ __global__ void __launch_bounds__(kVmaxSlots) k_step_head(StepParams *p, SkinSta
         if (dt > p->dt_max) dt = p->dt_max;
         set_dt_dev(p, dt);
     }
-    step_record(p, skin);
+    step_record(p);
 }
-void launch_step_head(const LaunchCtx &lc, StepParams *sp, SkinState *skin) {
-    k_step_head<<<1, kVmaxSlots, 0, lc.stream>>>(sp, skin);
+void launch_step_head(const LaunchCtx &lc, StepParams *sp) {
+    k_step_head<<<1, kVmaxSlots, 0, lc.stream>>>(sp);
 }
 // steps taken and simulated time into a sample record (stage machine thermo output)
 __global__ void k_clock_sample(const StepParams *p, double *out) {
@@ -2743,7 +2779,11 @@ __device__ __forceinline__ void border_put(Inter &in, int q, const double p3[3],
 __global__ void __launch_bounds__(kManageThreads) k_inter_manage(Geom g, Slots s, Inter in, int mask, bool mixed, StepParams *sp) {
     extern __shared__ long long sm_keys[];
     const int tid = threadIdx.x, nthr = blockDim.x;
-    if ((mask & MANAGE_CLOCK) && tid == 0) step_record(sp, s.skin);
+    if ((mask & MANAGE_CLOCK) && tid == 0) step_record(sp);
+    if ((mask & MANAGE_DECIDE) && s.kx && tid == 0) {  // the positions are firststep's now
+        s.skin->wild = s.skin->wild_next;
+        s.skin->wild_next = 0;
+    }
 
     // The list counts are read once, by all threads before any is written, and then followed in
     // registers: every change to them is block-uniform (scan totals), and one global round trip
@@ -2795,6 +2835,7 @@ __global__ void __launch_bounds__(kManageThreads) k_inter_manage(Geom g, Slots s
                 s.type[sl] = kInvalid;
                 s.vx[sl] = 0.0; s.vy[sl] = 0.0; s.vz[sl] = 0.0;
                 s.u4[sidx(g, sl)] = vacant_u4();
+                if (s.kx) fix_put_vacant(g, s.fix + sidx(g, sl), s.kx, sl);
             }
             __syncthreads();
             n_inter = n0 + nd;
@@ -2838,6 +2879,7 @@ __global__ void __launch_bounds__(kManageThreads) k_inter_manage(Geom g, Slots s
                     double xs, ys, zs;
                     site_of(g, X, Y, Z, xs, ys, zs);
                     s.u4[sidx(g, sl)] = make_u4(g, in.x[a], in.y[a], in.z[a], xs, ys, zs, in.type[a]);
+                    if (s.kx) fix_put(s.fix + sidx(g, sl), s.kx, in.x[a], in.y[a], in.z[a], in.type[a]);
                 }
                 // A recombined atom may sit up to sqrt(5)/4 a0 from its new site. Every recombined atom
                 // joins this step's far list: the marks on its neighbourhood also make the density pass
@@ -3016,7 +3058,7 @@ void configure_manage_kernel() {
                          static_cast<int>(kSortSmemKeys * sizeof(long long)));
 }
 void launch_inter_manage(const LaunchCtx &lc, const Geom &g, Slots s, Inter in, int mask, bool mixed, StepParams *sp) {
-    k_inter_manage<<<1, kManageThreads, kSortSmemKeys * sizeof(long long), lc.stream>>>(g, s, in, mask, mixed, sp);
+    k_inter_manage<<<1, kManageThreads, kSortSmemKeys * sizeof(long long), lc.stream>>>(g, with_records(lc, s), in, mask, mixed, sp);
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -3227,7 +3269,7 @@ __global__ void __launch_bounds__(kInterThreads) k_ghost_copy(const NeighTables 
 }
 void launch_ghost_copy(const LaunchCtx &lc, const Geom &g, Slots s, Inter in, PotTables t, bool mixed, bool mark, bool inter) {
     const int n = (g.n_ghost_slots + kInterThreads - 1) / kInterThreads, e = inter ? inter_blocks(lc, g) : 0;
-    k_ghost_copy<<<n + e, kInterThreads, 0, lc.stream>>>(lc.ntd, g, s, in, t, mixed, mark, e);
+    k_ghost_copy<<<n + e, kInterThreads, 0, lc.stream>>>(lc.ntd, g, with_records(lc, s), in, t, mixed, mark, e);
 }
 // The copy of F' and what only needs F' of the box's own atoms: (advance) after a density pass with the group lists,
 // as launch_skin_advance; (inter_n blocks past the ghost slots') the forces on the inter atoms.
