@@ -82,6 +82,7 @@ struct mg_context {
     int fuse_steps = 16;
     cudaGraphExec_t graph_multi = nullptr;
     float4 *u4_main = nullptr, *u4_alt = nullptr;  // s.u4 and s.u4n outside fused graphs
+    FixRec *fix_main = nullptr, *fix_alt = nullptr;  // s.fix and s.fixn
     bool alt_bodies = false;        // capturing bodies that alternate u4 buffers
     bool graph_stale = true;
     uint64_t gen = 1;               // bumped whenever captured graphs of this context go stale
@@ -251,15 +252,18 @@ void seq_step(mg_context *ctx, Timer *t, bool fused_prev = false, bool fuse_next
                     fuse_next);
 }
 // steps of mg_simulate that run fused: the mixed form with a fixed dt
-bool fusable(const mg_context *ctx) { return ctx->fuse_steps >= 2 && ctx->mixed() && ctx->dx_max <= 0.0; }
-// Loop bodies in one graph launch (0: one body per launch). Bodies that are not fused still save the gap between two
-// launches, about 3 us (16k atoms FP64 58.0 -> 55.4 us per step with 4, 55.0 with 16; a graph of 4 costs 0.1 ms to
-// make, which runs of kMultiRun steps win back).
-constexpr int kPlainBodies = 4, kMultiRun = 40;
+bool fusable(const mg_context *ctx) { return ctx->fuse_steps >= 2 && (ctx->mixed() || ctx->lc().fp) && ctx->dx_max <= 0.0; }
+// Loop bodies in one graph launch of a run of that many steps (0: one body per launch). The mixed form: fuse_steps
+// fused bodies. The others kPlainBodies, since a graph costs about 25 us a body to make and their runs are short: bodies
+// of the FP64 form that are fused save a firststep each (2M atoms: 1959 -> 1926 us per step), and any saves the gap between two
+// launches, about 3 us (16k atoms FP64, per step: 58.0 -> 55.4 us with 4 bodies, 55.0 with 16).
+constexpr int kPlainBodies = 4;
+int multi_bodies(const mg_context *ctx) { return ctx->mixed() && fusable(ctx) ? ctx->fuse_steps : kPlainBodies; }
 int multi_steps(const mg_context *ctx, int64_t run) {
     if (ctx->fuse_steps < 2) return 0;
-    if (fusable(ctx)) return ctx->fuse_steps;
-    return ctx->graph_multi || run >= kMultiRun ? kPlainBodies : 0;
+    const bool pays = ctx->graph_multi || (ctx->mixed() && fusable(ctx)) || run >= 40 ||
+                      (fusable(ctx) && (run >= 20 || run * ctx->g.n_local >= 4000000));
+    return pays ? multi_bodies(ctx) : 0;
 }
 constexpr int kLaunchesPerStep = 8;
 
@@ -268,7 +272,7 @@ mg_status require_ready(mg_context *ctx) {
     return MG_OK;
 }
 
-// The FP64 form's fixed-point tables and arrays (40 bytes per slot), made for the first FP64 state that comes
+// The FP64 form's fixed-point tables and arrays (72 bytes per slot), made for the first FP64 state that comes
 // in under a potential. Where the tables do not suit the potential, or the arrays do not fit the device,
 // the passes run in FP64.
 void ensure_fix(mg_context *ctx) {
@@ -283,9 +287,10 @@ void ensure_fix(mg_context *ctx) {
     Slots &s = ctx->s;
     const size_t ns = static_cast<size_t>(ctx->g.n_slots);
     const size_t n[2] = {ft.rho.size(), ft.zg.size()};
-    void *tab = nullptr, *rec = s.fix, *df = s.dfq;
+    void *tab = nullptr, *rec = s.fix, *next = s.fixn, *df = s.dfq;
     cudaError_t e = cudaMalloc(&tab, (n[0] + n[1]) * sizeof(FixPoly));
     if (e == cudaSuccess && !rec) e = cudaMalloc(&rec, ns * sizeof(FixRec));
+    if (e == cudaSuccess && !next) e = cudaMalloc(&next, ns * sizeof(FixRec));
     if (e == cudaSuccess && !df) e = cudaMalloc(&df, ns * sizeof(i64));
     FixPoly *d = static_cast<FixPoly *>(tab);
     const FixPoly *src[2] = {ft.rho.data(), ft.zg.data()};
@@ -300,12 +305,15 @@ void ensure_fix(mg_context *ctx) {
         cudaGetLastError();
         cudaFree(tab);
         if (rec != s.fix) cudaFree(rec);
+        if (next != s.fixn) cudaFree(next);
         if (df != s.dfq) cudaFree(df);
         return;
     }
     if (!s.fix) ctx->dev_allocs.push_back(rec);
+    if (!s.fixn) ctx->dev_allocs.push_back(next);
     if (!s.dfq) ctx->dev_allocs.push_back(df);
-    s.fix = static_cast<FixRec *>(rec);
+    s.fix = ctx->fix_main = static_cast<FixRec *>(rec);
+    s.fixn = ctx->fix_alt = static_cast<FixRec *>(next);
     s.dfq = static_cast<i64 *>(df);
     ctx->fix_mem = tab;
     fp.rho = at[0];
@@ -481,12 +489,14 @@ mg_status build_graph(mg_context *ctx) {
     return MG_OK;
 }
 
-// The u4 buffers of body i of k fused bodies: its own and the next body's alternate, and the last
-// body's own is the context's usual one, so between launches u4 is where every other call expects it.
+// The u4 and fix buffers of body i of k fused bodies: its own and the next body's alternate, and the last
+// body's own are the context's usual ones, so between launches they are where every other call expects them.
 void set_body_buffers(mg_context *ctx, int64_t k, int64_t i) {
     const bool own_is_main = ((k - 1 - i) % 2) == 0;
     ctx->s.u4 = own_is_main ? ctx->u4_main : ctx->u4_alt;
     ctx->s.u4n = own_is_main ? ctx->u4_alt : ctx->u4_main;
+    ctx->s.fix = own_is_main ? ctx->fix_main : ctx->fix_alt;
+    ctx->s.fixn = own_is_main ? ctx->fix_alt : ctx->fix_main;
 }
 
 // Several loop bodies in one graph. Fused, the first takes its own firststep, the last does not take the
@@ -496,7 +506,7 @@ mg_status build_graph_multi(mg_context *ctx) {
     if (st != MG_OK || ctx->graph_multi) return st;
     cudaGraph_t graph;
     MG_CK(cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
-    const int k = fusable(ctx) ? ctx->fuse_steps : kPlainBodies;
+    const int k = multi_bodies(ctx);
     if (fusable(ctx)) {
         ctx->alt_bodies = true;
         for (int i = 0; i < k; i++) {
@@ -1015,7 +1025,7 @@ mg_status mg_simulate(mg_context *ctx, int64_t nsteps, int32_t sync) {
         }
         // the same fusion pattern as the graphs: blocks of fuse_steps bodies, then single bodies
         const bool fuse = fusable(ctx) && nsteps >= 2;
-        const int64_t k = fuse ? ctx->fuse_steps : 1, blocks = fuse ? nsteps / k : 0;
+        const int64_t k = fuse ? multi_bodies(ctx) : 1, blocks = fuse ? nsteps / k : 0;
         for (int64_t i = 0; i < nsteps; i++) {
             Timer t{ctx, i};
             const bool in_block = i < blocks * k;

@@ -118,6 +118,7 @@ struct Slots {
     float *df32;             // F'(rho) in float
     // FP64 form, the same layout (null: the passes run in FP64 throughout):
     FixRec *fix;             // fixed-point coordinates and type
+    FixRec *fixn;            // the next loop body's buffer when the force pass takes the next firststep
     int kx;                  // of a launch that keeps them: their unit's exponent (0: not kept)
     int wild_now;            // of a firststep over part of the box: SkinState::wild holds at once
     i64 *dfq;                // F'(rho) in fixed point, written wherever df is
@@ -325,8 +326,8 @@ void launch_spec_decide(const LaunchCtx &lc, const Geom &g, Slots s, Inter in, i
 // CNT_FAR = 0 and CNT_SPEC_VOID = 0 (after the previous far list's marks are cleared)
 void launch_spec_begin(const LaunchCtx &lc, Inter in);
 void launch_lat_df(const LaunchCtx &lc, const Geom &g, Slots s, PotTables t, bool mixed);
-// fuse_next (mixed form, kick, fixed dt): after the second half-kick each lattice atom also takes the
-// next step's firststep (into u4n), when no inter atoms exist
+// fuse_next (kick, fixed dt; not the FP64 loops): after the second half-kick each lattice atom also takes the
+// next step's firststep (into u4n and fixn), when no inter atoms exist
 void launch_lat_force(const LaunchCtx &lc, const Geom &g, Slots s, Inter in, PotTables t, StepParams *sp, bool kick,
                       bool mixed, bool hook, bool fuse_next = false, bool lists = false);
 // the force pass over the sites of both parities whose index within their parity is in [u0, u1):

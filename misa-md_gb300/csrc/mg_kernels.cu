@@ -502,7 +502,7 @@ __device__ __forceinline__ void skin_note(const Slots &s, float d2) {
 template <bool MOVE, bool DECIDE>
 __device__ __forceinline__ void first_half(const Geom &g, const Slots &s, const Inter &in, const StepParams *__restrict__ p,
                                            int sl, int t, int i, int j, int k, int ty, double vx, double vy, double vz,
-                                           double fx, double fy, double fz, float4 *u4_out, const float4 *u4_prev) {
+                                           double fx, double fy, double fz, float4 *u4_out, const float4 *u4_prev, FixRec *fix_out) {
     double x = s.x[sl], y = s.y[sl], z = s.z[sl];
     if (MOVE) {
         const double c = dt_inv_m_of(p, ty);
@@ -533,7 +533,7 @@ __device__ __forceinline__ void first_half(const Geom &g, const Slots &s, const 
         }
         u4_out[si] = nu;
         if (s.kx) {
-            fix_put(s.fix + si, s.kx, x, y, z, ty);
+            fix_put(fix_out + si, s.kx, x, y, z, ty);
             if (fix_wild(nu)) {
                 s.skin->wild_next = 1;
                 if (s.wild_now) s.skin->wild = 1;
@@ -578,8 +578,8 @@ __device__ __forceinline__ void inter_firststep(const Inter &in, const StepParam
 }
 
 // fused: the previous step's force pass already took this firststep for every local slot and wrote
-// its displacement records into this step's u4 buffer (when no inter atoms exist; else the work is
-// done here). Every local slot's u4 is written, vacancies included, so the two buffers a fused graph
+// its displacement records into this step's u4 buffer, and the FP64 form's records into this step's fix buffer
+// (when no inter atoms exist; else the work is done here). Every local slot's u4 is written, vacancies included, so the two buffers a fused graph
 // alternates between are always complete.
 // alt: inside a graph whose bodies alternate their u4 buffers, where the previous body's records are
 // in s.u4n
@@ -598,7 +598,7 @@ __global__ void __launch_bounds__(kFirstThreads) k_firststep(const NeighTables *
         inter_firststep(in, p, tid, stride);
         if (DECIDE) mark_far_neighbourhoods(*nt, g, in, 0, min(in.cnt[CNT_FAR], in.fcap), 0, tid, stride);
     }
-    if (fused && lattice_only(in)) return;
+    if (fused && lattice_only(in) && !(s.kx && s.skin->wild)) return;  // wild: as the force pass saw it
     for (int t = t0 + tid; t < t1; t += stride) {
         int i, j, k;
         const int sl = local_slot(g, t, i, j, k);
@@ -610,9 +610,9 @@ __global__ void __launch_bounds__(kFirstThreads) k_firststep(const NeighTables *
         }
         if (MOVE)
             first_half<true, DECIDE>(g, s, in, p, sl, t, i, j, k, ty, s.vx[sl], s.vy[sl], s.vz[sl], s.fx[sl], s.fy[sl],
-                                     s.fz[sl], s.u4, alt ? s.u4n : s.u4);
+                                     s.fz[sl], s.u4, alt ? s.u4n : s.u4, s.fix);
         else
-            first_half<false, DECIDE>(g, s, in, p, sl, t, i, j, k, ty, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, s.u4, s.u4);
+            first_half<false, DECIDE>(g, s, in, p, sl, t, i, j, k, ty, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, s.u4, s.u4, s.fix);
     }
 }
 
@@ -1759,17 +1759,33 @@ __device__ __forceinline__ void force_atom_fp64(const NeighTables &nt, const Geo
         else force_sum_fp64<0>(nt, g, s, pt, sl, ti, si, ui, xi, yi, zi, dfi, np, nf, fx, fy, fz);
     }
 }
-// stores the force and takes the second half-kick where the lattice pass may
-__device__ __forceinline__ void force_done_fp64(const Slots &s, const Inter &in, StepParams *sp, int sl, int ti, double fx,
-                                                double fy, double fz, bool kick, bool hook) {
-    s.fx[sl] = fx; s.fy[sl] = fy; s.fz[sl] = fz;
+// local coordinates and local index (k, j, i order) of a local slot
+__device__ __forceinline__ int local_index_of(const Geom &g, int sl, int &i, int &j, int &k) {
+    const int X = sl % g.Sx, r = sl / g.Sx;
+    i = X - g.gx;
+    j = r % g.Sy - g.gy;
+    k = r / g.Sy - g.gz;
+    return (k * g.by + j) * g.bx + i;
+}
+// Stores the force and takes the second half-kick where the lattice pass may; fused: also the next body's firststep.
+// A fused body's forces are used only in registers: the next body's firststep is taken here, and the last body of a
+// graph (never fused) stores the forces the state keeps between launches. The other threads of the pass still read
+// this atom's u4 and fix records, so the new ones go to the next body's buffers.
+__device__ __forceinline__ void force_done(const Geom &g, const Slots &s, const Inter &in, StepParams *sp, int sl, int si, int ti,
+                                           double fx, double fy, double fz, bool kick, bool hook, bool fused) {
+    if (!fused) { s.fx[sl] = fx; s.fy[sl] = fy; s.fz[sl] = fz; }
     if (kick && !hook && untouched(in, sl)) {
         const double c = dt_inv_m_of(sp, ti);
         const double vx = __dadd_rn(s.vx[sl], __dmul_rn(c, fx));
         const double vy = __dadd_rn(s.vy[sl], __dmul_rn(c, fy));
         const double vz = __dadd_rn(s.vz[sl], __dmul_rn(c, fz));
-        s.vx[sl] = vx; s.vy[sl] = vy; s.vz[sl] = vz;
+        if (!fused) { s.vx[sl] = vx; s.vy[sl] = vy; s.vz[sl] = vz; }  // else first_half writes the next v
         if (variable_dt(sp)) note_vmax2(sp, speed2(vx, vy, vz));
+        if (fused) {
+            int i, j, k;
+            const int tl = local_index_of(g, sl, i, j, k);
+            first_half<true, true>(g, s, in, sp, sl, tl, i, j, k, ti, vx, vy, vz, fx, fy, fz, s.u4n, s.u4, s.fixn);
+        }
     }
 }
 
@@ -1782,7 +1798,7 @@ __device__ __forceinline__ void k_lat_force_fp64_site(int t, const NeighTables &
     if (ti < 0) { s.fx[sl] = 0.0; s.fy[sl] = 0.0; s.fz[sl] = 0.0; return; }
     double fx, fy, fz;
     force_atom_fp64(nt, g, s, in, pt, sl, ti, par, fx, fy, fz);
-    force_done_fp64(s, in, sp, sl, ti, fx, fy, fz, kick, hook);
+    force_done(g, s, in, sp, sl, sidx(g, sl), ti, fx, fy, fz, kick, hook, false);
 }
 template <bool LOOP>  // LOOP: several sites per thread, one grid stride apart
 __global__ void __launch_bounds__(512) k_lat_force_fp64(const __grid_constant__ NeighTables nt, Geom g, Slots s, Inter in, PotTables pt,
@@ -1802,21 +1818,41 @@ struct FixForce {
     int df_hi;       // largest upper word of F'_i + F'_j met
     unsigned near;
 };
-// an atom's force over its near pairs, or (many) over all pairs, in FP64
+// An atom's force over its near pairs, or (many) over all pairs, in FP64, and over all pairs while the pass is wild.
+// But for that, the distance vectors come from the records: a fused pass changes the positions in place.
+__device__ __forceinline__ void fix_vector(const FixRec &i, const FixRec &j, double unit, double &dx, double &dy, double &dz) {
+    dx = (double) (i.x - j.x) * unit;
+    dy = (double) (i.y - j.y) * unit;
+    dz = (double) (i.z - j.z) * unit;
+}
 __device__ __noinline__ double3 force_near_fp64(const NeighTables &nt, const Geom &g, const Slots &s, const Inter &in,
-                                                const PotTables &pt, int sl, int ti, int par, unsigned near) {
+                                                const PotTables &pt, int kx, int sl, int ti, int par, unsigned near, bool wild) {
     double fx = 0.0, fy = 0.0, fz = 0.0;
-    if (near == kFixNearMany) {
+    if (wild) {
         force_atom_fp64(nt, g, s, in, pt, sl, ti, par, fx, fy, fz);
-    } else {
-        for (; near; near >>= 8) {
-            const int sj = sl + (par ? nt.lat[1][(near & 255u) - 1] : nt.lat[0][(near & 255u) - 1]);
-            const double dx = s.x[sl] - s.x[sj], dy = s.y[sl] - s.y[sj], dz = s.z[sl] - s.z[sj];
-            const double fpair = fpair_fp64(pt, dx * dx + dy * dy + dz * dz, ti, s.type[sj], s.df[sl], s.df[sj]);
-            fx += dx * fpair;
-            fy += dy * fpair;
-            fz += dz * fpair;
-        }
+        return make_double3(fx, fy, fz);
+    }
+    const bool many = near == kFixNearMany;
+    const double unit = scalbn(1.0, -kx), dfi = s.df[sl];
+    const int si = sidx(g, sl), end = many ? (in.far_flag[sl] ? nt.nfull : nt.npruned) : 4;
+    const FixRec me = ld_fix_rec(s.fix + si);
+    const float4 ui = s.u4[si];
+    for (int e = 0; e < end; e++) {
+        if (!many && !(near >> (8 * e))) break;
+        const int q = many ? e : (int) ((near >> (8 * e)) & 255u) - 1;
+        const float4 D = par ? nt.cand[1][q] : nt.cand[0][q];
+        const int oj = si + __float_as_int(D.w);
+        if (many && !near_f32(g, f2_pack(ui.x, ui.y), ui.z, D, s.u4[oj])) continue;
+        const FixRec j = ld_fix_rec(s.fix + oj);
+        const int sj = sl + (par ? nt.lat[1][q] : nt.lat[0][q]);
+        double dx, dy, dz;
+        fix_vector(me, j, unit, dx, dy, dz);
+        const double r2 = dx * dx + dy * dy + dz * dz;
+        if (!(r2 < g.rc2)) continue;
+        const double fpair = fpair_fp64(pt, r2, ti, (int) j.type, dfi, s.df[sj]);
+        fx += dx * fpair;
+        fy += dy * fpair;
+        fz += dz * fpair;
     }
     return make_double3(fx, fy, fz);
 }
@@ -1935,28 +1971,36 @@ __device__ __forceinline__ void force_fix_atom(const NeighTables &nt, const Geom
         f.z -= (double) a.z * fp.f_unit;
     }
 }
-// adds the near pairs, stores the force and takes the second half-kick where the lattice pass may
+// adds the near pairs; then as force_done_mixed
 __device__ __forceinline__ void force_done_fix(const NeighTables &nt, const Geom &g, const Slots &s, const Inter &in,
-                                               const PotTables &pt, StepParams *sp, int sl, int ti, int par, const FixForce &a,
-                                               double3 f, bool kick, bool hook) {
+                                               const PotTables &pt, StepParams *sp, int sl, int si, int ti, int par, const FixForce &a,
+                                               double3 f, bool kick, bool hook, bool fuse_next, bool wild) {
     const unsigned near = a.df_hi >= kFixBadHi ? kFixNearMany : a.near;
     if (near) {
-        const double3 n = force_near_fp64(nt, g, s, in, pt, sl, ti, par, near);
+        const double3 n = force_near_fp64(nt, g, s, in, pt, s.kx, sl, ti, par, near, wild);
         if (near == kFixNearMany) f = n;
         else { f.x += n.x; f.y += n.y; f.z += n.z; }
     }
-    force_done_fp64(s, in, sp, sl, ti, f.x, f.y, f.z, kick, hook);
+    force_done(g, s, in, sp, sl, si, ti, f.x, f.y, f.z, kick, hook, fuse_next && kick && !hook && !wild && lattice_only(in));
+}
+// a vacant site: no force, and in a fused body the next firststep's records of a vacancy
+__device__ __forceinline__ void force_vacant_fix(const Geom &g, const Slots &s, const Inter &in, int sl, int si, bool fuse_next, bool wild) {
+    s.fx[sl] = 0.0; s.fy[sl] = 0.0; s.fz[sl] = 0.0;
+    if (fuse_next && !wild && lattice_only(in)) {
+        s.u4n[si] = vacant_u4();
+        fix_put_vacant(g, s.fixn + si, s.kx, sl);
+    }
 }
 __device__ __forceinline__ void k_lat_force_fix_site(int t, const NeighTables &nt, const Geom &g, const Slots &s, const Inter &in,
                                                      const PotTables &pt, const FixParams &fp, StepParams *sp, bool kick, bool hook,
-                                                     int order, bool lists, bool wild) {
+                                                     int order, bool fuse_next, bool lists, bool wild) {
     int par, u;
     const int sl = gather_site(g, t, order, par, u);
     if (sl < 0) return;
     const int si = sidx(g, sl);
     const FixRec me = ld_fix_rec(s.fix + si);
     const int ti = (int) me.type;
-    if (ti < 0) { s.fx[sl] = 0.0; s.fy[sl] = 0.0; s.fz[sl] = 0.0; return; }
+    if (ti < 0) { force_vacant_fix(g, s, in, sl, si, fuse_next, wild); return; }
     FixForce a{0, 0, 0, 0, kFixNearMany};
     double3 f{0.0, 0.0, 0.0};
     if (!wild) {
@@ -1966,22 +2010,22 @@ __device__ __forceinline__ void k_lat_force_fix_site(int t, const NeighTables &n
         if (par) force_fix_atom<1>(nt, g, s, fp, si, ti, me, list, far, a, f);
         else force_fix_atom<0>(nt, g, s, fp, si, ti, me, list, far, a, f);
     }
-    force_done_fix(nt, g, s, in, pt, sp, sl, ti, par, a, f, kick, hook);
+    force_done_fix(nt, g, s, in, pt, sp, sl, si, ti, par, a, f, kick, hook, fuse_next, wild);
 }
 template <bool LOOP>  // LOOP: several sites per thread, one grid stride apart (no group lists)
 __global__ void __launch_bounds__(512, 2) k_lat_force_fix(const __grid_constant__ NeighTables nt, const __grid_constant__ Geom g,
                                                           const __grid_constant__ Slots s, const __grid_constant__ Inter in,
                                                           const __grid_constant__ PotTables pt, const __grid_constant__ FixParams fp,
                                                           StepParams *sp, bool kick, bool hook, int order, int tbase, int nthreads,
-                                                          bool lists) {
+                                                          bool fuse_next, bool lists) {
     const int t0 = tbase + blockIdx.x * blockDim.x + threadIdx.x;  // threads [tbase, nthreads)
     const bool wild = s.skin->wild != 0;
     if (!LOOP) {
-        if (t0 < nthreads) k_lat_force_fix_site(t0, nt, g, s, in, pt, fp, sp, kick, hook, order, lists && !wild, wild);
+        if (t0 < nthreads) k_lat_force_fix_site(t0, nt, g, s, in, pt, fp, sp, kick, hook, order, fuse_next, lists && !wild, wild);
         return;
     }
     for (int t = t0; t < nthreads; t += gridDim.x * blockDim.x)
-        k_lat_force_fix_site(t, nt, g, s, in, pt, fp, sp, kick, hook, order, false, wild);
+        k_lat_force_fix_site(t, nt, g, s, in, pt, fp, sp, kick, hook, order, fuse_next, false, wild);
 }
 
 // Compensated force sums of the mixed form: each pair term d * fpair is added by Kahan's method
@@ -2068,20 +2112,9 @@ __device__ __forceinline__ void force_sum_listed(const NeighTables &nt, const Ge
             force_candidate<PAR>(nt, g, s, pt, si, ti, uixy, ui.z, dfi, 32 * k + __ffs(w) - 1, acc);
 }
 
-// local coordinates and local index (k, j, i order) of a local slot
-__device__ __forceinline__ int local_index_of(const Geom &g, int sl, int &i, int &j, int &k) {
-    const int X = sl % g.Sx, r = sl / g.Sx;
-    i = X - g.gx;
-    j = r % g.Sy - g.gy;
-    k = r / g.Sy - g.gz;
-    return (k * g.by + j) * g.bx + i;
-}
-
-// stores the force and takes the second half-kick where the lattice pass may; in a fused body also the next
-// body's firststep
+// the sums with their compensations, converted to FP64 once; then as force_done
 __device__ __forceinline__ void force_done_mixed(const Geom &g, const Slots &s, const Inter &in, StepParams *sp, int sl, int si, int ti,
                                                  const ForceAcc &acc, bool kick, bool hook, bool fuse_next) {
-    // each sum with its compensation, converted to FP64 once
     float sx, sy, mx, my;
     f2_unpack(acc.sxy, sx, sy);
     f2_unpack(acc.mxy, mx, my);
@@ -2089,26 +2122,7 @@ __device__ __forceinline__ void force_done_mixed(const Geom &g, const Slots &s, 
     const double fx = h * ((double) sx + (double) mx);
     const double fy = h * ((double) sy + (double) my);
     const double fz = h * ((double) acc.sz + (double) acc.mz);
-    const bool fused = fuse_next && kick && !hook && lattice_only(in);
-    // a fused body's forces are used only in registers: the next body's firststep is taken here, and
-    // the last body of a graph (never fused) stores the forces the state keeps between launches
-    if (!fused) { s.fx[sl] = fx; s.fy[sl] = fy; s.fz[sl] = fz; }
-    if (kick && !hook && untouched(in, sl)) {
-        const double c = dt_inv_m_of(sp, ti);
-        const double vx = __dadd_rn(s.vx[sl], __dmul_rn(c, fx));
-        const double vy = __dadd_rn(s.vy[sl], __dmul_rn(c, fy));
-        const double vz = __dadd_rn(s.vz[sl], __dmul_rn(c, fz));
-        if (!fused) { s.vx[sl] = vx; s.vy[sl] = vy; s.vz[sl] = vz; }  // else first_half writes the next v
-        if (variable_dt(sp)) note_vmax2(sp, speed2(vx, vy, vz));
-        if (fused) {
-            // the next loop body's firststep for this atom, with the force still in registers (the
-            // other threads of this pass still read this atom's u4, so the new record goes to the next
-            // body's buffer, u4n)
-            int i, j, k;
-            const int tl = local_index_of(g, sl, i, j, k);
-            first_half<true, true>(g, s, in, sp, sl, tl, i, j, k, ti, vx, vy, vz, fx, fy, fz, s.u4n, s.u4);
-        }
-    }
+    force_done(g, s, in, sp, sl, si, ti, fx, fy, fz, kick, hook, fuse_next && kick && !hook && lattice_only(in));
 }
 // a vacant site: no force, and in a fused body the next firststep's record of a vacancy
 __device__ __forceinline__ void force_vacant_mixed(const Geom &g, const Slots &s, const Inter &in, int sl, int si, bool fuse_next) {
@@ -2236,10 +2250,10 @@ struct SplitForce {
     int df_hi[W][32];
     unsigned near[W][32];
 };
-template <int W>
+template <int W, int U>
 __device__ __forceinline__ void force_fix_split(const NeighTables &nt, const float4 *cand, const Geom &g, const Slots &s,
                                                 const Inter &in, const PotTables &pt, const FixParams &fp, StepParams *sp,
-                                                const SplitSite &a, bool kick, bool hook, bool lists, bool far, bool wild,
+                                                const SplitSite &a, bool kick, bool hook, bool fuse_next, bool lists, bool far, bool wild,
                                                 SplitList &sh, SplitForce<W> &part) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int np = nt.npruned, end = wild ? 0 : __any_sync(0xffffffffu, far) ? nt.nfull : np;
@@ -2257,11 +2271,11 @@ __device__ __forceinline__ void force_fix_split(const NeighTables &nt, const flo
         FixForce m{0, 0, 0, 0, 0u};
         if (mine) {
             const int c1 = n * (warp + 1) / W;
-            for (int c = n * warp / W; c < c1; c += kFixForceAhead) {
-                int oj[kFixForceAhead], q[kFixForceAhead];
-                bool use[kFixForceAhead];
-                split_next<kFixForceAhead>(sh, a.si, q0, c, c1, oj, use, q);
-                force_fix_pairs<kFixForceAhead>(s, fp, oj, use, q, a.ti, xb, yb, zb, dfb, m);
+            for (int c = n * warp / W; c < c1; c += U) {
+                int oj[U], q[U];
+                bool use[U];
+                split_next<U>(sh, a.si, q0, c, c1, oj, use, q);
+                force_fix_pairs<U>(s, fp, oj, use, q, a.ti, xb, yb, zb, dfb, m);
             }
         }
         part.x[warp][lane] = m.x;
@@ -2286,26 +2300,27 @@ __device__ __forceinline__ void force_fix_split(const NeighTables &nt, const flo
         }
     }
     if (warp != 0 || a.sl < 0) return;
-    if (a.ti < 0) { s.fx[a.sl] = 0.0; s.fy[a.sl] = 0.0; s.fz[a.sl] = 0.0; return; }
-    force_done_fix(nt, g, s, in, pt, sp, a.sl, a.ti, a.par, tot, f, kick, hook);
+    if (a.ti < 0) { force_vacant_fix(g, s, in, a.sl, a.si, fuse_next, wild); return; }
+    force_done_fix(nt, g, s, in, pt, sp, a.sl, a.si, a.ti, a.par, tot, f, kick, hook, fuse_next, wild);
 }
-template <int W>
-__global__ void __launch_bounds__(32 * W, 20 / W) k_lat_force_fix_split(const __grid_constant__ NeighTables nt, const float4 *cand,
+// B: blocks an SM holds
+template <int W, int B, int U>
+__global__ void __launch_bounds__(32 * W, B) k_lat_force_fix_split(const __grid_constant__ NeighTables nt, const float4 *cand,
                                                                         const __grid_constant__ Geom g, const __grid_constant__ Slots s,
                                                                         const __grid_constant__ Inter in,
                                                                         const __grid_constant__ PotTables pt,
                                                                         const __grid_constant__ FixParams fp, StepParams *sp, bool kick,
-                                                                        bool hook, int u0, int u1, bool lists) {
+                                                                        bool hook, int u0, int u1, bool fuse_next, bool lists) {
     __shared__ SplitList sh;
     __shared__ SplitForce<W> part;
     const bool wild = s.skin->wild != 0;
     const SplitSite a = split_site(g, s, u0, u1);
     if (!__any_sync(0xffffffffu, a.ti >= 0)) {
-        if (threadIdx.x < 32 && a.sl >= 0) { s.fx[a.sl] = 0.0; s.fy[a.sl] = 0.0; s.fz[a.sl] = 0.0; }
+        if (threadIdx.x < 32 && a.sl >= 0) force_vacant_fix(g, s, in, a.sl, a.si, fuse_next, wild);
         return;
     }
     const bool far = a.ti >= 0 && in.far_flag[a.sl];
-    force_fix_split<W>(nt, cand + a.par * kMaxFull, g, s, in, pt, fp, sp, a, kick, hook, lists && !wild, far, wild, sh, part);
+    force_fix_split<W, U>(nt, cand + a.par * kMaxFull, g, s, in, pt, fp, sp, a, kick, hook, fuse_next, lists && !wild, far, wild, sh, part);
 }
 
 static void launch_lat_force_threads(const LaunchCtx &lc, const Geom &g, Slots s, Inter in, PotTables t, StepParams *p,
@@ -2314,14 +2329,15 @@ static void launch_lat_force_threads(const LaunchCtx &lc, const Geom &g, Slots s
     const int order = lc.force_order, b = lc.force_block;
     const int n = (te - tb + b * lc.force_apt - 1) / (b * lc.force_apt);
     if (n <= 0) return;
-    const bool fuse = fuse_next && mixed && kick && !hook;
+    const bool fuse = fuse_next && kick && !hook && (mixed || lc.fp);
+    s = with_records(lc, s);
     if (lc.force_apt > 1) {
         if (mixed) k_lat_force_mixed<true><<<n, b, 0, lc.stream>>>(*lc.nt, g, s, in, t, p, kick, hook, order, tb, te, fuse, false);
-        else if (lc.fp) k_lat_force_fix<true><<<n, b, 0, lc.stream>>>(*lc.nt, g, s, in, t, *lc.fp, p, kick, hook, order, tb, te, false);
+        else if (lc.fp) k_lat_force_fix<true><<<n, b, 0, lc.stream>>>(*lc.nt, g, s, in, t, *lc.fp, p, kick, hook, order, tb, te, fuse, false);
         else k_lat_force_fp64<true><<<n, b, 0, lc.stream>>>(*lc.nt, g, s, in, t, p, kick, hook, order, tb, te);
     } else {
         if (mixed) k_lat_force_mixed<false><<<n, b, 0, lc.stream>>>(*lc.nt, g, s, in, t, p, kick, hook, order, tb, te, fuse, lists);
-        else if (lc.fp) k_lat_force_fix<false><<<n, b, 0, lc.stream>>>(*lc.nt, g, s, in, t, *lc.fp, p, kick, hook, order, tb, te, lists);
+        else if (lc.fp) k_lat_force_fix<false><<<n, b, 0, lc.stream>>>(*lc.nt, g, s, in, t, *lc.fp, p, kick, hook, order, tb, te, fuse, lists);
         else k_lat_force_fp64<false><<<n, b, 0, lc.stream>>>(*lc.nt, g, s, in, t, p, kick, hook, order, tb, te);
     }
 }
@@ -2329,10 +2345,20 @@ template <int W>
 static void launch_force_split_w(const LaunchCtx &lc, const Geom &g, Slots s, Inter in, PotTables t, StepParams *p, bool kick, bool mixed,
                                  bool hook, int u0, int u1, bool fuse_next, bool lists) {
     const int n = split_groups(u0, u1);
+    const bool fuse = fuse_next && kick && !hook;
+    s = with_records(lc, s);
     if (mixed)
         k_lat_force_mixed_split<W><<<n, 32 * W, 0, lc.stream>>>(&lc.ntd->cand[0][0], lc.nt->npruned, lc.nt->nfull, g, s, in, t, p, kick, hook, u0, u1,
-                                                                fuse_next && kick && !hook, lists);
-    else k_lat_force_fix_split<W><<<n, 32 * W, 0, lc.stream>>>(*lc.nt, &lc.ntd->cand[0][0], g, s, in, t, *lc.fp, p, kick, hook, u0, u1, lists);
+                                                                fuse, lists);
+    else {
+        // 500 groups of 8 warps fit one wave at 64 registers, one candidate at a time: 29.1 -> 26.2 us
+        if constexpr (W == 8)
+            if (n * lc.share > 2 * lc.num_sms) {
+                k_lat_force_fix_split<W, 4, 1><<<n, 32 * W, 0, lc.stream>>>(*lc.nt, &lc.ntd->cand[0][0], g, s, in, t, *lc.fp, p, kick, hook, u0, u1, fuse, lists);
+                return;
+            }
+        k_lat_force_fix_split<W, 20 / W, kFixForceAhead><<<n, 32 * W, 0, lc.stream>>>(*lc.nt, &lc.ntd->cand[0][0], g, s, in, t, *lc.fp, p, kick, hook, u0, u1, fuse, lists);
+    }
 }
 static bool launch_lat_force_split(const LaunchCtx &lc, const Geom &g, Slots s, Inter in, PotTables t, StepParams *p, bool kick, bool mixed,
                                    bool hook, int u0, int u1, bool fuse_next, bool lists) {

@@ -51,3 +51,23 @@ def test_rule_switches_and_launch_lengths(pkg, wl, potentials, gpu_lib, prec, ru
         out.append((a.tobytes(), np.asarray(hist).tobytes(), ctx.clock()))
         ctx.close()
     assert out[0] == out[1]
+
+
+@pytest.mark.parametrize("temperature,kick,dt", [(1800.0, None, 0.001), (600.0, 300.0, 0.0002), (600.0, None, 0.001)])
+def test_fp64_fused_bodies_give_the_bits_of_single_steps(pkg, wl, potentials, gpu_lib, temperature, kick, dt):
+    """Hot crystals put pairs below the range of the tables (their distances come from the records, since a fused pass
+    changes the positions in place); a kicked atom makes inter atoms come and go, which bodies are not fused with."""
+    cells = (9, 8, 10)
+    atoms = wl.build_state(cells, A0, RCF, temperature=temperature, seed=12, cu_frac=0.05)
+    out = []
+    for single in (False, True):
+        ctx = _ctx(pkg, potentials["fecuni"], cells, atoms, "fp64", single)
+        ctx.set_timestep(dt)
+        if kick:
+            ctx.collision_step([4, 4, 5, 0], np.array([1.0, 3.0, 5.0]) / 35**0.5, kick)
+        for run in (40, 23, 1):
+            ctx.simulate(run)
+        a, inter = ctx.download()
+        out.append((a.tobytes(), inter.tobytes(), ctx.clock()))
+        ctx.close()
+    assert out[0] == out[1]
