@@ -2811,6 +2811,7 @@ __device__ __forceinline__ void border_put(Inter &in, int q, const double p3[3],
 
 __global__ void __launch_bounds__(kManageThreads) k_inter_manage(Geom g, Slots s, Inter in, int mask, bool mixed, StepParams *sp) {
     extern __shared__ long long sm_keys[];
+    __shared__ int sh_n, sh_d;
     const int tid = threadIdx.x, nthr = blockDim.x;
     if ((mask & MANAGE_CLOCK) && tid == 0) step_record(sp);
     if ((mask & MANAGE_DECIDE) && s.kx && tid == 0) {  // the positions are firststep's now
@@ -2849,10 +2850,10 @@ __global__ void __launch_bounds__(kManageThreads) k_inter_manage(Geom g, Slots s
         // (i) displaced lattice atoms join the list in scan order
         int nd = n_disp;
         if (nd > in.dcap) { if (tid == 0) set_error(in, MG_DEVERR_DISPLACED_OVERFLOW); nd = in.dcap; }
-        const int *order = block_sort_displaced(g, in, nd, reinterpret_cast<int *>(sm_keys));
         const int n0 = n_inter;
         if (nd > 0) {
             int room = in.cap - n0;
+            const int *order = block_sort_displaced(g, in, nd, reinterpret_cast<int *>(sm_keys));
             if (nd > room) { if (tid == 0) set_error(in, MG_DEVERR_INTER_OVERFLOW); nd = room; }
             for (int q = tid; q < nd; q += nthr) {
                 int i, j, k;
@@ -2926,9 +2927,36 @@ __global__ void __launch_bounds__(kManageThreads) k_inter_manage(Geom g, Slots s
                 }
             }
             __syncthreads();
-            // stable compaction of the survivors
+            // stable compaction of the survivors: a short list's records through one warp's registers
             int base = 0;
-            for (int c0 = 0; c0 < n; c0 += nthr) {
+            if (n <= 32) {
+                if (tid < 32) {
+                    const bool keep = tid < n && !won[tid];
+                    const unsigned kept = __ballot_sync(0xffffffffu, keep);
+                    double *const col[11] = {in.x, in.y, in.z, in.vx, in.vy, in.vz, in.fx, in.fy, in.fz, in.rho, in.df};
+                    double v[11];
+                    uint64_t id = 0;
+                    int type = 0;
+                    if (keep) {
+#pragma unroll
+                        for (int f = 0; f < 11; f++) v[f] = col[f][tid];
+                        id = in.id[tid];
+                        type = in.type[tid];
+                    }
+                    __syncwarp();
+                    const int to = __popc(kept & ((1u << tid) - 1u));
+                    if (keep && to != tid) {
+#pragma unroll
+                        for (int f = 0; f < 11; f++) col[f][to] = v[f];
+                        in.id[to] = id;
+                        in.type[to] = type;
+                    }
+                    if (tid == 0) sh_n = __popc(kept);
+                }
+                __syncthreads();
+                base = sh_n;
+            }
+            for (int c0 = 0; c0 < n && n > 32; c0 += nthr) {
                 const int a = c0 + tid;
                 const int keep = (a < n && !won[a]) ? 1 : 0;
                 int ex;
@@ -2937,7 +2965,8 @@ __global__ void __launch_bounds__(kManageThreads) k_inter_manage(Geom g, Slots s
                 base += tot;
             }
             __syncthreads();
-            for (int a = tid; a < base; a += nthr) inter_restore(in, a, a);
+            if (n > 32)
+                for (int a = tid; a < base; a += nthr) inter_restore(in, a, a);
             n_inter = base;
             if (tid == 0) in.cnt[CNT_INTER] = base;
         }
@@ -2949,8 +2978,14 @@ __global__ void __launch_bounds__(kManageThreads) k_inter_manage(Geom g, Slots s
         // an atom's out-of-box flags are found once and kept until a partition moves and shifts the
         // records (each thread keeps the same atoms from one dimension to the next)
         uint32_t *flags = reinterpret_cast<uint32_t *>(in.scratch_i + 2 * in.cap);
-        bool flags_valid = false;
-        for (int d = 0; d < 3; d++) {
+        uint32_t outside = 0;
+        for (int a = tid; a < n_inter; a += nthr) {
+            flags[a] = is_out_box(g, in.x[a], in.y[a], in.z[a]);
+            outside |= flags[a];
+        }
+        bool flags_valid = true;
+        const bool leaving = __syncthreads_or(outside != 0);
+        for (int d = 0; d < 3 && leaving; d++) {
             const int n = n_inter;
             int *cls = in.scratch_i + in.cap;  // 0 stay, 1 lower, 2 higher
             int leaves = 0;
@@ -3000,7 +3035,52 @@ __global__ void __launch_bounds__(kManageThreads) k_inter_manage(Geom g, Slots s
         // keeps the same entries in both passes, and cap + gcap ints fit in the 13 * cap doubles of
         // scratch_d.
         int *mk = reinterpret_cast<int *>(in.scratch_d);
-        for (int d = 0; d < 3; d++) {
+        int d0 = 0;
+        if (n_inter + n_ghost <= 32) {
+            // one warp, an entry per lane, no block barriers; an entry's nearest site is found once
+            if (tid < 32) {
+                int d = 0, ng = n_ghost, ty = 0, root = 0;
+                double p3[3] = {0.0, 0.0, 0.0};
+                long long c[3] = {0, 0, 0};
+                bool found = false;
+#pragma unroll
+                for (int dd = 0; dd < 3; dd++) {
+                    const int total = n_inter + ng;
+                    if (total > 32) break;
+                    if (tid < total && !found) {
+                        border_entry(in, n_inter, tid, p3, ty, root);
+                        near_lat_coord(g, p3[0], p3[1], p3[2], c);
+                        found = true;
+                    }
+                    int m = 0;
+#pragma unroll
+                    for (int r = 0; r < 2; r++) {
+                        int lo[3], hi[3];
+                        region_fw(g, dd, r, lo, hi);
+                        if (tid < total && c[0] >= lo[0] && c[0] < hi[0] && c[1] >= lo[1] && c[1] < hi[1] && c[2] >= lo[2] && c[2] < hi[2])
+                            m |= 1 << r;
+                    }
+                    const unsigned b0 = __ballot_sync(0xffffffffu, m & 1), b1 = __ballot_sync(0xffffffffu, m & 2);
+                    const unsigned below = (1u << tid) - 1u;
+                    const int base1 = min(ng + __popc(b0), in.gcap);
+                    if (m & 1) border_put(in, ng + __popc(b0 & below), p3, dd, g.L[dd], ty, root);
+                    if (m & 2) border_put(in, base1 + __popc(b1 & below), p3, dd, -g.L[dd], ty, root);
+                    ng = min(base1 + __popc(b1), in.gcap);
+                    d = dd + 1;
+                    __syncwarp();
+                }
+                if (tid == 0) {
+                    sh_d = d;
+                    sh_n = ng;
+                    in.cnt[CNT_GHOST] = ng;
+                }
+            }
+            __syncthreads();
+            d0 = sh_d;
+            n_ghost = sh_n;
+            __syncthreads();
+        }
+        for (int d = d0; d < 3; d++) {
             const int n_loc = n_inter;
             const int total = n_loc + n_ghost;
             int lo[2][3], hi[2][3];
@@ -3062,6 +3142,7 @@ __global__ void __launch_bounds__(kManageThreads) k_inter_manage(Geom g, Slots s
         const int n_loc = n_inter;
         const int n_gh = n_ghost;
         const int total = n_loc + n_gh;
+        long long mine = LLONG_MAX;
         for (int e = tid; e < total; e += nthr) {
             double px, py, pz;
             int ref;
@@ -3076,7 +3157,17 @@ __global__ void __launch_bounds__(kManageThreads) k_inter_manage(Geom g, Slots s
             } else {
                 key = lin(g, (int) c[0], (int) c[1], (int) c[2]);
             }
-            in.bucket[e] = (key << 32) | (long long) ref;
+            mine = (key << 32) | (long long) ref;
+            if (total > 32) in.bucket[e] = mine;
+        }
+        if (total <= 32) {  // ranked by one warp
+            if (tid < 32) {
+                int r = 0;
+                for (int k = 0; k < 32; k++) r += __shfl_sync(0xffffffffu, mine, k) < mine;
+                if (tid < total) in.bucket[r] = mine;
+                if (tid == 0) *in.n_bucket = total;
+            }
+            return;
         }
         __syncthreads();
         if (total <= kSortSmemKeys) block_bitonic_sort_smem(in.bucket, total, sm_keys);
