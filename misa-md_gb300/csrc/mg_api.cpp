@@ -37,6 +37,8 @@ namespace mg {
 void set_global_error(const char *msg) { g_create_error = msg ? msg : ""; }
 }  // namespace mg
 
+constexpr int kWideForce = 1500000;  // sites from which the mixed force pass takes blocks of 512 (mg_context::tune)
+
 struct mg_context {
     int device = 0;
     int precision = MG_PREC_FP64;
@@ -105,9 +107,12 @@ struct mg_context {
 
     // [precision][rho, force] = {thread order, block size, atoms per thread}. Order 1 until an autotune: its
     // warps cover whole 32-site groups in every box, so the group lists serve boxes with an odd number of sites
-    // of a parity as well (order 0 visits all 112 candidates there). Blocks of 256; the FP64 density pass, at 56
-    // registers, fills the SMs better with 128 (2M atoms: 720 -> 682 us).
-    int tune[2][2][3] = {{{1, 128, 1}, {1, 256, 1}}, {{1, 256, 1}, {1, 256, 1}}};
+    // of a parity as well (order 0 visits all 112 candidates there). Block sizes by measurement: the FP64 density pass
+    // 128 (2M atoms: 720 us with 256, 682 with 128), its force pass 256 (128: 2M atoms -0.2%, 304k atoms +1%); the
+    // mixed density pass 512 (2M atoms 233 -> 228 us, 221k atoms 40.2 -> 38.3, elsewhere even); the mixed force pass
+    // 256, from kWideForce sites on 512, whose groups share more of L1 (2M atoms 427 -> 419 us; 1M atoms 264 -> 267
+    // and 315k atoms 103 -> 107, by their last wave).
+    int tune[2][2][3] = {{{1, 128, 1}, {1, 256, 1}}, {{1, 512, 1}, {1, 256, 1}}};
     int share = 1;                  // contexts stepping side by side (while a batch captures)
     LaunchCtx lc() const {
         LaunchCtx l{stream, num_sms};
@@ -251,7 +256,7 @@ void seq_step(mg_context *ctx, Timer *t, bool fused_prev = false, bool fuse_next
     seq_compute_eam(ctx, true, true, MANAGE_DECIDE | MANAGE_CLEAR_GHOST | MANAGE_EXCHANGE | MANAGE_BORDER | (variable ? 0 : MANAGE_CLOCK), t,
                     fuse_next);
 }
-// steps of mg_simulate that run fused: the mixed form with a fixed dt
+// runs whose force passes may take the next firststep: a fixed dt, in the mixed or the fixed-point form
 bool fusable(const mg_context *ctx) { return ctx->fuse_steps >= 2 && (ctx->mixed() || ctx->lc().fp) && ctx->dx_max <= 0.0; }
 // Loop bodies in one graph launch of a run of that many steps (0: one body per launch). The mixed form: fuse_steps
 // fused bodies. The others kPlainBodies, since a graph costs about 25 us a body to make and their runs are short: bodies
@@ -583,6 +588,7 @@ mg_status mg_create(const int64_t phase_space[3], double lattice_const, double r
     g.half = g.n_slots / 2;  // Sx is even, so slot parity is x parity
     g.nxh = g.bx / 2;
     g.n_local_half = g.n_local / 2;
+    if (g.n_local >= kWideForce) ctx->tune[MG_PREC_MIXED][1][1] = 512;
     for (int d = 0; d < 3; d++) g.cells[d] = (int) phase_space[d];
     g.a0 = lattice_const;
     g.rc = lattice_const * rcf;  // atom::atom, src/atom.cpp:14-19
