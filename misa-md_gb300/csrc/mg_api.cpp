@@ -52,6 +52,7 @@ struct mg_context {
     bool pot_ready = false;
     HostPotential hp;               // the spline coefficients in use
     int types_ok_mask = 0;          // bit t set: the potential has the element of atom type t
+    bool one_type = false;          // all types have the same tables (a potential of one element)
     std::vector<void *> dev_allocs;
     void *pot_mem = nullptr;
     OffsetTable offs;
@@ -119,6 +120,7 @@ struct mg_context {
         l.share = share;
         l.nt = &nt;
         l.ntd = d_nt;
+        l.one_type = one_type;
         l.fp = !mixed() && fp.on && s.fix ? &fp : nullptr;
         l.rho_order = tune[precision][0][0];
         l.rho_block = tune[precision][0][1];
@@ -387,6 +389,7 @@ mg_status install_potential(mg_context *ctx, const HostPotential &hp) {
         if (e >= 0) ctx->types_ok_mask |= 1 << t;
         ele_of_type[t] = e >= 0 ? e : 0;
     }
+    ctx->one_type = ele_of_type[1] == ele_of_type[0] && ele_of_type[2] == ele_of_type[0];
     if ((hp.nr - 1) * hp.dr + 1e-12 < ctx->g.rc) {  // the hit test uses rc = a0 * cutoff_radius_factor
         ctx->err = "potential r-table shorter than the cutoff radius";
         return MG_ERR_POTENTIAL;

@@ -264,6 +264,7 @@ struct LaunchCtx {
     const NeighTables *ntd = nullptr;        // the same in device memory
     const FixParams *fp = nullptr;           // FP64 form: scales and tables of the fixed-point pair arithmetic
     int share = 1;                           // contexts that step side by side (a batch's members)
+    bool one_type = false;                   // all types have the same tables
 };
 
 // Mass table shared by all contexts (atom types are fixed).

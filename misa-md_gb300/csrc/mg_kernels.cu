@@ -1262,7 +1262,7 @@ __global__ void __launch_bounds__(32 * W) k_lat_rho_mixed_split(const float4 *ca
 // FP64 form in fixed point (mg_fixed.h): the pair sums in 64-bit integers. Bound by integer issue and by the
 // table records' L1 wavefronts. A pair costs about 60 (density) and 110 (force) integer and single-precision
 // operations at one or two issue slots each; its FP64 operations cost 64 slots apiece, which bound the FP64
-// loops (2M atoms, step: 14.2 -> 2.1 ms; 300k atoms: 2.2 -> 0.50 ms; 16k atoms: 0.32 -> 0.14 ms). They stay
+// loops (2M atoms, step: 14.2 -> 1.93 ms; 304k atoms: 2.2 -> 0.40 ms; 16k atoms: 0.32 -> 0.05 ms). They stay
 // for the cases below and for tables the fixed point does not suit. Its errors are half the FP64 loops'
 // (thermal crystals against 113-bit arithmetic: force rms 2.4e-15 -> 1.1e-15 of the rms force).
 // The group lists of the mixed form serve here as well: 66 candidates are visited instead of 112.
@@ -1912,7 +1912,8 @@ __device__ __forceinline__ void force_fix_pairs(const Slots &s, const FixParams 
         a.z = fix_mul_add(d[u].zh, d[u].zl, fh, fl, a.z);
     }
 }
-// candidate q, at index oj
+// candidate q, at index oj. ONE: every atom is of the one type that the potential has
+template <bool ONE>
 __device__ __forceinline__ void force_fix_candidate(const Slots &s, const FixParams &fp, int oj, int ti, i64 xb,
                                                     i64 yb, i64 zb, i64 dfb, int q, FixForce &a) {
     const FixRec j = ld_fix_rec(s.fix + oj);
@@ -1922,16 +1923,19 @@ __device__ __forceinline__ void force_fix_candidate(const Slots &s, const FixPar
         const i64 dfj = __ldg(s.dfq + oj);
         int m;
         const FixCoord t = fix_locate(fp, r2, m);
-        const int tj = (int) j.type;
+        const int tj = ONE ? ti : (int) j.type;
         const FixPoly *rec = fp.zg + 2 * ((ti * 3 + tj) * fp.nr1 + m);
-        const i64 gj = fix_poly(ld_fix_poly(rec), t, fp.e3_g);
-        i64 f = fix_poly(ld_fix_poly(rec + 1), t, fp.e3_h);
+        const FixPoly pg = ld_fix_poly(rec), ph = ld_fix_poly(rec + 1);
+        FixPoly pi;
+        if (tj != ti) pi = ld_fix_poly(fp.zg + 2 * ((tj * 3 + ti) * fp.nr1 + m));
+        const i64 gj = fix_poly(pg, t, fp.e3_g);
+        i64 f = fix_poly(ph, t, fp.e3_h);
         const i64 both = dfb + dfj;  // biased
         a.df_hi = max(a.df_hi, fix_hi(both));
         if (tj == ti) {
             f = fix_mul_add(fix_hi(both), fix_lo(both), fix_hi(gj), fix_lo(gj), f);
         } else {
-            const i64 gi = fix_poly(ld_fix_poly(fp.zg + 2 * ((tj * 3 + ti) * fp.nr1 + m)), t, fp.e3_g);
+            const i64 gi = fix_poly(pi, t, fp.e3_g);
             const i64 djb = dfj + kFixBias;
             f = fix_mul_add(fix_hi(dfb), fix_lo(dfb), fix_hi(gj), fix_lo(gj), f);
             f = fix_mul_add(fix_hi(djb), fix_lo(djb), fix_hi(gi), fix_lo(gi), f);
@@ -1944,7 +1948,7 @@ __device__ __forceinline__ void force_fix_candidate(const Slots &s, const FixPar
         fix_note_near(a.near, q);
     }
 }
-template <int PAR>
+template <int PAR, bool ONE>
 __device__ __forceinline__ void force_fix_range(const NeighTables &nt, const Geom &g, const Slots &s, const FixParams &fp, int si,
                                                 int ti, float4 ui, i64 xb, i64 yb, i64 zb, i64 dfb, int q0, int q1, FixForce &a) {
     const f2 uixy = f2_pack(ui.x, ui.y);
@@ -1952,10 +1956,10 @@ __device__ __forceinline__ void force_fix_range(const NeighTables &nt, const Geo
     for (int q = q0; q < q1; q++) {
         const float4 D = nt.cand[PAR][q];
         if (near_f32(g, uixy, ui.z, D, __ldg(s.u4 + si + __float_as_int(D.w))))
-            force_fix_candidate(s, fp, si + __float_as_int(D.w), ti, xb, yb, zb, dfb, q, a);
+            force_fix_candidate<ONE>(s, fp, si + __float_as_int(D.w), ti, xb, yb, zb, dfb, q, a);
     }
 }
-template <int PAR>
+template <int PAR, bool ONE>
 __device__ __forceinline__ void force_fix_atom(const NeighTables &nt, const Geom &g, const Slots &s, const FixParams &fp, int si,
                                                int ti, const FixRec &me, const unsigned *list, bool far, FixForce &a, double3 &f) {
     const i64 xb = me.x + kFixBias, yb = me.y + kFixBias, zb = me.z + kFixBias, dfb = s.dfq[si] + kFixBias;
@@ -1964,15 +1968,15 @@ __device__ __forceinline__ void force_fix_atom(const NeighTables &nt, const Geom
         for (int k = 0; k * 32 < np; k++)
             for (unsigned w = list[k]; w; w &= w - 1) {
                 const int q = 32 * k + __ffs(w) - 1;
-                force_fix_candidate(s, fp, si + __float_as_int(nt.cand[PAR][q].w), ti, xb, yb, zb, dfb, q, a);
+                force_fix_candidate<ONE>(s, fp, si + __float_as_int(nt.cand[PAR][q].w), ti, xb, yb, zb, dfb, q, a);
             }
     } else {
-        force_fix_range<PAR>(nt, g, s, fp, si, ti, s.u4[si], xb, yb, zb, dfb, 0, np, a);
+        force_fix_range<PAR, ONE>(nt, g, s, fp, si, ti, s.u4[si], xb, yb, zb, dfb, 0, np, a);
     }
     f = make_double3(-(double) a.x * fp.f_unit, -(double) a.y * fp.f_unit, -(double) a.z * fp.f_unit);
     if (far) {  // each part fits the integers by itself
         a.x = 0; a.y = 0; a.z = 0;
-        force_fix_range<PAR>(nt, g, s, fp, si, ti, s.u4[si], xb, yb, zb, dfb, np, nt.nfull, a);
+        force_fix_range<PAR, ONE>(nt, g, s, fp, si, ti, s.u4[si], xb, yb, zb, dfb, np, nt.nfull, a);
         f.x -= (double) a.x * fp.f_unit;
         f.y -= (double) a.y * fp.f_unit;
         f.z -= (double) a.z * fp.f_unit;
@@ -1998,6 +2002,7 @@ __device__ __forceinline__ void force_vacant_fix(const Geom &g, const Slots &s, 
         fix_put_vacant(g, s.fixn + si, s.kx, sl);
     }
 }
+template <bool ONE>
 __device__ __forceinline__ void k_lat_force_fix_site(int t, const NeighTables &nt, const Geom &g, const Slots &s, const Inter &in,
                                                      const PotTables &pt, const FixParams &fp, StepParams *sp, bool kick, bool hook,
                                                      int order, bool fuse_next, bool lists, bool wild) {
@@ -2014,12 +2019,12 @@ __device__ __forceinline__ void k_lat_force_fix_site(int t, const NeighTables &n
         a.near = 0u;
         const unsigned *list = lists ? group_list(g, s, par, u) : nullptr;
         const bool far = in.far_flag[sl];
-        if (par) force_fix_atom<1>(nt, g, s, fp, si, ti, me, list, far, a, f);
-        else force_fix_atom<0>(nt, g, s, fp, si, ti, me, list, far, a, f);
+        if (par) force_fix_atom<1, ONE>(nt, g, s, fp, si, ti, me, list, far, a, f);
+        else force_fix_atom<0, ONE>(nt, g, s, fp, si, ti, me, list, far, a, f);
     }
     force_done_fix(nt, g, s, in, pt, sp, sl, si, ti, par, a, f, kick, hook, fuse_next, wild);
 }
-template <bool LOOP>  // LOOP: several sites per thread, one grid stride apart (no group lists)
+template <bool LOOP, bool ONE>  // LOOP: several sites per thread, one grid stride apart (no group lists)
 __global__ void __launch_bounds__(512, 2) k_lat_force_fix(const __grid_constant__ NeighTables nt, const __grid_constant__ Geom g,
                                                           const __grid_constant__ Slots s, const __grid_constant__ Inter in,
                                                           const __grid_constant__ PotTables pt, const __grid_constant__ FixParams fp,
@@ -2028,11 +2033,11 @@ __global__ void __launch_bounds__(512, 2) k_lat_force_fix(const __grid_constant_
     const int t0 = tbase + blockIdx.x * blockDim.x + threadIdx.x;  // threads [tbase, nthreads)
     const bool wild = s.skin->wild != 0;
     if (!LOOP) {
-        if (t0 < nthreads) k_lat_force_fix_site(t0, nt, g, s, in, pt, fp, sp, kick, hook, order, fuse_next, lists && !wild, wild);
+        if (t0 < nthreads) k_lat_force_fix_site<ONE>(t0, nt, g, s, in, pt, fp, sp, kick, hook, order, fuse_next, lists && !wild, wild);
         return;
     }
     for (int t = t0; t < nthreads; t += gridDim.x * blockDim.x)
-        k_lat_force_fix_site(t, nt, g, s, in, pt, fp, sp, kick, hook, order, fuse_next, false, wild);
+        k_lat_force_fix_site<ONE>(t, nt, g, s, in, pt, fp, sp, kick, hook, order, fuse_next, false, wild);
 }
 
 // Compensated force sums of the mixed form: each pair term d * fpair is added by Kahan's method
@@ -2085,8 +2090,9 @@ __device__ __forceinline__ float fpair_mixed(const Geom &g, const PotTables &pt,
     const float psip = __fmaf_rn(dphi, rinv, __fmaf_rn(dfi, rhojp, __fmul_rn(dfj, rhoip)));
     return __fmul_rn(-psip, rinv);
 }
-// one candidate of the force pass: the pair term when inside the cutoff (false for vacancies, NaN)
-template <int PAR>
+// one candidate of the force pass: the pair term when inside the cutoff (false for vacancies, NaN); ONE: as
+// force_fix_candidate
+template <int PAR, bool ONE>
 __device__ __forceinline__ void force_candidate(const NeighTables &nt, const Geom &g, const Slots &s, const PotTables &pt, int si,
                                                 int ti, f2 uixy, float uiz, float dfi, int q, ForceAcc &acc) {
     const float4 D = nt.cand[PAR][q];
@@ -2095,28 +2101,28 @@ __device__ __forceinline__ void force_candidate(const NeighTables &nt, const Geo
     f2 dxy; float dz;
     const float r2 = pair_r2(uixy, uiz, D, uj, dxy, dz);
     if (r2 < g.rc2_h) {
-        const int tj = __float_as_int(uj.w);
+        const int tj = ONE ? ti : __float_as_int(uj.w);
         force_acc_add(acc, dxy, dz, fpair_mixed(g, pt, pair_record(pt, r2, ti, tj), ti, tj, dfi, __ldg(s.df32 + oj)));
     }
 }
-template <int PAR>
+template <int PAR, bool ONE>
 __device__ __forceinline__ void force_sum_mixed(const NeighTables &nt, const Geom &g, const Slots &s, const PotTables &pt, int si, int ti,
                                                 float4 ui, float dfi, int q0, int q1, ForceAcc &acc) {
     const f2 uixy = f2_pack(ui.x, ui.y);
 #pragma unroll 1  // 2, 3, 4 and full unrolling measured slower
-    for (int q = q0; q < q1; q++) force_candidate<PAR>(nt, g, s, pt, si, ti, uixy, ui.z, dfi, q, acc);
+    for (int q = q0; q < q1; q++) force_candidate<PAR, ONE>(nt, g, s, pt, si, ti, uixy, ui.z, dfi, q, acc);
 }
 // the candidates of the warp's group list, in table order: the density pass of this step checked or
 // rebuilt the list, so it holds every pruned candidate inside the cutoff for any site of the group
 // (the cutoff is tested again here with the same rounding, so the pairs summed are those of the full
 // loop, in the same order)
-template <int PAR>
+template <int PAR, bool ONE>
 __device__ __forceinline__ void force_sum_listed(const NeighTables &nt, const Geom &g, const Slots &s, const PotTables &pt, int si,
                                                  int ti, float4 ui, float dfi, const unsigned *words, ForceAcc &acc) {
     const f2 uixy = f2_pack(ui.x, ui.y);
     for (int k = 0; k * 32 < nt.npruned; k++)
         for (unsigned w = words[k]; w; w &= w - 1)
-            force_candidate<PAR>(nt, g, s, pt, si, ti, uixy, ui.z, dfi, 32 * k + __ffs(w) - 1, acc);
+            force_candidate<PAR, ONE>(nt, g, s, pt, si, ti, uixy, ui.z, dfi, 32 * k + __ffs(w) - 1, acc);
 }
 
 // the sums with their compensations, converted to FP64 once; then as force_done
@@ -2136,6 +2142,7 @@ __device__ __forceinline__ void force_vacant_mixed(const Geom &g, const Slots &s
     s.fx[sl] = 0.0; s.fy[sl] = 0.0; s.fz[sl] = 0.0;
     if (fuse_next && lattice_only(in)) s.u4n[si] = vacant_u4();
 }
+template <bool ONE>
 __device__ __forceinline__ void k_lat_force_mixed_site(int t, const NeighTables &nt, const Geom &g, const Slots &s, const Inter &in,
                                                 const PotTables &pt, StepParams *sp, bool kick, bool hook, int order,
                                                 bool fuse_next, bool lists) {
@@ -2152,30 +2159,30 @@ __device__ __forceinline__ void k_lat_force_mixed_site(int t, const NeighTables 
     const int np = nt.npruned;
     if (lists) {
         const unsigned *w = group_list(g, s, par, u);
-        if (par) force_sum_listed<1>(nt, g, s, pt, si, ti, ui, dfi, w, acc);
-        else force_sum_listed<0>(nt, g, s, pt, si, ti, ui, dfi, w, acc);
+        if (par) force_sum_listed<1, ONE>(nt, g, s, pt, si, ti, ui, dfi, w, acc);
+        else force_sum_listed<0, ONE>(nt, g, s, pt, si, ti, ui, dfi, w, acc);
     } else {
-        if (par) force_sum_mixed<1>(nt, g, s, pt, si, ti, ui, dfi, 0, np, acc);
-        else force_sum_mixed<0>(nt, g, s, pt, si, ti, ui, dfi, 0, np, acc);
+        if (par) force_sum_mixed<1, ONE>(nt, g, s, pt, si, ti, ui, dfi, 0, np, acc);
+        else force_sum_mixed<0, ONE>(nt, g, s, pt, si, ti, ui, dfi, 0, np, acc);
     }
     if (in.far_flag[sl]) {
         const int nf = nt.nfull;
-        if (par) force_sum_mixed<1>(nt, g, s, pt, si, ti, ui, dfi, np, nf, acc);
-        else force_sum_mixed<0>(nt, g, s, pt, si, ti, ui, dfi, np, nf, acc);
+        if (par) force_sum_mixed<1, ONE>(nt, g, s, pt, si, ti, ui, dfi, np, nf, acc);
+        else force_sum_mixed<0, ONE>(nt, g, s, pt, si, ti, ui, dfi, np, nf, acc);
     }
     force_done_mixed(g, s, in, sp, sl, si, ti, acc, kick, hook, fuse_next);
 }
-template <bool LOOP>  // LOOP: several sites per thread, one grid stride apart
+template <bool LOOP, bool ONE>  // LOOP: several sites per thread, one grid stride apart
 __global__ void __launch_bounds__(512, 3) k_lat_force_mixed(const __grid_constant__ NeighTables nt, Geom g, Slots s, Inter in, PotTables pt,
                                                          StepParams *sp, bool kick, bool hook, int order, int tbase,
                                                          int nthreads, bool fuse_next, bool lists) {
     const int t0 = tbase + blockIdx.x * blockDim.x + threadIdx.x;  // threads [tbase, nthreads)
     if (!LOOP) {
-        if (t0 < nthreads) k_lat_force_mixed_site(t0, nt, g, s, in, pt, sp, kick, hook, order, fuse_next, lists);
+        if (t0 < nthreads) k_lat_force_mixed_site<ONE>(t0, nt, g, s, in, pt, sp, kick, hook, order, fuse_next, lists);
         return;
     }
     for (int t = t0; t < nthreads; t += gridDim.x * blockDim.x)
-        k_lat_force_mixed_site(t, nt, g, s, in, pt, sp, kick, hook, order, fuse_next, false);
+        k_lat_force_mixed_site<ONE>(t, nt, g, s, in, pt, sp, kick, hook, order, fuse_next, false);
 }
 
 // ---- the force passes of small boxes and thin slabs: see rho_mixed_split (500 groups: 30 -> 14 us; FP64 form 58 ->
@@ -2330,6 +2337,9 @@ __global__ void __launch_bounds__(32 * W, B) k_lat_force_fix_split(const __grid_
     force_fix_split<W, U>(nt, cand + a.par * kMaxFull, g, s, in, pt, fp, sp, a, kick, hook, fuse_next, lists && !wild, far, wild, sh, part);
 }
 
+// Where every type has the same tables (one_type), the force passes drop the third record of a pair of two types, its
+// branch and the types: by the spills it saves as much as by the branch (2M atoms: mixed 419 -> 399 us, FP64 1227 -> 1163).
+// With several, a pair's three FP64 records are loaded together (3 elements, 2M atoms: 1535 -> 1504 us).
 static void launch_lat_force_threads(const LaunchCtx &lc, const Geom &g, Slots s, Inter in, PotTables t, StepParams *p,
                                      bool kick, bool mixed, bool hook, int tb, int te, bool fuse_next = false,
                                      bool lists = false) {
@@ -2339,12 +2349,14 @@ static void launch_lat_force_threads(const LaunchCtx &lc, const Geom &g, Slots s
     const bool fuse = fuse_next && kick && !hook && (mixed || lc.fp);
     s = with_records(lc, s);
     if (lc.force_apt > 1) {
-        if (mixed) k_lat_force_mixed<true><<<n, b, 0, lc.stream>>>(*lc.nt, g, s, in, t, p, kick, hook, order, tb, te, fuse, false);
-        else if (lc.fp) k_lat_force_fix<true><<<n, b, 0, lc.stream>>>(*lc.nt, g, s, in, t, *lc.fp, p, kick, hook, order, tb, te, fuse, false);
+        if (mixed) k_lat_force_mixed<true, false><<<n, b, 0, lc.stream>>>(*lc.nt, g, s, in, t, p, kick, hook, order, tb, te, fuse, false);
+        else if (lc.fp) k_lat_force_fix<true, false><<<n, b, 0, lc.stream>>>(*lc.nt, g, s, in, t, *lc.fp, p, kick, hook, order, tb, te, fuse, false);
         else k_lat_force_fp64<true><<<n, b, 0, lc.stream>>>(*lc.nt, g, s, in, t, p, kick, hook, order, tb, te);
     } else {
-        if (mixed) k_lat_force_mixed<false><<<n, b, 0, lc.stream>>>(*lc.nt, g, s, in, t, p, kick, hook, order, tb, te, fuse, lists);
-        else if (lc.fp) k_lat_force_fix<false><<<n, b, 0, lc.stream>>>(*lc.nt, g, s, in, t, *lc.fp, p, kick, hook, order, tb, te, fuse, lists);
+        if (mixed && lc.one_type) k_lat_force_mixed<false, true><<<n, b, 0, lc.stream>>>(*lc.nt, g, s, in, t, p, kick, hook, order, tb, te, fuse, lists);
+        else if (mixed) k_lat_force_mixed<false, false><<<n, b, 0, lc.stream>>>(*lc.nt, g, s, in, t, p, kick, hook, order, tb, te, fuse, lists);
+        else if (lc.fp && lc.one_type) k_lat_force_fix<false, true><<<n, b, 0, lc.stream>>>(*lc.nt, g, s, in, t, *lc.fp, p, kick, hook, order, tb, te, fuse, lists);
+        else if (lc.fp) k_lat_force_fix<false, false><<<n, b, 0, lc.stream>>>(*lc.nt, g, s, in, t, *lc.fp, p, kick, hook, order, tb, te, fuse, lists);
         else k_lat_force_fp64<false><<<n, b, 0, lc.stream>>>(*lc.nt, g, s, in, t, p, kick, hook, order, tb, te);
     }
 }
