@@ -148,8 +148,8 @@ mg_status mg_dt_history(mg_context *ctx, double *out, int64_t cap, int64_t *n_ou
 mg_status mg_prepare(mg_context *ctx);
 /* nsteps iterations of the loop body (src/simulation.cpp:165-193): firststep, decide, exchangeInter,
  * borderInter, exchangeAtom, computeEam, secondstep. Asynchronous on the context stream unless
- * sync != 0. The step sequence is captured once as a CUDA graph and replayed; in the mixed form with
- * a fixed dt, runs of 16 bodies replay one fused graph (mg_set_step_fusion). */
+ * sync != 0. The step sequence is captured once as a CUDA graph and replayed; with a fixed dt, runs of
+ * 16 bodies (mixed form) or 4 (FP64 form) replay one fused graph (mg_set_step_fusion). */
 mg_status mg_simulate(mg_context *ctx, int64_t nsteps, int32_t sync);
 /* One phase of the loop body, for parity checks: 0 firststep, 1 decide, 2 exchangeInter,
  * 3 borderInter, 4 exchangeAtom, 5 computeEam, 6 secondstep. */
@@ -197,7 +197,7 @@ mg_status mg_clear_errors(mg_context *ctx);
 mg_status mg_step_host(mg_context *ctx, mg_atom_element *atoms, int64_t n_slots, mg_atom_element *inter,
                        int64_t inter_cap, int64_t *n_inter, int64_t nsteps);
 /* Loop bodies per CUDA graph launch of mg_simulate in the mixed form with a fixed dt (default 16; 0 or
- * 1: one body per launch). Inside a launch, each force pass but the last also takes the next body's
+ * 1: one body per launch, in every form; otherwise the FP64 form launches 4 at a time). Inside a launch, each force pass but the last also takes the next body's
  * firststep for its atoms (when no inter atoms exist; the kernels check on the device), which saves
  * the separate firststep pass. The state between launches is the end of a loop body as always, and
  * results are bit-identical either way. mg_run_stages uses the same graph for runs of bodies with
