@@ -1863,8 +1863,8 @@ __device__ __noinline__ double3 force_near_fp64(const NeighTables &nt, const Geo
     }
     return make_double3(fx, fy, fz);
 }
-// U candidates, as rho_fix_pairs
-template <int U>
+// U candidates, as rho_fix_pairs. ONE: every type has the same tables
+template <int U, bool ONE>
 __device__ __forceinline__ void force_fix_pairs(const Slots &s, const FixParams &fp, const int (&oj)[U], const bool (&use)[U],
                                                 const int (&q)[U], int ti, i64 xb, i64 yb, i64 zb, i64 dfb, FixForce &a) {
     FixRec j[U];
@@ -1886,7 +1886,7 @@ __device__ __forceinline__ void force_fix_pairs(const Slots &s, const FixParams 
         in[u] = use[u] && (unsigned long long) (r2 - fp.lo) < (unsigned long long) (fp.rc2 - fp.lo);
         if (use[u] && (unsigned long long) r2 < (unsigned long long) fp.lo) fix_note_near(a.near, q[u]);
         t[u] = fix_locate(fp, in[u] ? r2 : fp.rc2 - 1, m[u]);
-        tj[u] = in[u] ? (int) j[u].type : ti;
+        tj[u] = !ONE && in[u] ? (int) j[u].type : ti;
         const FixPoly *rec = fp.zg + 2 * ((ti * 3 + tj[u]) * fp.nr1 + m[u]);
         pg[u] = ld_fix_poly(rec);
         ph[u] = ld_fix_poly(rec + 1);
@@ -1897,7 +1897,7 @@ __device__ __forceinline__ void force_fix_pairs(const Slots &s, const FixParams 
         i64 f = fix_poly(ph[u], t[u], fp.e3_h);
         const i64 both = dfb + dfj[u];  // biased
         if (in[u]) a.df_hi = max(a.df_hi, fix_hi(both));
-        if (tj[u] == ti) {
+        if (ONE || tj[u] == ti) {
             f = fix_mul_add(fix_hi(both), fix_lo(both), fix_hi(gj), fix_lo(gj), f);
         } else {
             const i64 gi = fix_poly(ld_fix_poly(fp.zg + 2 * ((tj[u] * 3 + ti) * fp.nr1 + m[u])), t[u], fp.e3_g);
@@ -2264,7 +2264,7 @@ struct SplitForce {
     int df_hi[W][32];
     unsigned near[W][32];
 };
-template <int W, int U>
+template <int W, int U, bool ONE>
 __device__ __forceinline__ void force_fix_split(const NeighTables &nt, const float4 *cand, const Geom &g, const Slots &s,
                                                 const Inter &in, const PotTables &pt, const FixParams &fp, StepParams *sp,
                                                 const SplitSite &a, bool kick, bool hook, bool fuse_next, bool lists, bool far, bool wild,
@@ -2289,7 +2289,7 @@ __device__ __forceinline__ void force_fix_split(const NeighTables &nt, const flo
                 int oj[U], q[U];
                 bool use[U];
                 split_next<U>(sh, a.si, q0, c, c1, oj, use, q);
-                force_fix_pairs<U>(s, fp, oj, use, q, a.ti, xb, yb, zb, dfb, m);
+                force_fix_pairs<U, ONE>(s, fp, oj, use, q, a.ti, xb, yb, zb, dfb, m);
             }
         }
         part.x[warp][lane] = m.x;
@@ -2318,7 +2318,7 @@ __device__ __forceinline__ void force_fix_split(const NeighTables &nt, const flo
     force_done_fix(nt, g, s, in, pt, sp, a.sl, a.si, a.ti, a.par, tot, f, kick, hook, fuse_next, wild);
 }
 // B: blocks an SM holds
-template <int W, int B, int U>
+template <int W, int B, int U, bool ONE>
 __global__ void __launch_bounds__(32 * W, B) k_lat_force_fix_split(const __grid_constant__ NeighTables nt, const float4 *cand,
                                                                         const __grid_constant__ Geom g, const __grid_constant__ Slots s,
                                                                         const __grid_constant__ Inter in,
@@ -2334,7 +2334,7 @@ __global__ void __launch_bounds__(32 * W, B) k_lat_force_fix_split(const __grid_
         return;
     }
     const bool far = a.ti >= 0 && in.far_flag[a.sl];
-    force_fix_split<W, U>(nt, cand + a.par * kMaxFull, g, s, in, pt, fp, sp, a, kick, hook, fuse_next, lists && !wild, far, wild, sh, part);
+    force_fix_split<W, U, ONE>(nt, cand + a.par * kMaxFull, g, s, in, pt, fp, sp, a, kick, hook, fuse_next, lists && !wild, far, wild, sh, part);
 }
 
 // Where every type has the same tables (one_type), the force passes drop the third record of a pair of two types, its
@@ -2360,6 +2360,20 @@ static void launch_lat_force_threads(const LaunchCtx &lc, const Geom &g, Slots s
         else k_lat_force_fp64<false><<<n, b, 0, lc.stream>>>(*lc.nt, g, s, in, t, p, kick, hook, order, tb, te);
     }
 }
+// one element: a step of 16k atoms 50.2 -> 49.5 us, 65k 108.1 -> 103.9, 128k 172.4 -> 166.6
+template <int W, bool ONE>
+static void launch_force_fix_split(const LaunchCtx &lc, const Geom &g, Slots s, Inter in, PotTables t, StepParams *p, bool kick, bool hook,
+                                   int u0, int u1, bool fuse, bool lists) {
+    const int n = split_groups(u0, u1);
+    const float4 *cand = &lc.ntd->cand[0][0];
+    // 500 groups of 8 warps fit one wave at 64 registers, one candidate at a time: 29.1 -> 26.2 us
+    if constexpr (W == 8)
+        if (n * lc.share > 2 * lc.num_sms) {
+            k_lat_force_fix_split<W, 4, 1, ONE><<<n, 32 * W, 0, lc.stream>>>(*lc.nt, cand, g, s, in, t, *lc.fp, p, kick, hook, u0, u1, fuse, lists);
+            return;
+        }
+    k_lat_force_fix_split<W, 20 / W, kFixForceAhead, ONE><<<n, 32 * W, 0, lc.stream>>>(*lc.nt, cand, g, s, in, t, *lc.fp, p, kick, hook, u0, u1, fuse, lists);
+}
 template <int W>
 static void launch_force_split_w(const LaunchCtx &lc, const Geom &g, Slots s, Inter in, PotTables t, StepParams *p, bool kick, bool mixed,
                                  bool hook, int u0, int u1, bool fuse_next, bool lists) {
@@ -2369,15 +2383,8 @@ static void launch_force_split_w(const LaunchCtx &lc, const Geom &g, Slots s, In
     if (mixed)
         k_lat_force_mixed_split<W><<<n, 32 * W, 0, lc.stream>>>(&lc.ntd->cand[0][0], lc.nt->npruned, lc.nt->nfull, g, s, in, t, p, kick, hook, u0, u1,
                                                                 fuse, lists);
-    else {
-        // 500 groups of 8 warps fit one wave at 64 registers, one candidate at a time: 29.1 -> 26.2 us
-        if constexpr (W == 8)
-            if (n * lc.share > 2 * lc.num_sms) {
-                k_lat_force_fix_split<W, 4, 1><<<n, 32 * W, 0, lc.stream>>>(*lc.nt, &lc.ntd->cand[0][0], g, s, in, t, *lc.fp, p, kick, hook, u0, u1, fuse, lists);
-                return;
-            }
-        k_lat_force_fix_split<W, 20 / W, kFixForceAhead><<<n, 32 * W, 0, lc.stream>>>(*lc.nt, &lc.ntd->cand[0][0], g, s, in, t, *lc.fp, p, kick, hook, u0, u1, fuse, lists);
-    }
+    else if (lc.one_type) launch_force_fix_split<W, true>(lc, g, s, in, t, p, kick, hook, u0, u1, fuse, lists);
+    else launch_force_fix_split<W, false>(lc, g, s, in, t, p, kick, hook, u0, u1, fuse, lists);
 }
 static bool launch_lat_force_split(const LaunchCtx &lc, const Geom &g, Slots s, Inter in, PotTables t, StepParams *p, bool kick, bool mixed,
                                    bool hook, int u0, int u1, bool fuse_next, bool lists) {

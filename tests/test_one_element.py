@@ -1,4 +1,4 @@
-"""The force passes over whole groups leave the types out where every type has the same tables (a potential of one
+"""The force passes leave the types out where every type has the same tables (a potential of one
 element). A potential with that element's tables under three names takes the general passes; iron alone gives the
 same operations in both, so the same bits."""
 import numpy as np
@@ -21,9 +21,11 @@ def _three_names(path, out):
     return str(out)
 
 
-# 8116 groups with short last ones, and 62500 of 32 sites (the mixed form's wider blocks)
+# 8116 groups with short last ones, and 62500 of 32 sites (the mixed form's wider blocks); 18, 430, 1014 and 3906 groups
+# for the split passes
 @pytest.mark.parametrize("prec", ["fp64", "mixed"])
-@pytest.mark.parametrize("cells,steps", [((53, 50, 49), 21), ((100, 100, 100), 3)])
+@pytest.mark.parametrize("cells,steps", [((53, 50, 49), 21), ((100, 100, 100), 3), ((6, 6, 8), 21), ((13, 17, 31), 21),
+                                         ((24, 25, 27), 21), ((40, 39, 40), 21)])
 def test_one_element_gives_the_same_bits(pkg, wl, potentials, gpu_lib, tmp_path, prec, cells, steps):
     atoms = wl.build_state(cells, A0, RCF, temperature=900.0, seed=12)
     got = []
