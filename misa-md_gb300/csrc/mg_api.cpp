@@ -1363,7 +1363,8 @@ mg_status mg_clear_errors(mg_context *ctx) {
 // 2.69 -> 2.44 ms). The thin slabs at the periodic z seam
 // (two of 4 planes at each end) wait for the ghost planes, copied after the last chunk. Per atom the
 // kernels and their order are those of the unpipelined path, so the result is bit-identical to it. If a
-// chunk's decide met a displaced atom that does not go straight back to its own site, the step is void:
+// chunk's decide met a displaced atom that does not go straight back to its own site, or its firststep one too far off
+// for the fixed-point records, the step is void:
 // it runs again in full from the kept input, as mg_upload + one loop body + mg_download would.
 // S >= 6 in-chunks and 6 <= SS <= bz / 4 density slabs, at least 32 sites of a parity per plane.
 static mg_status step_host_overlapped(mg_context *ctx, mg_atom_element *atoms, mg_atom_element *inter,
@@ -1381,7 +1382,8 @@ static mg_status step_host_overlapped(mg_context *ctx, mg_atom_element *atoms, m
     mg_status st;
     if ((st = ensure_aos(ctx)) != MG_OK) return st;
     if (!ctx->d_aos_in) MG_CK(dalloc(ctx, &ctx->d_aos_in, static_cast<size_t>(g.n_slots)));
-    const LaunchCtx lc = ctx->lc();
+    LaunchCtx lc = ctx->lc();
+    lc.spec = true;
     LaunchCtx lf = lc;  // force slabs and packs
     lf.stream = ctx->side;
     const bool mx = ctx->mixed();
@@ -1515,7 +1517,7 @@ static mg_status step_host_overlapped(mg_context *ctx, mg_atom_element *atoms, m
     ctx->energy_valid = false;
     if (cnt[CNT_SPEC_VOID]) {
         // the whole loop body again from the kept input (the step head has run once already)
-        launch_unpack_aos(lc, g, ctx->d_aos_in, ctx->s, ctx->in, ctx->types_ok_mask, mx);
+        launch_unpack_aos(ctx->lc(), g, ctx->d_aos_in, ctx->s, ctx->in, ctx->types_ok_mask, mx);
         launch_set_counts(lc, ctx->in, 0);
         seq_firststep(ctx, true, nullptr);
         seq_compute_eam(ctx, true, true, MANAGE_DECIDE | MANAGE_CLEAR_GHOST | MANAGE_EXCHANGE | MANAGE_BORDER, nullptr);

@@ -29,7 +29,8 @@ constexpr uint32_t kInBox = 0, kXLow = 1u, kXHigh = 2u, kYLow = 4u, kYHigh = 8u,
 // device counters / flags word indices
 // CNT_TOUCHED: lattice owners listed by an inter-atom pass for the ordered owner gather that follows;
 // CNT_TOUCH_DONE: blocks of that gather finished (the last one resets both words)
-// CNT_SPEC_VOID: the overlapped host step met a displaced atom whose decide it cannot take per chunk
+// CNT_SPEC_VOID: the overlapped host step met a displaced atom whose decide it cannot take per chunk, or one too far
+// from its site for the fixed-point records
 enum {
     CNT_INTER = 0, CNT_GHOST = 1, CNT_DISPLACED = 2, CNT_ERRORS = 3, CNT_FAR = 4, CNT_TOUCHED = 5, CNT_TOUCH_DONE = 6,
     CNT_SPEC_VOID = 7, CNT_WORDS = 8
@@ -120,7 +121,7 @@ struct Slots {
     FixRec *fix;             // fixed-point coordinates and type
     FixRec *fixn;            // the next loop body's buffer when the force pass takes the next firststep
     int kx;                  // of a launch that keeps them: their unit's exponent (0: not kept)
-    int wild_now;            // of a firststep over part of the box: SkinState::wild holds at once
+    int spec;                // of a launch of the overlapped host step: see LaunchCtx::spec
     i64 *dfq;                // F'(rho) in fixed point, written wherever df is
 };
 
@@ -265,6 +266,9 @@ struct LaunchCtx {
     const FixParams *fp = nullptr;           // FP64 form: scales and tables of the fixed-point pair arithmetic
     int share = 1;                           // contexts that step side by side (a batch's members)
     bool one_type = false;                   // all types have the same tables
+    // The overlapped host step: its force slabs run beside the unpack and firststep of later chunks, so none of its
+    // kernels reads or writes SkinState::wild. An atom that far off voids the step (CNT_SPEC_VOID) and is a vacancy to it.
+    bool spec = false;
 };
 
 // Mass table shared by all contexts (atom types are fixed).

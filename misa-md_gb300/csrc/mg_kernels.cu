@@ -373,9 +373,12 @@ __device__ __forceinline__ bool fix_wild(float4 u) {
 // with the FP64 form's records (off when the launch's form keeps none)
 inline Slots with_records(const LaunchCtx &lc, Slots s) {
     s.kx = lc.fp ? lc.fp->kx : 0;
-    s.wild_now = 0;
+    s.spec = lc.spec;
     return s;
 }
+// whether a pass takes every atom in FP64: the same in every thread of its grid, since nothing writes the word while a
+// pass that reads it runs
+__device__ __forceinline__ bool pass_wild(const Slots &s) { return !s.spec && s.skin->wild != 0; }
 
 // ------------------------------------------------------------------------------------------------
 // AoS <-> SoA (the reference's AtomElement array crosses the boundary as raw records)
@@ -405,7 +408,7 @@ __global__ void k_unpack_aos(Geom g, const mg_atom_element *aos, Slots s, Inter 
         if (s.kx && a.type < 0) fix_put_vacant(g, s.fix + si, s.kx, t);
         else if (s.kx) {
             fix_put(s.fix + si, s.kx, a.x[0], a.x[1], a.x[2], a.type);
-            if (fix_wild(u)) s.skin->wild = 1;
+            if (fix_wild(u) && !s.spec) s.skin->wild = 1;
         }
     }
     if (mixed) s.df32[sidx(g, t)] = (float) a.df;
@@ -535,8 +538,13 @@ __device__ __forceinline__ void first_half(const Geom &g, const Slots &s, const 
         if (s.kx) {
             fix_put(fix_out + si, s.kx, x, y, z, ty);
             if (fix_wild(nu)) {
-                s.skin->wild_next = 1;
-                if (s.wild_now) s.skin->wild = 1;
+                if (!s.spec) {
+                    s.skin->wild_next = 1;
+                } else {  // its wrapped coordinates could meet a vacancy's
+                    in.cnt[CNT_SPEC_VOID] = 1;
+                    u4_out[si] = vacant_u4();
+                    fix_put_vacant(g, fix_out + si, s.kx, sl);
+                }
             }
         }
     }
@@ -660,7 +668,6 @@ void launch_firststep(const LaunchCtx &lc, const Geom &g, Slots s, Inter in, con
     if (t1 <= t0) return;
     const int b = kFirstThreads, n = std::min((t1 - t0 + b - 1) / b, lc.num_sms * 8);
     s = with_records(lc, s);
-    s.wild_now = !whole;  // a part's passes may come before the list manager
     if (decide) k_firststep<true, true><<<n, b, 0, lc.stream>>>(lc.ntd, g, s, in, p, t0, t1, fused, alt, whole);
     else k_firststep<true, false><<<n, b, 0, lc.stream>>>(lc.ntd, g, s, in, p, t0, t1, fused, alt, whole);
 }
@@ -1475,7 +1482,7 @@ __global__ void __launch_bounds__(512, 2) k_lat_rho_fix(const __grid_constant__ 
                                                         const __grid_constant__ PotTables pt, const __grid_constant__ FixParams fp,
                                                         bool hook, int order, int tbase, int nthreads, bool lists) {
     const int t0 = tbase + blockIdx.x * blockDim.x + threadIdx.x;  // threads [tbase, nthreads)
-    const bool wild = s.skin->wild != 0;  // the same in every thread of the grid: set before the pass
+    const bool wild = pass_wild(s);
     if (LOOP) {
         for (int t = t0; t < nthreads; t += gridDim.x * blockDim.x)
             k_lat_rho_fix_site(t, true, nt, g, s, in, pt, fp, hook, order, false, true, wild);
@@ -1555,7 +1562,7 @@ __global__ void __launch_bounds__(32 * W, 32 / W) k_lat_rho_fix_split(const __gr
     __shared__ SplitList sh;
     __shared__ i64 part[W][32];
     __shared__ unsigned part_near[W][32];
-    const bool wild = s.skin->wild != 0;
+    const bool wild = pass_wild(s);
     bool full = lists && !wild && skin_full(g, s);
     if (lists && blockIdx.x == 0 && threadIdx.x == 0) {
         if (wild) s.skin->dirty = 1;  // groups near a recombined atom did not rebuild their lists
@@ -1605,6 +1612,7 @@ template <int W>
 static void launch_rho_split_w(const LaunchCtx &lc, const Geom &g, Slots s, Inter in, PotTables t, bool mixed, bool hook, int u0, int u1,
                                bool lists) {
     const int n = split_groups(u0, u1);
+    s = with_records(lc, s);
     if (mixed)
         k_lat_rho_mixed_split<W><<<n, 32 * W, 0, lc.stream>>>(&lc.ntd->cand[0][0], lc.nt->npruned, lc.nt->nfull, g, s, in, t, hook, u0, u1, lists);
     else k_lat_rho_fix_split<W><<<n, 32 * W, 0, lc.stream>>>(*lc.nt, &lc.ntd->cand[0][0], g, s, in, t, *lc.fp, hook, u0, u1, lists);
@@ -1624,6 +1632,7 @@ static void launch_lat_rho_threads(const LaunchCtx &lc, const Geom &g, Slots s, 
     const int order = lc.rho_order, b = lc.rho_block;
     const int n = (te - tb + b * lc.rho_apt - 1) / (b * lc.rho_apt);
     if (n <= 0) return;
+    s = with_records(lc, s);
     if (lc.rho_apt > 1) {
         if (mixed) k_lat_rho_mixed<true><<<n, b, 0, lc.stream>>>(*lc.nt, g, s, in, t, hook, order, tb, te, false);
         else if (lc.fp) k_lat_rho_fix<true><<<n, b, 0, lc.stream>>>(*lc.nt, g, s, in, t, *lc.fp, hook, order, tb, te, false);
@@ -2031,7 +2040,7 @@ __global__ void __launch_bounds__(512, 2) k_lat_force_fix(const __grid_constant_
                                                           StepParams *sp, bool kick, bool hook, int order, int tbase, int nthreads,
                                                           bool fuse_next, bool lists) {
     const int t0 = tbase + blockIdx.x * blockDim.x + threadIdx.x;  // threads [tbase, nthreads)
-    const bool wild = s.skin->wild != 0;
+    const bool wild = pass_wild(s);
     if (!LOOP) {
         if (t0 < nthreads) k_lat_force_fix_site<ONE>(t0, nt, g, s, in, pt, fp, sp, kick, hook, order, fuse_next, lists && !wild, wild);
         return;
@@ -2327,7 +2336,7 @@ __global__ void __launch_bounds__(32 * W, B) k_lat_force_fix_split(const __grid_
                                                                         bool hook, int u0, int u1, bool fuse_next, bool lists) {
     __shared__ SplitList sh;
     __shared__ SplitForce<W> part;
-    const bool wild = s.skin->wild != 0;
+    const bool wild = pass_wild(s);
     const SplitSite a = split_site(g, s, u0, u1);
     if (!__any_sync(0xffffffffu, a.ti >= 0)) {
         if (threadIdx.x < 32 && a.sl >= 0) force_vacant_fix(g, s, in, a.sl, a.si, fuse_next, wild);
