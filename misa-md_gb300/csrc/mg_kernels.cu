@@ -540,6 +540,7 @@ __device__ __forceinline__ void first_half(const Geom &g, const Slots &s, const 
             if (fix_wild(nu)) {
                 if (!s.spec) {
                     s.skin->wild_next = 1;
+                    if (!DECIDE) s.skin->wild = 1;  // firststep as a phase of its own: no decide need follow
                 } else {  // its wrapped coordinates could meet a vacancy's
                     in.cnt[CNT_SPEC_VOID] = 1;
                     u4_out[si] = vacant_u4();
