@@ -225,11 +225,13 @@ mg_status mg_skin_stats(mg_context *ctx, int64_t *passes, int64_t *rebuilds);
 mg_status mg_ws_map(mg_context *ctx, const double *xyz, int64_t n, int64_t *coords, uint32_t *flags,
                     int64_t *index);
 
-/* Autotuner: times the density and force passes of the current precision on the resident state for
- * every gather thread order (0: all even sites then all odd; 1: even/odd warps interleaved per 32
- * sites), block size (128, 256, 512) and number of sites per thread (1, 2, 4; a thread's sites are
- * one grid stride apart), reps launches each, and keeps the fastest. Results are cached per
- * (box, precision) for the life of the process. out (may be NULL) receives {rho order, rho block,
+/* Autotuner: times the density and force passes of the current precision on the resident state, as a
+ * step launches them, for every gather thread order (0: all even sites then all odd; 1: even/odd warps
+ * interleaved per 32 sites), block size (128, 256, 512) and number of sites per thread (1, 2, 4; a
+ * thread's sites are one grid stride apart) under which the group candidate lists stay in use, reps
+ * launches each, and keeps the fastest. Small boxes, whose passes share a group among several warps, have
+ * no shapes to choose: they get the default ones. Results are cached per box, candidate table, precision
+ * and kind of potential for the life of the process. out (may be NULL) receives {rho order, rho block,
  * rho sites per thread, force order, force block, force sites per thread}. Needs mg_prepare first. */
 mg_status mg_autotune(mg_context *ctx, int32_t reps, int32_t out[6]);
 /* Sets the six tuning values directly (same layout as mg_autotune's out). */

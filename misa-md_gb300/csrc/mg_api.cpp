@@ -37,8 +37,6 @@ namespace mg {
 void set_global_error(const char *msg) { g_create_error = msg ? msg : ""; }
 }  // namespace mg
 
-constexpr int kWideForce = 1500000;  // sites from which the mixed force pass takes blocks of 512 (mg_context::tune)
-
 struct mg_context {
     int device = 0;
     int precision = MG_PREC_FP64;
@@ -106,14 +104,7 @@ struct mg_context {
     uint64_t stage_dump_interval = 0;
     std::string origin_path;
 
-    // [precision][rho, force] = {thread order, block size, atoms per thread}. Order 1 until an autotune: its
-    // warps cover whole 32-site groups in every box, so the group lists serve boxes with an odd number of sites
-    // of a parity as well (order 0 visits all 112 candidates there). Block sizes by measurement: the FP64 density pass
-    // 128 (2M atoms: 720 us with 256, 682 with 128), its force pass 256 (128: 2M atoms -0.2%, 304k atoms +1%); the
-    // mixed density pass 512 (2M atoms 233 -> 228 us, 221k atoms 40.2 -> 38.3, elsewhere even); the mixed force pass
-    // 256, from kWideForce sites on 512, whose groups share more of L1 (2M atoms 427 -> 419 us; 1M atoms 264 -> 267
-    // and 315k atoms 103 -> 107, by their last wave).
-    int tune[2][2][3] = {{{1, 128, 1}, {1, 256, 1}}, {{1, 512, 1}, {1, 256, 1}}};
+    int tune[2][2][3];              // [precision][rho, force] = {thread order, block size, atoms per thread}
     int share = 1;                  // contexts stepping side by side (while a batch captures)
     LaunchCtx lc() const {
         LaunchCtx l{stream, num_sms};
@@ -163,6 +154,20 @@ void set_skin(Geom &g, double skin) {
     g.skin_h = static_cast<float>(skin * g.inv_h);
     const double r = (g.rc + skin) * g.inv_h;
     g.rcs2_h = skin > 0.0 ? static_cast<float>(r * r) : g.rc2_h;
+}
+
+// The launch shapes until an autotune. Order 1: its
+// warps cover whole 32-site groups in every box, so the group lists serve boxes with an odd number of sites
+// of a parity as well (order 0 visits all 112 candidates there). Block sizes by measurement: the FP64 density pass
+// 128 (2M atoms: 720 us with 256, 682 with 128), its force pass 256 (128: 2M atoms -0.2%, 304k atoms +1%); the
+// mixed density pass 512 (2M atoms 233 -> 228 us, 221k atoms 40.2 -> 38.3, elsewhere even); the mixed force pass
+// 256, from kWideForce sites on 512, whose groups share more of L1 (2M atoms 427 -> 419 us; 1M atoms 264 -> 267
+// and 315k atoms 103 -> 107, by their last wave).
+constexpr int kWideForce = 1500000;
+void default_shapes(mg_context *ctx, int precision) {
+    const bool mixed = precision == MG_PREC_MIXED;
+    const int shapes[2][3] = {{1, mixed ? 512 : 128, 1}, {1, mixed && ctx->g.n_local >= kWideForce ? 512 : 256, 1}};
+    std::memcpy(ctx->tune[precision], shapes, sizeof(shapes));
 }
 
 int next_pow2(int n) {
@@ -591,7 +596,8 @@ mg_status mg_create(const int64_t phase_space[3], double lattice_const, double r
     g.half = g.n_slots / 2;  // Sx is even, so slot parity is x parity
     g.nxh = g.bx / 2;
     g.n_local_half = g.n_local / 2;
-    if (g.n_local >= kWideForce) ctx->tune[MG_PREC_MIXED][1][1] = 512;
+    default_shapes(ctx, MG_PREC_FP64);
+    default_shapes(ctx, MG_PREC_MIXED);
     for (int d = 0; d < 3; d++) g.cells[d] = (int) phase_space[d];
     g.a0 = lattice_const;
     g.rc = lattice_const * rcf;  // atom::atom, src/atom.cpp:14-19
@@ -1772,78 +1778,98 @@ mg_status mg_ws_map(mg_context *ctx, const double *xyz, int64_t n, int64_t *coor
     return MG_OK;
 }
 
-// Autotuner: times each gather kernel of the current precision for every (thread order, block size)
-// on the resident state and keeps the fastest; results are cached per (box, precision) for the process.
+// Autotuner: times each gather pass of the current precision as the step launches it, for every (thread order, block
+// size, sites per thread) that keeps what the step gains from its group lists, on the resident state, and keeps the
+// fastest. Shapes that lose the lists are left out: with them every candidate is searched in every step (16k atoms mixed:
+// 40 -> 54 us per step, FP64 50 -> 62). Split passes (small boxes) take their own shapes, so there the default
+// shapes stand. Results are cached for the process, by what decides which kernels run and on how many groups.
 namespace {
 struct TuneKey {
-    int cells[3], precision;
+    int cells[3], precision, n_pruned;
+    bool fixed, one_type;  // the passes' form
     bool operator==(const TuneKey &o) const {
-        return cells[0] == o.cells[0] && cells[1] == o.cells[1] && cells[2] == o.cells[2] && precision == o.precision;
+        return cells[0] == o.cells[0] && cells[1] == o.cells[1] && cells[2] == o.cells[2] && precision == o.precision &&
+               n_pruned == o.n_pruned && fixed == o.fixed && one_type == o.one_type;
     }
 };
 std::vector<std::pair<TuneKey, std::array<int, 6>>> g_tune_cache;
 std::mutex g_tune_mutex;
+
+// every shape for the density pass, then for the force pass
+mg_status time_shapes(mg_context *ctx, int reps, cudaEvent_t e0, cudaEvent_t e1) {
+    const Geom &g = ctx->g;
+    const int p = ctx->precision, blocks[3] = {128, 256, 512}, apts[3] = {1, 2, 4};
+    const bool keep = lat_lists(ctx->lc(), g, ctx->mixed());
+    for (int kern = 0; kern < 2; kern++) {
+        float best_ms = 1e30f;
+        int *tune = ctx->tune[p][kern], best[3] = {tune[0], tune[1], tune[2]};
+        for (int order = 0; order < 2; order++) {
+            for (int b : blocks) for (int apt : apts) {
+                tune[0] = order;
+                tune[1] = b;
+                tune[2] = apt;
+                const LaunchCtx lc = ctx->lc();
+                if (keep && !lat_lists(lc, g, ctx->mixed())) continue;
+                auto run = [&]() {
+                    if (kern == 0) launch_lat_rho(lc, g, ctx->s, ctx->in, ctx->pt, ctx->mixed(), false, true);
+                    else launch_lat_force(lc, g, ctx->s, ctx->in, ctx->pt, ctx->d_sp, false, ctx->mixed(), false, false, true);
+                };
+                run();  // warm
+                MG_CK(cudaEventRecord(e0, ctx->stream));
+                for (int r = 0; r < reps; r++) run();
+                MG_CK(cudaEventRecord(e1, ctx->stream));
+                MG_CK(cudaEventSynchronize(e1));
+                float ms = 0.f;
+                MG_CK(cudaEventElapsedTime(&ms, e0, e1));
+                if (ms < best_ms) { best_ms = ms; best[0] = order; best[1] = b; best[2] = apt; }
+            }
+        }
+        for (int c = 0; c < 3; c++) tune[c] = best[c];
+    }
+    return check_launch(ctx);
+}
 }  // namespace
 
 mg_status mg_autotune(mg_context *ctx, int32_t reps, int32_t out[6]) {
     if (!ctx) return MG_ERR_ARG;
     if (!ctx->prepared) { ctx->err = "mg_prepare must run before mg_autotune"; return MG_ERR_STATE; }
     const int p = ctx->precision;
-    const TuneKey key{{ctx->g.cells[0], ctx->g.cells[1], ctx->g.cells[2]}, p};
+    const TuneKey key{{ctx->g.cells[0], ctx->g.cells[1], ctx->g.cells[2]}, p, ctx->n_pruned, ctx->lc().fp != nullptr, ctx->one_type};
+    std::array<int, 6> best{};
+    bool known = false;
     {
         std::lock_guard<std::mutex> lock(g_tune_mutex);
         for (auto &kv : g_tune_cache) {
             if (kv.first == key) {
-                for (int k = 0; k < 2; k++)
-                    for (int c = 0; c < 3; c++) ctx->tune[p][k][c] = kv.second[3 * k + c];
-                if (out) for (int k = 0; k < 6; k++) out[k] = kv.second[k];
-                ctx->graph_stale = true;
-                ctx->gen++;
-                return MG_OK;
+                best = kv.second;
+                known = true;
+                break;
             }
         }
     }
-    if (reps < 1) reps = 3;
-    cudaEvent_t e0, e1;
-    MG_CK(cudaEventCreate(&e0));
-    MG_CK(cudaEventCreate(&e1));
-    const int blocks[3] = {128, 256, 512}, apts[3] = {1, 2, 4};
-    std::array<int, 6> best{};
-    for (int kern = 0; kern < 2; kern++) {
-        float best_ms = 1e30f;
-        for (int order = 0; order < 2; order++) {
-            for (int b : blocks) for (int apt : apts) {
-                ctx->tune[p][kern][0] = order;
-                ctx->tune[p][kern][1] = b;
-                ctx->tune[p][kern][2] = apt;
-                const LaunchCtx lc = ctx->lc();
-                auto run = [&]() {
-                    if (kern == 0) launch_lat_rho(lc, ctx->g, ctx->s, ctx->in, ctx->pt, ctx->mixed(), false);
-                    else launch_lat_force(lc, ctx->g, ctx->s, ctx->in, ctx->pt, ctx->d_sp, false, ctx->mixed(), false);
-                };
-                run();  // warm
-                cudaEventRecord(e0, ctx->stream);
-                for (int r = 0; r < reps; r++) run();
-                cudaEventRecord(e1, ctx->stream);
-                MG_CK(cudaEventSynchronize(e1));
-                float ms = 0.f;
-                cudaEventElapsedTime(&ms, e0, e1);
-                if (ms < best_ms) { best_ms = ms; best[3 * kern] = order; best[3 * kern + 1] = b; best[3 * kern + 2] = apt; }
+    ctx->graph_stale = true;
+    ctx->gen++;  // the captured graph holds the old launch shapes
+    if (known) {
+        for (int k = 0; k < 6; k++) ctx->tune[p][k / 3][k % 3] = best[k];
+    } else {
+        default_shapes(ctx, p);
+        if (!lat_split(ctx->lc(), ctx->g, ctx->mixed())) {
+            cudaEvent_t e0 = nullptr, e1 = nullptr;
+            MG_CK(cudaEventCreate(&e0));
+            if (cudaEventCreate(&e1) != cudaSuccess) { cudaEventDestroy(e0); ctx->err = "cudaEventCreate"; return MG_ERR_CUDA; }
+            const mg_status st = time_shapes(ctx, reps < 1 ? 3 : reps, e0, e1);
+            cudaEventDestroy(e0);
+            cudaEventDestroy(e1);
+            if (st != MG_OK) {
+                default_shapes(ctx, p);
+                return st;
             }
         }
-        for (int c = 0; c < 3; c++) ctx->tune[p][kern][c] = best[3 * kern + c];
-    }
-    cudaEventDestroy(e0);
-    cudaEventDestroy(e1);
-    mg_status st = check_launch(ctx);
-    if (st != MG_OK) return st;
-    {
+        for (int k = 0; k < 6; k++) best[k] = ctx->tune[p][k / 3][k % 3];
         std::lock_guard<std::mutex> lock(g_tune_mutex);
         g_tune_cache.push_back({key, best});
     }
     if (out) for (int k = 0; k < 6; k++) out[k] = best[k];
-    ctx->graph_stale = true;
-    ctx->gen++;  // the captured graph holds the old launch shapes
     return MG_OK;
 }
 

@@ -309,6 +309,10 @@ void launch_ghost_df(const LaunchCtx &lc, const Geom &g, Slots s, Inter in, PotT
 // leaves to launch_inter_rho_owners.
 bool launch_lat_rho(const LaunchCtx &lc, const Geom &g, Slots s, Inter in, PotTables t, bool mixed, bool hook,
                     bool lists = false);
+// Whether the step's passes over the whole box use the group lists under these launch shapes, and whether they are split
+// passes, which take their own shapes.
+bool lat_lists(const LaunchCtx &lc, const Geom &g, bool mixed);
+bool lat_split(const LaunchCtx &lc, const Geom &g, bool mixed);
 // the density pass over the sites [u0, u1) of both parities (as launch_lat_force_sites)
 void launch_lat_rho_sites(const LaunchCtx &lc, const Geom &g, Slots s, Inter in, PotTables t, bool mixed, int u0, int u1,
                           bool lists = false);

@@ -1650,6 +1650,10 @@ void launch_skin_dirty(const LaunchCtx &lc, Slots s) { cudaMemsetAsync(&s.skin->
 
 // whether a pass can use the group lists: the mixed form, and the FP64 form's fixed-point passes
 static bool has_lists(const LaunchCtx &lc, bool mixed) { return mixed || lc.fp; }
+bool lat_lists(const LaunchCtx &lc, const Geom &g, bool mixed) { return has_lists(lc, mixed) && lists_ok(lc, g); }
+bool lat_split(const LaunchCtx &lc, const Geom &g, bool mixed) {
+    return split_warps(lc, mixed, lat_lists(lc, g, mixed), split_groups(0, g.n_local_half)) != 0;
+}
 // A pass with the group lists is followed by the skin's advance, which the caller launches (true: it is due). A
 // pass without them leaves the lists behind the positions, so the next pass with them rebuilds them.
 bool launch_lat_rho(const LaunchCtx &lc, const Geom &g, Slots s, Inter in, PotTables t, bool mixed, bool hook, bool lists) {
