@@ -1826,6 +1826,8 @@ mg_status time_shapes(mg_context *ctx, int reps, cudaEvent_t e0, cudaEvent_t e1)
         }
         for (int c = 0; c < 3; c++) tune[c] = best[c];
     }
+    // the lattice passes alone leave out what inter atoms add to densities and forces
+    seq_compute_eam(ctx, false, false, 0, nullptr);
     return check_launch(ctx);
 }
 }  // namespace
