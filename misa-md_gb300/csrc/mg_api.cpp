@@ -46,7 +46,8 @@ struct mg_context {
     PotTables pt{};
     FixParams fp{};                 // fixed-point pair arithmetic of the FP64 form (on when the tables suit it)
     void *fix_mem = nullptr;        // its tables
-    bool fix_built = false;         // tables made for the potential in use (by the first FP64 state)
+    void *fix_slots = nullptr;      // s.fix, s.fixn and s.dfq
+    bool fix_built = false;         // tables made, or found not to fit, for the potential in use (by the first FP64 state)
     bool pot_ready = false;
     HostPotential hp;               // the spline coefficients in use
     int types_ok_mask = 0;          // bit t set: the potential has the element of atom type t
@@ -124,6 +125,36 @@ struct mg_context {
     bool mixed() const { return precision == MG_PREC_MIXED; }
 };
 
+namespace {
+// The FP64 form's fixed-point arrays and tables, which its passes can do without; false when there are none. Launches are
+// taken from the context afterwards.
+bool drop_optional(mg_context *ctx) {
+    if (!ctx->fix_slots && !ctx->fix_mem) return false;
+    if (ctx->stream) cudaStreamSynchronize(ctx->stream);
+    cudaFree(ctx->fix_slots);
+    cudaFree(ctx->fix_mem);
+    ctx->fix_slots = ctx->fix_mem = nullptr;
+    ctx->s.fix = ctx->s.fixn = ctx->fix_main = ctx->fix_alt = nullptr;
+    ctx->s.dfq = nullptr;
+    ctx->fp = FixParams{};
+    ctx->graph_stale = true;
+    ctx->gen++;
+    return true;
+}
+}  // namespace
+
+namespace mg {
+// Memory that the caller's work cannot do without: where the device has none left, the arrays above are given back for it.
+cudaError_t needed_malloc(mg_context *ctx, void **p, size_t bytes) {
+    cudaError_t e = cudaMalloc(p, bytes);
+    if (e == cudaErrorMemoryAllocation && drop_optional(ctx)) {
+        cudaGetLastError();
+        e = cudaMalloc(p, bytes);
+    }
+    return e;
+}
+}  // namespace mg
+
 #define MG_CK(call)                                                                             \
     do {                                                                                        \
         cudaError_t e_ = (call);                                                                \
@@ -138,7 +169,7 @@ namespace {
 template <class T>
 cudaError_t dalloc(mg_context *ctx, T **p, size_t n) {
     void *q = nullptr;
-    cudaError_t e = cudaMalloc(&q, n * sizeof(T) + 16);
+    cudaError_t e = needed_malloc(ctx, &q, n * sizeof(T) + 16);
     if (e == cudaSuccess) {
         ctx->dev_allocs.push_back(q);
         *p = static_cast<T *>(q);
@@ -285,8 +316,9 @@ mg_status require_ready(mg_context *ctx) {
 }
 
 // The FP64 form's fixed-point tables and arrays (72 bytes per slot), made for the first FP64 state that comes
-// in under a potential. Where the tables do not suit the potential, or the arrays do not fit the device,
-// the passes run in FP64.
+// in under a potential. Where the tables do not suit the potential, or the arrays do not fit the device beside what the
+// calls need, the passes run in FP64.
+constexpr size_t kFixBytes = 2 * sizeof(FixRec) + sizeof(i64);
 void ensure_fix(mg_context *ctx) {
     if (ctx->mixed() || !ctx->pot_ready || ctx->fix_built) return;
     ctx->fix_built = true;
@@ -299,12 +331,10 @@ void ensure_fix(mg_context *ctx) {
     Slots &s = ctx->s;
     const size_t ns = static_cast<size_t>(ctx->g.n_slots);
     const size_t n[2] = {ft.rho.size(), ft.zg.size()};
-    void *tab = nullptr, *rec = s.fix, *next = s.fixn, *df = s.dfq;
-    cudaError_t e = cudaMalloc(&tab, (n[0] + n[1]) * sizeof(FixPoly));
-    if (e == cudaSuccess && !rec) e = cudaMalloc(&rec, ns * sizeof(FixRec));
-    if (e == cudaSuccess && !next) e = cudaMalloc(&next, ns * sizeof(FixRec));
-    if (e == cudaSuccess && !df) e = cudaMalloc(&df, ns * sizeof(i64));
-    FixPoly *d = static_cast<FixPoly *>(tab);
+    const bool kept = ctx->fix_slots;  // a former potential's
+    cudaError_t e = cudaMalloc(&ctx->fix_mem, (n[0] + n[1]) * sizeof(FixPoly));
+    if (e == cudaSuccess && !kept) e = cudaMalloc(&ctx->fix_slots, ns * kFixBytes);
+    FixPoly *d = static_cast<FixPoly *>(ctx->fix_mem);
     const FixPoly *src[2] = {ft.rho.data(), ft.zg.data()};
     const FixPoly *at[2];
     for (int k = 0; k < 2; k++) {
@@ -312,22 +342,16 @@ void ensure_fix(mg_context *ctx) {
         if (e == cudaSuccess) e = cudaMemcpy(d, src[k], n[k] * sizeof(FixPoly), cudaMemcpyHostToDevice);
         if (d) d += n[k];
     }
-    if (e == cudaSuccess && !s.dfq) e = cudaMemsetAsync(df, 0, ns * sizeof(i64), ctx->stream);
+    FixRec *rec = static_cast<FixRec *>(ctx->fix_slots);
+    if (e == cudaSuccess && !kept) e = cudaMemsetAsync(rec + 2 * ns, 0, ns * sizeof(i64), ctx->stream);
     if (e != cudaSuccess) {
         cudaGetLastError();
-        cudaFree(tab);
-        if (rec != s.fix) cudaFree(rec);
-        if (next != s.fixn) cudaFree(next);
-        if (df != s.dfq) cudaFree(df);
+        drop_optional(ctx);
         return;
     }
-    if (!s.fix) ctx->dev_allocs.push_back(rec);
-    if (!s.fixn) ctx->dev_allocs.push_back(next);
-    if (!s.dfq) ctx->dev_allocs.push_back(df);
-    s.fix = ctx->fix_main = static_cast<FixRec *>(rec);
-    s.fixn = ctx->fix_alt = static_cast<FixRec *>(next);
-    s.dfq = static_cast<i64 *>(df);
-    ctx->fix_mem = tab;
+    s.fix = ctx->fix_main = rec;
+    s.fixn = ctx->fix_alt = rec + ns;
+    s.dfq = reinterpret_cast<i64 *>(rec + 2 * ns);
     fp.rho = at[0];
     fp.zg = at[1];
     ctx->fp = fp;
@@ -338,9 +362,8 @@ void ensure_fix(mg_context *ctx) {
 }
 
 mg_status ensure_aos(mg_context *ctx) {
+    if (!ctx->d_aos) MG_CK(dalloc(ctx, &ctx->d_aos, static_cast<size_t>(ctx->g.n_slots)));
     ensure_fix(ctx);
-    if (ctx->d_aos) return MG_OK;
-    MG_CK(dalloc(ctx, &ctx->d_aos, static_cast<size_t>(ctx->g.n_slots)));
     return MG_OK;
 }
 
@@ -436,7 +459,7 @@ mg_status install_potential(mg_context *ctx, const HostPotential &hp) {
         }
     }
     const size_t bytes = n_rec * (2 * sizeof(Knot64) + 2 * sizeof(float4)) + zr.size() * sizeof(float);
-    MG_CK(cudaMalloc(&ctx->pot_mem, bytes));
+    MG_CK(needed_malloc(ctx, &ctx->pot_mem, bytes));
     Knot64 *d_vd = static_cast<Knot64 *>(ctx->pot_mem);
     Knot64 *d_dd = d_vd + n_rec;
     float4 *d_vf = reinterpret_cast<float4 *>(d_dd + n_rec);
@@ -730,6 +753,7 @@ mg_status mg_destroy(mg_context *ctx) {
     for (void *p : ctx->dev_allocs) cudaFree(p);
     if (ctx->pot_mem) cudaFree(ctx->pot_mem);
     if (ctx->fix_mem) cudaFree(ctx->fix_mem);
+    if (ctx->fix_slots) cudaFree(ctx->fix_slots);
     if (ctx->stream) cudaStreamDestroy(ctx->stream);
     delete ctx;
     return MG_OK;

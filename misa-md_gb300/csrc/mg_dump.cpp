@@ -183,12 +183,14 @@ mg_status mg_dump_open(mg_context *ctx, const char *path, int32_t by_frame, int6
     d->max_records = src.max_records;
     const size_t frame_bytes = static_cast<size_t>(src.max_records) * sizeof(mg_dump_record);
     const size_t pin_bytes = static_cast<size_t>(std::min<int64_t>(d->chunk, static_cast<int64_t>(frame_bytes)));
+    auto dmalloc = [ctx](auto **p, size_t bytes) {
+        return needed_malloc(ctx, reinterpret_cast<void **>(p), bytes) == cudaSuccess;
+    };
     bool ok = cudaStreamCreateWithFlags(&d->io, cudaStreamNonBlocking) == cudaSuccess &&
-              cudaMalloc(&d->d_count, 2 * sizeof(unsigned long long)) == cudaSuccess &&
-              cudaMalloc(&d->scratch, static_cast<size_t>(src.scratch_ints) * sizeof(int)) == cudaSuccess &&
+              dmalloc(&d->d_count, 2 * sizeof(unsigned long long)) && dmalloc(&d->scratch, static_cast<size_t>(src.scratch_ints) * sizeof(int)) &&
               cudaHostAlloc(&d->h_count, sizeof(unsigned long long), cudaHostAllocDefault) == cudaSuccess;
     for (int k = 0; k < 2 && ok; k++) {
-        ok = cudaMalloc(&d->stage[k], frame_bytes) == cudaSuccess &&
+        ok = dmalloc(&d->stage[k], frame_bytes) &&
              cudaEventCreateWithFlags(&d->packed[k], cudaEventDisableTiming) == cudaSuccess &&
              cudaEventCreateWithFlags(&d->copied[k], cudaEventDisableTiming) == cudaSuccess &&
              cudaHostAlloc(&d->pin[k], pin_bytes, cudaHostAllocDefault) == cudaSuccess;

@@ -389,6 +389,7 @@ struct DumpSource {
     int scratch_ints;
 };
 DumpSource dump_source(const mg_context *ctx);
+cudaError_t needed_malloc(mg_context *ctx, void **p, size_t bytes);  // cudaMalloc, in place of what the context can do without
 mg_status dump_pack(mg_context *ctx, mg_dump_record *out, unsigned long long *count, int *scratch, uint64_t step);
 void dump_detach(mg_context *ctx, const mg_dump *d);  // mg_dump_close: the stage machine forgets d
 void dump_note_error(mg_context *ctx, const std::string &why);  // mg_last_error(ctx) reports it

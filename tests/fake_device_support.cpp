@@ -1,0 +1,50 @@
+// A device for CPU tests of the host code: memory of a fixed size on the heap, copies at once, kernels that do nothing
+// (the launch functions and the rest of the runtime are stubs that return 0).
+#include <cuda_runtime.h>
+
+#include <cstdlib>
+#include <cstring>
+#include <map>
+
+static size_t g_limit = ~size_t(0), g_used = 0;
+static std::map<void *, size_t> g_blocks;
+
+extern "C" {
+void fake_limit(size_t bytes) { g_limit = bytes; }
+size_t fake_used() { return g_used; }
+
+cudaError_t cudaMalloc(void **p, size_t n) {
+    if (n > g_limit || g_used > g_limit - n) return cudaErrorMemoryAllocation;
+    *p = std::calloc(n, 1);
+    if (!*p) return cudaErrorMemoryAllocation;
+    g_blocks[*p] = n;
+    g_used += n;
+    return cudaSuccess;
+}
+cudaError_t cudaFree(void *p) {
+    auto it = g_blocks.find(p);
+    if (it != g_blocks.end()) {
+        g_used -= it->second;
+        g_blocks.erase(it);
+        std::free(p);
+    }
+    return cudaSuccess;
+}
+cudaError_t cudaMemcpy(void *d, const void *s, size_t n, cudaMemcpyKind) {
+    std::memcpy(d, s, n);
+    return cudaSuccess;
+}
+cudaError_t cudaMemcpyAsync(void *d, const void *s, size_t n, cudaMemcpyKind, cudaStream_t) {
+    std::memcpy(d, s, n);
+    return cudaSuccess;
+}
+cudaError_t cudaHostAlloc(void **p, size_t n, unsigned) {
+    *p = std::calloc(n, 1);
+    return cudaSuccess;
+}
+cudaError_t cudaFreeHost(void *p) {
+    std::free(p);
+    return cudaSuccess;
+}
+const char *cudaGetErrorString(cudaError_t) { return "fake device"; }
+}
