@@ -410,6 +410,10 @@ mg_status upload_tables(mg_context *ctx) {
 mg_status install_potential(mg_context *ctx, const HostPotential &hp) {
     // Tables by atom type (3 x nr / nrho knots) and by type pair (9 x nr, ti * 3 + tj); types whose
     // element the file lacks point at element 0 and are rejected at upload (types_ok_mask).
+    if ((hp.nr - 1) * hp.dr + 1e-12 < ctx->g.rc) {  // the hit test uses rc = a0 * cutoff_radius_factor
+        ctx->err = "potential r-table shorter than the cutoff radius";
+        return MG_ERR_POTENTIAL;
+    }
     int ele_of_type[3];
     ctx->types_ok_mask = 0;
     for (int t = 0; t < 3; t++) {
@@ -418,10 +422,6 @@ mg_status install_potential(mg_context *ctx, const HostPotential &hp) {
         ele_of_type[t] = e >= 0 ? e : 0;
     }
     ctx->one_type = ele_of_type[1] == ele_of_type[0] && ele_of_type[2] == ele_of_type[0];
-    if ((hp.nr - 1) * hp.dr + 1e-12 < ctx->g.rc) {  // the hit test uses rc = a0 * cutoff_radius_factor
-        ctx->err = "potential r-table shorter than the cutoff radius";
-        return MG_ERR_POTENTIAL;
-    }
     const size_t nr = hp.nr, nrho = hp.nrho;
     const size_t n_rec = 3 * nr + 3 * nrho + 9 * nr;
     std::vector<Knot64> vd(n_rec), dd(n_rec);
