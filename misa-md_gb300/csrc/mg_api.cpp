@@ -7,6 +7,7 @@
 #include <cstddef>
 #include <cstdio>
 #include <cstring>
+#include <exception>
 #include <string>
 #include <array>
 #include <mutex>
@@ -327,7 +328,11 @@ void ensure_fix(mg_context *ctx) {
     for (int t = 0; t < 3; t++) ele_of_type[t] = std::max(0, hp.ele(type_key(t)));
     FixParams fp;
     FixTables ft;
-    if (!build_fixed(hp, ele_of_type, ctx->g.a0, ctx->g.rc / ctx->g.a0, std::max(ctx->n_pruned, ctx->n_full - ctx->n_pruned), fp, ft, false)) return;
+    try {  // no host memory for the tables: as where they do not suit the potential
+        if (!build_fixed(hp, ele_of_type, ctx->g.a0, ctx->g.rc / ctx->g.a0, std::max(ctx->n_pruned, ctx->n_full - ctx->n_pruned), fp, ft, false)) return;
+    } catch (const std::exception &) {
+        return;
+    }
     Slots &s = ctx->s;
     const size_t ns = static_cast<size_t>(ctx->g.n_slots);
     const size_t n[2] = {ft.rho.size(), ft.zg.size()};

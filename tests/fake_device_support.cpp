@@ -5,6 +5,18 @@
 #include <cstdlib>
 #include <cstring>
 #include <map>
+#include <new>
+
+// host memory: requests above a size fail
+static size_t g_largest = ~size_t(0);
+extern "C" void fake_largest(size_t bytes) { g_largest = bytes; }
+void *operator new(size_t n) {
+    void *p = n <= g_largest ? std::malloc(n ? n : 1) : nullptr;
+    if (!p) throw std::bad_alloc();
+    return p;
+}
+void operator delete(void *p) noexcept { std::free(p); }
+void operator delete(void *p, size_t) noexcept { std::free(p); }
 
 static size_t g_limit = ~size_t(0), g_used = 0;
 static std::map<void *, size_t> g_blocks;

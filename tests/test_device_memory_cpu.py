@@ -37,6 +37,7 @@ def lib(tmp_path_factory, pkg):
     lib = ctypes.CDLL(so)
     lib.fake_used.restype = ctypes.c_size_t
     lib.fake_limit.argtypes = [ctypes.c_size_t]
+    lib.fake_largest.argtypes = [ctypes.c_size_t]
     lib.mg_last_error.restype = ctypes.c_char_p
     yield lib
     lib.fake_limit(2**63)
@@ -103,4 +104,15 @@ def test_dump_takes_the_fixed_point_arrays_room(lib, wl, potentials, tmp_path):
     d = ctypes.c_void_p()
     assert c.call("mg_dump_open", os.fsencode(str(tmp_path / "d.bin")), 0, ctypes.c_int64(0), ctypes.byref(d)) == 0
     assert lib.mg_dump_close(d) == 0
+    c.close()
+
+
+@pytest.mark.parametrize("largest", [1000, 50000, 300000])  # bytes; the tables and what they are made from take more
+def test_no_host_memory_for_the_tables(lib, wl, potentials, largest):
+    c = Ctx(lib, wl, potentials["fe"], lambda n: n * (RECORD + FIX) + SLACK)
+    lib.fake_largest(largest)
+    st = c.upload()
+    lib.fake_largest(2**63)
+    assert st == 0, c.call("mg_last_error")
+    assert c.taken() < RECORD * c.n + SLACK
     c.close()
