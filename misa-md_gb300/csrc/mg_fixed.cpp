@@ -11,6 +11,7 @@
 // do not meet the error bound that every record is checked against, and the FP64 loops stay in use for them.
 
 #include <algorithm>
+#include <array>
 #include <cmath>
 #include <future>
 
@@ -144,10 +145,10 @@ int exponent_for(double bound, int bits) {
 
 // the largest values of the functions from a knot on to the cutoff, over elements and pairs
 struct Largest {
-    double rho, g, h, phi, rg, rh, f_typ;
+    double rho, g, h, phi, rg, rh;
 };
 // at[m]: from knot m on (m_from <= m <= nr - 2); one pass serves every inner end that is tried
-std::vector<Largest> largest_from(const HostPotential &hp, int m_from, double nn) {
+std::vector<Largest> largest_from(const HostPotential &hp, int m_from) {
     std::vector<Largest> at(hp.nr - 1, Largest{});
     Largest v{};
     for (int m = hp.nr - 2; m >= m_from; m--) {
@@ -163,7 +164,6 @@ std::vector<Largest> largest_from(const HostPotential &hp, int m_from, double nn
                 v.phi = std::max(v.phi, std::fabs(phi));
                 v.h = std::max(v.h, h);
                 v.rh = std::max(v.rh, r * h);
-                if (r >= 0.97 * nn) v.f_typ = std::max(v.f_typ, r * h);
             }
         }
         at[m] = v;
@@ -174,9 +174,89 @@ int first_knot(double r_lo, double dr) { return std::max(1, (int) (r_lo / dr) - 
 
 }  // namespace
 
-// build_fixed for one inner end r_lo of the tables' range; tab null: the scales only
-static bool build_from(const HostPotential &hp, const int ele_of_type[3], double a0, double rcf, int n_part, double r_lo,
-                       const std::vector<Largest> &largest, FixParams &fp, FixTables *tab, bool want_phi) {
+// A perfect crystal's neighbours of a site in the order the loops visit them (in half lattice constants, BCC: all even or
+// all odd), and the largest |F'(rho)| of an element on a site whose neighbours are of one element.
+struct Crystal {
+    std::vector<std::array<int, 3>> near;
+    double df_most = 0.0;
+};
+static double distance_of(const std::array<int, 3> &n, double a0) {
+    return 0.5 * a0 * std::sqrt((double) (n[0] * n[0] + n[1] * n[1] + n[2] * n[2]));
+}
+static double crystal_rho(const HostPotential &hp, const Crystal &c, double a0, int b) {
+    const HostSpline &s = hp.rho[b];
+    double rho = 0.0;
+    for (const auto &n : c.near) {
+        const double x = distance_of(n, a0) * s.inv_delta;
+        const int m = std::min((int) x, hp.nr - 2);
+        rho += cubic_at(dd(x - m), s.c0[m], s.c1[m], s.c2[m], s.c3[m]).h;
+    }
+    return rho;
+}
+static double embedding_df(const HostPotential &hp, int a, double rho) {
+    const HostSpline &F = hp.F[a];
+    const int m = std::max(0, std::min((int) (rho * F.inv_delta), hp.nrho - 2));
+    return cubic_at(dd(std::min(rho * F.inv_delta - m, 1.0)), F.d0[m], F.d1[m], F.d2[m], 0.0).h;
+}
+static Crystal crystal_of(const HostPotential &hp, double a0, double rc) {
+    Crystal c;
+    const int n = 2 * ((int) (rc / a0) + 1);
+    for (int k = -n; k <= n; k++)
+        for (int j = -n; j <= n; j++)
+            for (int i = -n; i <= n; i++)
+                if (!(((i ^ j) | (j ^ k)) & 1) && (i || j || k) && distance_of({i, j, k}, a0) < rc) c.near.push_back({i, j, k});
+    for (int b = 0; b < hp.n_ele; b++) {
+        const double rho = crystal_rho(hp, c, a0, b);
+        if (!(rho <= (hp.nrho - 1) * hp.drho)) continue;  // past the embedding tables: no crystal to judge by
+        for (int a = 0; a < hp.n_ele; a++) {
+            const double df = std::fabs(embedding_df(hp, a, rho));
+            c.df_most = std::max(c.df_most, df);
+        }
+    }
+    return c;
+}
+// The FP64 loops' rms error in a component of the force on an atom: what each pair's roundings make of its force, near
+// its crystal distance, against double-double arithmetic, and the roundings of the sum. The least over crystals of one
+// element.
+static double fp64_error(const HostPotential &hp, const Crystal &c, double a0, double rc) {
+    const double dir[3] = {0.48, 0.6, 0.64}, inv = hp.rho[0].inv_delta;
+    double least = HUGE_VAL;
+    for (int a = 0; a < hp.n_ele; a++) {
+        const HostSpline &s = hp.rho[a], &z = hp.z2[HostPotential::pair_index(a, a)];
+        const double df2 = 2.0 * embedding_df(hp, a, crystal_rho(hp, c, a0, a));
+        double sum = 0.0, part[3] = {0.0, 0.0, 0.0};
+        int at = 0;
+        for (const auto &n : c.near) {
+            // distances within 2% of the crystal's, another for each neighbour
+            const double r0 = distance_of(n, a0), want = r0 * (1.0 + 0.04 * (std::fmod(0.618034 * ++at, 1.0) - 0.5));
+            const double x = want * dir[0], y = want * dir[1], w = want * dir[2];
+            const double r2 = std::fma(w, w, std::fma(y, y, x * x));
+            if (r2 >= rc * rc) continue;
+            const double ri = 1.0 / std::sqrt(r2), r = r2 * ri;
+            const int m = std::min((int) (r * inv), hp.nr - 2);
+            const double p = r * inv - m;
+            const double rhop = std::fma(std::fma(s.d2[m], p, s.d1[m]), p, s.d0[m]);
+            const double phi = std::fma(std::fma(std::fma(z.c3[m], p, z.c2[m]), p, z.c1[m]), p, z.c0[m]) * ri;
+            const double phip = std::fma(std::fma(z.d2[m], p, z.d1[m]), p, z.d0[m]) * ri - phi * ri;
+            const double f = (df2 * rhop + phip) * ri;
+            const Place q = place(root(dd(x) * dd(x) + dd(y) * dd(y) + dd(w) * dd(w)), inv, m);
+            const double err = (dd(f) - (dd(df2) * value_at(s, m, FN_G, q) + value_at(z, m, FN_H, q))).h * r;
+            sum += err * err;
+            for (int d = 0; d < 3; d++) {
+                part[d] += 0.5 * a0 * n[d] * f;
+                const double unit = part[d] != 0.0 ? std::ldexp(1.0, std::ilogb(part[d]) - 52) : 0.0;
+                sum += unit * unit / 12.0;
+            }
+        }
+        least = std::min(least, std::sqrt(sum / 3.0));
+    }
+    return least;
+}
+
+// build_fixed for one inner end r_lo of the tables' range and F'(rho) in units of 2^-kd; exact: the FP64 loops' error;
+// tab null: the scales only
+static bool build_from(const HostPotential &hp, const int ele_of_type[3], double a0, double rcf, int n_part, double r_lo, int kd,
+                       double exact, const std::vector<Largest> &largest, FixParams &fp, FixTables *tab, bool want_phi) {
     fp = FixParams{};
     const double rc = a0 * rcf, dr = hp.dr;
     const int nr = hp.nr;
@@ -212,13 +292,12 @@ static bool build_from(const HostPotential &hp, const int ele_of_type[3], double
     const double inv_dr = hp.rho[0].inv_delta;
     const Largest &top = largest[m_lo];
     const double rho_max = top.rho, g_max = top.g, h_max = top.h, phi_max = top.phi, rg_max = top.rg, rh_max = top.rh;
-    const double f_typ = top.f_typ;
-    if (!(rho_max > 0) || !(g_max > 0) || !(h_max > 0) || !(f_typ > 0) || !std::isfinite(rho_max + g_max + h_max + phi_max))
+    if (!(rho_max > 0) || !(g_max > 0) || !(h_max > 0) || !std::isfinite(rho_max + g_max + h_max + phi_max))
         return false;
     const double room = 1.01;  // values between the knots
-    // F'(rho) below 1 (alloy tables in eV; others scale with the density's unit): |F' g| at the unit bound
-    // is the pair force of a bond at full embedding, so the product's unit follows from both
-    fp.kd = 60;
+    // F'(rho) below 2^(60 - kd): |F' g| at the bound is the pair force of a bond at full embedding, so the
+    // product's unit follows from both
+    fp.kd = kd;
     const int kg = exponent_for(g_max * room, 62);
     const int kf = fp.kd + kg - 64;                 // pair factor (F'_i + F'_j) g + h
     const int kF = fp.kx + kf - 64;                 // force sums
@@ -227,7 +306,8 @@ static bool build_from(const HostPotential &hp, const int ele_of_type[3], double
     const int kphi = exponent_for(n_part * phi_max * room, 62);
     if ((df2 * g_max + h_max) * room >= std::ldexp(1.0, 62 - kf)) return false;
     if (n_part * (df2 * rg_max + rh_max) * room >= std::ldexp(1.0, 63 - kF)) return false;
-    if (std::ldexp(1.0, -kF) > std::ldexp(f_typ, -48)) return false;  // the force sums' unit against a bond's force
+    // the sums are to be no less exact than the FP64 loops'; their rms error in thermal crystals is 2.3 to 2.5 units
+    if (2.5 * std::ldexp(1.0, -kF) > exact) return false;
     fp.rho_unit = std::ldexp(1.0, -krho);
     fp.e_unit = std::ldexp(1.0, -kphi);
     fp.f_unit = std::ldexp(1.0, -kF);
@@ -382,21 +462,30 @@ static bool build_from(const HostPotential &hp, const int ele_of_type[3], double
 // finest that any end up to 0.86 of the nearest-neighbour distance allows, as close as the tables' error
 // bound admits. The closer it is, the fewer pairs of a hot crystal take the FP64 terms; at 320 K about one
 // pair in 1e5 is closer than 0.82.
+// F' stays below 1 in most tables (in eV; others scale with the density's unit). Where the bound of 1 leaves the force sums' unit too coarse, a lower one serves if it is two and a
+// half times a crystal's F' or more (next to a vacancy F' grows by a tenth).
 bool build_fixed(const HostPotential &hp, const int ele_of_type[3], double a0, double rcf, int n_part, FixParams &fp,
                  FixTables &tab, bool want_phi) {
     fp = FixParams{};
     if (hp.nr < 64 || hp.nr > 20000) return false;
     const double nn = 0.5 * std::sqrt(3.0) * a0, percent = 0.01 * nn;
     const int m_from = std::min(first_knot(70 * percent, hp.dr), hp.nr - 1);
-    const std::vector<Largest> largest = largest_from(hp, m_from, nn);
+    const std::vector<Largest> largest = largest_from(hp, m_from);
+    const Crystal crystal = crystal_of(hp, a0, a0 * rcf);
+    if (!(crystal.df_most > 0.0)) return false;
+    const double exact = fp64_error(hp, crystal, a0, a0 * rcf);
+    int kd = 60;
     double finest = 0.0;
-    for (int f = 70; f <= 86; f += 2)
-        if (build_from(hp, ele_of_type, a0, rcf, n_part, f * percent, largest, fp, nullptr, want_phi) &&
-            (finest == 0.0 || fp.f_unit < finest))
-            finest = fp.f_unit;
+    for (int k = 60; k <= 80 && finest == 0.0 && (k == 60 || std::ldexp(2.5 * crystal.df_most, k - 60) <= 1.0); k++) {
+        kd = k;
+        for (int f = 70; f <= 86; f += 2)
+            if (build_from(hp, ele_of_type, a0, rcf, n_part, f * percent, kd, exact, largest, fp, nullptr, want_phi) &&
+                (finest == 0.0 || fp.f_unit < finest))
+                finest = fp.f_unit;
+    }
     for (int f = 70; f <= 86 && finest > 0.0; f += 2)
-        if (build_from(hp, ele_of_type, a0, rcf, n_part, f * percent, largest, fp, nullptr, want_phi) && fp.f_unit == finest &&
-            build_from(hp, ele_of_type, a0, rcf, n_part, f * percent, largest, fp, &tab, want_phi))
+        if (build_from(hp, ele_of_type, a0, rcf, n_part, f * percent, kd, exact, largest, fp, nullptr, want_phi) && fp.f_unit == finest &&
+            build_from(hp, ele_of_type, a0, rcf, n_part, f * percent, kd, exact, largest, fp, &tab, want_phi))
             return true;
     fp = FixParams{};
     return false;
