@@ -175,10 +175,11 @@ int first_knot(double r_lo, double dr) { return std::max(1, (int) (r_lo / dr) - 
 }  // namespace
 
 // A perfect crystal's neighbours of a site in the order the loops visit them (in half lattice constants, BCC: all even or
-// all odd), and the largest |F'(rho)| of an element on a site whose neighbours are of one element.
+// all odd), and |F'(rho)| of an element on a site whose neighbours are of one element: the least and the largest over the
+// elements.
 struct Crystal {
     std::vector<std::array<int, 3>> near;
-    double df_most = 0.0;
+    double df_least = HUGE_VAL, df_most = 0.0;
 };
 static double distance_of(const std::array<int, 3> &n, double a0) {
     return 0.5 * a0 * std::sqrt((double) (n[0] * n[0] + n[1] * n[1] + n[2] * n[2]));
@@ -210,6 +211,7 @@ static Crystal crystal_of(const HostPotential &hp, double a0, double rc) {
         if (!(rho <= (hp.nrho - 1) * hp.drho)) continue;  // past the embedding tables: no crystal to judge by
         for (int a = 0; a < hp.n_ele; a++) {
             const double df = std::fabs(embedding_df(hp, a, rho));
+            c.df_least = std::min(c.df_least, df);
             c.df_most = std::max(c.df_most, df);
         }
     }
@@ -462,7 +464,9 @@ static bool build_from(const HostPotential &hp, const int ele_of_type[3], double
 // finest that any end up to 0.86 of the nearest-neighbour distance allows, as close as the tables' error
 // bound admits. The closer it is, the fewer pairs of a hot crystal take the FP64 terms; at 320 K about one
 // pair in 1e5 is closer than 0.82.
-// F' stays below 1 in most tables (in eV; others scale with the density's unit). Where the bound of 1 leaves the force sums' unit too coarse, a lower one serves if it is two and a
+// F' stays below 1 in most tables (in eV; others scale with the density's unit). An atom above the bound takes the FP64
+// loop after its fixed-point one, and so does every neighbour, so where every perfect crystal is at it already, the
+// tables are refused. Where the bound of 1 leaves the force sums' unit too coarse, a lower one serves if it is two and a
 // half times a crystal's F' or more (next to a vacancy F' grows by a tenth).
 bool build_fixed(const HostPotential &hp, const int ele_of_type[3], double a0, double rcf, int n_part, FixParams &fp,
                  FixTables &tab, bool want_phi) {
@@ -472,7 +476,7 @@ bool build_fixed(const HostPotential &hp, const int ele_of_type[3], double a0, d
     const int m_from = std::min(first_knot(70 * percent, hp.dr), hp.nr - 1);
     const std::vector<Largest> largest = largest_from(hp, m_from);
     const Crystal crystal = crystal_of(hp, a0, a0 * rcf);
-    if (!(crystal.df_most > 0.0)) return false;
+    if (!(1.05 * crystal.df_least < 1.0)) return false;
     const double exact = fp64_error(hp, crystal, a0, a0 * rcf);
     int kd = 60;
     double finest = 0.0;

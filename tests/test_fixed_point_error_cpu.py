@@ -1,5 +1,6 @@
 """Whatever potential the fixed-point tables are made for, the forces they give are no further from the exact ones than the
-FP64 loops': on the CPU, over density units, embedding and pair strengths, knots, and crystals of each element."""
+FP64 loops', and the atoms of a crystal do not fall back to those: on the CPU, over density units, embedding and
+pair strengths, knots, and crystals of each element."""
 import ctypes
 import os
 import subprocess
@@ -38,7 +39,8 @@ def _write(wl, path, n_ele, nr, density, embed, pair):
     (1, 5000, 1.0, 1.0, 1.0, True), (3, 5000, 1.0, 1.0, 1.0, True), (1, 4500, 1.0, 1.0, 1.0, True), (1, 20000, 1.0, 1.0, 1.0, True),
     (1, 5000, 0.2, 1.0, 1.0, True), (3, 5000, 0.3, 1.0, 1.0, True), (1, 5000, 4.0, 1.0, 1.0, None), (1, 5000, 10.0, 1.0, 1.0, None),
     (3, 5000, 8.0, 1.0, 1.0, None), (1, 5000, 1.0, 0.1, 1.0, None), (1, 5000, 1.0, 6.0, 1.0, None), (1, 5000, 1.0, 1.0, 0.1, None),
-    (1, 5000, 1.0, 1.0, 0.3, None), (1, 5000, 1.0, 1.0, 3.0, None)])
+    (1, 5000, 1.0, 1.0, 0.3, None), (1, 5000, 1.0, 1.0, 3.0, None),
+    (1, 5000, 1.0, 10.0, 1.0, False)])  # F' of 1.2 at the crystal's density
 def test_forces_are_no_less_exact_than_the_fp64_loops(lib, wl, tmp_path, n_ele, nr, density, embed, pair, fixed):
     path = _write(wl, tmp_path / "p.setfl", n_ele, nr, density, embed, pair)
     for spread in (0.02, 0.08):
