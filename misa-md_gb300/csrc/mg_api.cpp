@@ -79,18 +79,37 @@ struct mg_context {
     int64_t *d_ws_coords = nullptr, *d_ws_index = nullptr;
     uint32_t *d_ws_flags = nullptr;
     int64_t ws_cap = 0;
-    cudaGraphExec_t graph_exec = nullptr;
-    // multi-step graph: kPlainBodies loop bodies, or (fused) fuse_steps whose force passes (all but the last) take the
-    // next firststep (mixed form, fixed dt); < 2: off
-    int fuse_steps = 16;
-    cudaGraphExec_t graph_multi = nullptr;
+    // captured steps, of each timestep rule (fixed, variable): a step's kernels differ by the rule, and a program may
+    // switch between them
+    struct Graphs {
+        cudaGraphExec_t one = nullptr;  // one loop body
+        // kPlainBodies loop bodies, or (fused) fuse_steps whose force passes (all but the last) take the next firststep
+        // (mixed form, fixed dt)
+        cudaGraphExec_t multi = nullptr;
+        int launches = 0;               // kernels of one body
+    } graphs[2];
+    int fuse_steps = 16;            // < 2: no graphs of several bodies
+    Graphs &steps() { return graphs[dx_max > 0.0]; }
+    const Graphs &steps() const { return graphs[dx_max > 0.0]; }
+    void drop_multi() {
+        for (Graphs &g : graphs) {
+            if (g.multi) cudaGraphExecDestroy(g.multi);
+            g.multi = nullptr;
+        }
+    }
+    void drop_graphs() {
+        drop_multi();
+        for (Graphs &g : graphs) {
+            if (g.one) cudaGraphExecDestroy(g.one);
+            g = Graphs{};
+        }
+    }
     float4 *u4_main = nullptr, *u4_alt = nullptr;  // s.u4 and s.u4n outside fused graphs
     FixRec *fix_main = nullptr, *fix_alt = nullptr;  // s.fix and s.fixn
     bool alt_bodies = false;        // capturing bodies that alternate u4 buffers
     bool graph_stale = true;
     uint64_t gen = 1;               // bumped whenever captured graphs of this context go stale
     int graph_prec = -1;
-    int launches_per_step = 0;
     bool timing = false;
     std::vector<cudaEvent_t> ev;       // kNumTimers + 1 events per timed step
     std::vector<double> timer_ms;      // accumulated per kernel
@@ -221,10 +240,6 @@ mg_status check_launch(mg_context *ctx) {
 // record; dx_max > 0 switches to the variable rule, which the step head applies from the next step
 void set_dt(mg_context *ctx, double dt, double dx_max = 0.0, double dt_min = 0.0, double dt_max = 0.0) {
     ctx->dt = dt;
-    if ((dx_max > 0.0) != (ctx->dx_max > 0.0)) {  // steps captured under the other rule
-        ctx->graph_stale = true;
-        ctx->gen++;
-    }
     ctx->dx_max = dx_max;
     ctx->dt_min = dt_min;
     ctx->dt_max = dt_max;
@@ -305,7 +320,7 @@ constexpr int kPlainBodies = 4;
 int multi_bodies(const mg_context *ctx) { return ctx->mixed() && fusable(ctx) ? ctx->fuse_steps : kPlainBodies; }
 int multi_steps(const mg_context *ctx, int64_t run) {
     if (ctx->fuse_steps < 2) return 0;
-    const bool pays = ctx->graph_multi || (ctx->mixed() && fusable(ctx)) || run >= 40 ||
+    const bool pays = (ctx->steps().multi && !ctx->graph_stale) || (ctx->mixed() && fusable(ctx)) || run >= 40 ||
                       (fusable(ctx) && (run >= 20 || run * ctx->g.n_local >= 4000000));
     return pays ? multi_bodies(ctx) : 0;
 }
@@ -511,22 +526,23 @@ mg_status check_types(mg_context *ctx, const mg_atom_element *atoms, int64_t n) 
     return MG_OK;
 }
 
+// the graphs of the timestep rule in use
 mg_status build_graph(mg_context *ctx) {
-    if (ctx->graph_exec && !ctx->graph_stale && ctx->graph_prec == ctx->precision) return MG_OK;
-    if (ctx->graph_exec) { cudaGraphExecDestroy(ctx->graph_exec); ctx->graph_exec = nullptr; }
-    if (ctx->graph_multi) { cudaGraphExecDestroy(ctx->graph_multi); ctx->graph_multi = nullptr; }
+    if (ctx->graph_stale || ctx->graph_prec != ctx->precision) ctx->drop_graphs();
+    ctx->graph_stale = false;
+    ctx->graph_prec = ctx->precision;
+    mg_context::Graphs &g = ctx->steps();
+    if (g.one) return MG_OK;
     cudaGraph_t graph;
     MG_CK(cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
     seq_step(ctx, nullptr);
     MG_CK(cudaStreamEndCapture(ctx->stream, &graph));
     size_t n_nodes = 0;
     cudaGraphGetNodes(graph, nullptr, &n_nodes);
-    ctx->launches_per_step = static_cast<int>(n_nodes);
-    cudaError_t e = cudaGraphInstantiate(&ctx->graph_exec, graph, 0);
+    g.launches = static_cast<int>(n_nodes);
+    cudaError_t e = cudaGraphInstantiate(&g.one, graph, 0);
     cudaGraphDestroy(graph);
     if (e != cudaSuccess) { ctx->err = std::string("graph instantiate: ") + cudaGetErrorString(e); return MG_ERR_CUDA; }
-    ctx->graph_stale = false;
-    ctx->graph_prec = ctx->precision;
     return MG_OK;
 }
 
@@ -544,7 +560,8 @@ void set_body_buffers(mg_context *ctx, int64_t k, int64_t i) {
 // next one, so the state between launches is the end of a loop body as always
 mg_status build_graph_multi(mg_context *ctx) {
     mg_status st = build_graph(ctx);
-    if (st != MG_OK || ctx->graph_multi) return st;
+    mg_context::Graphs &g = ctx->steps();
+    if (st != MG_OK || g.multi) return st;
     cudaGraph_t graph;
     MG_CK(cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
     const int k = multi_bodies(ctx);
@@ -560,7 +577,7 @@ mg_status build_graph_multi(mg_context *ctx) {
         for (int i = 0; i < k; i++) seq_step(ctx, nullptr);
     }
     MG_CK(cudaStreamEndCapture(ctx->stream, &graph));
-    cudaError_t e = cudaGraphInstantiate(&ctx->graph_multi, graph, 0);
+    cudaError_t e = cudaGraphInstantiate(&g.multi, graph, 0);
     cudaGraphDestroy(graph);
     if (e != cudaSuccess) { ctx->err = std::string("graph instantiate: ") + cudaGetErrorString(e); return MG_ERR_CUDA; }
     return MG_OK;
@@ -748,8 +765,7 @@ mg_status mg_create(const int64_t phase_space[3], double lattice_const, double r
 mg_status mg_destroy(mg_context *ctx) {
     if (!ctx) return MG_ERR_ARG;
     if (ctx->stream) cudaStreamSynchronize(ctx->stream);
-    if (ctx->graph_exec) cudaGraphExecDestroy(ctx->graph_exec);
-    if (ctx->graph_multi) cudaGraphExecDestroy(ctx->graph_multi);
+    ctx->drop_graphs();
     for (cudaEvent_t e : ctx->ev) cudaEventDestroy(e);
     for (cudaEvent_t e : ctx->pipe_ev) cudaEventDestroy(e);
     if (ctx->copy_in) cudaStreamDestroy(ctx->copy_in);
@@ -1097,9 +1113,9 @@ mg_status mg_simulate(mg_context *ctx, int64_t nsteps, int32_t sync) {
         const int64_t k = multi_steps(ctx, nsteps);
         if (k >= 2 && nsteps >= k) {
             if ((st = build_graph_multi(ctx)) != MG_OK) return st;
-            for (; i + k <= nsteps; i += k) MG_CK(cudaGraphLaunch(ctx->graph_multi, ctx->stream));
+            for (; i + k <= nsteps; i += k) MG_CK(cudaGraphLaunch(ctx->steps().multi, ctx->stream));
         }
-        for (; i < nsteps; i++) MG_CK(cudaGraphLaunch(ctx->graph_exec, ctx->stream));
+        for (; i < nsteps; i++) MG_CK(cudaGraphLaunch(ctx->steps().one, ctx->stream));
     }
     ctx->energy_valid = false;
     if (sync) {
@@ -1244,7 +1260,6 @@ mg_status mg_run_stages(mg_context *ctx, const mg_stage *stages, int32_t n_stage
         ctx->n_samples_cap = want;
     }
     mg_status st;
-    if ((st = build_graph(ctx)) != MG_OK) return st;
     const LaunchCtx lc = ctx->lc();
     int64_t cur_stage_steps = 0, stage_len = 0, taken = 0;
     int32_t next = 0;
@@ -1290,12 +1305,12 @@ mg_status mg_run_stages(mg_context *ctx, const mg_stage *stages, int32_t n_stage
         }
         if (fused) {
             if ((st = build_graph_multi(ctx)) != MG_OK) return st;
-            MG_CK(cudaGraphLaunch(ctx->graph_multi, ctx->stream));
+            MG_CK(cudaGraphLaunch(ctx->steps().multi, ctx->stream));
             cur_stage_steps += k - 1;
             step += k - 1;
         } else {
-            if ((st = build_graph(ctx)) != MG_OK) return st;  // a stage's dt ends the variable rule
-            MG_CK(cudaGraphLaunch(ctx->graph_exec, ctx->stream));
+            if ((st = build_graph(ctx)) != MG_OK) return st;
+            MG_CK(cudaGraphLaunch(ctx->steps().one, ctx->stream));
         }
         cur_stage_steps++;
         if (ctx->stage_dump && ctx->stage_dump_interval && (step + 1) % ctx->stage_dump_interval == 0) {
@@ -1743,7 +1758,7 @@ static mg_status step_host_pipelined(mg_context *ctx, mg_atom_element *atoms, mg
 mg_status mg_set_step_fusion(mg_context *ctx, int32_t steps_per_graph) {
     if (!ctx || steps_per_graph < 0 || steps_per_graph > 256) return MG_ERR_ARG;
     ctx->fuse_steps = steps_per_graph;
-    if (ctx->graph_multi) { cudaGraphExecDestroy(ctx->graph_multi); ctx->graph_multi = nullptr; }
+    ctx->drop_multi();
     return MG_OK;
 }
 
@@ -1753,7 +1768,6 @@ mg_status mg_set_neighbour_skin(mg_context *ctx, double skin) {
     launch_skin_dirty(ctx->lc(), ctx->s);
     ctx->graph_stale = true;  // the captured kernels hold the old geometry
     ctx->gen++;
-    if (ctx->graph_multi) { cudaGraphExecDestroy(ctx->graph_multi); ctx->graph_multi = nullptr; }
     return check_launch(ctx);
 }
 
@@ -1935,7 +1949,7 @@ mg_status mg_kernel_times(const mg_context *ctx, double *ms, int32_t cap, int32_
 
 mg_status mg_launches_per_step(const mg_context *ctx, int32_t *n) {
     if (!ctx || !n) return MG_ERR_ARG;
-    *n = ctx->launches_per_step > 0 ? ctx->launches_per_step : kLaunchesPerStep;
+    *n = ctx->steps().launches > 0 ? ctx->steps().launches : kLaunchesPerStep;
     return MG_OK;
 }
 
@@ -1949,11 +1963,25 @@ struct mg_batch {
     std::vector<uint64_t> gens;          // each context's generation when the graphs were captured
     int steps_per_launch = 1;
     cudaStream_t stream = nullptr;
-    cudaGraphExec_t exec_k = nullptr;    // steps_per_launch loop bodies of every replica
-    cudaGraphExec_t exec_1 = nullptr;    // one loop body of every replica (remainders)
+    // captured steps: of the replicas' timestep rules in use, and of those before them, which a program may go back to
+    struct Graphs {
+        std::vector<bool> variable;      // each replica's rule
+        cudaGraphExec_t exec_k = nullptr;  // steps_per_launch loop bodies of every replica
+        cudaGraphExec_t exec_1 = nullptr;  // one loop body of every replica (remainders)
+        int launches = 0;                // kernels of one body of every replica
+        bool matches(const std::vector<mg_context *> &ctxs) const {
+            for (size_t r = 0; r < ctxs.size(); r++)
+                if (variable.size() != ctxs.size() || variable[r] != (ctxs[r]->dx_max > 0.0)) return false;
+            return true;
+        }
+        void drop() {
+            if (exec_k) cudaGraphExecDestroy(exec_k);
+            if (exec_1) cudaGraphExecDestroy(exec_1);
+            *this = Graphs{};
+        }
+    } now, before;
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
     std::vector<cudaEvent_t> ev_ctx;
-    int launches_per_step = 0;
     std::string err;
 };
 
@@ -2002,15 +2030,22 @@ mg_status capture_batch(mg_batch *b, int steps, cudaGraphExec_t *exec, int *n_no
     return MG_OK;
 }
 
-mg_status batch_capture_all(mg_batch *b) {
-    if (b->exec_k) { cudaGraphExecDestroy(b->exec_k); b->exec_k = nullptr; }
-    if (b->exec_1) { cudaGraphExecDestroy(b->exec_1); b->exec_1 = nullptr; }
+// graphs of the replicas' rules in use into b->now (at most one other set is kept); stale: none of the present ones holds
+mg_status batch_capture_all(mg_batch *b, bool stale) {
+    std::swap(b->now, b->before);
+    if (!stale && b->now.matches(b->ctxs)) return MG_OK;
+    b->now.drop();
+    if (stale) b->before.drop();
     for (mg_context *ctx : b->ctxs) MB_CK(cudaStreamSynchronize(ctx->stream));
     int nk = 0, n1 = 0;
-    mg_status st = capture_batch(b, b->steps_per_launch, &b->exec_k, &nk);
-    if (st == MG_OK && b->steps_per_launch > 1) st = capture_batch(b, 1, &b->exec_1, &n1);
-    if (st != MG_OK) return st;
-    b->launches_per_step = b->steps_per_launch > 1 ? n1 : nk;
+    mg_status st = capture_batch(b, b->steps_per_launch, &b->now.exec_k, &nk);
+    if (st == MG_OK && b->steps_per_launch > 1) st = capture_batch(b, 1, &b->now.exec_1, &n1);
+    if (st != MG_OK) {
+        b->now.drop();
+        return st;
+    }
+    b->now.launches = b->steps_per_launch > 1 ? n1 : nk;
+    for (mg_context *ctx : b->ctxs) b->now.variable.push_back(ctx->dx_max > 0.0);
     for (size_t r = 0; r < b->ctxs.size(); r++) b->gens[r] = b->ctxs[r]->gen;
     return MG_OK;
 }
@@ -2042,7 +2077,7 @@ mg_status mg_batch_create(mg_context *const *ctxs, int32_t n, int32_t steps_per_
         mg_batch_destroy(b);
         return MG_ERR_CUDA;
     }
-    if (batch_capture_all(b) != MG_OK) {
+    if (batch_capture_all(b, true) != MG_OK) {
         g_create_error = b->err;
         mg_batch_destroy(b);
         return MG_ERR_CUDA;
@@ -2053,13 +2088,14 @@ mg_status mg_batch_create(mg_context *const *ctxs, int32_t n, int32_t steps_per_
 
 mg_status mg_batch_run(mg_batch *b, int64_t nsteps, int32_t sync) {
     if (!b || nsteps < 0) return MG_ERR_ARG;
+    bool stale = false;  // precision, tuning or potential changed since the capture
     for (size_t r = 0; r < b->ctxs.size(); r++) {
         if (!b->ctxs[r]->prepared) { b->err = "replica " + std::to_string(r) + " is not prepared"; return MG_ERR_STATE; }
-        if (b->ctxs[r]->gen != b->gens[r]) {  // precision, tuning or potential changed since the capture
-            mg_status st = batch_capture_all(b);
-            if (st != MG_OK) return st;
-            break;
-        }
+        stale = stale || b->ctxs[r]->gen != b->gens[r];
+    }
+    if (stale || !b->now.matches(b->ctxs)) {
+        mg_status st = batch_capture_all(b, stale);
+        if (st != MG_OK) return st;
     }
     // the batch runs after each replica's pending work, and each replica's later work after the batch
     for (size_t r = 0; r < b->ctxs.size(); r++) {
@@ -2072,8 +2108,8 @@ mg_status mg_batch_run(mg_batch *b, int64_t nsteps, int32_t sync) {
         MB_CK(cudaStreamWaitEvent(b->stream, b->ev_ctx[r], 0));
     }
     const int64_t k = b->steps_per_launch;
-    for (int64_t i = 0; i < nsteps / k; i++) MB_CK(cudaGraphLaunch(b->exec_k, b->stream));
-    for (int64_t i = 0; i < nsteps % k; i++) MB_CK(cudaGraphLaunch(b->exec_1, b->stream));
+    for (int64_t i = 0; i < nsteps / k; i++) MB_CK(cudaGraphLaunch(b->now.exec_k, b->stream));
+    for (int64_t i = 0; i < nsteps % k; i++) MB_CK(cudaGraphLaunch(b->now.exec_1, b->stream));
     MB_CK(cudaEventRecord(b->ev_join, b->stream));
     for (mg_context *ctx : b->ctxs) {
         MB_CK(cudaStreamWaitEvent(ctx->stream, b->ev_join, 0));
@@ -2096,7 +2132,7 @@ mg_status mg_batch_run(mg_batch *b, int64_t nsteps, int32_t sync) {
 
 mg_status mg_batch_launches_per_step(const mg_batch *b, int32_t *n) {
     if (!b || !n) return MG_ERR_ARG;
-    *n = b->launches_per_step;
+    *n = b->now.launches;
     return MG_OK;
 }
 
@@ -2107,8 +2143,8 @@ const char *mg_batch_last_error(const mg_batch *b) { return b ? b->err.c_str() :
 mg_status mg_batch_destroy(mg_batch *b) {
     if (!b) return MG_ERR_ARG;
     if (b->stream) cudaStreamSynchronize(b->stream);
-    if (b->exec_k) cudaGraphExecDestroy(b->exec_k);
-    if (b->exec_1) cudaGraphExecDestroy(b->exec_1);
+    b->now.drop();
+    b->before.drop();
     if (b->ev_fork) cudaEventDestroy(b->ev_fork);
     if (b->ev_join) cudaEventDestroy(b->ev_join);
     for (cudaEvent_t e : b->ev_ctx) if (e) cudaEventDestroy(e);

@@ -59,4 +59,17 @@ cudaError_t cudaFreeHost(void *p) {
     return cudaSuccess;
 }
 const char *cudaGetErrorString(cudaError_t) { return "fake device"; }
+
+static int g_graphs_made = 0, g_graphs_alive = 0;
+int fake_graphs_made() { return g_graphs_made; }
+int fake_graphs_alive() { return g_graphs_alive; }
+cudaError_t cudaGraphInstantiate(cudaGraphExec_t *e, cudaGraph_t, unsigned long long) {
+    *e = reinterpret_cast<cudaGraphExec_t>(static_cast<size_t>(++g_graphs_made));
+    g_graphs_alive++;
+    return cudaSuccess;
+}
+cudaError_t cudaGraphExecDestroy(cudaGraphExec_t) {
+    g_graphs_alive--;
+    return cudaSuccess;
+}
 }
