@@ -255,10 +255,13 @@ static double fp64_error(const HostPotential &hp, const Crystal &c, double a0, d
     return least;
 }
 
-// build_fixed for one inner end r_lo of the tables' range and F'(rho) in units of 2^-kd; exact: the FP64 loops' error;
-// tab null: the scales only
+// build_fixed for one inner end r_lo of the tables' range and F'(rho) in units of 2^-kd; exact: the FP64 loops' error.
+// depth: the scales only, whether the innermost intervals (where the quartics are at their worst) meet the bound, or
+// everything into tab
+enum Depth { SCALES, INNERMOST, TABLES };
 static bool build_from(const HostPotential &hp, const int ele_of_type[3], double a0, double rcf, int n_part, double r_lo, int kd,
-                       double exact, const std::vector<Largest> &largest, FixParams &fp, FixTables *tab, bool want_phi) {
+                       double exact, const std::vector<Largest> &largest, FixParams &fp, FixTables *tab, bool want_phi,
+                       Depth depth) {
     fp = FixParams{};
     const double rc = a0 * rcf, dr = hp.dr;
     const int nr = hp.nr;
@@ -315,7 +318,8 @@ static bool build_from(const HostPotential &hp, const int ele_of_type[3], double
     fp.f_unit = std::ldexp(1.0, -kF);
     fp.lo = (i64) (std::ldexp((m_lo + 1) * dr * (m_lo + 1) * dr, kr - 32) + 1.0) << 32;
 
-    if (!tab) return true;
+    if (depth == SCALES) return true;
+    const int m_end = depth == INNERMOST ? std::min(m_lo + 16, fp.nr1) : fp.nr1;
 
     // the intervals; the records past the last one (a cutoff at the table's end, found a knot too far)
     // continue its cubic
@@ -323,8 +327,8 @@ static bool build_from(const HostPotential &hp, const int ele_of_type[3], double
         return root(scaled(dd((double) (v >> 31)) * dd(2147483648.0) + dd((double) (v & 0x7fffffff)), -kr));
     };
     const Series sq = power(1);
-    std::vector<Interval> iv(fp.nr1);
-    for (int m = m_lo; m < fp.nr1; m++) {
+    std::vector<Interval> iv(m_end);
+    for (int m = m_lo; m < m_end; m++) {
         Interval &v = iv[m];
         v.m = std::min(m, m_hi);
         v.sc = -fix_centre_sub(fp, m, 0);
@@ -366,9 +370,9 @@ static bool build_from(const HostPotential &hp, const int ele_of_type[3], double
     const int first[4] = {add(FN_RHO, krho, false, rho_max), add(FN_G, kg, true, g_max), add(FN_H, kf, true, h_max),
                           want_phi ? add(FN_PHI, kphi, false, phi_max) : 0};
     auto expand = [&](Table &t) {
-        t.w.resize(fp.nr1);
-        t.out.assign(fp.nr1, FixPoly{});
-        for (int m = m_lo; m < fp.nr1; m++) {
+        t.w.resize(m_end);
+        t.out.assign(m_end, FixPoly{});
+        for (int m = m_lo; m < m_end; m++) {
             const Interval &v = iv[m];
             Series &w = t.w[m] = expanded(*t.s, t.fn, v);
             double f = 1.0;
@@ -385,7 +389,7 @@ static bool build_from(const HostPotential &hp, const int ele_of_type[3], double
         }
     };
     auto round_all = [&](Table &t, int e3) {
-        for (int m = m_lo; m < fp.nr1; m++) {
+        for (int m = m_lo; m < m_end; m++) {
             const Interval &v = iv[m];
             // What the coarse units of c4 and c3 leave over goes to the lower coefficients, as T4 and T3 put it:
             // x^4 = xm^2 x^2 - xm^4 / 8 and x^3 = (3/4) xm^2 x, to xm^4 / 8 and xm^3 / 4.
@@ -419,6 +423,10 @@ static bool build_from(const HostPotential &hp, const int ele_of_type[3], double
         t.ok = true;
     };
     auto side_by_side = [&](auto &&work) {
+        if (depth == INNERMOST) {
+            for (Table &t : tables) work(t);
+            return;
+        }
         std::vector<std::future<void>> f;
         for (Table &t : tables) f.push_back(std::async([&work, &t] { work(t); }));  // (in turn where no thread can be had)
         for (auto &x : f) x.get();
@@ -436,6 +444,7 @@ static bool build_from(const HostPotential &hp, const int ele_of_type[3], double
     side_by_side([&](Table &t) { round_all(t, e3[t.fn]); });
     for (const Table &t : tables)
         if (!t.ok) return false;
+    if (depth == INNERMOST) return true;
     fp.e3_rho = e3[FN_RHO];
     fp.e3_g = e3[FN_G];
     fp.e3_h = e3[FN_H];
@@ -479,18 +488,17 @@ bool build_fixed(const HostPotential &hp, const int ele_of_type[3], double a0, d
     if (!(1.05 * crystal.df_least < 1.0)) return false;
     const double exact = fp64_error(hp, crystal, a0, a0 * rcf);
     int kd = 60;
+    auto from = [&](int f, Depth depth) {
+        return build_from(hp, ele_of_type, a0, rcf, n_part, f * percent, kd, exact, largest, fp, &tab, want_phi, depth);
+    };
     double finest = 0.0;
     for (int k = 60; k <= 80 && finest == 0.0 && (k == 60 || std::ldexp(2.5 * crystal.df_most, k - 60) <= 1.0); k++) {
         kd = k;
         for (int f = 70; f <= 86; f += 2)
-            if (build_from(hp, ele_of_type, a0, rcf, n_part, f * percent, kd, exact, largest, fp, nullptr, want_phi) &&
-                (finest == 0.0 || fp.f_unit < finest))
-                finest = fp.f_unit;
+            if (from(f, SCALES) && (finest == 0.0 || fp.f_unit < finest)) finest = fp.f_unit;
     }
     for (int f = 70; f <= 86 && finest > 0.0; f += 2)
-        if (build_from(hp, ele_of_type, a0, rcf, n_part, f * percent, kd, exact, largest, fp, nullptr, want_phi) && fp.f_unit == finest &&
-            build_from(hp, ele_of_type, a0, rcf, n_part, f * percent, kd, exact, largest, fp, &tab, want_phi))
-            return true;
+        if (from(f, SCALES) && fp.f_unit == finest && from(f, INNERMOST) && from(f, TABLES)) return true;
     fp = FixParams{};
     return false;
 }
