@@ -237,7 +237,8 @@ mg_status mg_autotune(mg_context *ctx, int32_t reps, int32_t out[6]);
 /* Sets the six tuning values directly (same layout as mg_autotune's out). */
 mg_status mg_set_tuning(mg_context *ctx, const int32_t tune[6]);
 
-/* Measured kernel times of the last mg_simulate call with timing enabled (ms per step per kernel). */
+/* Measured times of the parts of a step in the last mg_simulate call with timing enabled (ms per step). A part whose work
+ * other kernels have taken over (inter_firststep, lat_df, secondstep) reads 0; theirs include it. */
 mg_status mg_enable_timing(mg_context *ctx, int32_t on);
 mg_status mg_kernel_times(const mg_context *ctx, double *ms, int32_t cap, int32_t *n, const char **names);
 /* Number of kernel launches per loop-body step in the captured graph. */

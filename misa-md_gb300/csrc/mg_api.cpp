@@ -21,15 +21,22 @@ namespace {
 
 thread_local std::string g_create_error;
 
-constexpr int kNumTimers = 9;  // events per timed step; the kernels between consecutive events are:
-const char *kTimerNames[kNumTimers - 1] = {"firststep",     // the step head (variable dt) and firststep
-                                           "inter_manage",  // the list manager
-                                           "ghost_copy",    // and the far atoms' marks and the inter atoms' densities
-                                           "lat_rho",
-                                           "inter_rho",     // the density shares of lattice atoms near inter atoms
-                                           "ghost_df",      // and the forces on the inter atoms
-                                           "lat_force",
-                                           "inter_force"};  // the force shares of those atoms, and their half-kicks
+constexpr int kNumTimers = 9;  // events per timed step
+// The parts of a step that are reported, and the interval between events that holds each: -1 where its work is in another
+// part's kernels, and reported there.
+constexpr int kNumParts = 11;
+const struct { const char *name; int interval; } kParts[kNumParts] = {
+    {"firststep", 0},          // the step head (variable dt), firststep, the inter atoms' firststep
+    {"inter_firststep", -1},
+    {"inter_manage", 1},       // the list manager
+    {"ghost_copy", 2},         // and the far atoms' marks and the inter atoms' densities
+    {"lat_rho", 3},            // and dF/drho of the atoms no inter atom is near
+    {"inter_rho", 4},          // the density shares of lattice atoms near inter atoms, and their dF/drho
+    {"lat_df", -1},
+    {"ghost_df", 5},           // and the forces on the inter atoms
+    {"lat_force", 6},          // and the second half-kick of the atoms no inter atom is near
+    {"inter_force", 7},        // the force shares of the others, their half-kicks and the inter atoms'
+    {"secondstep", -1}};
 
 }  // namespace
 
@@ -1939,10 +1946,11 @@ mg_status mg_enable_timing(mg_context *ctx, int32_t on) {
 
 mg_status mg_kernel_times(const mg_context *ctx, double *ms, int32_t cap, int32_t *n, const char **names) {
     if (!ctx || !n) return MG_ERR_ARG;
-    *n = kNumTimers - 1;
-    for (int k = 0; k < kNumTimers - 1 && k < cap; k++) {
-        if (ms) ms[k] = ctx->timed_steps ? ctx->timer_ms.size() > (size_t) k ? ctx->timer_ms[k] / ctx->timed_steps : 0.0 : 0.0;
-        if (names) names[k] = kTimerNames[k];
+    *n = kNumParts;
+    for (int k = 0; k < kNumParts && k < cap; k++) {
+        const int at = kParts[k].interval;
+        if (ms) ms[k] = at >= 0 && ctx->timed_steps ? ctx->timer_ms[at] / ctx->timed_steps : 0.0;
+        if (names) names[k] = kParts[k].name;
     }
     return MG_OK;
 }
