@@ -241,7 +241,7 @@ mg_status mg_set_tuning(mg_context *ctx, const int32_t tune[6]);
  * other kernels have taken over (inter_firststep, lat_df, secondstep) reads 0; theirs include it. */
 mg_status mg_enable_timing(mg_context *ctx, int32_t on);
 mg_status mg_kernel_times(const mg_context *ctx, double *ms, int32_t cap, int32_t *n, const char **names);
-/* Number of kernel launches per loop-body step in the captured graph. */
+/* Number of kernel launches per loop-body step in the captured graph of the timestep rule in use. */
 mg_status mg_launches_per_step(const mg_context *ctx, int32_t *n);
 /* CUDA stream of the context (a cudaStream_t), for callers timing on it. */
 void *mg_stream(const mg_context *ctx);

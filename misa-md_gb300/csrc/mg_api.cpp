@@ -331,7 +331,7 @@ int multi_steps(const mg_context *ctx, int64_t run) {
                       (fusable(ctx) && (run >= 20 || run * ctx->g.n_local >= 4000000));
     return pays ? multi_bodies(ctx) : 0;
 }
-constexpr int kLaunchesPerStep = 8;
+constexpr int kLaunchesPerStep = 8;  // and the step head under the variable rule
 
 mg_status require_ready(mg_context *ctx) {
     if (!ctx->pot_ready) { ctx->err = "potential not initialised"; return MG_ERR_POTENTIAL; }
@@ -1957,7 +1957,7 @@ mg_status mg_kernel_times(const mg_context *ctx, double *ms, int32_t cap, int32_
 
 mg_status mg_launches_per_step(const mg_context *ctx, int32_t *n) {
     if (!ctx || !n) return MG_ERR_ARG;
-    *n = ctx->steps().launches > 0 ? ctx->steps().launches : kLaunchesPerStep;
+    *n = ctx->steps().launches > 0 ? ctx->steps().launches : kLaunchesPerStep + (ctx->dx_max > 0.0 ? 1 : 0);
     return MG_OK;
 }
 
