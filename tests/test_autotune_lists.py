@@ -29,3 +29,21 @@ def test_steps_after_autotune_use_the_lists(pkg, wl, potentials, gpu_lib, prec, 
     for got in out[1:]:
         for f in ("x", "v", "f", "rho", "df"):
             assert np.array_equal(got[f], out[0][f]), f
+
+
+@pytest.mark.parametrize("pot,cells", [("fe", (99, 100, 101)), ("fecuni", (99, 100, 101)), ("fe", (70, 70, 70))])  # 512, 256, 256
+def test_default_blocks_keep_the_bits(pkg, wl, potentials, gpu_lib, pot, cells):
+    """The mixed force pass's default block follows from the box and the potential, and changes no bits."""
+    atoms = wl.build_state(cells, A0, RCF, temperature=300.0, seed=6)
+    out = []
+    for tune in (None, (1, 512, 1, 256), (1, 512, 1, 512)):
+        ctx = pkg.Context(cells, A0, RCF, precision="mixed")
+        if tune:
+            ctx.set_tuning(*tune)
+        ctx.pot_init_setfl(potentials[pot])
+        ctx.upload(atoms)
+        ctx.prepare()
+        ctx.simulate(2)
+        out.append(ctx.download()[0]["f"])
+        ctx.close()
+    assert np.array_equal(out[0], out[1]) and np.array_equal(out[0], out[2])
