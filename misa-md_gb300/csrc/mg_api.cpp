@@ -322,16 +322,18 @@ void seq_step(mg_context *ctx, Timer *t, bool fused_prev = false, bool fuse_next
 }
 // runs whose force passes may take the next firststep: a fixed dt, in the mixed or the fixed-point form
 bool fusable(const mg_context *ctx) { return ctx->fuse_steps >= 2 && (ctx->mixed() || ctx->lc().fp) && ctx->dx_max <= 0.0; }
-// Loop bodies in one graph launch of a run of that many steps (0: one body per launch). The mixed form: fuse_steps
-// fused bodies. The others kPlainBodies, since a graph costs about 25 us a body to make and their runs are short: bodies
-// of the FP64 form that are fused save a firststep each (2M atoms: 1959 -> 1926 us per step), and any saves the gap between two
-// launches, about 3 us (16k atoms FP64, per step: 58.0 -> 55.4 us with 4 bodies, 55.0 with 16).
+// Loop bodies in one graph launch of a run of that many steps (0: one body per launch). The mixed form with a fixed dt:
+// fuse_steps fused bodies. The others kPlainBodies, since a graph costs about 25 us a body to make and their runs are short.
+// A context makes it for the first run that it pays for within, at 100 us for four bodies. Gain per step over single
+// launches, us: the FP64 form with a fixed dt, whose bodies are fused (a firststep saved each), 3.8 at 2k sites, 3.7 at
+// 16k, 3.0 at 65k, 12.6 at 686k, 41 at 2M; the variable rule, which saves the gaps between launches only, FP64 1.1 / 4.2 /
+// 1.7 / 1.9 / 3.2, mixed 0.3 / 2.8 / 1.2 / 0.9 / 1.5.
 constexpr int kPlainBodies = 4;
 int multi_bodies(const mg_context *ctx) { return ctx->mixed() && fusable(ctx) ? ctx->fuse_steps : kPlainBodies; }
 int multi_steps(const mg_context *ctx, int64_t run) {
     if (ctx->fuse_steps < 2) return 0;
-    const bool pays = (ctx->steps().multi && !ctx->graph_stale) || (ctx->mixed() && fusable(ctx)) || run >= 40 ||
-                      (fusable(ctx) && (run >= 20 || run * ctx->g.n_local >= 4000000));
+    const double gain = fusable(ctx) ? 3.4 + 1.8e-5 * ctx->g.n_local : 1.8;
+    const bool pays = (ctx->steps().multi && !ctx->graph_stale) || (ctx->mixed() && fusable(ctx)) || run * gain >= 100.0;
     return pays ? multi_bodies(ctx) : 0;
 }
 constexpr int kLaunchesPerStep = 8;  // and the step head under the variable rule
