@@ -188,7 +188,8 @@ mg_status mg_clear_errors(mg_context *ctx);
  * One loop body with a fixed dt and no inter atoms in (*n_inter == 0) is pipelined: the slot array
  * moves in z-chunks of whole planes. In boxes of at least 24 planes the density and force slabs run
  * as their planes arrive and go back out while later chunks still come in. Decide is taken per chunk
- * for displaced atoms that return to their own site; any other displaced atom makes the call run the
+ * for displaced atoms that return to their own site; any other displaced atom (in the FP64 form also one
+ * more than 0.6 a0 from its site along an axis) makes the call run the
  * loop body again in full from its kept input (an extra device copy of the slot array). Thinner boxes
  * overlap the copies in with firststep and the copies out with the force slabs. The result is
  * bit-identical to the unpipelined path. With a pinned slot array (mg_host_register) the copies run
@@ -197,23 +198,28 @@ mg_status mg_clear_errors(mg_context *ctx);
 mg_status mg_step_host(mg_context *ctx, mg_atom_element *atoms, int64_t n_slots, mg_atom_element *inter,
                        int64_t inter_cap, int64_t *n_inter, int64_t nsteps);
 /* Loop bodies per CUDA graph launch of mg_simulate in the mixed form with a fixed dt (default 16; 0 or
- * 1: one body per launch, in every form; otherwise the FP64 form launches 4 at a time). Inside a launch, each force pass but the last also takes the next body's
- * firststep for its atoms (when no inter atoms exist; the kernels check on the device), which saves
- * the separate firststep pass. The state between launches is the end of a loop body as always, and
- * results are bit-identical either way. mg_run_stages uses the same graph for runs of bodies with
+ * 1: one body per launch, in every form). Otherwise the FP64 form, and both forms under the variable
+ * timestep, launch 4 at a time once a run is long enough to pay for capturing them. With a fixed dt each
+ * force pass of a launch but the last (FP64 form: where its fixed-point passes are in use) also takes the
+ * next body's firststep for its atoms (when no inter atoms exist; the kernels check on the device), which
+ * saves the separate firststep pass. The state between launches is the end of a loop body as always, and
+ * results are bit-identical either way. mg_run_stages uses the same graphs for runs of bodies with
  * no stage event between them. */
 mg_status mg_set_step_fusion(mg_context *ctx, int32_t steps_per_graph);
-/* Number of z-chunks of mg_step_host's pipeline (default: by the box's size, up to 16; 0 or 1: no pipelining). */
+/* Number of z-chunks of mg_step_host's pipeline (0 or 1: no pipelining). Until the first call they follow from the
+ * box's size, up to 16; there is no value that goes back to that. */
 mg_status mg_set_host_pipeline(mg_context *ctx, int32_t chunks);
-/* Verlet skin of the mixed form's candidate lists, in Angstrom (default 0.2; 0: off; at most a0).
+/* Verlet skin of the candidate lists (mixed form, and the FP64 form's fixed-point passes), in Angstrom
+ * (default 0.2; 0: off; at most a0).
  * Each group of 32 sites keeps the pruned candidates that some site of the group had within
  * rc + skin when the list was built. The density pass then visits only those, until the sum of the
  * per-step maximum displacements, doubled, reaches the skin; a record written by an upload or by
  * recombination also forces a rebuild. Every pair inside the cutoff is visited either way, in the
  * same order, so results are bit-identical for every skin. Captured graphs are rebuilt. */
 mg_status mg_set_neighbour_skin(mg_context *ctx, double skin);
-/* Density passes that used the mixed form's candidate lists, and how many of them rebuilt the lists
- * (diagnostics). Syncs. */
+/* Density passes that used the candidate lists, and how many of them rebuilt the lists (diagnostics).
+ * The FP64 loops, which serve potentials that the fixed-point tables do not suit, use none: passes that
+ * do not count in the FP64 form show which of the two is in use. Syncs. */
 mg_status mg_skin_stats(mg_context *ctx, int64_t *passes, int64_t *rebuilds);
 
 /* ---------------------------------------------------------------------------------------------

@@ -416,7 +416,7 @@ class Context:
         self._check(self.lib.mg_set_step_fusion(self.h, int(steps_per_graph)))
 
     def set_neighbour_skin(self, skin):
-        """Verlet skin (Angstrom) of the mixed form's candidate lists (0: off); results do not depend on it."""
+        """Verlet skin (Angstrom) of the candidate lists (0: off); results do not depend on it."""
         self._check(self.lib.mg_set_neighbour_skin(self.h, float(skin)))
 
     def skin_stats(self):

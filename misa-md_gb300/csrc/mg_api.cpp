@@ -90,8 +90,7 @@ struct mg_context {
     // switch between them
     struct Graphs {
         cudaGraphExec_t one = nullptr;  // one loop body
-        // kPlainBodies loop bodies, or (fused) fuse_steps whose force passes (all but the last) take the next firststep
-        // (mixed form, fixed dt)
+        // several loop bodies (multi_bodies); with a fixed dt the force passes of all but the last take the next firststep
         cudaGraphExec_t multi = nullptr;
         int launches = 0;               // kernels of one body
     } graphs[2];
@@ -205,7 +204,7 @@ cudaError_t dalloc(mg_context *ctx, T **p, size_t n) {
     return e;
 }
 
-// Verlet skin of the group candidate lists (mixed form), Angstrom. The lists then hold about the
+// Verlet skin of the group candidate lists, Angstrom. The lists then hold about the
 // sixth shell besides the 58 neighbours inside the cutoff; at 600 K and dt = 1 fs they last about 8
 // steps (0.15 to 0.25 A measured within 0.3% of each other on 16M atoms, 0.2 the fastest).
 constexpr double kDefaultSkin = 0.2;

@@ -83,7 +83,7 @@ struct Geom {
     int n_site_half;
 };
 
-// Verlet skin on the group candidate lists (mixed form). The density pass of some step built the
+// Verlet skin on the group candidate lists. The density pass of some step built the
 // lists from the displacement records of that step. Until `dirty` is set, no record has changed since
 // then except through firststep (or through recombination, whose neighbourhood marks make the groups
 // that can see the atom rebuild their own lists), and every change of a record is at most the
@@ -182,7 +182,7 @@ struct PotTables {
 };
 
 // Per-step parameters, resident in device memory (one record per context). Kernels read dt and the
-// half-kick factors dt/(2m) from here, so a new timestep needs no new graph. In variable-timestep
+// half-kick factors dt/(2m) from here, so a new timestep needs no new graph (each timestep rule has its own). In variable-timestep
 // mode the step-head kernel rewrites them every step from the largest speed the previous kick left.
 constexpr int kVmaxSlots = 1024;    // spread max-words: one per (warp index mod kVmaxSlots)
 constexpr int kDtHistory = 65536;   // ring of the most recent timesteps
@@ -302,9 +302,9 @@ void launch_far_mark(const LaunchCtx &lc, const Geom &g, Inter in);
 void launch_ghost_copy(const LaunchCtx &lc, const Geom &g, Slots s, Inter in, PotTables t, bool mixed, bool mark, bool inter);
 // also the forces on the inter atoms; advance: also as launch_skin_advance
 void launch_ghost_df(const LaunchCtx &lc, const Geom &g, Slots s, Inter in, PotTables t, bool mixed, bool advance);
-// lists (mixed form): check or rebuild, per 32-site group, the list of pruned candidates that some site
-// of the group has inside rc + skin, and visit only those (when lists_ok; the force pass of the same
-// step must get the same flag)
+// lists (mixed form, and the FP64 form's fixed-point passes): check or rebuild, per 32-site group, the list of pruned
+// candidates that some site of the group has inside rc + skin, and visit only those (when lists_ok; the force pass of the
+// same step must get the same flag)
 // true: the skin's advance is due. Inter atoms: after launch_ghost_copy, which lists the owners whose F' the pass
 // leaves to launch_inter_rho_owners.
 bool launch_lat_rho(const LaunchCtx &lc, const Geom &g, Slots s, Inter in, PotTables t, bool mixed, bool hook,

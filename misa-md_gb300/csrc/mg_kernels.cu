@@ -1272,7 +1272,8 @@ __global__ void __launch_bounds__(32 * W) k_lat_rho_mixed_split(const float4 *ca
 // operations at one or two issue slots each; its FP64 operations cost 64 slots apiece, which bound the FP64
 // loops (2M atoms, step: 14.2 -> 1.93 ms; 304k atoms: 2.2 -> 0.40 ms; 16k atoms: 0.32 -> 0.05 ms). They stay
 // for the cases below and for tables the fixed point does not suit. Its errors are half the FP64 loops'
-// (thermal crystals against 113-bit arithmetic: force rms 2.4e-15 -> 1.1e-15 of the rms force).
+// (thermal crystals against 113-bit arithmetic: force rms 2.4e-15 -> 1.1e-15 of the rms force); build_fixed refuses tables
+// where they would be larger.
 // The group lists of the mixed form serve here as well: 66 candidates are visited instead of 112.
 // Pairs closer than the tables reach (hot crystals, cascades) are kept per thread and summed in FP64 after
 // the loop; an atom with more than four of them, or with an F'(rho) too large for its fixed-point
@@ -2380,7 +2381,9 @@ static void launch_force_fix_split(const LaunchCtx &lc, const Geom &g, Slots s, 
                                    int u0, int u1, bool fuse, bool lists) {
     const int n = split_groups(u0, u1);
     const float4 *cand = &lc.ntd->cand[0][0];
-    // 500 groups of 8 warps fit one wave at 64 registers, one candidate at a time: 29.1 -> 26.2 us
+    // From two groups per SM on, one candidate at a time: at 64 registers the blocks of 8 warps still fit one wave. Force pass
+    // with two -> one, us, one element: 307 groups 25.8 -> 22.6, 364 27.9 -> 22.9, 500 28.1 -> 26.0, 578 28.7 -> 26.5; three:
+    // 28.4 -> 26.2, 31.9 -> 27.0, 32.7 -> 30.7, 33.4 -> 30.8. Below it two hide more of the loads.
     if constexpr (W == 8)
         if (n * lc.share > 2 * lc.num_sms) {
             k_lat_force_fix_split<W, 4, 1, ONE><<<n, 32 * W, 0, lc.stream>>>(*lc.nt, cand, g, s, in, t, *lc.fp, p, kick, hook, u0, u1, fuse, lists);
