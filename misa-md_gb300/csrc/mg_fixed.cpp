@@ -487,6 +487,7 @@ bool build_fixed(const HostPotential &hp, const int ele_of_type[3], double a0, d
     const Crystal crystal = crystal_of(hp, a0, a0 * rcf);
     if (!(1.05 * crystal.df_least < 1.0)) return false;
     const double exact = fp64_error(hp, crystal, a0, a0 * rcf);
+    if (!std::isfinite(exact)) return false;  // no crystal of one element to hold the sums against
     int kd = 60;
     auto from = [&](int f, Depth depth) {
         return build_from(hp, ele_of_type, a0, rcf, n_part, f * percent, kd, exact, largest, fp, &tab, want_phi, depth);
