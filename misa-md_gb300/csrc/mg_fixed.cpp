@@ -475,8 +475,8 @@ static bool build_from(const HostPotential &hp, const int ele_of_type[3], double
 // pair in 1e5 is closer than 0.82.
 // F' stays below 1 in most tables (in eV; others scale with the density's unit). An atom above the bound takes the FP64
 // loop after its fixed-point one, and so does every neighbour, so where every perfect crystal is at it already, the
-// tables are refused. Where the bound of 1 leaves the force sums' unit too coarse, a lower one serves if it is two and a
-// half times a crystal's F' or more (next to a vacancy F' grows by a tenth).
+// tables are refused. Where the bound of 1 leaves the force sums' unit too coarse, a lower one serves if it is five
+// quarters of a crystal's F' or more (next to a vacancy F' grows by a tenth).
 bool build_fixed(const HostPotential &hp, const int ele_of_type[3], double a0, double rcf, int n_part, FixParams &fp,
                  FixTables &tab, bool want_phi) {
     fp = FixParams{};
@@ -493,7 +493,7 @@ bool build_fixed(const HostPotential &hp, const int ele_of_type[3], double a0, d
         return build_from(hp, ele_of_type, a0, rcf, n_part, f * percent, kd, exact, largest, fp, &tab, want_phi, depth);
     };
     double finest = 0.0;
-    for (int k = 60; k <= 80 && finest == 0.0 && (k == 60 || std::ldexp(2.5 * crystal.df_most, k - 60) <= 1.0); k++) {
+    for (int k = 60; k <= 80 && finest == 0.0 && (k == 60 || std::ldexp(1.25 * crystal.df_most, k - 60) <= 1.0); k++) {
         kd = k;
         for (int f = 70; f <= 86; f += 2)
             if (from(f, SCALES) && (finest == 0.0 || fp.f_unit < finest)) finest = fp.f_unit;
