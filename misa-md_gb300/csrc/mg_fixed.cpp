@@ -175,11 +175,11 @@ int first_knot(double r_lo, double dr) { return std::max(1, (int) (r_lo / dr) - 
 }  // namespace
 
 // A perfect crystal's neighbours of a site in the order the loops visit them (in half lattice constants, BCC: all even or
-// all odd), and |F'(rho)| of an element on a site whose neighbours are of one element: the least and the largest over the
-// elements.
+// all odd), and over the elements: the least density of crystals of one of them, and the least and the largest |F'(rho)|
+// of an element on a site whose neighbours are of one.
 struct Crystal {
     std::vector<std::array<int, 3>> near;
-    double df_least = HUGE_VAL, df_most = 0.0;
+    double rho_least = HUGE_VAL, df_least = HUGE_VAL, df_most = 0.0;
 };
 static double distance_of(const std::array<int, 3> &n, double a0) {
     return 0.5 * a0 * std::sqrt((double) (n[0] * n[0] + n[1] * n[1] + n[2] * n[2]));
@@ -208,6 +208,7 @@ static Crystal crystal_of(const HostPotential &hp, double a0, double rc) {
                 if (!(((i ^ j) | (j ^ k)) & 1) && (i || j || k) && distance_of({i, j, k}, a0) < rc) c.near.push_back({i, j, k});
     for (int b = 0; b < hp.n_ele; b++) {
         const double rho = crystal_rho(hp, c, a0, b);
+        c.rho_least = std::min(c.rho_least, rho);
         if (!(rho <= (hp.nrho - 1) * hp.drho)) continue;  // past the embedding tables: no crystal to judge by
         for (int a = 0; a < hp.n_ele; a++) {
             const double df = std::fabs(embedding_df(hp, a, rho));
@@ -255,13 +256,14 @@ static double fp64_error(const HostPotential &hp, const Crystal &c, double a0, d
     return least;
 }
 
-// build_fixed for one inner end r_lo of the tables' range and F'(rho) in units of 2^-kd; exact: the FP64 loops' error.
+// build_fixed for one inner end r_lo of the tables' range and F'(rho) in units of 2^-kd; exact: the FP64 loops' error in a
+// force.
 // depth: the scales only, whether the innermost intervals (where the quartics are at their worst) meet the bound, or
 // everything into tab
 enum Depth { SCALES, INNERMOST, TABLES };
 static bool build_from(const HostPotential &hp, const int ele_of_type[3], double a0, double rcf, int n_part, double r_lo, int kd,
-                       double exact, const std::vector<Largest> &largest, FixParams &fp, FixTables *tab, bool want_phi,
-                       Depth depth) {
+                       double exact, const Crystal &crystal, const std::vector<Largest> &largest, FixParams &fp, FixTables *tab,
+                       bool want_phi, Depth depth) {
     fp = FixParams{};
     const double rc = a0 * rcf, dr = hp.dr;
     const int nr = hp.nr;
@@ -311,8 +313,9 @@ static bool build_from(const HostPotential &hp, const int ele_of_type[3], double
     const int kphi = exponent_for(n_part * phi_max * room, 62);
     if ((df2 * g_max + h_max) * room >= std::ldexp(1.0, 62 - kf)) return false;
     if (n_part * (df2 * rg_max + rh_max) * room >= std::ldexp(1.0, 63 - kF)) return false;
-    // the sums are to be no less exact than the FP64 loops'; their rms error in thermal crystals is 2.3 to 2.5 units
-    if (2.5 * std::ldexp(1.0, -kF) > exact) return false;
+    // The sums are to be no less exact than the FP64 loops'. Rms errors in thermal crystals: forces 2.3 to 2.5 units, densities
+    // (all elements' in one unit, which the largest sets) 5.5 units against the loops' 2.1e-16 to 2.8e-16 of the density.
+    if (2.5 * std::ldexp(1.0, -kF) > exact || 5.5 * std::ldexp(1.0, -krho) > 2.1e-16 * crystal.rho_least) return false;
     fp.rho_unit = std::ldexp(1.0, -krho);
     fp.e_unit = std::ldexp(1.0, -kphi);
     fp.f_unit = std::ldexp(1.0, -kF);
@@ -490,7 +493,7 @@ bool build_fixed(const HostPotential &hp, const int ele_of_type[3], double a0, d
     if (!std::isfinite(exact)) return false;  // no crystal of one element to hold the sums against
     int kd = 60;
     auto from = [&](int f, Depth depth) {
-        return build_from(hp, ele_of_type, a0, rcf, n_part, f * percent, kd, exact, largest, fp, &tab, want_phi, depth);
+        return build_from(hp, ele_of_type, a0, rcf, n_part, f * percent, kd, exact, crystal, largest, fp, &tab, want_phi, depth);
     };
     double finest = 0.0;
     for (int k = 60; k <= 80 && finest == 0.0 && (k == 60 || std::ldexp(1.25 * crystal.df_most, k - 60) <= 1.0); k++) {

@@ -33,7 +33,7 @@ static int knot(T x, double inv, int n, T &p) {
 
 // spread: standard deviation of the displacements (A); pure: every atom's type (or -1: 80 / 10 / 10 %). Returns 0 where
 // the tables are refused. out: rms errors of the force components by the FP64 operations and in fixed point; atoms whose
-// F' is past the fixed-point bound; the force sums' unit.
+// F' is past the fixed-point bound; the force sums' unit; rms errors of the densities, relative, by both.
 extern "C" int force_errors(const char *path, double spread, int pure, double *out) {
     HostPotential P;
     std::string err;
@@ -91,6 +91,7 @@ extern "C" int force_errors(const char *path, double spread, int pure, double *o
     std::vector<double> df(n), dfx(n);
     std::vector<ld> dfl(n);
     int past = 0;
+    ld r64 = 0.0L, rfx = 0.0L, rr = 0.0L;
     for (int i = 0; i < n; i++) {
         double rho = 0.0, close = 0.0, d[3], p;
         ld rhol = 0.0L, dl[3], pl;
@@ -116,7 +117,11 @@ extern "C" int force_errors(const char *path, double spread, int pure, double *o
         const HostSpline &F = P.F[ele[at[i].type]];
         int m = knot(rho, F.inv_delta, P.nrho, p);
         df[i] = slope(F, m, p);
-        m = knot((double) sum * fp.rho_unit + close, F.inv_delta, P.nrho, p);
+        const double rhox = (double) sum * fp.rho_unit + close;
+        r64 += ((ld) rho - rhol) * ((ld) rho - rhol);
+        rfx += ((ld) rhox - rhol) * ((ld) rhox - rhol);
+        rr += rhol * rhol;
+        m = knot(rhox, F.inv_delta, P.nrho, p);
         dfx[i] = slope(F, m, p);
         m = knot(rhol, F.inv_delta, P.nrho, pl);
         dfl[i] = slope(F, m, pl);
@@ -175,5 +180,7 @@ extern "C" int force_errors(const char *path, double spread, int pure, double *o
     out[1] = (double) std::sqrt(efx / (3 * n));
     out[2] = past;
     out[3] = fp.f_unit;
+    out[4] = (double) std::sqrt(r64 / rr);
+    out[5] = (double) std::sqrt(rfx / rr);
     return 1;
 }

@@ -22,13 +22,14 @@ def lib(tmp_path_factory, pkg):
     return ctypes.CDLL(so)
 
 
-def _write(wl, path, n_ele, nr, density, embed, pair):
-    """The density, with its unit, times `density`; the embedding and pair energies times the others."""
+def _write(wl, path, n_ele, nr, density, embed, pair, second=1.0):
+    """The density, with its unit, times `density`; the embedding and pair energies times the others; the second element's
+    density alone times `second`."""
     F, rho, rphi, drho, dr = wl.potential_tables(wl.PotentialSpec(n_ele=n_ele, seed=5, nr=nr))
     lines = ["", "", "", "%d %s" % (n_ele, " ".join(("Fe", "Cu", "Ni")[:n_ele])), "%d %.17g %d %.17g 5.6" % (len(F[0]), drho * density, nr, dr)]
     for e, z in zip(range(n_ele), (26, 29, 28)):
         lines.append("%d 55.845 2.855 bcc" % z)
-        lines += ["%.17g" % v for v in np.concatenate([np.asarray(F[e]) * embed, np.asarray(rho[e]) * density])]
+        lines += ["%.17g" % v for v in np.concatenate([np.asarray(F[e]) * embed, np.asarray(rho[e]) * density * (second if e == 1 else 1.0)])]
     for p in rphi:
         lines += ["%.17g" % v for v in np.asarray(p) * pair]
     path.write_text("\n".join(lines) + "\n")
@@ -45,9 +46,23 @@ def test_forces_are_no_less_exact_than_the_fp64_loops(lib, wl, tmp_path, n_ele, 
     path = _write(wl, tmp_path / "p.setfl", n_ele, nr, density, embed, pair)
     for spread in (0.02, 0.08):
         for pure in ((-1, 0, 1, 2) if n_ele == 3 else (-1,)):
-            out = (ctypes.c_double * 4)()
+            out = (ctypes.c_double * 6)()
             st = lib.force_errors(os.fsencode(path), ctypes.c_double(spread), pure, out)
             assert st >= 0 and fixed in (None, bool(st))
             if st:
                 assert out[2] == 0
                 assert out[1] <= out[0], (spread, pure, out[0], out[1], out[3])
+                assert out[5] <= out[4], (spread, pure, out[4], out[5])
+
+
+@pytest.mark.parametrize("second,embed,pair", [(0.3, 1.0, 1.0), (0.1, 0.3, 4.0), (0.03, 0.3, 4.0), (0.01, 0.1, 4.0), (3.0, 1.0, 1.0),
+                                               (10.0, 1.0, 4.0)])
+def test_elements_of_unlike_densities(lib, wl, tmp_path, second, embed, pair):
+    """The sums of all elements have one unit, set by the largest density; crystals of the element with a smaller one."""
+    path = _write(wl, tmp_path / "p.setfl", 3, 5000, 1.0, embed, pair, second)
+    for pure in (-1, 0, 1, 2):
+        out = (ctypes.c_double * 6)()
+        st = lib.force_errors(os.fsencode(path), ctypes.c_double(0.06), pure, out)
+        assert st >= 0
+        if st:
+            assert out[1] <= out[0] and out[5] <= out[4], (pure, list(out))
