@@ -266,8 +266,8 @@ struct LaunchCtx {
     const FixParams *fp = nullptr;           // FP64 form: scales and tables of the fixed-point pair arithmetic
     int share = 1;                           // contexts that step side by side (a batch's members)
     bool one_type = false;                   // all types have the same tables
-    // The overlapped host step: its force slabs run beside the unpack and firststep of later chunks, so none of its
-    // kernels reads or writes SkinState::wild. An atom that far off voids the step (CNT_SPEC_VOID) and is a vacancy to it.
+    // The overlapped host step: its force slabs run beside the unpack and firststep of later chunks, so those leave
+    // SkinState::wild at 0. An atom that far off voids the step (CNT_SPEC_VOID) and is a vacancy to its passes.
     bool spec = false;
 };
 

@@ -377,8 +377,8 @@ inline Slots with_records(const LaunchCtx &lc, Slots s) {
     return s;
 }
 // whether a pass takes every atom in FP64: the same in every thread of its grid, since nothing writes the word while a
-// pass that reads it runs
-__device__ __forceinline__ bool pass_wild(const Slots &s) { return !s.spec && s.skin->wild != 0; }
+// pass that reads it runs (the overlapped host step, whose passes run beside later chunks, leaves it at 0)
+__device__ __forceinline__ bool pass_wild(const Slots &s) { return s.skin->wild != 0; }
 
 // ------------------------------------------------------------------------------------------------
 // AoS <-> SoA (the reference's AtomElement array crosses the boundary as raw records)
@@ -501,8 +501,9 @@ __device__ __forceinline__ void skin_note(const Slots &s, float d2) {
 // test (src/atom.cpp:34-42): v += c f, x += dt v (each operation rounded as the reference rounds it),
 // the displacement record u4 (written to u4_out, parity-split index) and, where displaced, local index t
 // into the displaced list. MOVE = false: the test alone, on the current positions. u4_prev holds the record the last
-// density pass read (for the skin's displacement bound).
-template <bool MOVE, bool DECIDE>
+// density pass read (for the skin's displacement bound). PART: may be a launch of the overlapped host step (the force passes,
+// which take the next firststep in fused bodies, are not, and have no register to spare for it).
+template <bool MOVE, bool DECIDE, bool PART = false>
 __device__ __forceinline__ void first_half(const Geom &g, const Slots &s, const Inter &in, const StepParams *__restrict__ p,
                                            int sl, int t, int i, int j, int k, int ty, double vx, double vy, double vz,
                                            double fx, double fy, double fz, float4 *u4_out, const float4 *u4_prev, FixRec *fix_out) {
@@ -538,7 +539,7 @@ __device__ __forceinline__ void first_half(const Geom &g, const Slots &s, const 
         if (s.kx) {
             fix_put(fix_out + si, s.kx, x, y, z, ty);
             if (fix_wild(nu)) {
-                if (!s.spec) {
+                if (!PART || !s.spec) {
                     s.skin->wild_next = 1;
                     if (!DECIDE) s.skin->wild = 1;  // firststep as a phase of its own: no decide need follow
                 } else {  // its wrapped coordinates could meet a vacancy's
@@ -618,8 +619,8 @@ __global__ void __launch_bounds__(kFirstThreads) k_firststep(const NeighTables *
             continue;
         }
         if (MOVE)
-            first_half<true, DECIDE>(g, s, in, p, sl, t, i, j, k, ty, s.vx[sl], s.vy[sl], s.vz[sl], s.fx[sl], s.fy[sl],
-                                     s.fz[sl], s.u4, alt ? s.u4n : s.u4, s.fix);
+            first_half<true, DECIDE, true>(g, s, in, p, sl, t, i, j, k, ty, s.vx[sl], s.vy[sl], s.vz[sl], s.fx[sl], s.fy[sl],
+                                           s.fz[sl], s.u4, alt ? s.u4n : s.u4, s.fix);
         else
             first_half<false, DECIDE>(g, s, in, p, sl, t, i, j, k, ty, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, s.u4, s.u4, s.fix);
     }
@@ -1614,7 +1615,6 @@ template <int W>
 static void launch_rho_split_w(const LaunchCtx &lc, const Geom &g, Slots s, Inter in, PotTables t, bool mixed, bool hook, int u0, int u1,
                                bool lists) {
     const int n = split_groups(u0, u1);
-    s = with_records(lc, s);
     if (mixed)
         k_lat_rho_mixed_split<W><<<n, 32 * W, 0, lc.stream>>>(&lc.ntd->cand[0][0], lc.nt->npruned, lc.nt->nfull, g, s, in, t, hook, u0, u1, lists);
     else k_lat_rho_fix_split<W><<<n, 32 * W, 0, lc.stream>>>(*lc.nt, &lc.ntd->cand[0][0], g, s, in, t, *lc.fp, hook, u0, u1, lists);
@@ -1634,7 +1634,6 @@ static void launch_lat_rho_threads(const LaunchCtx &lc, const Geom &g, Slots s, 
     const int order = lc.rho_order, b = lc.rho_block;
     const int n = (te - tb + b * lc.rho_apt - 1) / (b * lc.rho_apt);
     if (n <= 0) return;
-    s = with_records(lc, s);
     if (lc.rho_apt > 1) {
         if (mixed) k_lat_rho_mixed<true><<<n, b, 0, lc.stream>>>(*lc.nt, g, s, in, t, hook, order, tb, te, false);
         else if (lc.fp) k_lat_rho_fix<true><<<n, b, 0, lc.stream>>>(*lc.nt, g, s, in, t, *lc.fp, hook, order, tb, te, false);
