@@ -132,7 +132,6 @@ struct mg_context {
     std::string origin_path;
 
     int tune[2][2][3];              // [precision][rho, force] = {thread order, block size, atoms per thread}
-    bool tuned[2] = {false, false};  // they are the caller's or an autotune's, not default_shapes'
     int share = 1;                  // contexts stepping side by side (while a batch captures)
     LaunchCtx lc() const {
         LaunchCtx l{stream, num_sms};
@@ -215,18 +214,18 @@ void set_skin(Geom &g, double skin) {
 }
 
 // The launch shapes until an autotune. Order 1: its warps cover whole 32-site groups in every box, so the group lists serve
-// boxes with an odd number of sites of a parity as well (order 0 visits all 112 candidates there). Block sizes by measurement: the FP64 density pass
-// 128 (2M atoms: 720 us with 256, 682 with 128), its force pass 256 (128: 2M atoms -0.2%, 304k atoms +1%); the
-// mixed density pass 512 (2M atoms 233 -> 228 us, 221k atoms 40.2 -> 38.3, elsewhere even). The mixed force pass: blocks of
-// 512 keep more of their neighbours in L1, blocks of 256 leave less of a last wave empty, which weighs less the more
-// waves there are. us per step with 256 -> 512, one element: 629k sites 239 -> 244, 1.02M 357 -> 358, 1.27M 433 -> 433,
-// 1.46M 485 -> 479, 2M 648 -> 638, 3.1M 989 -> 977, 8.2M 2483 -> 2446; three: 629k 292 -> 301, 1.27M 534 -> 538, 1.88M
-// 763 -> 767, 2.2M 878 -> 880, 3.1M 1220 -> 1220, 3.6M 1408 -> 1400, 8.2M 3081 -> 3066.
-constexpr int kWideForceOne = 1500000, kWideForce = 3500000;
+// boxes with an odd number of sites of a parity as well (order 0 visits all 112 candidates there). Block sizes by
+// measurement: the FP64 density pass 128 (2M atoms: 720 us with 256, 682 with 128), its force pass 256 (128: 2M atoms -0.2%,
+// 304k atoms +1%); the mixed density pass 512 (2M atoms 233 -> 228 us, 221k atoms 40.2 -> 38.3, elsewhere even). The mixed
+// force pass: blocks of 512 keep more of their neighbours in L1, blocks of 256 leave less of a last wave empty, which
+// weighs less the more waves there are. us per step with 256 -> 512, one element: 390k sites 165 -> 170, 629k 239 -> 244, 1.02M
+// 357 -> 358, 1.27M 433 -> 433, 1.46M 485 -> 479, 2M 648 -> 638, 3.1M 989 -> 977, 8.2M 2483 -> 2446; three: 390k 201 -> 210, 629k
+// 292 -> 301, 1.27M 534 -> 538, then from one box to the next between -0.5% and +0.6% (1.66M 680 -> 684, 1.77M 709 -> 706, 2M
+// 801 -> 797, 2.2M 878 -> 880, 3.1M 1220 -> 1220), 3.6M 1408 -> 1400, 8.2M 3081 -> 3066.
+constexpr int kWideForce = 1500000;
 void default_shapes(mg_context *ctx, int precision) {
     const bool mixed = precision == MG_PREC_MIXED;
-    const bool wide = mixed && ctx->g.n_local >= (ctx->one_type ? kWideForceOne : kWideForce);
-    const int shapes[2][3] = {{1, mixed ? 512 : 128, 1}, {1, wide ? 512 : 256, 1}};
+    const int shapes[2][3] = {{1, mixed ? 512 : 128, 1}, {1, mixed && ctx->g.n_local >= kWideForce ? 512 : 256, 1}};
     std::memcpy(ctx->tune[precision], shapes, sizeof(shapes));
 }
 
@@ -521,8 +520,6 @@ mg_status install_potential(mg_context *ctx, const HostPotential &hp) {
     if (ctx->fix_mem) { cudaFree(ctx->fix_mem); ctx->fix_mem = nullptr; }
     ctx->fp = FixParams{};
     ctx->fix_built = false;
-    for (int p = 0; p < 2; p++)
-        if (!ctx->tuned[p]) default_shapes(ctx, p);
     ctx->hp = hp;
     ctx->pot_ready = true;
     ctx->graph_stale = true;
@@ -1907,7 +1904,6 @@ mg_status mg_autotune(mg_context *ctx, int32_t reps, int32_t out[6]) {
     }
     ctx->graph_stale = true;
     ctx->gen++;  // the captured graph holds the old launch shapes
-    ctx->tuned[p] = true;
     if (known) {
         for (int k = 0; k < 6; k++) ctx->tune[p][k / 3][k % 3] = best[k];
     } else {
@@ -1940,7 +1936,6 @@ mg_status mg_set_tuning(mg_context *ctx, const int32_t tune[6]) {
     }
     for (int k = 0; k < 2; k++)
         for (int c = 0; c < 3; c++) ctx->tune[ctx->precision][k][c] = tune[3 * k + c];
-    ctx->tuned[ctx->precision] = true;
     ctx->graph_stale = true;
     ctx->gen++;
     return MG_OK;
